@@ -82,7 +82,11 @@ constexpr float kLog2e = 1.4426950408889634f;
 // done within one step.  D = 128 has room for three U stages and two W stages, except that the
 // key-stationary dropout instance needs 4 KB for its masks and stays at two and two.
 // DROP: 0 no dropout; 1 keep bits drawn by the kernel's own threads; 2 loaded from the call's bit buffer.
-template <int D, int MODE, int DROP>
+// PREC: 0 for calls with D = 64 or 128; 1 ("pair") for 16-bit calls with an additive bias or another head size (any
+// multiple of 8 up to 128, the tiles padded by TMA's zero fill): P and dS go back to tensor memory as hi + lo in the
+// inputs' own format and every accumulating MMA is issued for both, so they keep 17 (bf16) or 22 (fp16) significant
+// bits and no operand is converted.
+template <int D, int MODE, int DROP, int PREC>
 struct BwdCfg {
     static constexpr int kNBox = D / 64;
     static constexpr int kTileBytes = kNBox * kBoxBytes;
@@ -148,6 +152,13 @@ struct BwdArgs {
     const uint4* bits_q;           // [(b*H + h) * ceil128(Nk)/128 + key tile][nq_pad]: 128 keys of one query row
     const uint32_t* bits_k;        // [((b*H + h) * nq_pad/128 + query tile) * 4 + g][nk_pad]: 32 queries of one key row
     int nk_pad;
+    // PREC = 1:
+    int d;                         // head size (at most the template's D, a multiple of 8)
+    const float* bias;             // optional additive bias, element strides below (0 broadcasts)
+    int64_t bias_sb, bias_sn, bias_sh;
+    int bias_vec;                  // its rows can be read as float4
+    int ds_vec;                    // rows of d_scores can be written as float4
+    float* d_scores;               // optional dense (B, H, Nq, Nk) gradient of the scores (written by MODE 1)
 };
 
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
@@ -240,16 +251,18 @@ __device__ __forceinline__ CtaWork cta_work(int cols_per_group) {
 // INLINE (bf16 inputs only): the streamed tiles arrive as bf16 and the two spare warps convert them;
 // otherwise bf16 calls stream the fp16 copies the preprocess launch (Q, dO) and the dK/dV kernel (K:
 // map_aux, a by-product of its stationary tile) have written to the workspace.
-template <int D, bool BF16, int MODE, int NWG, int DROP, bool INLINE>
+template <int D, bool BF16, int MODE, int NWG, int DROP, bool INLINE, int PREC>
 __global__ void __launch_bounds__(128 * NWG + kExtraThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                  const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_out1, const __grid_constant__ CUtensorMap map_out2,
                  const __grid_constant__ CUtensorMap map_aux, const BwdArgs a) {
-    using Cfg = BwdCfg<D, MODE, DROP>;
+    using Cfg = BwdCfg<D, MODE, DROP, PREC>;
     constexpr bool KS = (MODE != 1);        // key-stationary: K, V stay, query tiles stream
     constexpr bool FUSED = (MODE == 2);     // key-stationary and dQ too
-    constexpr bool CONV = BF16;             // every MMA runs f16 x f16: bf16 tiles are converted
+    constexpr bool CONV = BF16 && PREC == 0;    // every MMA runs f16 x f16: bf16 tiles are converted
+    constexpr bool P_BF16 = BF16 && PREC == 1;  // ... except that pairs of bf16 need no conversion
+    static_assert(PREC == 0 || (MODE != 2 && !INLINE), "the pair instances are the two-pass form");
     constexpr bool STREAM_CONV = CONV && INLINE;             // ... the streamed ones by the spare warps
     constexpr bool XY_CONV = CONV && (KS || INLINE);         // ... the stationary ones by the elementwise warps
     constexpr bool ROWFORM = CONV && !INLINE;                // staged vectors are in the row form (see DoForm)
@@ -449,7 +462,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             constexpr bool T1_BF16 = BF16 && !CONV, T2_BF16 = BF16 && !(CONV && KS);
             constexpr uint32_t idesc_t1 = make_idesc_f16(T1_BF16, T1_BF16, kTile, kTile, false, false);
             constexpr uint32_t idesc_t2 = make_idesc_f16(T2_BF16, T2_BF16, kTile, kTile, false, false);
-            constexpr uint32_t idesc_acc = make_idesc_f16(false, false, kTile, D, false, true);
+            const uint32_t idesc_acc = PREC ? make_idesc_f16(P_BF16, P_BF16, kTile, (a.d + 15) & ~15, false, true)
+                                            : make_idesc_f16(false, false, kTile, D, false, true);
             constexpr int kUReady = STREAM_CONV ? Cfg::kUConv : Cfg::kUFull;
             constexpr int kWReady = (STREAM_CONV && KS) ? Cfg::kWConv : Cfg::kWFull;
             constexpr int kXYReady = XY_CONV ? Cfg::kXYConv : Cfg::kXYFull;
@@ -465,22 +479,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                     const uint32_t off = ((uint32_t)(kk >> 2) * kBoxBytes + (uint32_t)(kk & 3) * 32u) >> 4;
-                    mma_ss_f16(d_tmem, a0 + off, b0 + off, idesc_t, kk > 0);
+                    if (PREC == 0 || kk * 16 < a.d) mma_ss_f16(d_tmem, a0 + off, b0 + off, idesc_t, kk > 0);
                 }
             };
-            // acc (+)= A[TMEM] * B[smem tile, MN-major].  A holds 16-bit pairs: the thread group that owns
-            // columns [g*CPT, (g+1)*CPT) of T wrote its CPT values packed into columns [g*CPT, g*CPT + CPT/2).
-            auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t strm_u, bool acc) {
-                const uint64_t b0 = dmn_major + (uint64_t)(strm_u >> 4);
-#pragma unroll
-                for (int kk = 0; kk < kTile / 16; ++kk) {
-                    const uint32_t a_col = (uint32_t)((16 * kk) / CPT) * CPT + (uint32_t)((16 * kk) % CPT) / 2u;
-                    mma_ts_f16(d_tmem, a_tmem + a_col, b0 + (uint64_t)((kk * 2048) >> 4), idesc_acc,
-                               (acc || kk > 0) ? 1u : 0u);
-                }
-            };
-            // the same product restricted to the first (hf = 0) or second 16 columns of every
-            // warpgroup's slice: K-steps kk = hf, hf + 2, hf + 4, hf + 6
+            // acc (+)= A[TMEM] * B[smem tile, MN-major], restricted to the first (hf = 0) or second 16 columns of
+            // every warpgroup's slice: K-steps kk = hf, hf + 2, hf + 4, hf + 6.  A holds 16-bit pairs: the group
+            // that owns columns [g*CPT, (g+1)*CPT) of T wrote its CPT values packed into columns
+            // [g*CPT, g*CPT + CPT/2); with pairs their low parts follow in [g*CPT + CPT/2, (g+1)*CPT).
             auto issue_acc_half = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t strm_u, bool acc, int hf) {
                 static_assert(CPT == 32, "one K-step of 16 per half slice");
                 const uint64_t b0 = dmn_major + (uint64_t)(strm_u >> 4);
@@ -490,6 +495,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     const uint32_t a_col = (uint32_t)g * CPT + (uint32_t)hf * 8u;
                     mma_ts_f16(d_tmem, a_tmem + a_col, b0 + (uint64_t)((kk * 2048) >> 4), idesc_acc,
                                (acc || hf > 0 || g > 0) ? 1u : 0u);
+                    if (PREC) mma_ts_f16(d_tmem, a_tmem + a_col + CPT / 2, b0 + (uint64_t)((kk * 2048) >> 4), idesc_acc, 1u);
                 }
             };
 
@@ -657,6 +663,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const float zk = a.inv_keep * sc.tt_mul;
         const uint64_t ladd2 = f2_pack(sc.l_add, sc.l_add);
         my_ndelta *= sc.nd_mul;
+        // PREC = 1, query-stationary: my row of d loss / d scores, and what undoes dS' = dS * 2^g
+        [[maybe_unused]] float* ds_row = (PREC && MODE == 1 && a.d_scores)
+            ? a.d_scores + (((int64_t)b * a.H + head_x) * a.Nq + row_g) * (int64_t)a.Nk : nullptr;
+        [[maybe_unused]] const float ds_mul = sc.acc1_mul / a.scale;
         bool ok = true;
         if (XY_CONV && n_iter > 0) {
             // the stationary tiles, once per CTA: K_j and V_j, or Q_i (dO_i is only ever multiplied
@@ -707,6 +717,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const int col_g0 = strm_tile * kTile + cb;                          // global index of my first column
             const int head_q = (KS) ? head_x * group + hg : head_x;
             const uint32_t bh = dropout_column(a.rng, b, head_q);
+            [[maybe_unused]] const float* bias_h = PREC ? a.bias + b * a.bias_sb + head_q * a.bias_sh : nullptr;
             // key-stationary: -lse*log2(e) and -delta of this step's 128 queries (slot it & 1)
             const float* lse_s = sVec + (it & 1) * 256;
             const float* del_s = lse_s + 128;
@@ -816,7 +827,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             const bool tail = tile * kTile + kTile > nk;            // the tile holds padding keys
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                uint32_t pk[2][4];                                  // [h][2j' + k], j' = j - 2hf
+                uint32_t pk[2][4], pl[2][4];                        // [h][2j' + k], j' = j - 2hf; pairs: the low parts
 #pragma unroll
                 for (int jj = 0; jj < 2; ++jj) {
                     const int j = 2 * hf + jj;
@@ -839,6 +850,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             const int i0 = 4 * j + 2 * k;
                             float x0, x1;
                             f2_unpack(f2_fma(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), sc2, L), x0, x1);
+                            if (PREC && a.bias) {
+                                // bias[query][key]: eight lanes read eight neighbouring keys of one query
+                                const int key = tile * kTile + rbase + 16 * h + 8 * k, qr = col_g0 + 8 * j + 2 * lq;
+                                const float* bp = bias_h + (int64_t)qr * a.bias_sn + key;
+                                if (key < a.Nk && qr < a.Nq) x0 = fmaf(bp[0], kLog2e, x0);
+                                if (key < a.Nk && qr + 1 < a.Nq) x1 = fmaf(bp[a.bias_sn], kLog2e, x1);
+                            }
                             pf[h][i0] = __float_as_uint(ex2(x0));
                             pf[h][i0 + 1] = __float_as_uint(ex2(x1));
                         }
@@ -874,7 +892,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 if (!(kw & 1u)) z0 = 0.f;
                                 if (!(kw & 2u)) z1 = 0.f;
                             }
-                            pk[h][2 * jj + k] = pack2<false>(z0, z1);
+                            if (PREC) pack2_pair<P_BF16>(z0, z1, pk[h][2 * jj + k], pl[h][2 * jj + k]);
+                            else      pk[h][2 * jj + k] = pack2<false>(z0, z1);
                         }
                 if (drop && hf == 1) {
                     tmem_wait_st();
@@ -883,6 +902,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 tmem_st_16x128b_x2(tT1 + t_lo + hf * 8, pk[0]);
                 tmem_st_16x128b_x2(tT1 + t_hi + hf * 8, pk[1]);
+                if (PREC) {
+                    tmem_st_16x128b_x2(tT1 + t_lo + 16 + hf * 8, pl[0]);
+                    tmem_st_16x128b_x2(tT1 + t_hi + 16 + hf * 8, pl[1]);
+                }
             }
             tmem_wait_st();
             tc_fence_before_sync();
@@ -899,7 +922,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_ld();
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    uint32_t pk[2][4];
+                    uint32_t pk[2][4], pl[2][4];
 #pragma unroll
                     for (int jj = 0; jj < 2; ++jj) {
                         const int j = 2 * hf + jj;
@@ -924,7 +947,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 }
                                 float d0, d1;
                                 f2_unpack(f2_mul(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), tt), d0, d1);
-                                pk[h][2 * jj + k] = pack2<false>(d0, d1);
+                                if (PREC) pack2_pair<P_BF16>(d0, d1, pk[h][2 * jj + k], pl[h][2 * jj + k]);
+                                else      pk[h][2 * jj + k] = pack2<false>(d0, d1);
                             }
                     }
                     if (drop && hf == 1) {
@@ -934,6 +958,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     }
                     tmem_st_16x128b_x2(tT2 + t_lo + hf * 8, pk[0]);
                     tmem_st_16x128b_x2(tT2 + t_hi + hf * 8, pk[1]);
+                    if (PREC) {
+                        tmem_st_16x128b_x2(tT2 + t_lo + 16 + hf * 8, pl[0]);
+                        tmem_st_16x128b_x2(tT2 + t_hi + 16 + hf * 8, pl[1]);
+                    }
                 }
                 tmem_wait_st();
             }
@@ -1016,10 +1044,27 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_st();
             } else {
                 const uint64_t neg2 = f2_pack(my_nlse2, my_nlse2);
+                [[maybe_unused]] float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < CPT; c += 2) {
                     float x0, x1;
                     f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), sc2, neg2), x0, x1);
+                    if constexpr (PREC != 0) {
+                        if (a.bias) {
+                            const float* bp = bias_h + (int64_t)(row_g < a.Nq ? row_g : a.Nq - 1) * a.bias_sn + col_g0 + c;
+                            if (a.bias_vec && col_g0 + (c & ~3) + 4 <= a.Nk) {
+                                if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(bp);
+                                x0 = fmaf((c & 2) ? bv.z : bv.x, kLog2e, x0);
+                                x1 = fmaf((c & 2) ? bv.w : bv.y, kLog2e, x1);
+                            } else {
+                                if (col_g0 + c < a.Nk) x0 = fmaf(bp[0], kLog2e, x0);
+                                if (col_g0 + c + 1 < a.Nk) x1 = fmaf(bp[1], kLog2e, x1);
+                            }
+                        }
+                        PSET(c, ex2(x0));
+                        PSET(c + 1, ex2(x1));
+                        continue;
+                    }
                     // a quarter of the exponentials as a polynomial on the FMA pipes (this kernel keeps the
                     // special-function unit busiest; measured 0.7 % over the backward, half: 0.2 %)
                     if (((c >> 1) & 3) == 0) {
@@ -1074,7 +1119,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const uint64_t my_nd2 = f2_pack(my_ndelta, my_ndelta);
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    uint32_t pk[CPT / 4];
+                    uint32_t pk[CPT / 4], pl[CPT / 4];
                     if (hf == 1) {
                         tmem_wait_st();                            // the first half, stored just now
                         tc_fence_before_sync();
@@ -1107,10 +1152,30 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         float d0, d1, d2v, d3;
                         f2_unpack(f2_mul(f2_pack(PF(c), PF(c + 1)), ta), d0, d1);
                         f2_unpack(f2_mul(f2_pack(PF(c + 2), PF(c + 3)), tb), d2v, d3);
-                        pk[(c4 - hf * (CPT / 8)) * 2 + 0] = pack2<false>(d0, d1);
-                        pk[(c4 - hf * (CPT / 8)) * 2 + 1] = pack2<false>(d2v, d3);
+                        if constexpr (PREC != 0) {
+                            const int e = (c4 - hf * (CPT / 8)) * 2;
+                            pack2_pair<P_BF16>(d0, d1, pk[e], pl[e]);
+                            pack2_pair<P_BF16>(d2v, d3, pk[e + 1], pl[e + 1]);
+                            if (ds_row && row_g < a.Nq) {
+                                // d loss / d scores, the power of two of dS' taken out (exact)
+                                float* dst = ds_row + col_g0 + c;
+                                if (a.ds_vec) {
+                                    if (col_g0 + c < a.Nk)
+                                        *reinterpret_cast<float4*>(dst) = make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
+                                } else {
+                                    if (col_g0 + c < a.Nk) dst[0] = d0 * ds_mul;
+                                    if (col_g0 + c + 1 < a.Nk) dst[1] = d1 * ds_mul;
+                                    if (col_g0 + c + 2 < a.Nk) dst[2] = d2v * ds_mul;
+                                    if (col_g0 + c + 3 < a.Nk) dst[3] = d3 * ds_mul;
+                                }
+                            }
+                        } else {
+                            pk[(c4 - hf * (CPT / 8)) * 2 + 0] = pack2<false>(d0, d1);
+                            pk[(c4 - hf * (CPT / 8)) * 2 + 1] = pack2<false>(d2v, d3);
+                        }
                     }
                     tmem_st_32x8(tD + lane_off + cb + hf * (CPT / 4), pk);
+                    if (PREC) tmem_st_32x8(tD + lane_off + cb + CPT / 2 + hf * (CPT / 4), pl);
                     if (FUSED) {
                         // the same dS^T values as a shared-memory tile [key row][query], 64-query boxes with
                         // the 128-byte swizzle: the A operand (MN-major) of the dQ MMA.  The previous
@@ -1240,9 +1305,10 @@ struct PreprocessCopies {
     const void* q; int64_t q_sb, q_sn, q_sh;
     uint16_t* q16; uint16_t* do16; float* erow;
 };
+// A head size below D (pair instances) leaves the lanes beyond it idle.
 template <typename T, int D, bool COPIES>
 __global__ void __launch_bounds__(256)
-bwd_preprocess_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const float* __restrict__ lse,
+bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o, const float* __restrict__ lse,
                       float* __restrict__ lse2, float* __restrict__ delta, float* __restrict__ ranges,
                       int B, int Nq, int H, int Hkv, int nq_pad,
                       int64_t o_sb, int64_t o_sn, int64_t o_sh, int64_t g_sb, int64_t g_sn, int64_t g_sh,
@@ -1260,7 +1326,7 @@ bwd_preprocess_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const 
         const int nk = kv_len_of(kv_len, b, Nk);
         uint32_t m = 0u;
         const int j_end = min(nk, (slab + 1) * kVRows);
-        for (int j = slab * kVRows + (int)(threadIdx.x / LPR); j < j_end; j += 256 / LPR)
+        for (int j = slab * kVRows + (int)(threadIdx.x / LPR); j < j_end && sub * 8 < d; j += 256 / LPR)
             m = absmax16_acc(m, *reinterpret_cast<const uint4*>(v + b * v_sb + (int64_t)j * v_sn + hk * v_sh + sub * 8));
         absmax16_commit<T>(m, ranges + 2 * (int64_t)col + 1, red);
         return;
@@ -1284,7 +1350,7 @@ bwd_preprocess_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const 
         const int64_t row = bh * nq_pad + i;
         const bool in = i < Nq;
         uint4 vo = make_uint4(0, 0, 0, 0), vg = vo, vl = vo, vq = vo;
-        if (in) {
+        if (in && sub * 8 < d) {
             vo = *reinterpret_cast<const uint4*>(op + (int64_t)i * o_sn);
             vg = *reinterpret_cast<const uint4*>(gp + (int64_t)i * g_sn);
             if (lp) vl = *reinterpret_cast<const uint4*>(lp + (int64_t)i * cp.l_sn);
@@ -1358,21 +1424,22 @@ bwd_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, int Nq,
 // convert their tiles themselves.
 // the kernel instance and its shared memory for a dropout form (0 none, 1 drawn in the kernel, 2 loaded;
 // the converting-in-kernel instances, which serve the entry without a workspace, never load)
-template <int D, bool BF16, int MODE, bool INLINE>
+template <int D, bool BF16, int MODE, bool INLINE, int PREC>
 auto pick_kernel(int drop) {
-    if (drop == 2 && !INLINE) return bwd_sm100_kernel<D, BF16, MODE, kNWG, INLINE ? 1 : 2, INLINE>;
-    return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE>;
+    if (drop == 2 && !INLINE) return bwd_sm100_kernel<D, BF16, MODE, kNWG, INLINE ? 1 : 2, INLINE, PREC>;
+    return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE, PREC> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;
 }
-template <int D, int MODE>
+template <int D, int MODE, int PREC>
 int pick_smem(int drop) {
-    return drop == 2 ? BwdCfg<D, MODE, 2>::kSmemBytes : (drop ? BwdCfg<D, MODE, 1>::kSmemBytes : BwdCfg<D, MODE, 0>::kSmemBytes);
+    return drop == 2 ? BwdCfg<D, MODE, 2, PREC>::kSmemBytes
+                     : (drop ? BwdCfg<D, MODE, 1, PREC>::kSmemBytes : BwdCfg<D, MODE, 0, PREC>::kSmemBytes);
 }
 
-template <int D, bool BF16, bool INLINE>
+template <int D, bool BF16, bool INLINE, int PREC>
 int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     using T = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
     const CUtensorMapDataType dt = BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    constexpr bool COPIES = BF16 && !INLINE;
+    constexpr bool COPIES = BF16 && !INLINE && PREC == 0;
     cudaStream_t st = (cudaStream_t)p.stream;
     const int nq_pad = (int)align_up((size_t)p.Nq, 128);
     char* wsp = (char*)p.workspace;
@@ -1405,7 +1472,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
             cp.erow = (float*)(wsp + ws.erow_off);
         }
         bwd_preprocess_kernel<T, D, COPIES><<<(unsigned)n_blocks, 256, 0, st>>>(
-            (const T*)p.o.ptr, (const T*)p.d_o.ptr, p.lse, lse2, delta, ranges, p.B, p.Nq, p.H, p.Hkv, nq_pad,
+            p.D, (const T*)p.o.ptr, (const T*)p.d_o.ptr, p.lse, lse2, delta, ranges, p.B, p.Nq, p.H, p.Hkv, nq_pad,
             p.o.stride_b, p.o.stride_n, p.o.stride_h, p.d_o.stride_b, p.d_o.stride_n, p.d_o.stride_h,
             (const T*)p.v.ptr, p.v.stride_b, p.v.stride_n, p.v.stride_h, p.Nk, p.kv_lengths, n_row_blocks, v_slabs, cp);
         FA_CUDA_CHECK(cudaGetLastError());
@@ -1414,7 +1481,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     CUtensorMap mq, mk, mv, mg, mdq, mdk, mdv, mq16, mg16, mk16;
     int r;
     auto mk_map = [&](CUtensorMap* m, const fa_b200_tensor& t, int N, int H) {
-        return cached_tmap_bnhd(m, t.ptr, dt, 2, p.B, N, H, D, t.stride_b, t.stride_n, t.stride_h, 128, 64, true);
+        return cached_tmap_bnhd(m, t.ptr, dt, 2, p.B, N, H, p.D, t.stride_b, t.stride_n, t.stride_h, 128, 64, true);
     };
     // a dense fp16 (B, N, H, D) copy in the workspace
     auto mk_copy = [&](CUtensorMap* m, size_t off, int N, int H) {
@@ -1458,6 +1525,12 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     a.bits_q = (const uint4*)p.dropout_bits;
     a.bits_k = (const uint32_t*)((const char*)p.dropout_bits + bits_one);
     a.nk_pad = (int)align_up((size_t)p.Nk, 128);
+    a.d = p.D;
+    a.bias = (const float*)p.bias.ptr;
+    a.bias_sb = p.bias.stride_b; a.bias_sn = p.bias.stride_n; a.bias_sh = p.bias.stride_h;
+    a.bias_vec = (((uintptr_t)p.bias.ptr & 15u) == 0 && (p.bias.stride_b | p.bias.stride_n | p.bias.stride_h) % 4 == 0) ? 1 : 0;
+    a.d_scores = p.d_scores;
+    a.ds_vec = (p.Nk % 4 == 0 && ((uintptr_t)p.d_scores & 15u) == 0) ? 1 : 0;
     if (drop == 2 && !p.dropout_bits_ready && (phases & 1)) {
         int rc = launch_dropout_bits(p, (void*)a.bits_q, (void*)a.bits_k);
         if (rc) return rc;
@@ -1468,10 +1541,10 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     constexpr int kThreads = 128 * kNWG + kExtraThreads;
     const dim3 grid_kv((p.Nk + kTile - 1) / kTile, p.Hkv, p.B);
     const dim3 grid_q((p.Nq + kTile - 1) / kTile, p.H, p.B);
-    if constexpr (D == 64) if (fused) {
+    if constexpr (D == 64 && PREC == 0) if (fused) {
         // one key-stationary kernel for dK, dV and the fp32 dQ sums, then the conversion of dQ
-        auto k2 = pick_kernel<D, BF16, 2, INLINE>(drop);
-        const int smem2 = pick_smem<D, 2>(drop);
+        auto k2 = pick_kernel<D, BF16, 2, INLINE, PREC>(drop);
+        const int smem2 = pick_smem<D, 2, PREC>(drop);
         FA_CUDA_CHECK(set_smem_limit_once(k2, smem2, p.device, &smem_done[6 + drop], &smem_mu));
         if (phases & 2) {
             k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, a);
@@ -1486,9 +1559,9 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         return FA_OK;
     }
     if (COPIES && ws.k16_bytes == 0) { set_error("workspace layout lacks the fp16 copy of K"); return FA_EWORKSPACE; }
-    auto k0 = pick_kernel<D, BF16, 0, INLINE>(drop);
-    auto k1 = pick_kernel<D, BF16, 1, INLINE>(drop);
-    const int smem0 = pick_smem<D, 0>(drop), smem1 = pick_smem<D, 1>(drop);
+    auto k0 = pick_kernel<D, BF16, 0, INLINE, PREC>(drop);
+    auto k1 = pick_kernel<D, BF16, 1, INLINE, PREC>(drop);
+    const int smem0 = pick_smem<D, 0, PREC>(drop), smem1 = pick_smem<D, 1, PREC>(drop);
     FA_CUDA_CHECK(set_smem_limit_once(k0, smem0, p.device, &smem_done[drop], &smem_mu));
     FA_CUDA_CHECK(set_smem_limit_once(k1, smem1, p.device, &smem_done[3 + drop], &smem_mu));
     if (phases & 2) {
@@ -1518,6 +1591,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
 
 }  // namespace
 
+#ifndef FA_PAIR_INSTANCES
 bool sm100_bwd_fused_supported(const fa_b200_params& p) {
     // D = 64 only.  At D = 128 tensor memory is full (S^T, dP^T, dK, dV), the per-step dQ tile has
     // to share dP^T's columns, which serialises the step, and the fp32 additions (64 KB per step)
@@ -1528,10 +1602,17 @@ bool sm100_bwd_fused_supported(const fa_b200_params& p) {
 
 int sm100_bwd(const fa_b200_params& p, const BwdWorkspace& ws) {
     if (p.dtype == FA_B200_BF16) {
-        if (ws.q16_bytes == 0) return p.D == 128 ? launch<128, true, true>(p, ws) : launch<64, true, true>(p, ws);
-        return p.D == 128 ? launch<128, true, false>(p, ws) : launch<64, true, false>(p, ws);
+        if (ws.q16_bytes == 0) return p.D == 128 ? launch<128, true, true, 0>(p, ws) : launch<64, true, true, 0>(p, ws);
+        return p.D == 128 ? launch<128, true, false, 0>(p, ws) : launch<64, true, false, 0>(p, ws);
     }
-    return p.D == 128 ? launch<128, false, false>(p, ws) : launch<64, false, false>(p, ws);
+    return p.D == 128 ? launch<128, false, false, 0>(p, ws) : launch<64, false, false, 0>(p, ws);
 }
+
+#else
+int sm100_pair_bwd(const fa_b200_params& p, const BwdWorkspace& ws) {
+    if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, false, 1>(p, ws) : launch<64, true, false, 1>(p, ws);
+    return p.D > 64 ? launch<128, false, false, 1>(p, ws) : launch<64, false, false, 1>(p, ws);
+}
+#endif
 
 }  // namespace fa

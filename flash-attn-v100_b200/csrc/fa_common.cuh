@@ -77,6 +77,9 @@ struct BwdWorkspace {
 };
 BwdWorkspace bwd_workspace_layout(const fa_b200_params& p, int variant, bool inline_conversion = false);
 
+// What AUTO resolves to besides the public variants: the pair instances of the tensor-core kernels.
+constexpr int kVariantPair = 16;
+
 // ---- kernel families ---------------------------------------------------------
 // CUDA-core tiles (simt_kernels.cu)
 int simt_fwd(const fa_b200_params& p);
@@ -87,6 +90,11 @@ bool simt_supports(const fa_b200_params& p);
 int sm100_fwd(const fa_b200_params& p);
 int sm100_bwd(const fa_b200_params& p, const BwdWorkspace& ws);
 bool sm100_supports(const fa_b200_params& p, bool backward, const char** why);
+// The same kernels with P and dS as hi + lo pairs (fwd_pair_sm100.cu, bwd_pair_sm100.cu): 16-bit calls with an
+// additive bias, or a head size other than 64 and 128.
+int sm100_pair_fwd(const fa_b200_params& p);
+int sm100_pair_bwd(const fa_b200_params& p, const BwdWorkspace& ws);
+bool sm100_pair_supports(const fa_b200_params& p, bool backward, const char** why);
 // fp32 forward on the tensor cores (fwd_tf32_sm100.cu): TF32 products taken three times
 int sm100_tf32_fwd(const fa_b200_params& p);
 bool sm100_tf32_fwd_supports(const fa_b200_params& p, const char** why);

@@ -25,8 +25,8 @@ BwdWorkspace bwd_workspace_layout(const fa_b200_params& p, int variant, bool inl
     BwdWorkspace w;
     memset(&w, 0, sizeof(w));
     const size_t nq_pad = align_up((size_t)p.Nq, 128);
-    const bool tc = (variant == FA_B200_VARIANT_TCGEN05 || variant == FA_B200_VARIANT_TCGEN05_2PASS);
-    const bool copies = tc && p.dtype == FA_B200_BF16 && !inline_conversion;
+    const bool tc = variant != FA_B200_VARIANT_SIMT;
+    const bool copies = tc && variant != kVariantPair && p.dtype == FA_B200_BF16 && !inline_conversion;
     const bool one_kernel = (variant == FA_B200_VARIANT_TCGEN05 && sm100_bwd_fused_supported(p));
     size_t at = 0;
     auto region = [&](size_t* off, size_t* bytes, size_t n) { *off = at; *bytes = n; at = align_up(at + n, 256); };
@@ -202,6 +202,7 @@ int choose_variant(const fa_b200_params& p, bool backward, int* variant) {
     // AUTO is the deterministic form: every gradient element is summed by one CTA in a fixed order.
     // The one-kernel backward (dQ tiles summed with unordered global additions) is opt-in (TCGEN05).
     if (p.variant == FA_B200_VARIANT_AUTO && tc) { *variant = FA_B200_VARIANT_TCGEN05_2PASS; return FA_OK; }
+    if (p.variant == FA_B200_VARIANT_AUTO && sm100_pair_supports(p, backward, &why)) { *variant = kVariantPair; return FA_OK; }
     if (!simt_supports(p)) {
         set_error("no kernel covers D=%d (CUDA-core tiles need D <= 128; tensor-core tiles: %s)", p.D, why);
         return FA_EUNSUPPORTED;
@@ -267,6 +268,7 @@ int fa_b200_fwd(const fa_b200_params* p) {
     if ((rc = choose_variant(*p, false, &variant))) return rc;
     GuardDevice g(p->device);
     if (!g.ok) { set_error("cudaSetDevice(%d) failed", p->device); return FA_ECUDA; }
+    if (variant == kVariantPair) return sm100_pair_fwd(*p);
     return variant != FA_B200_VARIANT_SIMT ? sm100_fwd(*p) : simt_fwd(*p);
 }
 
@@ -299,6 +301,8 @@ size_t fa_b200_bwd_workspace_bytes(const fa_b200_params* p) {
     q.variant = FA_B200_VARIANT_AUTO;
     if (p->variant != FA_B200_VARIANT_SIMT && sm100_supports(q, true, &why))
         variant = (p->variant == FA_B200_VARIANT_TCGEN05) ? FA_B200_VARIANT_TCGEN05 : FA_B200_VARIANT_TCGEN05_2PASS;
+    else if (p->variant == FA_B200_VARIANT_AUTO && sm100_pair_supports(q, true, &why))
+        variant = kVariantPair;
     return bwd_workspace_layout(*p, variant).total;
 }
 
@@ -309,7 +313,8 @@ size_t fa_b200_dropout_bits_bytes(const fa_b200_params* p) {
     fa_b200_params q = *p;
     q.variant = FA_B200_VARIANT_AUTO;
     const char* why = "";
-    if (!sm100_supports(q, false, &why) && !sm100_supports(q, true, &why)) return 0;
+    if (!sm100_supports(q, false, &why) && !sm100_supports(q, true, &why) &&
+        !(p->variant == FA_B200_VARIANT_AUTO && sm100_pair_supports(q, false, &why))) return 0;
     return 2 * dropout_bits_bytes(*p);
 }
 
@@ -334,6 +339,7 @@ int fa_b200_bwd(const fa_b200_params* p) {
     GuardDevice g(p->device);
     if (!g.ok) { set_error("cudaSetDevice(%d) failed", p->device); return FA_ECUDA; }
     if (p->Nq == 0) return zero_dk_dv(p);      // no queries: dK = dV = 0
+    if (variant == kVariantPair) return sm100_pair_bwd(*p, ws);
     return variant != FA_B200_VARIANT_SIMT ? sm100_bwd(*p, ws) : simt_bwd(*p, ws);
 }
 
@@ -411,6 +417,7 @@ int fa_b200_bwd_static(const fa_b200_params* p) {
     q.workspace_bytes = kStaticScratchBytes;
     // Nothing in the scratch has to start at zero: the preprocess launch writes
     // every delta / lse entry (padding included) before the main kernels read them.
+    if (variant == kVariantPair) return sm100_pair_bwd(q, ws);
     return variant != FA_B200_VARIANT_SIMT ? sm100_bwd(q, ws) : simt_bwd(q, ws);
 }
 

@@ -1,8 +1,8 @@
 // CUDA-core attention tiles: the shape-generic kernel family of the library.
 //
 // Serves what the tensor-core family does not: fp32 inputs (computed in exact
-// fp32 FMA arithmetic, no TF32 rounding), head dims other than 64/128 (any
-// D <= 128), grouped K/V heads.  Same math as the tensor-core family:
+// fp32 FMA arithmetic, no TF32 rounding), head dims that are no multiple of 8 (any
+// D <= 128), unaligned views.  Same math as the tensor-core family:
 //
 //   forward  (replaces kernels/forward_kernel.py:18-243 of the reference)
 //     per 64-row query tile, for each 64-row key tile at or below the diagonal:

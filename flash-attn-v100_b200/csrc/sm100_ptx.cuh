@@ -377,6 +377,26 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return r;
 }
 
+// packed 16-bit pair -> two floats (`lo` from bits 0-15)
+template <bool BF16>
+__device__ __forceinline__ void unpack2(uint32_t v, float& lo, float& hi) {
+    if (BF16) {
+        lo = __uint_as_float(v << 16);
+        hi = __uint_as_float(v & 0xFFFF0000u);
+    } else {
+        asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}"
+            : "=f"(lo), "=f"(hi) : "r"(v));
+    }
+}
+// Two floats as packed 16-bit pairs hi + lo: hi the rounded values, lo what the rounding dropped, rounded once more.
+template <bool BF16>
+__device__ __forceinline__ void pack2_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+    hi = pack2<BF16>(x0, x1);
+    float h0, h1;
+    unpack2<BF16>(hi, h0, h1);
+    lo = pack2<BF16>(x0 - h0, x1 - h1);
+}
+
 // ---- bf16 -> fp16 in shared memory ---------------------------------------------------------------
 // tcgen05.mma kind::f16 wants both operands in one 16-bit format.  A product whose A operand is a
 // probability (or dS) tile rounded to bf16 carries that rounding, 2^-9 relative, into the result
@@ -417,18 +437,6 @@ __device__ __forceinline__ void convert_tile_bf16_to_f16(uint8_t* tile, int byte
             v.z = bf16x2_to_f16x2(v.z); v.w = bf16x2_to_f16x2(v.w);
         }
         p[i * nthreads] = v;
-    }
-}
-
-// packed 16-bit pair -> two floats (`lo` from bits 0-15)
-template <bool BF16>
-__device__ __forceinline__ void unpack2(uint32_t v, float& lo, float& hi) {
-    if (BF16) {
-        lo = __uint_as_float(v << 16);
-        hi = __uint_as_float(v & 0xFFFF0000u);
-    } else {
-        asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}"
-            : "=f"(lo), "=f"(hi) : "r"(v));
     }
 }
 

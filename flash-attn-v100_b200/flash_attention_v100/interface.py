@@ -272,7 +272,7 @@ def flash_attention_v100(
         scale: defaults to 1/sqrt(head_dim)
         dropout_p: drop probability of the attention weights (quantised to 1/256)
         bias: additive score bias, (B|1, H|1, Nq|1, Nk): scores = scale * q.k + bias before the causal mask;
-            -inf entries mask keys.  Served by the CUDA-core kernels; its gradient is returned
+            -inf entries mask keys.  Its gradient is returned
         key_lengths: (not in the reference) int tensor (B,): batch entry b attends to its first
             key_lengths[b] keys only (right-padded batches); key blocks beyond are skipped on every
             kernel family, dK / dV of the padding are zero

@@ -118,7 +118,7 @@ class EnhancedMultiHeadAttention(nn.Module):
         of each batch entry; the call stays on the tensor-core kernels and skips the padding's key
         blocks.  A boolean key_padding_mask alone (no attn_mask, is_causal False) gets there too, by moving
         the kept keys to the front (compact_keys); combined with other masks, or as a float mask, it
-        becomes a bias and runs on the CUDA-core kernels."""
+        becomes a bias."""
         if not self.batch_first:
             query = query.transpose(0, 1)
             key = key.transpose(0, 1) if key is not None else None

@@ -214,7 +214,7 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
         o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
         lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
     p = _base_params(q, k, v, o, lse, scale, causal, dropout_p, seed, offset, causal_shift, dropout_origin)
-    p.bias, _keep = _bias_operand(bias)        # scores = scale * q.k + bias (CUDA-core kernels)
+    p.bias, _keep = _bias_operand(bias)        # scores = scale * q.k + bias
     p.kv_lengths, _keep_len = _lengths_operand(key_lengths, q)
     if o_residual is not None:
         _check_residual(o_residual, o)

@@ -125,7 +125,8 @@ typedef struct fa_b200_params {
        fp32, logical shape (B, H, Nq, Nk): stride_b / stride_h / stride_n are the element strides over
        batch, head and QUERY index, the key index has stride 1; a stride of 0 broadcasts (a key-padding
        mask is (B, 1, 1, Nk): stride_h = stride_n = 0).  -inf entries mask keys.  ptr = NULL: no bias.
-       Calls with a bias are served by the CUDA-core kernels. */
+       With 16-bit inputs and a head size that is a multiple of 8 the tensor-core kernels serve such calls (P and
+       dS as hi + lo pairs); other calls with a bias run on the CUDA-core kernels. */
     fa_b200_tensor bias;
     /* backward, optional: dense (B, H, Nq, Nk) fp32 buffer, zero-filled by the caller, that receives
        d(loss)/d(scores) = P o (dP o Z - delta); the caller sums it over the bias' broadcast
