@@ -87,7 +87,9 @@ int simt_bwd(const fa_b200_params& p, const BwdWorkspace& ws);
 bool simt_supports(const fa_b200_params& p);
 
 // TMA + tcgen05 (fwd_sm100.cu, bwd_sm100.cu)
-int sm100_fwd(const fa_b200_params& p);
+// The forward's scratch is optional: with it (at least sm100_fwd_workspace_bytes) the work may be divided anew.
+int sm100_fwd(const fa_b200_params& p, void* ws, size_t ws_bytes);
+size_t sm100_fwd_workspace_bytes(const fa_b200_params& p);
 int sm100_bwd(const fa_b200_params& p, const BwdWorkspace& ws);
 bool sm100_supports(const fa_b200_params& p, bool backward, const char** why);
 // The same kernels with P and dS as hi + lo pairs (fwd_pair_sm100.cu, bwd_pair_sm100.cu): 16-bit calls with an

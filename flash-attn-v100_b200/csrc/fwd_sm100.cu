@@ -78,11 +78,18 @@ static_assert(tile::kFwdQTilesPerCta == 2, "the kernel is written for two query 
 //      tiles are padded to 64 or 128 columns by TMA's zero fill, the MMA K-steps and N stop at the head
 //      size).  P is handed over as hi + lo in the inputs' own format, two MMAs per K-step of P V, so P keeps
 //      17 (bf16) or 22 (fp16) significant bits and a bf16 V needs no conversion.
-template <int D, int PREC>
+// SCHED: how the work is divided (plan_schedule).
+//   0  whole pairs of 128-row tiles, round robin (kernel comment above)
+//   1  the split schedule, with packed tiles or plain ones
+//   2  the same for a call whose rows fit one tile (decoding): the tile's even key blocks go through S_0, P_0 and O_0,
+//      the odd ones through S_1, P_1 and O_1, and the two sums are put together in the epilogue; the room of the
+//      second query tile goes to the K and V rings.
+template <int D, int PREC, int SCHED>
 struct FwdCfg {
     static constexpr int kNBox = D / 64;
     static constexpr int kTileBytes = kNBox * kBoxBytes;
-    static constexpr int kStages = tile::fwd_kv_stages(D);
+    static constexpr int kQTiles = SCHED == 2 ? 1 : 2;
+    static constexpr int kStages = SCHED == 2 ? tile::fwd_one_tile_kv_stages(D) : tile::fwd_kv_stages(D);
     // barrier slots
     static constexpr int kQFull = 0;                       // [2]
     static constexpr int kQEmpty = 2;                      // [2] last S MMA of the pair has read Q_t
@@ -95,8 +102,13 @@ struct FwdCfg {
     static constexpr int kODone = kPFull + 2;              // [2]
     static constexpr int kPHalf = kODone + 2;              // [2] first 64 keys of P_t stored (one arrival per warp)
     static constexpr int kVConv = kPHalf + 2;              // [kStages] V_j converted to fp16 (one arrival per converting warp)
-    static constexpr int kNumBars = kVConv + kStages;
-    static constexpr int kSmemBytes = (2 + 2 * kStages) * kTileBytes + kNumBars * 8 + 64 + 1024;
+    static constexpr int kMlFull = kVConv + kStages;       // SCHED = 2: the odd blocks' maxima and sums are in shared memory
+    static constexpr int kORead = kMlFull + 1;             // SCHED = 2: O_1 has been read (both: one arrival per warp of a warpgroup)
+    static constexpr int kNumBars = kORead + 1;
+    static constexpr int kMlBytes = SCHED == 2 ? kBlockM * 8 : 0;
+    static constexpr int kWalkBytes = SCHED ? 8 * 40 : 0;  // a WalkRecord per softmax warp
+    static constexpr int kSmemBytes = (kQTiles + 2 * kStages) * kTileBytes + kNumBars * 8 + 64 + kMlBytes + kWalkBytes + 1024;
+    static_assert(kSmemBytes <= 232448, "shared-memory plan does not fit");
 };
 
 struct FwdArgs {
@@ -110,7 +122,7 @@ struct FwdArgs {
     int B, Nq, Nk, H, Hkv;
     int causal;
     int shift;                     // key j is visible to query i iff j <= i + shift
-    int n_pairs;                   // ceil(Nq / 256)
+    int n_pairs;                   // ceil(query tiles / 2)
     int items_per_head;            // causal: ceil(n_pairs / 2) mirrored items; else n_pairs
     int n_items;                   // items_per_head * B * H
     int wait_limit_ms;             // limit of one mbarrier wait (0: the default)
@@ -125,35 +137,196 @@ struct FwdArgs {
     int bias_vec;                  // its rows can be read as float4
     const uint4* mq;               // DROP = 2: keep bits, [(b*H + h) * n_kblocks + key block][padded query row]
     int nq_pad, n_kblocks;
+    // Rows of a query tile: `pack` query heads of one K/V head times `q_per_tile` queries, the heads fastest
+    // (1 and 128 unless the call is packed, see plan_schedule()).  `heads` = H / pack columns per batch entry.
+    int pack, q_per_tile, heads;
+    // Split schedule: the call's (pair, key block) units are cut into gridDim.x equal ranges; a pair that lies in
+    // several ranges leaves partial results for fwd_merge_kernel.
+    int part_rows;                 // rows a partial's slot holds
+    float4* part_o;                // [2 * gridDim.x slots][D / 4][part_rows], sums not yet divided
+    float2* part_ml;               // [2 * gridDim.x slots][part_rows]: maximum (log2 units), row sum (< 0: no block visited)
+    int4* part_meta;               // [gridDim.x]: batch, column, pair, number of ranges (0: none starts here)
 };
 
-struct Pair { int pair, h, b; };
+// A stretch of work: key blocks [j0, j1) of a pair.  n[t]: blocks the pair's tile t has in all
+// (0: no rows); count(t): how many of them lie in this stretch.
+struct Stretch {
+    int pair, h, b, nk, j0, j1, n[2];
+    __device__ __forceinline__ int count(int t) const { const int e = n[t] < j1 ? n[t] : j1; return e > j0 ? e - j0 : 0; }
+    __device__ __forceinline__ bool whole() const { return j0 == 0 && j1 >= n[0] && j1 >= n[1]; }
+};
 
-// Sub-item u (0 or 1) of work item w; false if the item has no such sub-item.
-__device__ __forceinline__ bool decode_work(const FwdArgs& a, int w, int u, Pair& out) {
-    const int bh = w / a.items_per_head, slot = w - bh * a.items_per_head;
-    int pair;
-    if (a.causal) {
-        const int heavy = a.n_pairs - 1 - slot;           // more key blocks: first
-        if (u == 0) pair = heavy;
-        else { if (slot == heavy) return false; pair = slot; }
-    } else {
-        if (u == 1) return false;
-        pair = slot;
-    }
-    out.pair = pair;
-    out.h = bh % a.H;
-    out.b = bh / a.H;
-    return true;
-}
-
-// key blocks tile t of a pair visits
-__device__ __forceinline__ int num_blocks(const FwdArgs& a, int pair, int t, int nk) {
-    const int row0 = (pair * 2 + t) * kBlockM;
+// key blocks tile t of a pair of tiles with q_per_tile queries visits
+__device__ __forceinline__ int num_blocks(const FwdArgs& a, int q_per_tile, int pair, int t, int nk) {
+    const int row0 = (pair * 2 + t) * q_per_tile;
     int kv_end = nk;               // keys this batch entry attends to
-    if (a.causal && row0 + kBlockM + a.shift < kv_end) kv_end = row0 + kBlockM + a.shift;
+    if (a.causal && row0 + q_per_tile + a.shift < kv_end) kv_end = row0 + q_per_tile + a.shift;
     return (row0 < a.Nq) ? (kv_end + kBlockN - 1) / kBlockN : 0;
 }
+__device__ __forceinline__ int pair_blocks(const FwdArgs& a, int pair, int nk) {
+    const int n0 = num_blocks(a, a.q_per_tile, pair, 0, nk), n1 = num_blocks(a, a.q_per_tile, pair, 1, nk);
+    return n0 > n1 ? n0 : n1;
+}
+
+// Where a CTA's range of units starts and how long it is (split schedule), left in shared memory for every role.
+// `ctas`: CTAs that have a range (with per-batch key counts the units can be fewer than the CTAs; every range has one).
+struct RangeStart { int b, h, pair, block, units, total, ctas; };
+__device__ __forceinline__ int range_begin(int cta, int ctas, int total) { return (int)((int64_t)cta * total / ctas); }
+
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) { const int o = __shfl_up_sync(0xffffffffu, v, off); if (lane >= off) v += o; }
+    return v;
+}
+// The index i < n whose cost range holds unit `target` of the costs laid end to end; target becomes the offset in it.
+template <typename Cost>
+__device__ __forceinline__ int warp_find(int n, int lane, int& target, Cost cost) {
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const int c = i0 + lane < n ? cost(i0 + lane) : 0;
+        const int incl = warp_scan(c, lane);
+        const uint32_t hit = __ballot_sync(0xffffffffu, target < incl);
+        if (hit) {
+            const int l = __ffs((int)hit) - 1;
+            target -= __shfl_sync(0xffffffffu, incl - c, l);
+            return i0 + l;
+        }
+        target -= __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return n - 1;
+}
+// One warp: the costs are the pairs' key blocks; with per-batch key counts a batch entry has a total of its own.
+__device__ __forceinline__ void find_range(const FwdArgs& a, int lane, volatile RangeStart* out) {
+    auto column = [&](int b) {                       // units of one (batch, column): serial, every lane its own b
+        const int nk = kv_len_of(a.kv_len, b, a.Nk);
+        int sum = 0;
+        for (int pr = 0; pr < a.n_pairs; ++pr) sum += pair_blocks(a, pr, nk);
+        return sum;
+    };
+    int total = 0, col = 0;
+    if (a.kv_len) {
+        for (int b = lane; b < a.B; b += 32) total += a.heads * column(b);
+        total = __shfl_sync(0xffffffffu, warp_scan(total, lane), 31);
+    } else {
+        for (int pr = lane; pr < a.n_pairs; pr += 32) col += pair_blocks(a, pr, a.Nk);
+        col = __shfl_sync(0xffffffffu, warp_scan(col, lane), 31);
+        total = a.B * a.heads * col;
+    }
+    const int ctas = total < (int)gridDim.x ? total : (int)gridDim.x;
+    if ((int)blockIdx.x >= ctas) { if (lane == 0) out->units = 0; return; }
+    const int first = range_begin((int)blockIdx.x, ctas, total);
+    const int units = range_begin((int)blockIdx.x + 1, ctas, total) - first;
+    int at = first, b;
+    if (a.kv_len) {
+        b = warp_find(a.B, lane, at, [&](int i) { return a.heads * column(i); });
+        col = column(b);
+    } else {
+        b = at / (a.heads * col);
+        at -= b * a.heads * col;
+    }
+    const int h = at / col;
+    at -= h * col;
+    const int nk = kv_len_of(a.kv_len, b, a.Nk);
+    const int pair = warp_find(a.n_pairs, lane, at, [&](int i) { return pair_blocks(a, i, nk); });
+    if (lane == 0) {
+        out->b = b; out->h = h; out->pair = pair; out->block = at; out->units = units; out->total = total; out->ctas = ctas;
+    }
+}
+
+// A role's walk over the CTA's work; every role runs one of its own and sees the same stretches:
+//     for (WorkLoop<SCHED> wl(a, range); wl.more(a); wl.advance()) for (u = 0; u < wl.kSub; ++u) if (wl.get(a, u, st)) ...
+// Two walks and not one with a switch, because the softmax threads have no register to spare: one walk for
+// both made the kernel of whole pairs spill more and cost it 1-2 % (B4 N4096 H32 D128).
+template <int SCHED> struct WorkLoop;
+template <> struct WorkLoop<0> {       // whole pairs, round robin
+    static constexpr int kSub = 2;     // causal: a pair and its mirror
+    int w;
+    __device__ __forceinline__ WorkLoop(const FwdArgs&, const volatile RangeStart*) : w(blockIdx.x) {}
+    __device__ __forceinline__ bool more(const FwdArgs& a) const { return w < a.n_items; }
+    __device__ __forceinline__ void advance() { w += gridDim.x; }
+    __device__ __forceinline__ bool get(const FwdArgs& a, int u, Stretch& s) const {
+        const int bh = w / a.items_per_head, slot = w - bh * a.items_per_head;
+        int pair;
+        if (a.causal) {
+            const int heavy = a.n_pairs - 1 - slot;           // more key blocks: first
+            if (u == 0) pair = heavy;
+            else { if (slot == heavy) return false; pair = slot; }
+        } else {
+            if (u == 1) return false;
+            pair = slot;
+        }
+        s.pair = pair;
+        s.h = bh % a.H;
+        s.b = bh / a.H;
+        s.nk = kv_len_of(a.kv_len, s.b, a.Nk);
+        s.n[0] = num_blocks(a, kBlockM, pair, 0, s.nk); s.n[1] = num_blocks(a, kBlockM, pair, 1, s.nk);
+        s.j0 = 0;
+        s.j1 = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
+        return true;
+    }
+};
+template <> struct WorkLoop<1> {       // split schedule: the CTA's range of units
+    static constexpr int kSub = 1;
+    int b, h, pair, block, units;
+    __device__ __forceinline__ WorkLoop(const FwdArgs&, const volatile RangeStart* r)
+        : b(r->b), h(r->h), pair(r->pair), block(r->block), units(r->units) {}
+    __device__ __forceinline__ bool more(const FwdArgs&) const { return units > 0; }
+    __device__ __forceinline__ void advance() {}
+    __device__ __forceinline__ bool get(const FwdArgs& a, int, Stretch& s) {
+        s.pair = pair; s.h = h; s.b = b;
+        s.nk = kv_len_of(a.kv_len, b, a.Nk);
+        s.n[0] = num_blocks(a, a.q_per_tile, pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, pair, 1, s.nk);
+        const int n = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
+        s.j0 = block;
+        s.j1 = n - block < units ? n : block + units;
+        units -= s.j1 - s.j0;
+        block = 0;
+        if (++pair == a.n_pairs) { pair = 0; if (++h == a.heads) { h = 0; ++b; } }
+        return true;
+    }
+};
+template <> struct WorkLoop<2> : WorkLoop<1> { using WorkLoop<1>::WorkLoop; };
+
+// The softmax warps' form of the walk: its state and the current stretch lie in shared memory, a record per warp, and
+// the epilogue reads the stretch again, so that no register holds them while a block's 128 scores are worked on.
+// Held in registers, the D = 128 kernel spilled 424 bytes instead of 60 and the chunk below took 152 us instead of 112.
+struct WalkRecord { int b, h, pair, block, units, cur_pair, cur_h, cur_b, cur_j0, cur_j1; };
+template <int SCHED> struct SoftmaxLoop : WorkLoop<SCHED> {
+    __device__ __forceinline__ SoftmaxLoop(const FwdArgs& a, const volatile RangeStart* r, volatile WalkRecord*) : WorkLoop<SCHED>(a, r) {}
+    __device__ __forceinline__ void again(const FwdArgs&, Stretch&) const {}
+};
+struct SplitSoftmaxLoop {
+    static constexpr int kSub = 1;
+    volatile WalkRecord* rec;
+    __device__ __forceinline__ SplitSoftmaxLoop(const FwdArgs&, const volatile RangeStart* r, volatile WalkRecord* w) : rec(w) {
+        rec->b = r->b; rec->h = r->h; rec->pair = r->pair; rec->block = r->block; rec->units = r->units;    // every lane the same
+        __syncwarp();
+    }
+    __device__ __forceinline__ bool more(const FwdArgs&) const { return rec->units > 0; }
+    __device__ __forceinline__ void advance() {}
+    __device__ __forceinline__ bool get(const FwdArgs& a, int, Stretch& s) {
+        int b = rec->b, h = rec->h, pair = rec->pair;
+        const int block = rec->block, units = rec->units;
+        s.pair = pair; s.h = h; s.b = b;
+        s.nk = kv_len_of(a.kv_len, b, a.Nk);
+        s.n[0] = num_blocks(a, a.q_per_tile, pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, pair, 1, s.nk);
+        const int n = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
+        s.j0 = block;
+        s.j1 = n - block < units ? n : block + units;
+        if (++pair == a.n_pairs) { pair = 0; if (++h == a.heads) { h = 0; ++b; } }
+        __syncwarp();                                  // every lane has read
+        rec->b = b; rec->h = h; rec->pair = pair; rec->block = 0; rec->units = units - (s.j1 - s.j0);
+        rec->cur_pair = s.pair; rec->cur_h = s.h; rec->cur_b = s.b; rec->cur_j0 = s.j0; rec->cur_j1 = s.j1;
+        __syncwarp();
+        return true;
+    }
+    __device__ __forceinline__ void again(const FwdArgs& a, Stretch& s) const {
+        s.pair = rec->cur_pair; s.h = rec->cur_h; s.b = rec->cur_b; s.j0 = rec->cur_j0; s.j1 = rec->cur_j1;
+        s.nk = kv_len_of(a.kv_len, s.b, a.Nk);
+        s.n[0] = num_blocks(a, a.q_per_tile, s.pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, s.pair, 1, s.nk);
+    }
+};
+template <> struct SoftmaxLoop<1> : SplitSoftmaxLoop { using SplitSoftmaxLoop::SplitSoftmaxLoop; };
+template <> struct SoftmaxLoop<2> : SplitSoftmaxLoop { using SplitSoftmaxLoop::SplitSoftmaxLoop; };
 
 // P is stored as 2^(S c - m + kPShift): with the lazily refreshed maximum P <= 2^8, so the shifted value
 // stays below 2^14 in fp16 and entries down to 2^-20 of the row's largest keep full precision.
@@ -161,11 +334,13 @@ constexpr float kPShift = 6.0f;
 
 // DROP: 0 no dropout; 1 the keep bits are drawn here, by the softmax threads (no workspace);
 // 2 they are loaded from the workspace, where dropout_bits_kernel has written the call's bits.
-template <int D, bool BF16, int DROP, int PREC>
+// SCHED: see FwdCfg.
+template <int D, bool BF16, int DROP, int PREC, int SCHED>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const FwdArgs a) {
-    using Cfg = FwdCfg<D, PREC>;
+    using Cfg = FwdCfg<D, PREC, SCHED>;
+    constexpr bool FREE = SCHED != 0, TWIN = SCHED == 2;
     constexpr int ST = Cfg::kStages;
     constexpr int TILE = Cfg::kTileBytes;
     // tcgen05.mma kind::f16 wants A and B in one format (an fp16 A next to a bf16 B raises an
@@ -177,18 +352,19 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = smem;
-    uint8_t* sK = sQ + 2 * TILE;
+    uint8_t* sK = sQ + Cfg::kQTiles * TILE;
     uint8_t* sV = sK + ST * TILE;
     uint64_t* bars = (uint64_t*)(sV + ST * TILE);
     uint32_t* tmem_slot = (uint32_t*)(bars + Cfg::kNumBars);
     volatile uint32_t* abort_flag = (volatile uint32_t*)(tmem_slot + 1);
+    [[maybe_unused]] float2* sMl = (float2*)((uint8_t*)(bars + Cfg::kNumBars) + 64);      // SCHED = 2: [128]
+    volatile RangeStart* range = (volatile RangeStart*)(tmem_slot + 4);      // seven words of the 64 bytes behind the barriers
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int group = a.H / a.Hkv;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < Cfg::kNumBars; ++i) {
-            const bool wg_bar = (i >= Cfg::kPFull && i < Cfg::kPFull + 2) || (i >= Cfg::kPHalf && i < Cfg::kPHalf + 2);
+            const bool wg_bar = (i >= Cfg::kPFull && i < Cfg::kPFull + 2) || (i >= Cfg::kPHalf && i < Cfg::kPHalf + 2) || i >= Cfg::kMlFull;
             const bool conv_bar = (i >= Cfg::kVConv && i < Cfg::kVConv + ST);
             mbar_init(&bars[i], wg_bar ? 4u : (conv_bar ? 2u : 1u));
         }
@@ -204,11 +380,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         prefetch_tensormap(&map_k);
         prefetch_tensormap(&map_v);
     }
+    if (FREE && warp == 11) find_range(a, lane, range);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
+    if (FREE) grid_launch_dependents();       // fwd_merge_kernel, which waits for this grid's end
 
+    const int pack = FREE ? a.pack : 1, q_per_tile = FREE ? a.q_per_tile : kBlockM;
     if (warp >= 8) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
       if (warp == 9) {
@@ -217,29 +396,27 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             int kvc = 0;                    // K/V blocks loaded so far (ring index = count % ST)
             int q_loads[2] = {0, 0};
             bool ok = true;
-            for (int w = blockIdx.x; w < a.n_items && ok; w += gridDim.x) {
-                for (int u = 0; u < 2 && ok; ++u) {
-                    Pair pr;
-                    if (!decode_work(a, w, u, pr)) continue;
-                    const int hk = pr.h / group;
-                    const int q0 = pr.pair * 2 * kBlockM;
-                    const int nk = kv_len_of(a.kv_len, pr.b, a.Nk);
-                    const int n0 = num_blocks(a, pr.pair, 0, nk), n1 = num_blocks(a, pr.pair, 1, nk);
-                    const int nmax = n0 > n1 ? n0 : n1;
+            const uint32_t q_bytes = FREE ? (uint32_t)(Cfg::kNBox * 128 * pack * q_per_tile) : TILE;
+            for (WorkLoop<SCHED> wl(a, range); wl.more(a) && ok; wl.advance()) {
+                for (int u = 0; u < wl.kSub && ok; ++u) {
+                    Stretch st;
+                    if (!wl.get(a, u, st)) continue;
+                    const int hk = st.h * pack / (a.H / a.Hkv);
+                    const int q0 = st.pair * 2 * q_per_tile;
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
-                        if ((t == 0 ? n0 : n1) == 0) continue;
+                        if (st.count(t) == 0) continue;
                         // Q_t of the previous pair must have been read by its last S MMA
                         ok = mbar_wait(&bars[Cfg::kQEmpty + t], ((uint32_t)q_loads[t] & 1u) ^ 1u, abort_flag);
                         if (!ok) break;
-                        mbar_expect_tx(&bars[Cfg::kQFull + t], TILE);
+                        mbar_expect_tx(&bars[Cfg::kQFull + t], q_bytes);
 #pragma unroll
                         for (int bx = 0; bx < Cfg::kNBox; ++bx)
                             tma_load_4d(sQ + t * TILE + bx * kBoxBytes, &map_q, &bars[Cfg::kQFull + t],
-                                        bx * 64, pr.h, q0 + t * kBlockM, pr.b);
+                                        bx * 64, st.h * pack, q0 + t * q_per_tile, st.b);
                         ++q_loads[t];
                     }
-                    for (int j = 0; j < nmax && ok; ++j, ++kvc) {
+                    for (int j = st.j0; j < st.j1 && ok; ++j, ++kvc) {
                         const int s = kvc % ST;
                         const uint32_t ph = (uint32_t)(kvc / ST) & 1u;
                         ok = mbar_wait(&bars[Cfg::kKEmpty + s], ph ^ 1u, abort_flag);
@@ -248,7 +425,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                         for (int bx = 0; bx < Cfg::kNBox; ++bx)
                             tma_load_4d(sK + s * TILE + bx * kBoxBytes, &map_k, &bars[Cfg::kKFull + s],
-                                        bx * 64, hk, j * kBlockN, pr.b);
+                                        bx * 64, hk, j * kBlockN, st.b);
                         ok = mbar_wait(&bars[Cfg::kVEmpty + s], ph ^ 1u, abort_flag);
                         if (!ok) {
                             // K of this block is in flight: let it land before giving up shared memory
@@ -259,7 +436,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                         for (int bx = 0; bx < Cfg::kNBox; ++bx)
                             tma_load_4d(sV + s * TILE + bx * kBoxBytes, &map_v, &bars[Cfg::kVFull + s],
-                                        bx * 64, hk, j * kBlockN, pr.b);
+                                        bx * 64, hk, j * kBlockN, st.b);
                     }
                 }
             }
@@ -326,13 +503,55 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             int q_uses[2] = {0, 0};         // pairs that used tile t (Q_full phase)
             int p_waits[2] = {0, 0};        // P_t hand-offs so far (P_full phase)
             bool ok = true;
-            for (int w = blockIdx.x; w < a.n_items && ok; w += gridDim.x) {
-                for (int u = 0; u < 2 && ok; ++u) {
-                    Pair pr;
-                    if (!decode_work(a, w, u, pr)) continue;
-                    const int nk = kv_len_of(a.kv_len, pr.b, a.Nk);
-                    int nblk[2] = {num_blocks(a, pr.pair, 0, nk), num_blocks(a, pr.pair, 1, nk)};
-                    const int nmax = nblk[0] > nblk[1] ? nblk[0] : nblk[1];
+            for (WorkLoop<SCHED> wl(a, range); TWIN && wl.more(a) && ok; wl.advance()) {
+                Stretch st;
+                wl.get(a, 0, st);
+                // one tile: block j of the stretch belongs to accumulator set j & 1
+                const int nb = st.j1 - st.j0;
+                ok = mbar_wait(&bars[Cfg::kQFull], (uint32_t)q_uses[0] & 1u, abort_flag);
+                ++q_uses[0];
+                auto s_block = [&](int j) {
+                    const int c = kvc + j;
+                    if (!mbar_wait(&bars[Cfg::kKFull + c % ST], (uint32_t)(c / ST) & 1u, abort_flag)) return false;
+                    tc_fence_after_sync();
+                    const uint64_t b0 = dK + (uint64_t)(((c % ST) * TILE) >> 4);
+                    const uint32_t d = tmem + (uint32_t)(j & 1) * 128u;
+#pragma unroll
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t off = ((uint32_t)(kk >> 2) * kBoxBytes + (uint32_t)(kk & 3) * 32u) >> 4;
+                        mma_ss_f16(d, dQ + off, b0 + off, idesc_s, kk > 0);
+                    }
+                    mma_commit(&bars[Cfg::kSFull + (j & 1)]);
+                    mma_commit(&bars[Cfg::kKEmpty + c % ST]);
+                    if (j == nb - 1) mma_commit(&bars[Cfg::kQEmpty]);
+                    return true;
+                };
+                if (ok) ok = s_block(0);
+                if (ok && nb > 1) ok = s_block(1);
+                for (int j = 0; j < nb && ok; ++j) {
+                    const int t = j & 1, c = kvc + j, vs = c % ST;
+                    ok = mbar_wait(&bars[(CONV ? Cfg::kVConv : Cfg::kVFull) + vs], (uint32_t)(c / ST) & 1u, abort_flag);
+                    if (ok) ok = mbar_wait(&bars[Cfg::kPHalf + t], (uint32_t)p_waits[t] & 1u, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    issue_pv(t, vs, j > 1, 0);
+                    ok = mbar_wait(&bars[Cfg::kPFull + t], (uint32_t)p_waits[t] & 1u, abort_flag);
+                    if (!ok) break;
+                    ++p_waits[t];
+                    tc_fence_after_sync();
+                    issue_pv(t, vs, j > 1, 1);
+                    if (j + 2 >= nb) mma_commit(&bars[Cfg::kODone + t]);
+                    mma_commit(&bars[Cfg::kVEmpty + vs]);
+                    if (j + 2 < nb) ok = s_block(j + 2);
+                }
+                kvc += nb;
+            }
+            for (WorkLoop<SCHED> wl(a, range); !TWIN && wl.more(a) && ok; wl.advance()) {
+                for (int u = 0; u < wl.kSub && ok; ++u) {
+                    Stretch st;
+                    if (!wl.get(a, u, st)) continue;
+                    const int nblk[2] = {st.count(0), st.count(1)};
+                    const int nmax = st.j1 - st.j0;
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {
                         if (nblk[t] == 0) continue;
@@ -401,14 +620,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const int ct = (warp - 10) * 32 + lane;
         int kvc = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < a.n_items && ok; w += gridDim.x) {
-            for (int u = 0; u < 2 && ok; ++u) {
-                Pair pr;
-                if (!decode_work(a, w, u, pr)) continue;
-                const int nk = kv_len_of(a.kv_len, pr.b, a.Nk);
-                const int n0 = num_blocks(a, pr.pair, 0, nk), n1 = num_blocks(a, pr.pair, 1, nk);
-                const int nmax = n0 > n1 ? n0 : n1;
-                for (int j = 0; j < nmax; ++j, ++kvc) {
+        for (WorkLoop<SCHED> wl(a, range); wl.more(a) && ok; wl.advance()) {
+            for (int u = 0; u < wl.kSub && ok; ++u) {
+                Stretch st;
+                if (!wl.get(a, u, st)) continue;
+                for (int j = st.j0; j < st.j1; ++j, ++kvc) {
                     const int sidx = kvc % ST;
                     ok = mbar_wait(&bars[Cfg::kVFull + sidx], (uint32_t)(kvc / ST) & 1u, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
@@ -429,35 +645,65 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
         const uint32_t tS = tmem + (uint32_t)t * 128u + lane_off;
         const uint32_t tO = tmem + 256u + (uint32_t)t * 128u + lane_off;
+        static_assert(sizeof(WalkRecord) == 40, "kWalkBytes");
+        volatile WalkRecord* walk = (volatile WalkRecord*)((uint8_t*)(bars + Cfg::kNumBars) + 64 + Cfg::kMlBytes) + warp;
         int s_waits = 0;                 // S_t hand-offs so far (S_full phase)
         int o_waits = 0;                 // pairs finished so far (O_done phase)
+        [[maybe_unused]] int stretches = 0;
         bool ok = true;
 
-        for (int w = blockIdx.x; w < a.n_items && ok; w += gridDim.x) {
-            for (int u = 0; u < 2 && ok; ++u) {
-                Pair pr;
-                if (!decode_work(a, w, u, pr)) continue;
-                const int nk = kv_len_of(a.kv_len, pr.b, a.Nk);
-                const int n = num_blocks(a, pr.pair, t, nk);
-                if (n == 0) continue;
-                const int tile = pr.pair * 2 + t;
-                const int i = tile * kBlockM + r;                    // global query row
-                const uint32_t bh = dropout_column(a.rng, pr.b, pr.h);
+        if (FREE && threadIdx.x == 0) a.part_meta[blockIdx.x] = make_int4(0, 0, 0, 0);
+        for (SoftmaxLoop<SCHED> wl(a, range, walk); wl.more(a) && ok; wl.advance()) {
+            for (int u = 0; u < wl.kSub && ok; ++u) {
+                Stretch st;
+                if (!wl.get(a, u, st)) continue;
+                // blocks [j0, n) are mine, with one tile every other one of them
+                constexpr int kStep = TWIN ? 2 : 1;
+                const int tile = TWIN ? 0 : st.pair * 2 + t;
+                const int first = st.j0 + (TWIN ? t : 0), n = TWIN ? st.j1 : st.j0 + st.count(t), nk = st.nk;
+                // my row: query i of head h; a packed tile may hold rows of no query (row_ok() is false)
+                int i = tile * q_per_tile + (FREE ? r / pack : r);
+                int h = FREE ? st.h * pack + r % pack : st.h;
+                auto row_ok = [&] { return i < a.Nq && (!FREE || r < pack * q_per_tile); };
+                if (FREE && !st.whole()) {
+                    // the slot my row's partial goes to: a range's first stretch takes slot 0 unless it starts a pair
+                    const int64_t slot = 2 * (int64_t)blockIdx.x + (st.j0 == 0 ? 1 : 0);
+                    if (!TWIN && n == st.j0 && row_ok()) a.part_ml[slot * a.part_rows + t * kBlockM + r] = make_float2(-INFINITY, -1.f);
+                    if (threadIdx.x == 0 && st.j0 == 0) {
+                        // the pair starts here and goes on in the ranges of the CTAs behind this one
+                        const int total = range->total, ctas = range->ctas;
+                        const int full = st.n[0] > st.n[1] ? st.n[0] : st.n[1];
+                        const int end = range_begin((int)blockIdx.x + 1, ctas, total) + (full - st.j1);
+                        int k = 1;
+                        while (range_begin((int)blockIdx.x + k, ctas, total) < end) ++k;
+                        a.part_meta[blockIdx.x] = make_int4(st.b, st.h, st.pair, k);
+                    }
+                }
+                if (!TWIN && n == st.j0) continue;
+                // a warp none of whose rows is a query of the call keeps the pipeline's hand-offs going and computes
+                // nothing: its rows of P are whatever tensor memory holds, and no other row of O depends on them
+                const bool idle = TWIN && __all_sync(0xffffffffu, !row_ok());
+                const uint32_t bh = dropout_column(a.rng, st.b, h);
                 float m = -INFINITY, l = 0.f;
                 // my row of the bias (a row beyond Nq, whose results nobody keeps, reads the last one)
                 const float* brow = nullptr;
                 if (PREC != 0 && a.bias)
-                    brow = a.bias + pr.b * a.bias_sb + pr.h * a.bias_sh + (int64_t)(i < a.Nq ? i : a.Nq - 1) * a.bias_sn;
+                    brow = a.bias + st.b * a.bias_sb + h * a.bias_sh + (int64_t)(i < a.Nq ? i : a.Nq - 1) * a.bias_sn;
 
-                for (int j = 0; j < n; ++j) {
+                for (int j = first; j < n; j += kStep) {
                     // DROP = 2: the block's 128 keep bits of my row, asked for before the wait for S
                     uint4 kb4 = make_uint4(0u, 0u, 0u, 0u);
                     if constexpr (DROP == 2)
-                        kb4 = a.mq[((int64_t)(pr.b * a.H + pr.h) * a.n_kblocks + j) * a.nq_pad + i];
+                        kb4 = a.mq[((int64_t)(st.b * a.H + h) * a.n_kblocks + j) * a.nq_pad + i];
                     ok = mbar_wait(&bars[Cfg::kSFull + t], (uint32_t)s_waits & 1u, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);      // the TMEM accesses below are warp-collective
                     if (!ok) break;
                     ++s_waits;
+                    if (idle) {
+                        mbar_arrive_warp(&bars[Cfg::kPHalf + t]);
+                        mbar_arrive_warp(&bars[Cfg::kPFull + t]);
+                        continue;
+                    }
                     tc_fence_after_sync();
                     uint32_t sr[4][32];                    // the row's 128 scores, then its 128 probabilities
 #define SF(c) __uint_as_float(sr[(c) >> 5][(c) & 31])
@@ -495,7 +741,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                             }
                         }
                     }
-                    const bool need_mask = (a.causal && col0 + kBlockN - 1 > tile * kBlockM + a.shift) || (col0 + kBlockN > nk);
+                    const bool need_mask = (a.causal && col0 + kBlockN - 1 > tile * q_per_tile + a.shift) || (col0 + kBlockN > nk);
                     if (need_mask) {
                         // my row sees the block's first `seen` columns: keys below the count, at most i + shift
                         int seen = nk - col0;
@@ -514,11 +760,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     const float m_new = fmaxf(m, mx);
                     const bool grow = (m_new - m) > kRescaleThreshold;   // first block: inf > 8
                     if (__any_sync(0xffffffffu, grow)) {
-                        // 0 on the first block; with a bias a row may have seen nothing but -inf so far
-                        const float alpha = (PREC && m_new == -INFINITY) ? 0.f : ex2(m - m_new);
+                        // 0 on the first block; a row may have seen nothing but -inf so far (a bias; a stretch of a pair)
+                        const float alpha = ((PREC || FREE) && m_new == -INFINITY) ? 0.f : ex2(m - m_new);
                         m = m_new;
                         l *= alpha;
-                        if (j > 0) {
+                        if (j > first) {
                             // S_t(j) complete implies PV_t(j-1) complete (same issuing thread, in order)
 #pragma unroll
                             for (int c0 = 0; c0 < D; c0 += 32) {
@@ -575,7 +821,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     // dropout P is packed to 16 bits as it is produced and each 64-key half is
                     // stored to TMEM as soon as it is complete, so conversion and store latency
                     // overlap the exponentials of the other half.
-                    const uint64_t c2 = f2_pack(a.scale_log2, a.scale_log2), nm2 = f2_pack(kPShift - m, kPShift - m);
+                    const float ms = kPShift - (FREE && m == -INFINITY ? 0.f : m);     // nothing seen yet: P = 0
+                    const uint64_t c2 = f2_pack(a.scale_log2, a.scale_log2), nm2 = f2_pack(ms, ms);
                     uint64_t la = 0ull, lb = 0ull;             // {0.f, 0.f}
 #pragma unroll
                     for (int c0 = 0; c0 < 2; ++c0) {
@@ -646,22 +893,96 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 if (!ok) break;
 
                 // ---- epilogue: O_t / l -> 16 bit -> global, straight from registers
-                ok = mbar_wait(&bars[Cfg::kODone + t], (uint32_t)o_waits & 1u, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                ++o_waits;
-                tc_fence_after_sync();
+                if constexpr (FREE) {
+                    wl.again(a, st);
+                    i = (TWIN ? 0 : st.pair * 2 + t) * q_per_tile + r / pack;
+                    h = st.h * pack + r % pack;
+                }
+                if (!TWIN || t == 0 || st.j1 - st.j0 > 1) {
+                    ok = mbar_wait(&bars[Cfg::kODone + t], (uint32_t)o_waits & 1u, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    ++o_waits;
+                    tc_fence_after_sync();
+                }
+                // one tile: O = w0 O_0 + w1 O_1, the other set's maximum and sum through shared memory.  The second
+                // warpgroup goes on, and lets O_1 be overwritten, when the first has read both.
+                [[maybe_unused]] float w0 = 1.f, w1 = 0.f;
+                if constexpr (TWIN) {
+                    const uint32_t ph = (uint32_t)stretches & 1u;
+                    ++stretches;
+                    if (t == 1) {
+                        sMl[r] = make_float2(m, st.j1 - st.j0 > 1 ? l : -1.f);
+                        tc_fence_before_sync();
+                        mbar_arrive_warp(&bars[Cfg::kMlFull]);
+                        ok = mbar_wait(&bars[Cfg::kORead], ph, abort_flag);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        continue;
+                    }
+                    ok = mbar_wait(&bars[Cfg::kMlFull], ph, abort_flag);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    const float2 o1 = sMl[r];
+                    if (o1.y >= 0.f || o1.y != o1.y) {          // (NaN: the row's result)
+                        const float m01 = fmaxf(m, o1.x);
+                        w0 = m == -INFINITY ? 0.f : ex2(m - m01);
+                        w1 = o1.x == -INFINITY ? 0.f : ex2(o1.x - m01);
+                        m = m01;
+                        l = fmaf(l, w0, o1.y * w1);
+                    }
+                }
+                // 32 columns of my row's sums
+                auto load_o = [&](int c0, uint32_t (&orr)[32]) {
+                    tmem_ld_32x32(tO + c0, orr);
+                    if constexpr (TWIN) {
+                        uint32_t o1[32];
+                        tmem_ld_32x32(tO + 128u + c0, o1);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) {
+                            const float x = __uint_as_float(orr[c]);
+                            orr[c] = __float_as_uint(st.j1 - st.j0 > 1 ? fmaf(x, w0, __uint_as_float(o1[c]) * w1) : x);
+                        }
+                        if (c0 + 32 == D) {
+                            tc_fence_before_sync();
+                            mbar_arrive_warp(&bars[Cfg::kORead]);
+                        }
+                    } else {
+                        tmem_wait_ld();
+                    }
+                };
+                if (FREE && !st.whole()) {
+                    // a part of the pair's keys: the sums as they are, four columns of neighbouring rows side by side
+                    const int64_t slot = 2 * (int64_t)blockIdx.x + (st.j0 == 0 ? 1 : 0);
+                    const int pr = t * kBlockM + r;
+                    if (row_ok()) a.part_ml[slot * a.part_rows + pr] = make_float2(m, l);
+                    float4* po = a.part_o + slot * (int64_t)(D / 4) * a.part_rows + pr;
+#pragma unroll
+                    for (int c0 = 0; c0 < D; c0 += 32) {
+                        uint32_t orr[32];
+                        load_o(c0, orr);
+                        if (row_ok()) {
+#pragma unroll
+                            for (int g = 0; g < 8; ++g)
+                                po[(int64_t)(c0 / 4 + g) * a.part_rows] =
+                                    make_float4(__uint_as_float(orr[4 * g]), __uint_as_float(orr[4 * g + 1]),
+                                                __uint_as_float(orr[4 * g + 2]), __uint_as_float(orr[4 * g + 3]));
+                        }
+                    }
+                    continue;
+                }
                 const float inv = a.inv_keep / l;
-                T16* orow = reinterpret_cast<T16*>(a.o) + (int64_t)pr.b * a.o_sb + (int64_t)i * a.o_sn +
-                            (int64_t)pr.h * a.o_sh;
-                T16* lrow = a.o_lo ? reinterpret_cast<T16*>(a.o_lo) + (int64_t)pr.b * a.l_sb + (int64_t)i * a.l_sn +
-                                         (int64_t)pr.h * a.l_sh : nullptr;
+                T16* orow = reinterpret_cast<T16*>(a.o) + (int64_t)st.b * a.o_sb + (int64_t)i * a.o_sn +
+                            (int64_t)h * a.o_sh;
+                T16* lrow = a.o_lo ? reinterpret_cast<T16*>(a.o_lo) + (int64_t)st.b * a.l_sb + (int64_t)i * a.l_sn +
+                                         (int64_t)h * a.l_sh : nullptr;
 #pragma unroll
                 for (int c0 = 0; c0 < D; c0 += 32) {
                     uint32_t orr[32];
-                    tmem_ld_32x32(tO + c0, orr);
-                    tmem_wait_ld();
-                    if (i < a.Nq) {
+                    load_o(c0, orr);
+                    if (row_ok()) {
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
                             if (PREC == 1 && c0 + g * 8 >= a.d) break;
@@ -687,7 +1008,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                 }
-                if (i < a.Nq) a.lse[((int64_t)pr.b * a.H + pr.h) * a.Nq + i] = kLn2 * ((m - kPShift) + log2f(l));
+                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = kLn2 * ((m - kPShift) + log2f(l));
                 // the O_t reads above are complete (wait::ld); the next pair's first PV_t MMA waits for
                 // this warpgroup's next P_t, so it cannot overwrite O_t earlier
             }
@@ -700,14 +1021,148 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 1);
 }
 
+// Put together the pairs that the split schedule cut: block (c, y) takes 32 rows of the pair that starts in CTA c's
+// range and goes on in others.  Its parts are read in the order of the ranges, so the result does not depend on
+// which CTA finished first.  A lane holds one row, a warp every eighth group of eight columns.
+template <int D, bool BF16>
+__global__ void __launch_bounds__(256) fwd_merge_kernel(const FwdArgs a) {
+    using T16 = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+    grid_dependency_wait();
+    const int4 meta = a.part_meta[blockIdx.x];
+    if (meta.w == 0) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rr = (int)blockIdx.y * 32 + lane, t = rr / kBlockM, r = rr % kBlockM;
+    const int i = (meta.z * 2 + t) * a.q_per_tile + r / a.pack, h = meta.y * a.pack + r % a.pack, b = meta.x;
+    if (i >= a.Nq || r >= a.pack * a.q_per_tile) return;
+    auto slot_of = [&](int k) { return 2 * ((int64_t)blockIdx.x + k) + (k == 0 ? 1 : 0); };
+    float m = -INFINITY;
+#pragma unroll 8
+    for (int k = 0; k < meta.w; ++k) m = fmaxf(m, a.part_ml[slot_of(k) * a.part_rows + rr].x);
+    constexpr int kGroups = (D / 8 + 7) / 8;           // column groups a warp takes
+    float acc[kGroups][8], l = 0.f;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[g][e] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < meta.w; ++k) {
+        const int64_t slot = slot_of(k);
+        const float2 ml = a.part_ml[slot * a.part_rows + rr];
+        if (ml.y < 0.f) continue;                      // none of the tile's blocks lay in this range
+        const float w = ml.x == -INFINITY ? 0.f : ex2(ml.x - m);
+        l = fmaf(w, ml.y, l);
+        const float4* po = a.part_o + slot * (int64_t)(D / 4) * a.part_rows + rr;
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g) {
+            const int c4 = (g * 8 + warp) * 2;
+            const float4 x = po[(int64_t)c4 * a.part_rows], y = po[(int64_t)(c4 + 1) * a.part_rows];
+            acc[g][0] = fmaf(w, x.x, acc[g][0]); acc[g][1] = fmaf(w, x.y, acc[g][1]);
+            acc[g][2] = fmaf(w, x.z, acc[g][2]); acc[g][3] = fmaf(w, x.w, acc[g][3]);
+            acc[g][4] = fmaf(w, y.x, acc[g][4]); acc[g][5] = fmaf(w, y.y, acc[g][5]);
+            acc[g][6] = fmaf(w, y.z, acc[g][6]); acc[g][7] = fmaf(w, y.w, acc[g][7]);
+        }
+    }
+    const float inv = a.inv_keep / l;
+    T16* orow = reinterpret_cast<T16*>(a.o) + (int64_t)b * a.o_sb + (int64_t)i * a.o_sn + (int64_t)h * a.o_sh;
+    T16* lrow = a.o_lo ? reinterpret_cast<T16*>(a.o_lo) + (int64_t)b * a.l_sb + (int64_t)i * a.l_sn + (int64_t)h * a.l_sh : nullptr;
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g) {
+        const int c0 = (g * 8 + warp) * 8;
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float x0 = acc[g][2 * e] * inv, x1 = acc[g][2 * e + 1] * inv;
+            float h0, h1;
+            hi[e] = pack2<BF16>(x0, x1);
+            unpack2<BF16>(hi[e], h0, h1);
+            lo[e] = pack2<BF16>(x0 - h0, x1 - h1);
+        }
+        *reinterpret_cast<uint4*>(orow + c0) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (lrow) *reinterpret_cast<uint4*>(lrow + c0) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+    if (warp == 0) a.lse[((int64_t)b * a.H + h) * a.Nq + i] = kLn2 * ((m - kPShift) + log2f(l));
+}
+
+// How a call's query rows are tiled and its work divided.
+struct FwdPlan {
+    int pack, q_per_tile, heads, n_pairs;
+    int sched;                     // FwdCfg's SCHED
+    int ctas, part_rows;           // split schedule: ranges, rows per slot
+    size_t ml_off, meta_off, bytes;        // workspace: partial sums | maxima and row sums | ranges' pairs
+};
+
+// units (key blocks walked by a pair of tiles) of one (batch, column), every batch entry with Nk keys
+int64_t column_units(const fa_b200_params& p, int q_per_tile, int n_pairs) {
+    const int64_t nk_blocks = (p.Nk + kBlockN - 1) / kBlockN;
+    if (!p.causal) return n_pairs * nk_blocks;
+    int64_t sum = 0;
+    for (int pr = 0; pr < n_pairs; ++pr) {
+        const int64_t q_end = (int64_t)(2 * pr + 1) * q_per_tile < p.Nq ? (int64_t)(2 * pr + 2) * q_per_tile : (int64_t)(2 * pr + 1) * q_per_tile;
+        const int64_t n = (q_end + p.causal_shift + kBlockN - 1) / kBlockN;
+        sum += n < nk_blocks ? n : nk_blocks;
+    }
+    return sum;
+}
+
+// `free`: the caller gave scratch and leaves the division of the work to the library.
+//
+// Packing.  The query heads that share a K/V head read the same keys, so with few queries they belong into one tile:
+// 128 / pack queries of `pack` = H / Hkv heads.  Taken when it leaves at least 5 % fewer (pair, key block) units;
+// with many queries both forms have the same number and the plain one stays.
+// Splitting.  Whole pairs dealt round robin leave SMs idle when there are few of them, or when a few keys of one
+// batch entry make one pair long.  The call's units are then cut into one equal range per SM.  What that costs
+// (partial sums through memory and a second launch) is about kMergeUnits units, so the ranges have to be that much
+// shorter than the longest round-robin share, and a tenth.  B200, before -> after, both rules together:
+// 32 requests of 2048-4096 keys, 1 query, H32 Hkv8 D128 bf16: 304 -> 84 us (403 MB of keys and values, 62 us at the
+// copy rate); 1 request, 700 queries on 8892 keys, same heads: 240 -> 112 us (98 GFLOP, 60 us at cuBLAS's rate).
+// Decoding as one pair per unit, without the one-tile kernel (SCHED = 2), took 116 us: S, softmax and P V of one tile
+// are a serial chain of about 2.7 us a block, and two stages of K and V cover too little of the memory's latency.
+constexpr int kMergeUnits = 4;
+FwdPlan plan_schedule(const fa_b200_params& p, int D, int sms, bool free) {
+    FwdPlan pl;
+    memset(&pl, 0, sizeof(pl));
+    auto pairs_of = [&](int qpt) { return (int)(((int64_t)p.Nq + 2 * qpt - 1) / (2 * qpt)); };
+    pl.pack = 1; pl.q_per_tile = kBlockM; pl.heads = p.H; pl.n_pairs = pairs_of(kBlockM);
+    if (!free || sms <= 0 || p.Nq > (1 << 20) || dropout_threshold(p.dropout_p) != 0u) return pl;
+    const int group = p.H / p.Hkv;
+    int64_t col = column_units(p, kBlockM, pl.n_pairs);
+    const int items = p.causal ? (pl.n_pairs + 1) / 2 : pl.n_pairs;              // per column: a pair, or a pair and its mirror
+    const int64_t n_items = (int64_t)items * p.B * p.H;
+    const int64_t whole = (n_items + sms - 1) / sms * ((col + items - 1) / items);
+    if (group > 1 && group <= kBlockM) {
+        const int qpt = kBlockM / group, pairs = pairs_of(qpt);
+        const int64_t packed = column_units(p, qpt, pairs);
+        if (packed * p.Hkv * 20 <= col * p.H * 19) { pl.pack = group; pl.q_per_tile = qpt; pl.heads = p.Hkv; pl.n_pairs = pairs; col = packed; }
+    }
+    const int64_t total = (int64_t)p.B * pl.heads * col;
+    pl.ctas = (int)(total < sms ? total : sms);
+    int64_t ranges = (total + pl.ctas - 1) / pl.ctas;
+    if (p.kv_lengths) ranges = (3 * ranges + 3) / 4;         // counts below Nk: the longest share is Nk's, a range the mean's
+    if (total < (1 << 30) && whole * 9 > (ranges + kMergeUnits) * 10) {
+        pl.sched = p.Nq <= pl.q_per_tile ? 2 : 1;
+        const int tiles = (int)(((int64_t)p.Nq + pl.q_per_tile - 1) / pl.q_per_tile);
+        const int rows = tiles > 1 ? 2 * kBlockM : p.Nq * pl.pack;
+        pl.part_rows = (int)align_up((size_t)rows, 32);
+        const size_t slots = 2 * (size_t)pl.ctas * pl.part_rows;
+        pl.ml_off = align_up(slots * D * sizeof(float), 256);
+        pl.meta_off = pl.ml_off + align_up(slots * sizeof(float2), 256);
+        pl.bytes = pl.meta_off + align_up((size_t)pl.ctas * sizeof(int4), 256);
+        return pl;
+    }
+    return plan_schedule(p, D, sms, false);
+}
+
 template <int D, bool BF16, int PREC>
-int launch(const fa_b200_params& p) {
-    using Cfg = FwdCfg<D, PREC>;
+int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
     const int d = p.D;
+    const int sms = sm_count(p.device);
+    if (sms <= 0) { set_error("cannot read the SM count of device %d", p.device); return FA_ECUDA; }
+    FwdPlan plan = plan_schedule(p, D, sms, ws != nullptr);
+    if (ws_bytes < plan.bytes || ((uintptr_t)ws & 255u) != 0) plan = plan_schedule(p, D, sms, false);
     const CUtensorMapDataType dt = BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     CUtensorMap mq, mk, mv;
     int r;
-    if ((r = cached_tmap_bnhd(&mq, p.q.ptr, dt, 2, p.B, p.Nq, p.H, d, p.q.stride_b, p.q.stride_n, p.q.stride_h, 128, 64, true)) ||
+    if ((r = cached_tmap_bnhd(&mq, p.q.ptr, dt, 2, p.B, p.Nq, p.H, d, p.q.stride_b, p.q.stride_n, p.q.stride_h, plan.q_per_tile, 64, true, plan.pack)) ||
         (r = cached_tmap_bnhd(&mk, p.k.ptr, dt, 2, p.B, p.Nk, p.Hkv, d, p.k.stride_b, p.k.stride_n, p.k.stride_h, 128, 64, true)) ||
         (r = cached_tmap_bnhd(&mv, p.v.ptr, dt, 2, p.B, p.Nk, p.Hkv, d, p.v.stride_b, p.v.stride_n, p.v.stride_h, 128, 64, true))) {
         set_error("cuTensorMapEncodeTiled failed (%d)", r);
@@ -725,10 +1180,15 @@ int launch(const fa_b200_params& p) {
     a.kv_len = p.kv_lengths;
     a.causal = p.causal;
     a.shift = p.causal ? p.causal_shift : 0;
-    a.n_pairs = (p.Nq + 2 * kBlockM - 1) / (2 * kBlockM);
+    a.pack = plan.pack; a.q_per_tile = plan.q_per_tile; a.heads = plan.heads;
+    a.n_pairs = plan.n_pairs;
+    a.part_rows = plan.part_rows;
+    a.part_o = (float4*)ws;
+    a.part_ml = (float2*)((char*)ws + plan.ml_off);
+    a.part_meta = (int4*)((char*)ws + plan.meta_off);
     a.items_per_head = p.causal ? (a.n_pairs + 1) / 2 : a.n_pairs;
-    const int64_t n_items = (int64_t)a.items_per_head * p.B * p.H;
-    if (n_items > 0x7fffffff) { set_error("too many work items"); return FA_EUNSUPPORTED; }
+    const int64_t n_items = (int64_t)a.items_per_head * p.B * plan.heads;
+    if (n_items > 0x7fffffff - 65536) { set_error("too many work items"); return FA_EUNSUPPORTED; }
     a.n_items = (int)n_items;
     a.scale_log2 = p.scale * kLog2e;
     a.d = d;
@@ -755,19 +1215,36 @@ int launch(const fa_b200_params& p) {
         a.mq = (const uint4*)p.dropout_bits;
         drop = 2;
     }
-    auto kernel = drop == 2 ? fwd_sm100_kernel<D, BF16, 2, PREC> : (drop == 1 ? fwd_sm100_kernel<D, BF16, 1, PREC> : fwd_sm100_kernel<D, BF16, 0, PREC>);
+    auto kernel = drop == 2 ? fwd_sm100_kernel<D, BF16, 2, PREC, 0>
+                            : (drop == 1 ? fwd_sm100_kernel<D, BF16, 1, PREC, 0> : fwd_sm100_kernel<D, BF16, 0, PREC, 0>);
+    int smem = FwdCfg<D, PREC, 0>::kSmemBytes;
+    if constexpr (PREC == 0) {
+        if (plan.sched == 1) kernel = fwd_sm100_kernel<D, BF16, 0, PREC, 1>;
+        if (plan.sched == 2) { kernel = fwd_sm100_kernel<D, BF16, 0, PREC, 2>; smem = FwdCfg<D, PREC, 2>::kSmemBytes; }
+    }
     {
         static std::mutex mu;
-        static uint64_t done[3] = {0, 0, 0};
-        FA_CUDA_CHECK(set_smem_limit_once(kernel, Cfg::kSmemBytes, p.device, &done[drop], &mu));
+        static uint64_t done[5] = {0, 0, 0, 0, 0};
+        FA_CUDA_CHECK(set_smem_limit_once(kernel, smem, p.device, &done[plan.sched ? 2 + plan.sched : drop], &mu));
     }
-    const int sms = sm_count(p.device);
-    if (sms <= 0) { set_error("cannot read the SM count of device %d", p.device); return FA_ECUDA; }
-    const int grid = a.n_items < sms ? a.n_items : sms;     // one persistent CTA per SM
-    kernel<<<grid, kThreads, Cfg::kSmemBytes, (cudaStream_t)p.stream>>>(mq, mk, mv, a);
+    const int grid = plan.sched ? plan.ctas : (a.n_items < sms ? a.n_items : sms);     // one persistent CTA per SM
+    kernel<<<grid, kThreads, smem, (cudaStream_t)p.stream>>>(mq, mk, mv, a);
     FA_CUDA_CHECK(cudaGetLastError());
+    if constexpr (PREC == 0) if (plan.sched) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)plan.ctas, (unsigned)(plan.part_rows / 32));
+        cfg.blockDim = dim3(256);
+        cfg.stream = (cudaStream_t)p.stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fwd_merge_kernel<D, BF16>, a));
+    }
     return FA_OK;
 }
+
 
 #ifndef FA_PAIR_INSTANCES
 bool tensor_ok(const fa_b200_tensor& t, int64_t B, int64_t N, int64_t H) {
@@ -812,17 +1289,20 @@ bool sm100_pair_supports(const fa_b200_params& p, bool backward, const char** wh
     return true;
 }
 
-int sm100_fwd(const fa_b200_params& p) {
+int sm100_fwd(const fa_b200_params& p, void* ws, size_t ws_bytes) {
     if (p.dtype == FA_B200_F32) return sm100_tf32_fwd(p);
-    if (p.dtype == FA_B200_BF16) return p.D == 128 ? launch<128, true, 0>(p) : launch<64, true, 0>(p);
-    return p.D == 128 ? launch<128, false, 0>(p) : launch<64, false, 0>(p);
+    if (p.dtype == FA_B200_BF16) return p.D == 128 ? launch<128, true, 0>(p, ws, ws_bytes) : launch<64, true, 0>(p, ws, ws_bytes);
+    return p.D == 128 ? launch<128, false, 0>(p, ws, ws_bytes) : launch<64, false, 0>(p, ws, ws_bytes);
+}
+size_t sm100_fwd_workspace_bytes(const fa_b200_params& p) {
+    return p.dtype == FA_B200_F32 ? 0 : plan_schedule(p, p.D, sm_count(p.device), true).bytes;
 }
 #else
 }  // namespace
 
 int sm100_pair_fwd(const fa_b200_params& p) {
-    if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, 1>(p) : launch<64, true, 1>(p);
-    return p.D > 64 ? launch<128, false, 1>(p) : launch<64, false, 1>(p);
+    if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, 1>(p, nullptr, 0) : launch<64, true, 1>(p, nullptr, 0);
+    return p.D > 64 ? launch<128, false, 1>(p, nullptr, 0) : launch<64, false, 1>(p, nullptr, 0);
 }
 #endif
 

@@ -258,7 +258,17 @@ int fa_b200_selftest_wait_timeout(int32_t* status_word, int limit_ms, int device
     return FA_OK;
 }
 
-int fa_b200_fwd(const fa_b200_params* p) {
+int fa_b200_fwd(const fa_b200_params* p) { return fa_b200_fwd_with_workspace(p, nullptr, 0); }
+
+size_t fa_b200_fwd_workspace_bytes(const fa_b200_params* p) {
+    if (!p || p->struct_bytes != sizeof(fa_b200_params)) return 0;
+    if (p->B <= 0 || p->Nq <= 0 || p->Nk <= 0 || p->H <= 0 || p->Hkv <= 0 || p->D <= 0 || p->H % p->Hkv != 0 || p->causal_shift < 0) return 0;
+    int variant;
+    if (choose_variant(*p, false, &variant) != FA_OK || variant == FA_B200_VARIANT_SIMT || variant == kVariantPair) return 0;
+    return sm100_fwd_workspace_bytes(*p);
+}
+
+int fa_b200_fwd_with_workspace(const fa_b200_params* p, void* workspace, size_t workspace_bytes) {
     int rc = validate_common(p, false);
     if (rc) return rc;
     if ((rc = refuse_after_timeout(p, "fa_b200_fwd"))) return rc;
@@ -269,7 +279,7 @@ int fa_b200_fwd(const fa_b200_params* p) {
     GuardDevice g(p->device);
     if (!g.ok) { set_error("cudaSetDevice(%d) failed", p->device); return FA_ECUDA; }
     if (variant == kVariantPair) return sm100_pair_fwd(*p);
-    return variant != FA_B200_VARIANT_SIMT ? sm100_fwd(*p) : simt_fwd(*p);
+    return variant != FA_B200_VARIANT_SIMT ? sm100_fwd(*p, workspace, workspace_bytes) : simt_fwd(*p);
 }
 
 int fa_b200_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch,

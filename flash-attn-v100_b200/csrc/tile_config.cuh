@@ -15,6 +15,7 @@ constexpr int kBlockN = 128;            // key rows per block
 constexpr int kFwdQTilesPerCta = 2;     // two query tiles in flight: the softmax of one hides the MMAs of the other
 constexpr int kFwdWarps = 12;           // 8 softmax + MMA + TMA + 2 converting (bf16) / spare (fp16) warps
 constexpr int fwd_kv_stages(int D) { return D == 128 ? 2 : 4; }      // K and V rings: what 227 KB hold
+constexpr int fwd_one_tile_kv_stages(int D) { return D == 128 ? 3 : 6; }   // one query tile: the other's room too
 constexpr int kFwdRegsSoftmax = 208;    // setmaxnreg split; best of 224/56, 216/72, 208/88, 200/104
 constexpr int kFwdRegsOther = 88;
 constexpr int kFwdPolyPeriod = 2;       // of every kFwdPolyPeriod groups of four exponentials, kFwdPolyCount

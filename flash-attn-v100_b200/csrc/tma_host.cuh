@@ -31,13 +31,13 @@ inline EncodeTiledFn encode_tiled_fn() {
 
 // Tensor map over a (B, N, H, D) tensor with element strides (sb, sn, sh, 1):
 // dimensions ordered (D, H, N, B); a box is `box_rows` sequence positions of
-// one head by `box_cols` elements of D; `swizzle`: 0 none, 1 the 128-byte swizzle (16-byte
+// `box_heads` heads (the heads vary faster) by `box_cols` elements of D; `swizzle`: 0 none, 1 the 128-byte swizzle (16-byte
 // pieces; box_cols * elem size must be 128 bytes), 2 the 128-byte swizzle in 32-byte pieces (what
 // tcgen05.mma wants for an MN-major 32-bit operand).  Out-of-range rows read as zero.
 // Returns 0 on success, else the CUresult (or -1 if the driver entry point is missing).
 inline int make_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataType dt, size_t elem_bytes,
                           int64_t B, int64_t N, int64_t H, int64_t D, int64_t sb, int64_t sn, int64_t sh,
-                          int box_rows, int box_cols, int swizzle) {
+                          int box_rows, int box_cols, int swizzle, int box_heads = 1) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return -1;
     // size-1 dimensions may carry arbitrary strides in a tensor view: give them a legal one
@@ -47,7 +47,7 @@ inline int make_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataType
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)B};
     cuuint64_t strides[3] = {(cuuint64_t)(sh * elem_bytes), (cuuint64_t)(sn * elem_bytes),
                              (cuuint64_t)(sb * elem_bytes)};
-    cuuint32_t box[4] = {(cuuint32_t)box_cols, 1u, (cuuint32_t)box_rows, 1u};
+    cuuint32_t box[4] = {(cuuint32_t)box_cols, (cuuint32_t)box_heads, (cuuint32_t)box_rows, 1u};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     CUresult r = fn(map, dt, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
@@ -65,7 +65,7 @@ inline int make_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataType
 struct TmapKey {
     uint64_t ptr;
     int64_t B, N, H, D, sb, sn, sh;
-    int32_t dt, box_rows, box_cols, swizzle;
+    int32_t dt, box_rows, box_cols, swizzle, box_heads, zero;
     bool operator==(const TmapKey& o) const { return memcmp(this, &o, sizeof(TmapKey)) == 0; }
 };
 struct TmapKeyHash {
@@ -80,7 +80,7 @@ static_assert(sizeof(TmapKey) % 8 == 0, "the key is hashed and compared as 64-bi
 
 inline int cached_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataType dt, size_t elem_bytes,
                             int64_t B, int64_t N, int64_t H, int64_t D, int64_t sb, int64_t sn, int64_t sh,
-                            int box_rows, int box_cols, int swizzle) {
+                            int box_rows, int box_cols, int swizzle, int box_heads = 1) {
     static std::mutex mu;
     static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
     TmapKey key;
@@ -88,12 +88,13 @@ inline int cached_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataTy
     key.ptr = (uint64_t)(uintptr_t)ptr;
     key.B = B; key.N = N; key.H = H; key.D = D; key.sb = sb; key.sn = sn; key.sh = sh;
     key.dt = (int32_t)dt; key.box_rows = box_rows; key.box_cols = box_cols; key.swizzle = swizzle;
+    key.box_heads = box_heads;
     {
         std::lock_guard<std::mutex> lock(mu);
         auto it = cache.find(key);
         if (it != cache.end()) { *map = it->second; return 0; }
     }
-    const int r = make_tmap_bnhd(map, ptr, dt, elem_bytes, B, N, H, D, sb, sn, sh, box_rows, box_cols, swizzle);
+    const int r = make_tmap_bnhd(map, ptr, dt, elem_bytes, B, N, H, D, sb, sn, sh, box_rows, box_cols, swizzle, box_heads);
     if (r == 0) {
         std::lock_guard<std::mutex> lock(mu);
         if (cache.size() >= 4096) cache.clear();          // bounded: start over rather than grow for ever

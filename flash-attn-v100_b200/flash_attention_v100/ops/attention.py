@@ -199,7 +199,7 @@ def _dropout_bits_operand(p, keep_bits, forward_only=False):
 
 def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=None, bias=None,
                    key_lengths=None, causal_shift=0, dropout_origin=None, o_residual=None, keep_bits=None,
-                   forward_only=True):
+                   forward_only=True, split_keys=False):
     """o, lse <- fa_b200_fwd.  Counterpart of flash_attention_forward_triton_enhanced
     (kernels/forward_kernel.py:246-387); returns (o, lse).  `out=(o, lse)` writes into
     caller-owned buffers (o like q, lse (B, H, Nq) fp32 contiguous) instead of allocating.
@@ -207,7 +207,9 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
     to launch_backward it removes that rounding from the gradients.  `keep_bits="new"` (or a
     (uint8 tensor, ready) pair) has the call's dropout bits written to a buffer once instead of drawn
     inside the kernel; the call then returns (o, lse, buffer), and launch_backward given
-    keep_bits=(buffer, True) reads the same bits (`forward_only=False` sizes the buffer for that)."""
+    keep_bits=(buffer, True) reads the same bits (`forward_only=False` sizes the buffer for that).
+    `split_keys`: scratch is allocated where the library asks for it, to share the keys of a call with few
+    queries out over the SMs; the result's last bits then depend on the call's batch and heads too."""
     if out is not None:
         o, lse = out
     else:
@@ -220,7 +222,13 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
         _check_residual(o_residual, o)
         p.o_lo = _tensor4(o_residual)
     bits = _dropout_bits_operand(p, keep_bits, forward_only)
-    rc = _cabi.load().fa_b200_fwd(ctypes.byref(p))
+    lib = _cabi.load()
+    nbytes = int(lib.fa_b200_fwd_workspace_bytes(ctypes.byref(p))) if split_keys else 0
+    if nbytes:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        rc = lib.fa_b200_fwd_with_workspace(ctypes.byref(p), ws.data_ptr(), nbytes)
+    else:
+        rc = lib.fa_b200_fwd(ctypes.byref(p))
     _cabi.raise_for_status(rc, "fa_b200_fwd")
     if keep_bits is not None:
         return o, lse, bits
@@ -348,7 +356,8 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
         # with dropout the call's keep bits are written to a buffer once; the backward reads the same bits
         res = launch_forward(q, k, v, scale, causal, dropout_p, seed, offset, bias=bias, key_lengths=key_lengths,
                              causal_shift=causal_shift, dropout_origin=dropout_origin, o_residual=o_lo,
-                             keep_bits="new" if dropout_p > 0.0 else None, forward_only=not needs_grad)
+                             keep_bits="new" if dropout_p > 0.0 else None, forward_only=not needs_grad,
+                             split_keys=not needs_grad)
         o, lse = res[0], res[1]
         ctx.keep_bits = res[2] if (len(res) > 2 and needs_grad) else None
         ctx.dropout_origin = dropout_origin
@@ -406,7 +415,8 @@ def flash_attention_forward_enhanced(q, k, v, scale: Optional[float] = None, cau
         o, lse = launch_forward(q, k, v, scale, causal, dropout_p, seed, offset, bias=bias,
                                 key_lengths=kwargs.get("key_lengths"), dropout_origin=kwargs.get("dropout_origin"),
                                 o_residual=kwargs.get("output_residual"),
-                                keep_bits="new" if dropout_p > 0.0 else None)[:2]
+                                keep_bits="new" if dropout_p > 0.0 else None,
+                                split_keys=kwargs.get("output_residual") is None)[:2]
     return (o, lse) if kwargs.get("return_softmax_lse", False) else o
 
 

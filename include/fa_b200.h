@@ -191,6 +191,15 @@ typedef struct fa_b200_tile {
  * kernels/forward_kernel.py:246-387 (launcher) and :18-243 (kernel). */
 int fa_b200_fwd(const fa_b200_params* p);
 
+/* Forward with optional scratch of its own (the workspace fields of *p stay the backward's).  With at least
+ * fa_b200_fwd_workspace_bytes(p) bytes, 256-byte aligned, the library may put the query heads of one K/V head into
+ * one tile and cut the keys of a call with few queries into ranges for all SMs, whose partial results (fp32, in the
+ * scratch) a second launch puts together in a fixed order.  Results are reproducible; their last bits can differ
+ * from fa_b200_fwd's, and between a call and a call over a slice of it.  With less, the same as fa_b200_fwd. */
+int fa_b200_fwd_with_workspace(const fa_b200_params* p, void* workspace, size_t workspace_bytes);
+/* 0: the call has no use for scratch.  Looks at the tensors' pointers and strides as the call itself does. */
+size_t fa_b200_fwd_workspace_bytes(const fa_b200_params* p);
+
 /* Backward: dq, dk, dv <- grad(q, k, v, o, lse, dO).  Replaces
  * kernels/backward_kernel.py:208-318 (launcher) and :17-205 (kernel).
  * With variant AUTO, SIMT or TCGEN05_2PASS every gradient element is summed in a fixed order: two
