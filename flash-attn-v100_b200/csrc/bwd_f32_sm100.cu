@@ -1,0 +1,542 @@
+// Attention backward for fp32 inputs on the sm_100a tensor cores: every fp32 operand as three bf16 planes.
+//
+// The reference runs its backward's products of fp32 inputs through tl.dot with TF32 allowed
+// (kernels/backward_kernel.py:118-176); one TF32 product misses this library's fp32 tolerance by more than an order
+// of magnitude, so fp32 gradients were CUDA-core work: 1.27 ms of the 1.33 ms that forward + backward of B2 N1024
+// H12 D64 causal took, at 9 TFLOP/s.  Here x = x1 + x2 + x3 with x1 = bf16(x), x2 = bf16(x - x1),
+// x3 = bf16(x - x1 - x2): 24 significant bits, and bf16 has fp32's exponents, so no range is lost.  A product takes
+// six of the nine partial products (those down to 2^-16 of the first); what is left out lies at 2^-25.  bf16 and not
+// TF32 halves because six bf16 products cost what three TF32 ones do, a 16-bit tile serves as K-major and as MN-major
+// operand alike (a 32-bit one would be needed twice), and three TF32 products stop at 2^-21.
+//
+// Accumulation.  The tensor core truncates when it adds to its fp32 accumulator, a bias that grows with every
+// addition.  So the five small partial products of a contraction go first, while the accumulator is small, and no
+// accumulator lives longer than one step: the step's dK, dV or dQ tile is added up in the threads' registers, where
+// fp32 additions round to nearest.
+//
+// Three launches, all outputs owned by one CTA and summed in a fixed order:
+//   1. split      Q, dO, K, V -> planes (p * B + b, N, H, 64); delta, lse padded
+//   2. MODE 0     one CTA per 128-key tile, 64 queries a step:  S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q
+//   3. MODE 1     one CTA per 128-query tile, 64 keys a step:   S = Q K^T, dP = dO V^T, dQ += dS K
+//
+//   warps 0-15   a thread owns one TMEM lane (row of T1 / T2); warpgroup g owns the step's columns [16 g, 16 g + 16)
+//   warp 16      MMA issuer      order  T1(0) T2(0) | T1(i+1) ACC2(i) T2(i+1) ACC1(i)
+//   warp 17      TMA producer    (18, 19 idle)
+// TMEM columns: T1 [0,64) and [448,512)  T2 [64,128)  P planes [128,224)  dS planes [224,320)  ACC1 [320,384)
+// ACC2 [384,448).  T1 is two sums over half the head each: an error of a score is an error of P at full size.
+// Shared memory: the stationary pair's planes 96 KB, two stages of the streamed pair's 96 KB, which is why head sizes
+// above 64 stay on the CUDA cores.  Every mbarrier wait is bounded (sm100_ptx.cuh).
+//
+// What bounds it: the 96 (MODE 0) or 72 MMAs of 128 x 64 x 16 a step and the threads' splitting of P and dS (about 25
+// instructions a score) are of the same length and overlap by one step.  B200, B2 N1024 H12 causal, CUDA cores -> here:
+// delta / split 11 -> 17 us, dK and dV 749 -> 59 us, dQ 522 -> 48 us.
+//
+// Error against float64 (rel-L2 of dq, dk, dv, the largest of the three; forward and lse from the TF32 kernel), CUDA
+// cores -> here: N2048 full 2.9e-6 -> 2.7e-6, N1024 causal 1.8e-6 -> 1.5e-6, with scores 16 times as large
+// 6.1e-5 -> 5.8e-5.  From a forward without error it would be 1.0e-6 -> 5.2e-7, 8.0e-7 -> 3.8e-7 and 3.6e-6 -> 7.3e-6:
+// inside one MMA the tensor core aligns sixteen products and drops what lies below, which shows when scores are large.
+// So the rule takes the one head size whose forward is the TF32 kernel, D = 64, and leaves the others, whose forward
+// is as exact as the CUDA cores', where they were.
+#include "fa_common.cuh"
+#include "sm100_ptx.cuh"
+#include "tma_host.cuh"
+
+namespace fa {
+namespace {
+
+using namespace ptx;
+
+constexpr int kRows = 128;                    // stationary rows of a CTA
+constexpr int kStep = 64;                     // streamed rows of a step
+constexpr int kDim = 64;                      // columns of a plane
+constexpr int kPlanes = 3;
+constexpr int kStatPlane = kRows * 128, kStrmPlane = kStep * 128;        // bytes: rows of 64 bf16
+constexpr int kStat = kPlanes * kStatPlane, kStrm = kPlanes * kStrmPlane;
+constexpr int kWorkers = 16;                  // elementwise warps
+constexpr int kThreads = 32 * (kWorkers + 4);
+constexpr float kLog2e = 1.4426950408889634f;
+// partial products, the small ones first: planes of the first and of the second operand
+constexpr int kPairs = 6;
+__device__ constexpr int kPairA[kPairs] = {0, 2, 1, 0, 1, 0};
+__device__ constexpr int kPairB[kPairs] = {2, 0, 1, 1, 0, 0};
+
+enum { kBarXY = 0, kBarU = 1 /*[2]*/, kBarW = 3 /*[2]*/, kBarUFree = 5 /*[2]*/, kBarWFree = 7 /*[2]*/, kBarT1 = 9, kBarT2 = 10,
+       kBarAcc = 11, kBarT1Read = 12, kBarT2Read = 13, kBarP = 14, kBarDs = 15, kNumBars = 16 };
+constexpr int kSmemBytes = 2 * kStat + 4 * kStrm + kNumBars * 8 + 64 + 1024;
+
+struct F32Args {
+    const float* lse;              // [B*H][nq_pad], +inf in the padding
+    const float* delta;            // [B*H][nq_pad], 0 in the padding
+    fa_b200_tensor out1, out2;     // MODE 0: dK, dV; MODE 1: dQ
+    const int32_t* kv_len;
+    int32_t* status;
+    int B, Nq, Nk, H, Hkv, nq_pad;
+    int causal, shift, vec, wait_limit_ms;
+    float scale;
+};
+
+// x -> three bf16 planes, two values packed per word
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t& a, uint32_t& b, uint32_t& c) {
+    float h0, h1;
+    a = pack2<true>(x0, x1);
+    unpack2<true>(a, h0, h1);
+    x0 -= h0; x1 -= h1;
+    b = pack2<true>(x0, x1);
+    unpack2<true>(b, h0, h1);
+    c = pack2<true>(x0 - h0, x1 - h1);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 1)
+bwd_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
+               const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w, const F32Args a) {
+    constexpr bool KS = MODE == 0;             // key-stationary
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sX = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t* sY = sX + kStat;
+    uint8_t* sU = sY + kStat;                  // two stages
+    uint8_t* sW = sU + 2 * kStrm;              // two stages
+    uint64_t* bars = (uint64_t*)(sW + 2 * kStrm);
+    uint32_t* tmem_slot = (uint32_t*)(bars + kNumBars);
+    volatile uint32_t* abort_flag = (volatile uint32_t*)(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // blocks start in linear order: columns fastest, the tiles with the most steps first
+    const int cols = (int)(gridDim.y * gridDim.z);
+    const int lin = (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z));
+    const int rank = lin / cols, col = lin - rank * cols;
+    const int tile = (!KS && a.causal) ? (int)gridDim.x - 1 - rank : rank;
+    const int head_x = col % (int)gridDim.y, b = col / (int)gridDim.y;
+    const int group = a.H / a.Hkv;
+    const int nk = kv_len_of(a.kv_len, b, a.Nk);
+    int it0 = 0, per_head, n_iter;
+    if (KS) {
+        if (a.causal && tile * kRows > a.shift) it0 = (tile * kRows - a.shift) / kStep;
+        const int steps = (a.Nq + kStep - 1) / kStep;
+        per_head = steps > it0 ? steps - it0 : 0;
+        if (tile * kRows >= nk) per_head = 0;                    // padding keys: dK = dV = 0
+        n_iter = per_head * group;
+    } else {
+        int kv_end = nk;
+        if (a.causal && tile * kRows + kRows + a.shift < kv_end) kv_end = tile * kRows + kRows + a.shift;
+        per_head = n_iter = (kv_end + kStep - 1) / kStep;
+    }
+    // streamed step `it`: its head and first row
+    auto strm_head = [&](int it) { return KS ? head_x * group + it / per_head : head_x / group; };
+    auto strm_row = [&](int it) { return (KS ? it0 + it % per_head : it) * kStep; };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kNumBars; ++i) mbar_init(&bars[i], i >= kBarT1Read ? kWorkers : 1u);
+        wait_control_init(abort_flag, a.wait_limit_ms);
+        fence_mbar_init();
+    }
+    if (warp == kWorkers) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    if (warp == kWorkers + 1 && lane == 0) {
+        prefetch_tensormap(&map_x); prefetch_tensormap(&map_y);
+        prefetch_tensormap(&map_u); prefetch_tensormap(&map_w);
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
+    const uint32_t tT1 = tmem, tT2 = tmem + 64u, tP = tmem + 128u, tDs = tmem + 224u, tAcc1 = tmem + 320u, tAcc2 = tmem + 384u, tT1b = tmem + 448u;
+
+    if (warp == kWorkers + 1) {
+        // ------------------------------------------------------------ TMA producer
+        if (elect_one() && n_iter > 0) {
+            mbar_expect_tx(&bars[kBarXY], 2 * kStat);
+#pragma unroll
+            for (int p = 0; p < kPlanes; ++p)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int at = p * kStatPlane + half * kStrmPlane, row = tile * kRows + half * kStep;
+                    tma_load_4d(sX + at, &map_x, &bars[kBarXY], 0, head_x, row, p * a.B + b);
+                    tma_load_4d(sY + at, &map_y, &bars[kBarXY], 0, head_x, row, p * a.B + b);
+                }
+            bool ok = true;
+            int u_done = 0, w_done = 0;
+            for (int it = 0; it < n_iter; ++it) {
+                const int s = it & 1;
+                const uint32_t ph = ((uint32_t)(it >> 1) & 1u) ^ 1u;
+                const int head = strm_head(it), row = strm_row(it);
+                ok = mbar_wait(&bars[kBarUFree + s], ph, abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(&bars[kBarU + s], kStrm);
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p)
+                    tma_load_4d(sU + s * kStrm + p * kStrmPlane, &map_u, &bars[kBarU + s], 0, head, row, p * a.B + b);
+                ++u_done;
+                ok = mbar_wait(&bars[kBarWFree + s], ph, abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(&bars[kBarW + s], kStrm);
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p)
+                    tma_load_4d(sW + s * kStrm + p * kStrmPlane, &map_w, &bars[kBarW + s], 0, head, row, p * a.B + b);
+                ++w_done;
+            }
+            if (!ok) {
+                // unwinding: let the copies in flight land before shared memory is given up
+                for (int s = 0; s < 2; ++s) {
+                    const int nu = (u_done + 1 - s) / 2, nw = (w_done + 1 - s) / 2;
+                    for (int spin = 0; spin < 4096 && nu > 0 && !mbar_try_wait(&bars[kBarU + s], (uint32_t)(nu - 1) & 1u); ++spin) {}
+                    for (int spin = 0; spin < 4096 && nw > 0 && !mbar_try_wait(&bars[kBarW + s], (uint32_t)(nw - 1) & 1u); ++spin) {}
+                }
+                for (int spin = 0; spin < 4096 && !mbar_try_wait(&bars[kBarXY], 0u); ++spin) {}
+            }
+        }
+        __syncwarp();
+    } else if (warp == kWorkers) {
+        // ------------------------------------------------------------ MMA issuer
+        if (elect_one() && n_iter > 0) {
+            constexpr uint32_t idesc_t = make_idesc_f16(true, true, kRows, kStep, false, false);
+            constexpr uint32_t idesc_acc = make_idesc_f16(true, true, kRows, kDim, false, true);
+            const uint64_t dk_major = make_smem_desc_sw128(0, 0, 1024), dmn_major = make_smem_desc_sw128(0, 8192, 1024);
+            const uint32_t sX_u = smem_u32(sX), sY_u = smem_u32(sY), sU_u = smem_u32(sU), sW_u = smem_u32(sW);
+            // T = stationary x streamed^T over the 64 columns of the head
+            auto issue_t = [&](uint32_t d_tmem, uint32_t stat_u, uint32_t strm_u, int k0, int k1) {
+                const uint64_t a0 = dk_major + (uint64_t)(stat_u >> 4), b0 = dk_major + (uint64_t)(strm_u >> 4);
+#pragma unroll
+                for (int pr = 0; pr < kPairs; ++pr)
+#pragma unroll
+                    for (int kk = k0; kk < k1; ++kk)
+                        mma_ss_f16(d_tmem, a0 + (uint64_t)((kPairA[pr] * kStatPlane + kk * 32) >> 4),
+                                   b0 + (uint64_t)((kPairB[pr] * kStrmPlane + kk * 32) >> 4), idesc_t, (pr > 0 || kk > k0) ? 1u : 0u);
+            };
+            // ACC = A[TMEM planes] x streamed tile read MN-major, over the step's 64 streamed rows
+            auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t strm_u) {
+                const uint64_t b0 = dmn_major + (uint64_t)(strm_u >> 4);
+#pragma unroll
+                for (int pr = 0; pr < kPairs; ++pr)
+#pragma unroll
+                    for (int kk = 0; kk < kStep / 16; ++kk)
+                        mma_ts_f16(d_tmem, a_tmem + (uint32_t)(kPairA[pr] * 32 + kk * 8),
+                                   b0 + (uint64_t)((kPairB[pr] * kStrmPlane + kk * 2048) >> 4), idesc_acc, (pr > 0 || kk > 0) ? 1u : 0u);
+            };
+            bool ok = mbar_wait(&bars[kBarXY], 0u, abort_flag);
+            if (ok) ok = mbar_wait(&bars[kBarU], 0u, abort_flag);
+            if (ok) ok = mbar_wait(&bars[kBarW], 0u, abort_flag);
+            if (ok) {
+                tc_fence_after_sync();
+                issue_t(tT1, sX_u, sU_u, 0, 2);
+                issue_t(tT1b, sX_u, sU_u, 2, 4);
+                mma_commit(&bars[kBarT1]);
+                issue_t(tT2, sY_u, sW_u, 0, 4);
+                mma_commit(&bars[kBarT2]);
+            }
+            for (int it = 0; it < n_iter && ok; ++it) {
+                const int s = it & 1, ns = s ^ 1;
+                const uint32_t ph = (uint32_t)it & 1u, nph = (uint32_t)((it + 1) >> 1) & 1u;
+                const bool more = it + 1 < n_iter;
+                if (more) {
+                    ok = mbar_wait(&bars[kBarT1Read], ph, abort_flag);
+                    if (ok) ok = mbar_wait(&bars[kBarU + ns], nph, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    issue_t(tT1, sX_u, sU_u + ns * kStrm, 0, 2);
+                    issue_t(tT1b, sX_u, sU_u + ns * kStrm, 2, 4);
+                    mma_commit(&bars[kBarT1]);
+                }
+                // P(it) is in its planes, and the sums of step it - 1 have been read
+                ok = mbar_wait(&bars[kBarP], ph, abort_flag);
+                if (!ok) break;
+                tc_fence_after_sync();
+                if (KS) issue_acc(tAcc2, tP, sW_u + s * kStrm);
+                if (more) {
+                    ok = mbar_wait(&bars[kBarT2Read], ph, abort_flag);
+                    if (ok) ok = mbar_wait(&bars[kBarW + ns], nph, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    issue_t(tT2, sY_u, sW_u + ns * kStrm, 0, 4);
+                    mma_commit(&bars[kBarT2]);
+                }
+                ok = mbar_wait(&bars[kBarDs], ph, abort_flag);
+                if (!ok) break;
+                tc_fence_after_sync();
+                issue_acc(tAcc1, tDs, sU_u + s * kStrm);
+                mma_commit(&bars[kBarAcc]);
+                mma_commit(&bars[kBarUFree + s]);
+                mma_commit(&bars[kBarWFree + s]);
+            }
+        }
+        __syncwarp();
+    } else if (warp < kWorkers) {
+        // ------------------------------------------------------------ P, dS, sums, epilogue
+        const int g = warp >> 2, r = (warp & 3) * 32 + lane;
+        const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+        const int row = tile * kRows + r;              // key (MODE 0) or query (MODE 1)
+        float my_lse = 0.f, my_delta = 0.f;
+        if (!KS) {
+            const int64_t at = ((int64_t)b * a.H + head_x) * a.nq_pad + row;
+            my_lse = a.lse[at];
+            my_delta = a.delta[at];
+        }
+        float acc1[16], acc2[KS ? 16 : 1];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) { acc1[c] = 0.f; if (KS) acc2[c] = 0.f; }
+        // the sums of a finished step, from tensor memory into the registers
+        auto fold = [&] {
+            uint32_t x[16];
+            tmem_ld_32x16(tAcc1 + lane_off + (uint32_t)(16 * g), x);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc1[c] += __uint_as_float(x[c]);
+            if constexpr (KS) {
+                tmem_ld_32x16(tAcc2 + lane_off + (uint32_t)(16 * g), x);
+                tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 16; ++c) acc2[c] += __uint_as_float(x[c]);
+            }
+        };
+        // 16 values -> the three planes of my row and columns
+        auto store_planes = [&](uint32_t t, const float (&x)[16]) {
+            uint32_t pa[8], pb[8], pc[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) split3(x[2 * c], x[2 * c + 1], pa[c], pb[c], pc[c]);
+            const uint32_t at = t + lane_off + (uint32_t)(8 * g);
+            tmem_st_32x8(at, pa);
+            tmem_st_32x8(at + 32u, pb);
+            tmem_st_32x8(at + 64u, pc);
+            tmem_wait_st();
+            tc_fence_before_sync();
+        };
+        bool ok = true;
+        for (int it = 0; it < n_iter; ++it) {
+            const uint32_t ph = (uint32_t)it & 1u;
+            const int col0 = strm_row(it) + 16 * g;    // my first streamed row: query (MODE 0) or key (MODE 1)
+            const int64_t at = KS ? ((int64_t)b * a.H + strm_head(it)) * a.nq_pad + col0 : 0;
+            float v[16];                               // lse, then delta of my columns' queries, asked for ahead of the waits
+            auto load_v = [&](const float* src) {
+#pragma unroll
+                for (int c = 0; c < 16; c += 4) {
+                    const float4 f = *reinterpret_cast<const float4*>(src + at + c);
+                    v[c] = f.x; v[c + 1] = f.y; v[c + 2] = f.z; v[c + 3] = f.w;
+                }
+            };
+            if (KS) load_v(a.lse);
+            ok = mbar_wait(&bars[kBarT1], ph, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            uint32_t t1[16], t1b[16];
+            tmem_ld_32x16(tT1 + lane_off + (uint32_t)(16 * g), t1);
+            tmem_ld_32x16(tT1b + lane_off + (uint32_t)(16 * g), t1b);
+            tmem_wait_ld();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&bars[kBarT1Read]);
+            float p[16];
+            // the difference is rounded once and small wherever P is not: base 2 comes after it
+#pragma unroll
+            for (int c = 0; c < 16; ++c) p[c] = ex2(fmaf(__uint_as_float(t1[c]) + __uint_as_float(t1b[c]), a.scale, -(KS ? v[c] : my_lse)) * kLog2e);
+            if (KS) {
+                const int hidden = a.causal ? row - a.shift - col0 : 0;       // my first columns do not see the key
+#pragma unroll
+                for (int c = 0; c < 16; ++c) if (c < hidden || row >= nk) p[c] = 0.f;
+                load_v(a.delta);
+            } else {
+                int seen = nk - col0;
+                if (a.causal && row + a.shift + 1 - col0 < seen) seen = row + a.shift + 1 - col0;
+#pragma unroll
+                for (int c = 0; c < 16; ++c) if (c >= seen) p[c] = 0.f;
+            }
+            if (it > 0) {
+                ok = mbar_wait(&bars[kBarAcc], ph ^ 1u, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after_sync();
+                fold();
+                tc_fence_before_sync();
+            }
+            if (KS) store_planes(tP, p);
+            mbar_arrive_warp(&bars[kBarP]);
+            ok = mbar_wait(&bars[kBarT2], ph, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+            uint32_t t2[16];
+            tmem_ld_32x16(tT2 + lane_off + (uint32_t)(16 * g), t2);
+            tmem_wait_ld();
+            tc_fence_before_sync();
+            mbar_arrive_warp(&bars[kBarT2Read]);
+#pragma unroll
+            for (int c = 0; c < 16; ++c) p[c] *= __uint_as_float(t2[c]) - (KS ? v[c] : my_delta);
+            store_planes(tDs, p);
+            mbar_arrive_warp(&bars[kBarDs]);
+        }
+        if (n_iter > 0 && ok) {
+            ok = mbar_wait(&bars[kBarAcc], (uint32_t)(n_iter - 1) & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (ok) {
+                tc_fence_after_sync();
+                fold();
+            }
+        }
+        if (ok && row < (KS ? a.Nk : a.Nq)) {
+            auto put = [&](const fa_b200_tensor& t, const float (&x)[16], float mul) {
+                float* dst = (float*)t.ptr + (int64_t)b * t.stride_b + (int64_t)row * t.stride_n + (int64_t)head_x * t.stride_h + 16 * g;
+                if (a.vec) {
+#pragma unroll
+                    for (int c = 0; c < 16; c += 4)
+                        *reinterpret_cast<float4*>(dst + c) = make_float4(x[c] * mul, x[c + 1] * mul, x[c + 2] * mul, x[c + 3] * mul);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) dst[c] = x[c] * mul;
+                }
+            };
+            put(a.out1, acc1, a.scale);
+            if constexpr (KS) put(a.out2, acc2, 1.f);
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kWorkers) tmem_dealloc(tmem, 512);
+    if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 6 + MODE);
+}
+
+// Planes of the four operands, delta and the padded lse: one warp per row, two columns per lane.  Rows [0, q_rows) are
+// (batch, padded query, head), the rest (batch, key, K/V head), heads fastest as in memory.
+struct SplitArgs {
+    fa_b200_tensor q, k, v, o, d_o;
+    const float* lse_in;
+    uint32_t *q16, *g16, *k16, *v16;      // planes, two columns per word
+    float *lse, *delta;
+    int B, Nq, Nk, H, Hkv, nq_pad;
+    int64_t q_rows, rows;
+};
+__global__ void __launch_bounds__(256) bwd_f32_split_kernel(const SplitArgs a) {
+    const int lane = threadIdx.x & 31, c = 2 * lane;
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= a.rows) return;
+    auto load = [&](const fa_b200_tensor& t, int b, int n, int h, float& x0, float& x1) {
+        const float* src = (const float*)t.ptr + (int64_t)b * t.stride_b + (int64_t)n * t.stride_n + (int64_t)h * t.stride_h + c;
+        x0 = src[0];
+        x1 = src[1];
+    };
+    auto store = [&](uint32_t* dst, int N, int H, int b, int n, int h, float x0, float x1) {
+        uint32_t p[kPlanes];
+        split3(x0, x1, p[0], p[1], p[2]);
+#pragma unroll
+        for (int i = 0; i < kPlanes; ++i)
+            dst[((((int64_t)i * a.B + b) * N + n) * H + h) * (kDim / 2) + lane] = p[i];
+    };
+    float x0, x1, y0, y1;
+    if (row < a.q_rows) {
+        const int h = (int)(row % a.H);
+        const int64_t rest = row / a.H;
+        const int i = (int)(rest % a.nq_pad), b = (int)(rest / a.nq_pad);
+        const int64_t at = ((int64_t)b * a.H + h) * a.nq_pad + i;
+        if (i >= a.Nq) {
+            if (lane == 0) { a.lse[at] = INFINITY; a.delta[at] = 0.f; }
+            return;
+        }
+        load(a.q, b, i, h, x0, x1);
+        store(a.q16, a.Nq, a.H, b, i, h, x0, x1);
+        load(a.d_o, b, i, h, x0, x1);
+        store(a.g16, a.Nq, a.H, b, i, h, x0, x1);
+        load(a.o, b, i, h, y0, y1);
+        float s = fmaf(x0, y0, x1 * y1);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) { a.lse[at] = a.lse_in[((int64_t)b * a.H + h) * a.Nq + i]; a.delta[at] = s; }
+    } else {
+        const int64_t kr = row - a.q_rows;
+        const int h = (int)(kr % a.Hkv);
+        const int64_t rest = kr / a.Hkv;
+        const int j = (int)(rest % a.Nk), b = (int)(rest / a.Nk);
+        load(a.k, b, j, h, x0, x1);
+        load(a.v, b, j, h, y0, y1);
+        store(a.k16, a.Nk, a.Hkv, b, j, h, x0, x1);
+        store(a.v16, a.Nk, a.Hkv, b, j, h, y0, y1);
+    }
+}
+
+struct F32Layout { size_t q, g, k, v, lse, delta, bytes; };
+F32Layout f32_layout(const fa_b200_params& p) {
+    F32Layout l;
+    size_t at = 0;
+    auto region = [&](size_t n) { const size_t r = at; at = align_up(at + n, 256); return r; };
+    const size_t q = (size_t)kPlanes * p.B * p.Nq * p.H * kDim * 2, k = (size_t)kPlanes * p.B * p.Nk * p.Hkv * kDim * 2;
+    const size_t rows = (size_t)p.B * p.H * align_up((size_t)p.Nq, 128) * sizeof(float);
+    l.q = region(q); l.g = region(q); l.k = region(k); l.v = region(k); l.lse = region(rows); l.delta = region(rows);
+    l.bytes = at;
+    return l;
+}
+
+}  // namespace
+
+// Which backward calls the planes serve, and the scratch they take (0: not served).  Other head sizes (kernel comment),
+// a bias and dropout stay on the CUDA cores.
+size_t sm100_f32_bwd_scratch_bytes(const fa_b200_params& p) {
+    if (p.dtype != FA_B200_F32 || p.variant != FA_B200_VARIANT_AUTO || p.D != kDim) return 0;
+    if (p.bias.ptr || p.d_scores || p.o_lo.ptr || dropout_threshold(p.dropout_p) != 0u) return 0;
+    if (p.B > 65535 / kPlanes || p.H > 65535 || p.B < 1 || p.Nq < 1 || p.Nk < 1) return 0;
+    return f32_layout(p).bytes;
+}
+
+int sm100_f32_bwd(const fa_b200_params& p, void* scratch) {
+    const F32Layout l = f32_layout(p);
+    char* ws = (char*)scratch;
+    cudaStream_t st = (cudaStream_t)p.stream;
+    const int nq_pad = (int)align_up((size_t)p.Nq, 128);
+    const int phases = p.bwd_phases ? p.bwd_phases : 7;
+    if (phases & 1) {
+        SplitArgs s;
+        s.q = p.q; s.k = p.k; s.v = p.v; s.o = p.o; s.d_o = p.d_o; s.lse_in = p.lse;
+        s.q16 = (uint32_t*)(ws + l.q); s.g16 = (uint32_t*)(ws + l.g); s.k16 = (uint32_t*)(ws + l.k); s.v16 = (uint32_t*)(ws + l.v);
+        s.lse = (float*)(ws + l.lse); s.delta = (float*)(ws + l.delta);
+        s.B = p.B; s.Nq = p.Nq; s.Nk = p.Nk; s.H = p.H; s.Hkv = p.Hkv; s.nq_pad = nq_pad;
+        s.q_rows = (int64_t)p.B * nq_pad * p.H;
+        s.rows = s.q_rows + (int64_t)p.B * p.Nk * p.Hkv;
+        const int64_t blocks = (s.rows + 7) / 8;
+        if (blocks > 0x7fffffff) { set_error("problem too large for the split grid"); return FA_EUNSUPPORTED; }
+        bwd_f32_split_kernel<<<(unsigned)blocks, 256, 0, st>>>(s);
+        FA_CUDA_CHECK(cudaGetLastError());
+    }
+    CUtensorMap mq, mg, mk, mv;
+    int r;
+    auto planes = [&](CUtensorMap* m, size_t off, int N, int H) {
+        return cached_tmap_bnhd(m, ws + off, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (int64_t)kPlanes * p.B, N, H, kDim, (int64_t)N * H * kDim,
+                                (int64_t)H * kDim, (int64_t)kDim, kStep, 64, 1);
+    };
+    if ((r = planes(&mq, l.q, p.Nq, p.H)) || (r = planes(&mg, l.g, p.Nq, p.H)) ||
+        (r = planes(&mk, l.k, p.Nk, p.Hkv)) || (r = planes(&mv, l.v, p.Nk, p.Hkv))) {
+        set_error("cuTensorMapEncodeTiled failed (%d)", r);
+        return FA_ECUDA;
+    }
+    F32Args a;
+    a.lse = (const float*)(ws + l.lse); a.delta = (const float*)(ws + l.delta);
+    a.kv_len = p.kv_lengths; a.status = p.status_word;
+    a.B = p.B; a.Nq = p.Nq; a.Nk = p.Nk; a.H = p.H; a.Hkv = p.Hkv; a.nq_pad = nq_pad;
+    a.causal = p.causal; a.shift = p.causal ? p.causal_shift : 0;
+    a.wait_limit_ms = p.wait_limit_ms;
+    a.scale = p.scale;
+    auto aligned = [&](const fa_b200_tensor& t) {
+        return ((uintptr_t)t.ptr & 15u) == 0 && t.stride_b % 4 == 0 && t.stride_n % 4 == 0 && t.stride_h % 4 == 0;
+    };
+    {
+        static std::mutex mu;
+        static uint64_t done[2] = {0, 0};
+        FA_CUDA_CHECK(set_smem_limit_once(bwd_f32_kernel<0>, kSmemBytes, p.device, &done[0], &mu));
+        FA_CUDA_CHECK(set_smem_limit_once(bwd_f32_kernel<1>, kSmemBytes, p.device, &done[1], &mu));
+    }
+    if (phases & 2) {
+        a.out1 = p.dk; a.out2 = p.dv;
+        a.vec = aligned(p.dk) && aligned(p.dv);
+        const dim3 grid((p.Nk + kRows - 1) / kRows, p.Hkv, p.B);
+        bwd_f32_kernel<0><<<grid, kThreads, kSmemBytes, st>>>(mk, mv, mq, mg, a);
+        FA_CUDA_CHECK(cudaGetLastError());
+    }
+    if (phases & 4) {
+        a.out1 = p.dq; a.out2 = p.dq;
+        a.vec = aligned(p.dq);
+        const dim3 grid((p.Nq + kRows - 1) / kRows, p.H, p.B);
+        bwd_f32_kernel<1><<<grid, kThreads, kSmemBytes, st>>>(mq, mg, mk, mv, a);
+        FA_CUDA_CHECK(cudaGetLastError());
+    }
+    return FA_OK;
+}
+
+}  // namespace fa

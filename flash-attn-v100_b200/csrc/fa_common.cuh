@@ -100,6 +100,9 @@ bool sm100_pair_supports(const fa_b200_params& p, bool backward, const char** wh
 // fp32 forward on the tensor cores (fwd_tf32_sm100.cu): TF32 products taken three times
 int sm100_tf32_fwd(const fa_b200_params& p);
 bool sm100_tf32_fwd_supports(const fa_b200_params& p, const char** why);
+// fp32 backward on the tensor cores, operands as three bf16 planes in caller-supplied scratch (0 bytes: not served)
+size_t sm100_f32_bwd_scratch_bytes(const fa_b200_params& p);
+int sm100_f32_bwd(const fa_b200_params& p, void* scratch);
 // Whether the one-kernel backward (dQ summed with global additions) covers a call the family supports.
 bool sm100_bwd_fused_supported(const fa_b200_params& p);
 

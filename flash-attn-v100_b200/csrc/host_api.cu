@@ -171,7 +171,7 @@ int refuse_after_timeout(const fa_b200_params* p, const char* what) {
     const int code = take_host_status(p->status_word);
     if (code == 0) return FA_OK;
     set_error("%s: an earlier call's device-side wait ran out (status %d: 1 forward, 2 dK/dV, 3 dQ, 4 one-kernel "
-              "backward, 5 fp32 forward, 8 shared memory, 9 self-test); its results are invalid.  The word has been cleared", what, code);
+              "backward, 5 fp32 forward, 6 fp32 dK/dV, 7 fp32 dQ, 8 shared memory, 9 self-test); its results are invalid.  The word has been cleared", what, code);
     return FA_ETIMEOUT;
 }
 
@@ -328,7 +328,14 @@ size_t fa_b200_dropout_bits_bytes(const fa_b200_params* p) {
     return 2 * dropout_bits_bytes(*p);
 }
 
-int fa_b200_bwd(const fa_b200_params* p) {
+int fa_b200_bwd(const fa_b200_params* p) { return fa_b200_bwd_with_scratch(p, nullptr, 0); }
+
+size_t fa_b200_bwd_scratch_bytes(const fa_b200_params* p) {
+    if (!p || p->struct_bytes != sizeof(fa_b200_params) || p->H <= 0 || p->Hkv <= 0 || p->D <= 0) return 0;
+    return sm100_f32_bwd_scratch_bytes(*p);
+}
+
+int fa_b200_bwd_with_scratch(const fa_b200_params* p, void* scratch, size_t scratch_bytes) {
     int rc = validate_common(p, true);
     if (rc) return rc;
     if ((rc = refuse_after_timeout(p, "fa_b200_bwd"))) return rc;
@@ -336,6 +343,12 @@ int fa_b200_bwd(const fa_b200_params* p) {
     if (p->Nk == 0) { set_error("Nk = 0: softmax over an empty key set is undefined"); return FA_EINVAL; }
     int variant;
     if ((rc = choose_variant(*p, true, &variant))) return rc;
+    const size_t planes = scratch && p->Nq > 0 && ((uintptr_t)scratch & 255u) == 0 ? sm100_f32_bwd_scratch_bytes(*p) : 0;
+    if (planes > 0 && scratch_bytes >= planes) {
+        GuardDevice g(p->device);
+        if (!g.ok) { set_error("cudaSetDevice(%d) failed", p->device); return FA_ECUDA; }
+        return sm100_f32_bwd(*p, scratch);
+    }
     BwdWorkspace ws = bwd_workspace_layout(*p, variant);
     if (!p->workspace || p->workspace_bytes < ws.total) {
         set_error("backward needs %zu bytes of workspace, got %zu", ws.total,

@@ -27,7 +27,7 @@ EXPORTS = (
     "fa_b200_dropout_mask_host", "fa_b200_dropout_mask_device", "fa_b200_dropout_effective_p",
     "fa_b200_philox4x32_10", "fa_b200_strerror", "fa_b200_last_error", "fa_b200_version", "fa_b200_combine",
     "fa_b200_copy_rows", "fa_b200_selftest_wait_timeout", "fa_b200_dropout_bits_bytes",
-    "fa_b200_fwd_with_workspace", "fa_b200_fwd_workspace_bytes",
+    "fa_b200_fwd_with_workspace", "fa_b200_fwd_workspace_bytes", "fa_b200_bwd_with_scratch", "fa_b200_bwd_scratch_bytes",
 )
 
 
@@ -112,6 +112,10 @@ def load():
         lib.fa_b200_fwd_with_workspace.restype = ctypes.c_int
         lib.fa_b200_fwd_workspace_bytes.argtypes = [pp]
         lib.fa_b200_fwd_workspace_bytes.restype = ctypes.c_size_t
+        lib.fa_b200_bwd_with_scratch.argtypes = [pp, ctypes.c_void_p, ctypes.c_size_t]
+        lib.fa_b200_bwd_with_scratch.restype = ctypes.c_int
+        lib.fa_b200_bwd_scratch_bytes.argtypes = [pp]
+        lib.fa_b200_bwd_scratch_bytes.restype = ctypes.c_size_t
         lib.fa_b200_bwd.argtypes = [pp]
         lib.fa_b200_bwd.restype = ctypes.c_int
         lib.fa_b200_bwd_static.argtypes = [pp]

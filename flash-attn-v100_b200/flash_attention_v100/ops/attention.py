@@ -241,7 +241,8 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
     """dq, dk, dv <- fa_b200_bwd.  Counterpart of
     flash_attention_backward_triton_enhanced (kernels/backward_kernel.py:208-318).
     `out=(dq, dk, dv)` and `workspace` (uint8, at least fa_b200_bwd_workspace_bytes)
-    use caller-owned buffers instead of allocating.  `fast`: allow the one-kernel backward where it
+    use caller-owned buffers instead of allocating (an fp32 call without a `workspace` gets more scratch and, where
+    they serve it, the tensor-core kernels).  `fast`: allow the one-kernel backward where it
     is faster (D = 64); dQ is then summed in no fixed order and is not bit-reproducible.
     `keep_bits`: as in launch_forward; (buffer, True) reuses the bits the forward wrote."""
     d_o = _last_dim_contiguous(d_o)
@@ -266,6 +267,14 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
             raise ValueError("d_scores must be a contiguous fp32 (B, H, Nq, Nk) tensor")
         p.d_scores = d_scores.data_ptr()
     lib = _cabi.load()
+    if workspace is None and q.dtype == torch.float32:
+        # planes for the tensor-core backward of fp32 calls; a caller with a workspace of its own gets the CUDA-core one
+        nbytes = int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
+        if nbytes:
+            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+            rc = lib.fa_b200_bwd_with_scratch(ctypes.byref(p), ws.data_ptr(), nbytes)
+            _cabi.raise_for_status(rc, "fa_b200_bwd")
+            return dq, dk, dv
     nbytes = int(lib.fa_b200_bwd_workspace_bytes(ctypes.byref(p)))
     if workspace is None:
         ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)

@@ -206,6 +206,13 @@ size_t fa_b200_fwd_workspace_bytes(const fa_b200_params* p);
  * runs give bit-identical dq, dk and dv.  Variant TCGEN05 at D = 64 trades that for speed (dq only). */
 int fa_b200_bwd(const fa_b200_params* p);
 
+/* Backward with optional scratch beside the workspace.  With at least fa_b200_bwd_scratch_bytes(p) bytes (256-byte
+ * aligned; 0: the call has no use for it), fp32 calls of variant AUTO with D = 64, without bias and dropout, run on
+ * the tensor cores, every fp32 operand split into three bf16 planes that the scratch holds, with an error no larger
+ * than the CUDA-core kernels' behind the same forward; the workspace is not used then.  With less, the same as fa_b200_bwd. */
+int fa_b200_bwd_with_scratch(const fa_b200_params* p, void* scratch, size_t scratch_bytes);
+size_t fa_b200_bwd_scratch_bytes(const fa_b200_params* p);
+
 /*
  * Backward that takes no workspace and allocates nothing.  It has no
  * counterpart in the reference.
