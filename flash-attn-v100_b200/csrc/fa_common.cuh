@@ -24,6 +24,20 @@ void set_error(const char* fmt, ...);
         }                                                                          \
     } while (0)
 
+// Makes `dev` the current device for a scope.
+struct GuardDevice {
+    int prev = -1;
+    bool ok = true;
+    explicit GuardDevice(int dev) {
+        if (cudaGetDevice(&prev) != cudaSuccess) { ok = false; return; }
+        if (prev != dev && cudaSetDevice(dev) != cudaSuccess) ok = false;
+    }
+    ~GuardDevice() {
+        int cur = -1;
+        if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
+    }
+};
+
 // ---- dtype helpers ---------------------------------------------------------
 template <typename T> __device__ __forceinline__ float to_f32(T x);
 template <> __device__ __forceinline__ float to_f32<float>(float x) { return x; }

@@ -59,19 +59,6 @@ int sm_count(int device) {
 
 namespace {
 
-struct GuardDevice {
-    int prev = -1;
-    bool ok = true;
-    explicit GuardDevice(int dev) {
-        if (cudaGetDevice(&prev) != cudaSuccess) { ok = false; return; }
-        if (prev != dev && cudaSetDevice(dev) != cudaSuccess) ok = false;
-    }
-    ~GuardDevice() {
-        int cur = -1;
-        if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
-    }
-};
-
 int check_tensor(const fa_b200_tensor& t, const char* name, bool required) {
     if (!t.ptr) {
         if (required) { set_error("%s pointer is null", name); return FA_EINVAL; }

@@ -28,6 +28,7 @@ EXPORTS = (
     "fa_b200_philox4x32_10", "fa_b200_strerror", "fa_b200_last_error", "fa_b200_version", "fa_b200_combine",
     "fa_b200_copy_rows", "fa_b200_selftest_wait_timeout", "fa_b200_dropout_bits_bytes",
     "fa_b200_fwd_with_workspace", "fa_b200_fwd_workspace_bytes", "fa_b200_bwd_with_scratch", "fa_b200_bwd_scratch_bytes",
+    "fa_b200_key_order", "fa_b200_permute_rows",
 )
 
 
@@ -129,6 +130,12 @@ def load():
         lib.fa_b200_copy_rows.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_size_t,
                                           ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p]
         lib.fa_b200_copy_rows.restype = ctypes.c_int
+        lib.fa_b200_key_order.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
+                                          ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+        lib.fa_b200_key_order.restype = ctypes.c_int
+        lib.fa_b200_permute_rows.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_int, ctypes.c_int, ctypes.c_size_t, ctypes.c_int,
+                                                                     ctypes.c_int, ctypes.c_void_p]
+        lib.fa_b200_permute_rows.restype = ctypes.c_int
         lib.fa_b200_selftest_wait_timeout.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
         lib.fa_b200_selftest_wait_timeout.restype = ctypes.c_int
         lib.fa_b200_tile_config.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(Tile)]

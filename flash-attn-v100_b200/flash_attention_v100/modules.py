@@ -28,6 +28,7 @@ import torch
 from torch import nn
 
 from .interface import flash_attention_v100
+from .kernels import _cabi
 
 
 def masks_to_bias(attn_mask: Optional[torch.Tensor], key_padding_mask: Optional[torch.Tensor],
@@ -76,6 +77,49 @@ def compact_keys(k: torch.Tensor, v: torch.Tensor, key_padding_mask: torch.Tenso
     counts = (~key_padding_mask).sum(dim=1).clamp_(min=1).to(torch.int32)
     index = order.view(order.shape[0], order.shape[1], 1, 1).expand(-1, -1, k.shape[2], k.shape[3])
     return k.gather(1, index), v.gather(1, index), counts
+
+
+def _permute_rows(a: torch.Tensor, b: torch.Tensor, order: torch.Tensor, scatter: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    x, y = torch.empty_like(a), torch.empty_like(b)
+    rc = _cabi.load().fa_b200_permute_rows(a.data_ptr(), b.data_ptr(), x.data_ptr(), y.data_ptr(), order.data_ptr(), a.shape[0], a.shape[1],
+                                           a.stride(1) * a.element_size(), int(scatter), a.device.index,
+                                           torch.cuda.current_stream(a.device).cuda_stream or None)
+    _cabi.raise_for_status(rc, "fa_b200_permute_rows")
+    return x, y
+
+
+class _CompactKeys(torch.autograd.Function):
+    """compact_keys on the GPU: one scan of the mask, one launch that moves the rows of K and V; the gradients go back
+    the same way.  For the layer only, whose attention op is an autograd Function like this one; compact_keys itself
+    stays differentiable twice, and under the transforms, as torch operations are."""
+
+    @staticmethod
+    def forward(ctx, k, v, mask):
+        B, N = mask.shape
+        if mask.stride(1) != 1 and N > 1:
+            mask = mask.contiguous()
+        order = torch.empty(B, N, dtype=torch.int32, device=k.device)
+        counts = torch.empty(B, dtype=torch.int32, device=k.device)
+        rc = _cabi.load().fa_b200_key_order(mask.data_ptr(), mask.stride(0), B, N, order.data_ptr(), counts.data_ptr(), k.device.index,
+                                            torch.cuda.current_stream(k.device).cuda_stream or None)
+        _cabi.raise_for_status(rc, "fa_b200_key_order")
+        k2, v2 = _permute_rows(k, v, order, False)
+        ctx.save_for_backward(order)
+        ctx.mark_non_differentiable(counts)
+        return k2, v2, counts
+
+    @staticmethod
+    def backward(ctx, gk, gv, _):
+        order, = ctx.saved_tensors
+        return _permute_rows(gk.contiguous(), gv.contiguous(), order, True) + (None,)
+
+
+def _rows_can_be_moved(k: torch.Tensor, v: torch.Tensor, mask: torch.Tensor) -> bool:
+    """Whether fa_b200_permute_rows takes these: dense tensors on one GPU, rows of whole 16-byte pieces."""
+    row = k.shape[2] * k.shape[3] * k.element_size()
+    return (k.is_cuda and v.device == k.device and mask.device == k.device and k.dtype == v.dtype and k.is_contiguous() and
+            v.is_contiguous() and k.numel() > 0 and row % 16 == 0 and k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0 and
+            k.shape[0] * k.shape[1] * (row // 16) < 1 << 32)
 
 
 class EnhancedMultiHeadAttention(nn.Module):
@@ -135,7 +179,10 @@ class EnhancedMultiHeadAttention(nn.Module):
                 and not is_causal and key_lengths is None:
             if tuple(key_padding_mask.shape) != (batch, seq_k):
                 raise ValueError(f"key_padding_mask shape {tuple(key_padding_mask.shape)}, expected {(batch, seq_k)}")
-            k, v, key_lengths = compact_keys(k, v, key_padding_mask)
+            if _rows_can_be_moved(k, v, key_padding_mask):
+                k, v, key_lengths = _CompactKeys.apply(k, v, key_padding_mask)
+            else:
+                k, v, key_lengths = compact_keys(k, v, key_padding_mask)
             key_padding_mask = None
         bias = masks_to_bias(attn_mask, key_padding_mask, batch, seq_q, seq_k)
         if need_weights:

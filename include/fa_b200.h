@@ -296,6 +296,19 @@ int fa_b200_combine(const fa_b200_combine_params* p);
 int fa_b200_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch,
                       size_t row_bytes, size_t rows, int device, void* stream);
 
+/*
+ * Keys a mask keeps first, for padding masks turned into kv_lengths.  key_order: from a (B, N) byte mask (non-zero
+ * hides; rows mask_stride_b bytes apart) order[b*N + p] = the key that comes p-th, kept keys in their order and then
+ * the hidden ones in theirs, and counts[b] = the kept keys, at least 1.  permute_rows: two dense (B, N, row_bytes)
+ * arrays at once, dst[b][p] = src[b][order[b][p]], or with `scatter` dst[b][order[b][p]] = src[b][p]; 16-byte aligned
+ * rows of a multiple of 16 bytes, fewer than 2^32 such pieces in all.  No counterpart in the reference, which expands
+ * the mask to a dense bias (examples/basic_usage.py:228-250).
+ */
+int fa_b200_key_order(const uint8_t* mask, int64_t mask_stride_b, int B, int N, int32_t* order, int32_t* counts,
+                      int device, void* stream);
+int fa_b200_permute_rows(const void* src0, const void* src1, void* dst0, void* dst1, const int32_t* order, int B, int N,
+                         size_t row_bytes, int scatter, int device, void* stream);
+
 /* Bytes of scratch fa_b200_bwd needs for these sizes (delta, fp32 dQ
  * accumulator, ...).  Counterpart of the 'delta' entry of
  * ops/memory.py:653-760 allocate_attention_workspace_enhanced. */
