@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import struct
 import threading
 from typing import Any, Dict, Optional, Tuple, Union
 
@@ -132,30 +133,52 @@ def _lengths_operand(key_lengths: Optional[torch.Tensor], q: torch.Tensor):
     return kl.data_ptr(), kl
 
 
+# The call's argument block up to `device`, packed in one go: forty attribute stores of a ctypes structure cost 8 us of
+# a call, packing them 2 us.
+_PREFIX = struct.Struct("@N" + 8 * "Pqqq" + "PPNPPQQ" + "10i")
+assert _PREFIX.size == _cabi.Params.scale.offset
+_NO_TENSOR = (0, 0, 0, 0)
+_U64 = 0xFFFFFFFFFFFFFFFF
+
+
+def _quad(t: Optional[torch.Tensor]) -> Tuple[int, int, int, int]:
+    """Pointer and element strides over batch, sequence and head."""
+    if t is None:
+        return _NO_TENSOR
+    sb, sn, sh, sd = t.stride()
+    assert sd == 1 or t.numel() == 0
+    return t.data_ptr(), sb, sn, sh
+
+
 def _base_params(q, k, v, o, lse, scale, causal, dropout_p, seed, offset, causal_shift=0,
-                 dropout_origin=None, variant=None) -> _cabi.Params:
+                 dropout_origin=None, variant=None, d_o=None, dq=None, dk=None, dv=None) -> _cabi.Params:
     p = _cabi.Params()
-    p.struct_bytes = ctypes.sizeof(_cabi.Params)
-    p.q, p.k, p.v, p.o = _tensor4(q), _tensor4(k), _tensor4(v), _tensor4(o)
-    p.lse = lse.data_ptr() or None
-    p.B, p.Nq, p.H, p.D = q.shape
-    p.Nk, p.Hkv = k.shape[1], k.shape[2]
-    p.dtype = dtype_enum(q.dtype)
-    p.causal = int(bool(causal))
-    p.causal_shift = int(causal_shift) if causal else 0
+    B, Nq, H, D = q.shape
+    _, Nk, Hkv, _ = k.shape
+    device = q.device.index if q.device.index is not None else torch.cuda.current_device()
     # an explicit kernel_variant() block wins; else the caller's choice (the autograd op's "speed" mode)
     override = getattr(_variant_override, "value", _cabi.VARIANT_AUTO)
-    p.variant = override if override != _cabi.VARIANT_AUTO else (variant or _cabi.VARIANT_AUTO)
-    p.device = q.device.index if q.device.index is not None else torch.cuda.current_device()
-    p.scale = float(scale)
-    p.dropout_p = float(dropout_p)
-    p.seed, p.offset = int(seed), int(offset)
-    p.stream = torch.cuda.current_stream(q.device).cuda_stream or None
-    p.status_word = _status_word(q.device).data_ptr()
+    if override != _cabi.VARIANT_AUTO:
+        variant = override
+    _PREFIX.pack_into(p, 0, _PARAMS_BYTES, *_quad(q), *_quad(k), *_quad(v), *_quad(o), *_quad(d_o), *_quad(dq), *_quad(dk), *_quad(dv),
+                      lse.data_ptr(), 0, 0, _status_word(q.device).data_ptr(), _raw_stream(device), int(seed) & _U64, int(offset) & _U64,
+                      B, Nq, Nk, H, Hkv, D, dtype_enum(q.dtype), int(bool(causal)), variant or _cabi.VARIANT_AUTO, device)
+    p.scale = scale
+    p.dropout_p = dropout_p
+    if causal and causal_shift:
+        p.causal_shift = int(causal_shift)
     if dropout_origin is not None:
         # the call is a slice of a larger problem: (batch offset, head offset, heads of the whole)
         p.rng_batch_offset, p.rng_head_offset, p.rng_heads = (int(x) for x in dropout_origin)
     return p
+
+
+_PARAMS_BYTES = ctypes.sizeof(_cabi.Params)
+
+
+def _raw_stream(device: int) -> int:
+    """The device's current stream as an integer (0: the default stream)."""
+    return torch._C._cuda_getCurrentRawStream(device)
 
 
 def _check_residual(o_residual: torch.Tensor, o: torch.Tensor) -> None:
@@ -213,11 +236,14 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
     if out is not None:
         o, lse = out
     else:
-        o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-        lse = torch.empty(q.shape[0], q.shape[2], q.shape[1], dtype=torch.float32, device=q.device)
+        B, Nq, H, _ = shape = q.shape
+        o = q.new_empty(shape)
+        lse = q.new_empty((B, H, Nq), dtype=torch.float32)
     p = _base_params(q, k, v, o, lse, scale, causal, dropout_p, seed, offset, causal_shift, dropout_origin)
-    p.bias, _keep = _bias_operand(bias)        # scores = scale * q.k + bias
-    p.kv_lengths, _keep_len = _lengths_operand(key_lengths, q)
+    if bias is not None:
+        p.bias, _keep = _bias_operand(bias)    # scores = scale * q.k + bias
+    if key_lengths is not None:
+        p.kv_lengths, _keep_len = _lengths_operand(key_lengths, q)
     if o_residual is not None:
         _check_residual(o_residual, o)
         p.o_lo = _tensor4(o_residual)
@@ -225,7 +251,7 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
     lib = _cabi.load()
     nbytes = int(lib.fa_b200_fwd_workspace_bytes(ctypes.byref(p))) if split_keys else 0
     if nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        ws = q.new_empty(nbytes, dtype=torch.uint8)
         rc = lib.fa_b200_fwd_with_workspace(ctypes.byref(p), ws.data_ptr(), nbytes)
     else:
         rc = lib.fa_b200_fwd(ctypes.byref(p))
@@ -249,14 +275,13 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
     if out is not None:
         dq, dk, dv = out
     else:
-        dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-        dk = torch.empty(k.shape, dtype=k.dtype, device=k.device)
-        dv = torch.empty(v.shape, dtype=v.dtype, device=v.device)
+        dq, dk, dv = q.new_empty(q.shape), k.new_empty(k.shape), v.new_empty(v.shape)
     p = _base_params(q, k, v, o, lse, scale, causal, dropout_p, seed, offset, causal_shift, dropout_origin,
-                     variant=_cabi.VARIANT_TCGEN05 if fast else None)
-    p.d_o, p.dq, p.dk, p.dv = _tensor4(d_o), _tensor4(dq), _tensor4(dk), _tensor4(dv)
-    p.bias, _keep = _bias_operand(bias)
-    p.kv_lengths, _keep_len = _lengths_operand(key_lengths, q)
+                     variant=_cabi.VARIANT_TCGEN05 if fast else None, d_o=d_o, dq=dq, dk=dk, dv=dv)
+    if bias is not None:
+        p.bias, _keep = _bias_operand(bias)
+    if key_lengths is not None:
+        p.kv_lengths, _keep_len = _lengths_operand(key_lengths, q)
     if o_residual is not None:
         _check_residual(o_residual, o)
         p.o_lo = _tensor4(o_residual)
@@ -271,13 +296,13 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
         # planes for the tensor-core backward of fp32 calls; a caller with a workspace of its own gets the CUDA-core one
         nbytes = int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
         if nbytes:
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+            ws = q.new_empty(nbytes, dtype=torch.uint8)
             rc = lib.fa_b200_bwd_with_scratch(ctypes.byref(p), ws.data_ptr(), nbytes)
             _cabi.raise_for_status(rc, "fa_b200_bwd")
             return dq, dk, dv
     nbytes = int(lib.fa_b200_bwd_workspace_bytes(ctypes.byref(p)))
     if workspace is None:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+        ws = q.new_empty(nbytes, dtype=torch.uint8)
     else:
         ws = workspace
         if ws.numel() < nbytes:
@@ -360,7 +385,7 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
         # causal_shift: key j is visible to query i iff j <= i + causal_shift (0: the reference's top-left
         # alignment; Nk - Nq: bottom-right)
         # the backward of a bf16 call also gets what rounding the output to bf16 dropped
-        needs_grad = any(t.requires_grad for t in (q, k, v)) or (bias is not None and bias.requires_grad)
+        needs_grad = q.requires_grad or k.requires_grad or v.requires_grad or (bias is not None and bias.requires_grad)
         o_lo = torch.empty_like(q) if (needs_grad and saves_output_residual(q.dtype)) else None
         # with dropout the call's keep bits are written to a buffer once; the backward reads the same bits
         res = launch_forward(q, k, v, scale, causal, dropout_p, seed, offset, bias=bias, key_lengths=key_lengths,

@@ -23,11 +23,13 @@ def cdiv(a: int, b: int) -> int:
 def _last_dim_contiguous(t: torch.Tensor) -> torch.Tensor:
     """Kernels need unit stride on the head dim and 16-byte aligned rows; head-
     or batch-sliced views pass through untouched, anything else is packed."""
-    if t.numel() == 0:
+    strides = t.stride()
+    bytes_ored = t.data_ptr()                    # low four bits: whether any address or row pitch is no multiple of 16
+    for s in strides[:-1]:
+        bytes_ored |= s * t.itemsize
+    if (strides[-1] == 1 and not bytes_ored & 15) or t.numel() == 0:
         return t
-    es = t.element_size()
-    ok = t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all((s * es) % 16 == 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
+    return t.contiguous()
 
 
 def validate_inputs(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
@@ -39,13 +41,14 @@ def validate_inputs(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     Same rules as reference utils.py:56-153; raises TypeError/ValueError with
     the reference's messages.
     """
-    if not all(isinstance(t, torch.Tensor) for t in (q, k, v)):
+    if not (isinstance(q, torch.Tensor) and isinstance(k, torch.Tensor) and isinstance(v, torch.Tensor)):
         raise TypeError("q, k, v must be torch.Tensor instances")
-    if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
+    qs, ks, vs = q.shape, k.shape, v.shape
+    if len(qs) != 4 or len(ks) != 4 or len(vs) != 4:
         raise ValueError("Input tensors must be 4-dimensional [batch, seq_len, num_heads, head_dim]")
-    b, nq, hq, dq = q.shape
-    bk, nk, hk, dk = k.shape
-    bv, nv, hv, dv = v.shape
+    b, nq, hq, dq = qs
+    bk, nk, hk, dk = ks
+    bv, nv, hv, dv = vs
     if not (b == bk == bv):
         raise ValueError(f"Batch sizes must match across Q, K, V. Got Q: {b}, K: {bk}, V: {bv}")
     if nk != nv:
