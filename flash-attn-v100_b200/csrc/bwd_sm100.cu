@@ -85,15 +85,17 @@ constexpr float kLog2e = 1.4426950408889634f;
 // PREC: 0 for calls with D = 64 or 128; 1 ("pair") for 16-bit calls with an additive bias or another head size (any
 // multiple of 8 up to 128, the tiles padded by TMA's zero fill): P and dS go back to tensor memory as hi + lo in the
 // inputs' own format and every accumulating MMA is issued for both, so they keep 17 (bf16) or 22 (fp16) significant
-// bits and no operand is converted.
+// bits and no operand is converted.  2: the same with the step's 128 x 128 bias tile brought to shared memory by TMA
+// (see the forward; here the key-stationary kernel would read a value, the other one 16 bytes of 32 lines, per load).
 template <int D, int MODE, int DROP, int PREC>
 struct BwdCfg {
     static constexpr int kNBox = D / 64;
     static constexpr int kTileBytes = kNBox * kBoxBytes;
     static constexpr bool kFused = (MODE == 2);
     static constexpr bool kMasks = DROP == 1 && MODE != 1;       // masks are built in shared memory when keys are rows
-    static constexpr int kUStages = tile::bwd_u_stages(D, kMasks);
-    static constexpr int kWStages = tile::bwd_w_stages(D);
+    static constexpr int kUStages = PREC == 2 ? tile::bwd_bias_u_stages(D) : tile::bwd_u_stages(D, kMasks);
+    static constexpr int kWStages = PREC == 2 ? tile::bwd_bias_w_stages(D) : tile::bwd_w_stages(D);
+    static constexpr int kBiasBytes = PREC == 2 ? 4 * kBoxBytes : 0;    // four boxes of 128 queries x 32 keys
     static constexpr int kMaskBytes = 2 * 128 * 8 * 2;          // two buffers of 128 x 8 uint16 keep masks
     static constexpr int kXYFull = 0;
     static constexpr int kUFull = 1;                             // [kUStages]
@@ -117,11 +119,13 @@ struct BwdCfg {
     static constexpr int kXYConv = kVEmpty + 2;                  // stationary tiles (elementwise warps)
     static constexpr int kUConv = kXYConv + 1;                   // [kUStages] streamed U (the two spare warps)
     static constexpr int kWConv = kUConv + kUStages;             // [kWStages] streamed W, key-stationary kernels only
-    static constexpr int kNumBars = kWConv + kWStages;
+    static constexpr int kBiasFull = kWConv + kWStages;          // PREC = 2: the step's bias tile has landed
+    static constexpr int kBiasEmpty = kBiasFull + 1;             // ... and has been read (one arrival per elementwise warp)
+    static constexpr int kNumBars = kBiasEmpty + 1;
     static constexpr int kVecBytes = (MODE != 1) ? 2 * 1024 : 0; // two slots of lse[128] | delta[128]
     static constexpr int kDsBytes = 128 * 128 * 2;               // fused kernel: dS^T tile for the dQ MMA
     // bytes used from the 1024-aligned base: X, Y, U ring, W ring, [dS], [vectors], barriers, TMEM slot + flag, [masks]
-    static constexpr int kUsedBytes = (2 + kUStages + kWStages) * kTileBytes + (kFused ? kDsBytes : 0) + kVecBytes +
+    static constexpr int kUsedBytes = (2 + kUStages + kWStages) * kTileBytes + kBiasBytes + (kFused ? kDsBytes : 0) + kVecBytes +
                                       kNumBars * 8 + 64 + (kMasks ? kMaskBytes : 0);
     static constexpr int kMaxSmem = 232448;                      // 227 KB: the most one CTA can ask for
     static_assert(128 * kNWG + 128 == 32 * tile::kBwdWarps, "thread count and table disagree");
@@ -157,6 +161,7 @@ struct BwdArgs {
     const float* bias;             // optional additive bias, element strides below (0 broadcasts)
     int64_t bias_sb, bias_sn, bias_sh;
     int bias_vec;                  // its rows can be read as float4
+    int bias_b, bias_h;            // PREC = 2: whether it has a batch / head dimension
     int ds_vec;                    // rows of d_scores can be written as float4
     float* d_scores;               // optional dense (B, H, Nq, Nk) gradient of the scores (written by MODE 1)
 };
@@ -256,12 +261,12 @@ __global__ void __launch_bounds__(128 * NWG + kExtraThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                  const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_out1, const __grid_constant__ CUtensorMap map_out2,
-                 const __grid_constant__ CUtensorMap map_aux, const BwdArgs a) {
+                 const __grid_constant__ CUtensorMap map_aux, const __grid_constant__ CUtensorMap map_bias, const BwdArgs a) {
     using Cfg = BwdCfg<D, MODE, DROP, PREC>;
     constexpr bool KS = (MODE != 1);        // key-stationary: K, V stay, query tiles stream
     constexpr bool FUSED = (MODE == 2);     // key-stationary and dQ too
     constexpr bool CONV = BF16 && PREC == 0;    // every MMA runs f16 x f16: bf16 tiles are converted
-    constexpr bool P_BF16 = BF16 && PREC == 1;  // ... except that pairs of bf16 need no conversion
+    constexpr bool P_BF16 = BF16 && PREC != 0;  // ... except that pairs of bf16 need no conversion
     static_assert(PREC == 0 || (MODE != 2 && !INLINE), "the pair instances are the two-pass form");
     constexpr bool STREAM_CONV = CONV && INLINE;             // ... the streamed ones by the spare warps
     constexpr bool XY_CONV = CONV && (KS || INLINE);         // ... the stationary ones by the elementwise warps
@@ -277,7 +282,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint8_t* sY = sX + TILE;
     uint8_t* sU = sY + TILE;                        // U ring
     uint8_t* sW = sU + UST * TILE;                  // W ring
-    uint8_t* sDs = sW + WST * TILE;                 // fused kernel only
+    uint8_t* sBias = sW + WST * TILE;               // PREC = 2
+    uint8_t* sDs = sBias + Cfg::kBiasBytes;         // fused kernel only
     float* sVec = (float*)(sDs + (FUSED ? Cfg::kDsBytes : 0));      // key-stationary only: 2 x (lse[128] | delta[128])
     uint64_t* bars = (uint64_t*)((uint8_t*)sVec + Cfg::kVecBytes);
     uint32_t* tmem_slot = (uint32_t*)(bars + Cfg::kNumBars);
@@ -336,8 +342,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int i = 0; i < Cfg::kNumBars; ++i) {
             const bool wide = (i == Cfg::kPReady || i == Cfg::kDsReady || i == Cfg::kMask || i == Cfg::kEpi ||
                                i == Cfg::kDqRead || i == Cfg::kPHalf || i == Cfg::kDsHalf ||
-                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i == Cfg::kXYConv);
-            const bool conv2 = i >= Cfg::kUConv;          // the two converting warps
+                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i == Cfg::kXYConv || i == Cfg::kBiasEmpty);
+            const bool conv2 = i >= Cfg::kUConv && i < Cfg::kBiasFull;          // the two converting warps
             mbar_init(&bars[i], wide ? 4u * NWG : (conv2 ? 2u : 1u));    // one arrival per elementwise warp
         }
         wait_control_init(abort_flag, a.wait_limit_ms);
@@ -634,6 +640,27 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (++us == UST) { us = 0; ++uph; }
             if (++ws == WST) { ws = 0; ++wph; }
         }
+      } else if (PREC == 2 && warp == kTmaWarp + 1) {
+        // ---------------------------------------------------------------- warp 18: the steps' bias tiles
+        if (elect_one()) {
+            int qi = 0, hg = 0, done = 0;
+            bool ok = true;
+            for (int it = 0; it < n_iter; ++it) {
+                const int head = KS ? head_x * group + hg : head_x;
+                const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : it) * kTile;
+                ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)it & 1u) ^ 1u, abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    tma_load_4d(sBias + c * kBoxBytes, &map_bias, &bars[Cfg::kBiasFull], k_col + 32 * c, a.bias_h ? head : 0, q_row,
+                                a.bias_b ? b : 0);
+                ++done;
+                if (++qi == n_per_head) { qi = 0; ++hg; }
+            }
+            for (int spin = 0; !ok && spin < 4096 && done > 0 && !mbar_try_wait(&bars[Cfg::kBiasFull], (uint32_t)(done - 1) & 1u); ++spin) {}
+        }
+        __syncwarp();
       }
     } else {
         // ---------------------------------------------------------------- P / dS and epilogue
@@ -790,6 +817,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
             ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)it & 1u, abort_flag);
             if (ok) ok = mbar_wait(&bars[Cfg::kVFull + (it & 1)], (uint32_t)(it >> 1) & 1u, abort_flag);
+            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)it & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -850,7 +878,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             const int i0 = 4 * j + 2 * k;
                             float x0, x1;
                             f2_unpack(f2_fma(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), sc2, L), x0, x1);
-                            if (PREC && a.bias) {
+                            if constexpr (PREC == 2) {
+                                // bias[query][key] from the tile: eight keys (two 16-byte pieces) of four queries a load,
+                                // which the swizzle spreads over all banks
+                                const int kk = lr + 16 * h + 8 * k;
+                                const uint8_t* bp = sBias + (warp & 3) * kBoxBytes + (cb + 8 * j + 2 * lq) * 128 + (kk & 3) * 4;
+                                x0 = fmaf(*reinterpret_cast<const float*>(bp + (((kk >> 2) ^ (2 * lq)) << 4)), kLog2e, x0);
+                                x1 = fmaf(*reinterpret_cast<const float*>(bp + 128 + (((kk >> 2) ^ (2 * lq + 1)) << 4)), kLog2e, x1);
+                            } else if (PREC && a.bias) {
                                 // bias[query][key]: eight lanes read eight neighbouring keys of one query
                                 const int key = tile * kTile + rbase + 16 * h + 8 * k, qr = col_g0 + 8 * j + 2 * lq;
                                 const float* bp = bias_h + (int64_t)qr * a.bias_sn + key;
@@ -861,6 +896,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             pf[h][i0 + 1] = __float_as_uint(ex2(x1));
                         }
                 }
+                if (PREC == 2 && hf == 1) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
                 if (diag || tail) {
                     // one branch for the whole half: the diagonal tile and a tile with padding keys are rare
 #pragma unroll
@@ -975,6 +1011,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             // ---- phase A: P from T1
             ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)it & 1u, abort_flag);
             if (KS && ok) ok = mbar_wait(&bars[Cfg::kVFull + (it & 1)], (uint32_t)(it >> 1) & 1u, abort_flag);
+            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)it & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1049,7 +1086,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 for (int c = 0; c < CPT; c += 2) {
                     float x0, x1;
                     f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), sc2, neg2), x0, x1);
-                    if constexpr (PREC != 0) {
+                    if constexpr (PREC == 2) {
+                        // my row's 32 keys are the wg-th box, its 16-byte pieces swizzled by the row
+                        if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4));
+                        PSET(c, ex2(fmaf((c & 2) ? bv.z : bv.x, kLog2e, x0)));
+                        PSET(c + 1, ex2(fmaf((c & 2) ? bv.w : bv.y, kLog2e, x1)));
+                        continue;
+                    }
+                    if constexpr (PREC == 1) {
                         if (a.bias) {
                             const float* bp = bias_h + (int64_t)(row_g < a.Nq ? row_g : a.Nq - 1) * a.bias_sn + col_g0 + c;
                             if (a.bias_vec && col_g0 + (c & ~3) + 4 <= a.Nk) {
@@ -1077,6 +1121,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         PSET(c + 1, ex2(x1));
                     }
                 }
+                if (PREC == 2) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
                 const bool diag = a.causal && strm_tile * kTile + kTile - 1 > tile * kTile + a.shift;
                 if (diag || strm_tile * kTile + kTile > nk) {
                     // my row sees my first `seen` columns: keys below the count, at most row + shift
@@ -1427,11 +1472,13 @@ bwd_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, int Nq,
 template <int D, bool BF16, int MODE, bool INLINE, int PREC>
 auto pick_kernel(int drop) {
     if (drop == 2 && !INLINE) return bwd_sm100_kernel<D, BF16, MODE, kNWG, INLINE ? 1 : 2, INLINE, PREC>;
-    return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE, PREC> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;
+    if constexpr (PREC == 2) return bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;       // bias_is_staged(): never drop = 1
+    else return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE, PREC> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;
 }
 template <int D, int MODE, int PREC>
 int pick_smem(int drop) {
-    return drop == 2 ? BwdCfg<D, MODE, 2, PREC>::kSmemBytes
+    if constexpr (PREC == 2) return drop ? BwdCfg<D, MODE, 2, PREC>::kSmemBytes : BwdCfg<D, MODE, 0, PREC>::kSmemBytes;
+    else return drop == 2 ? BwdCfg<D, MODE, 2, PREC>::kSmemBytes
                      : (drop ? BwdCfg<D, MODE, 1, PREC>::kSmemBytes : BwdCfg<D, MODE, 0, PREC>::kSmemBytes);
 }
 
@@ -1503,7 +1550,14 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
             return FA_ECUDA;
         }
     }
+    CUtensorMap mb = mq;
     BwdArgs a;
+    a.bias_b = p.bias.stride_b != 0 && p.B > 1; a.bias_h = p.bias.stride_h != 0 && p.H > 1;
+    if (PREC == 2 && (r = cached_tmap_bnhd(&mb, p.bias.ptr, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.bias_b ? p.B : 1, p.Nq, a.bias_h ? p.H : 1,
+                                           p.Nk, p.bias.stride_b, p.bias.stride_n, p.bias.stride_h, 128, 32, 1))) {
+        set_error("cuTensorMapEncodeTiled failed for the bias (%d)", r);
+        return FA_ECUDA;
+    }
     a.lse2 = lse2; a.delta = delta; a.ranges = ranges; a.dq_acc = dq_acc; a.status = p.status_word; a.wait_limit_ms = p.wait_limit_ms;
     a.erow = COPIES ? (const float*)(wsp + ws.erow_off) : nullptr;
     a.kv_len = p.kv_lengths;
@@ -1547,7 +1601,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         const int smem2 = pick_smem<D, 2, PREC>(drop);
         FA_CUDA_CHECK(set_smem_limit_once(k2, smem2, p.device, &smem_done[6 + drop], &smem_mu));
         if (phases & 2) {
-            k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, a);
+            k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, mb, a);
             FA_CUDA_CHECK(cudaGetLastError());
         }
         if (phases & 4) {
@@ -1567,7 +1621,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     if (phases & 2) {
         // stationary K_j, V_j; streamed Q_i, dO_i (bf16 with copies: their fp16 copies; the kernel leaves
         // the fp16 copy of K behind for the dQ kernel)
-        k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, a);
+        k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, mb, a);
         FA_CUDA_CHECK(cudaGetLastError());
     }
     if (phases & 4) {
@@ -1584,7 +1638,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         // that the dK/dV kernel is still writing.
         cfg.numAttrs = (!COPIES && (phases & 2) && (int64_t)p.Nk * D * 4 <= (int64_t)tile::kBwdOverlapMaxKvBytes) ? 1 : 0;
         // stationary Q_i (its fp16 copy), dO_i; streamed K_j (its fp16 copy), V_j
-        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k1, mq16, mg, mk16, mv, mdq, mdq, mdq, a));
+        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k1, mq16, mg, mk16, mv, mdq, mdq, mdq, mb, a));
     }
     return FA_OK;
 }
@@ -1610,6 +1664,10 @@ int sm100_bwd(const fa_b200_params& p, const BwdWorkspace& ws) {
 
 #else
 int sm100_pair_bwd(const fa_b200_params& p, const BwdWorkspace& ws) {
+    if (bias_is_staged(p, 2 * dropout_bits_bytes(p))) {
+        if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, false, 2>(p, ws) : launch<64, true, false, 2>(p, ws);
+        return p.D > 64 ? launch<128, false, false, 2>(p, ws) : launch<64, false, false, 2>(p, ws);
+    }
     if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, false, 1>(p, ws) : launch<64, true, false, 1>(p, ws);
     return p.D > 64 ? launch<128, false, false, 1>(p, ws) : launch<64, false, false, 1>(p, ws);
 }

@@ -110,6 +110,7 @@ bool sm100_supports(const fa_b200_params& p, bool backward, const char** why);
 // additive bias, or a head size other than 64 and 128.
 int sm100_pair_fwd(const fa_b200_params& p);
 int sm100_pair_bwd(const fa_b200_params& p, const BwdWorkspace& ws);
+bool bias_is_staged(const fa_b200_params& p, size_t bits);
 bool sm100_pair_supports(const fa_b200_params& p, bool backward, const char** why);
 // fp32 forward on the tensor cores (fwd_tf32_sm100.cu): TF32 products taken three times
 int sm100_tf32_fwd(const fa_b200_params& p);

@@ -78,6 +78,10 @@ static_assert(tile::kFwdQTilesPerCta == 2, "the kernel is written for two query 
 //      tiles are padded to 64 or 128 columns by TMA's zero fill, the MMA K-steps and N stop at the head
 //      size).  P is handed over as hi + lo in the inputs' own format, two MMAs per K-step of P V, so P keeps
 //      17 (bf16) or 22 (fp16) significant bits and a bf16 V needs no conversion.
+//   2  the same with the bias brought to shared memory by TMA, in chunks of 128 rows x 32 columns: a thread needs 32
+//      consecutive values of its own row, and read straight from global memory a warp's load touches 32 lines.
+//      Dense or batch / head broadcast biases whose rows TMA can address; one that is broadcast over the queries is
+//      the same value for a whole warp and stays with PREC = 1.
 // SCHED: how the work is divided (plan_schedule).
 //   0  whole pairs of 128-row tiles, round robin (kernel comment above)
 //   1  the split schedule, with packed tiles or plain ones
@@ -89,7 +93,10 @@ struct FwdCfg {
     static constexpr int kNBox = D / 64;
     static constexpr int kTileBytes = kNBox * kBoxBytes;
     static constexpr int kQTiles = SCHED == 2 ? 1 : 2;
-    static constexpr int kStages = SCHED == 2 ? tile::fwd_one_tile_kv_stages(D) : tile::fwd_kv_stages(D);
+    static constexpr int kStages = SCHED == 2 ? tile::fwd_one_tile_kv_stages(D)
+                                                 : (PREC == 2 ? tile::fwd_bias_kv_stages(D) : tile::fwd_kv_stages(D));
+    static constexpr int kBiasSlots = PREC == 2 ? tile::fwd_bias_slots(D) : 0;         // chunks of 16 KB per query tile
+    static constexpr int kBiasBytes = 2 * kBiasSlots * kBoxBytes;
     // barrier slots
     static constexpr int kQFull = 0;                       // [2]
     static constexpr int kQEmpty = 2;                      // [2] last S MMA of the pair has read Q_t
@@ -104,10 +111,12 @@ struct FwdCfg {
     static constexpr int kVConv = kPHalf + 2;              // [kStages] V_j converted to fp16 (one arrival per converting warp)
     static constexpr int kMlFull = kVConv + kStages;       // SCHED = 2: the odd blocks' maxima and sums are in shared memory
     static constexpr int kORead = kMlFull + 1;             // SCHED = 2: O_1 has been read (both: one arrival per warp of a warpgroup)
-    static constexpr int kNumBars = kORead + 1;
+    static constexpr int kBiasFull = kORead + 1;           // PREC = 2: [2 tiles][kBiasSlots]
+    static constexpr int kBiasEmpty = kBiasFull + 2 * kBiasSlots;      // ... one arrival per warp of the warpgroup
+    static constexpr int kNumBars = kBiasEmpty + 2 * kBiasSlots;
     static constexpr int kMlBytes = SCHED == 2 ? kBlockM * 8 : 0;
     static constexpr int kWalkBytes = SCHED ? 8 * 40 : 0;  // a WalkRecord per softmax warp
-    static constexpr int kSmemBytes = (kQTiles + 2 * kStages) * kTileBytes + kNumBars * 8 + 64 + kMlBytes + kWalkBytes + 1024;
+    static constexpr int kSmemBytes = (kQTiles + 2 * kStages) * kTileBytes + kBiasBytes + kNumBars * 8 + 64 + kMlBytes + kWalkBytes + 1024;
     static_assert(kSmemBytes <= 232448, "shared-memory plan does not fit");
 };
 
@@ -135,6 +144,7 @@ struct FwdArgs {
     const float* bias;             // PREC = 1: optional additive bias, element strides below (0 broadcasts)
     int64_t bias_sb, bias_sn, bias_sh;
     int bias_vec;                  // its rows can be read as float4
+    int bias_b, bias_h;            // PREC = 2: whether it has a batch / head dimension
     const uint4* mq;               // DROP = 2: keep bits, [(b*H + h) * n_kblocks + key block][padded query row]
     int nq_pad, n_kblocks;
     // Rows of a query tile: `pack` query heads of one K/V head times `q_per_tile` queries, the heads fastest
@@ -338,7 +348,7 @@ constexpr float kPShift = 6.0f;
 template <int D, bool BF16, int DROP, int PREC, int SCHED>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                 const __grid_constant__ CUtensorMap map_v, const FwdArgs a) {
+                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_bias, const FwdArgs a) {
     using Cfg = FwdCfg<D, PREC, SCHED>;
     constexpr bool FREE = SCHED != 0, TWIN = SCHED == 2;
     constexpr int ST = Cfg::kStages;
@@ -347,14 +357,15 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     // illegal-instruction fault).  P is always fp16; a bf16 V tile is converted to fp16 in shared memory.
     // With P as a pair (PREC = 1) P_hi + P_lo come in V's own format and nothing is converted.
     constexpr bool CONV = BF16 && PREC == 0;
-    constexpr bool P_BF16 = BF16 && PREC == 1;
+    constexpr bool P_BF16 = BF16 && PREC != 0;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = smem;
     uint8_t* sK = sQ + Cfg::kQTiles * TILE;
     uint8_t* sV = sK + ST * TILE;
-    uint64_t* bars = (uint64_t*)(sV + ST * TILE);
+    uint8_t* sBias = sV + ST * TILE;            // PREC = 2
+    uint64_t* bars = (uint64_t*)(sBias + Cfg::kBiasBytes);
     uint32_t* tmem_slot = (uint32_t*)(bars + Cfg::kNumBars);
     volatile uint32_t* abort_flag = (volatile uint32_t*)(tmem_slot + 1);
     [[maybe_unused]] float2* sMl = (float2*)((uint8_t*)(bars + Cfg::kNumBars) + 64);      // SCHED = 2: [128]
@@ -364,7 +375,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < Cfg::kNumBars; ++i) {
-            const bool wg_bar = (i >= Cfg::kPFull && i < Cfg::kPFull + 2) || (i >= Cfg::kPHalf && i < Cfg::kPHalf + 2) || i >= Cfg::kMlFull;
+            const bool wg_bar = (i >= Cfg::kPFull && i < Cfg::kPFull + 2) || (i >= Cfg::kPHalf && i < Cfg::kPHalf + 2) ||
+                                i == Cfg::kMlFull || i == Cfg::kORead || i >= Cfg::kBiasEmpty;
             const bool conv_bar = (i >= Cfg::kVConv && i < Cfg::kVConv + ST);
             mbar_init(&bars[i], wg_bar ? 4u : (conv_bar ? 2u : 1u));
         }
@@ -635,6 +647,37 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 }
             }
         }
+      } else if constexpr (PREC == 2) {
+        // ------------------------------------------------------------ warps 10-11: the bias chunks of tile 0, 1
+        const int t = warp - 10;
+        if (elect_one()) {
+            constexpr int NB = Cfg::kBiasSlots;
+            int slot = 0, done = 0;
+            uint32_t ph = 1u;                   // the slots start empty
+            bool ok = true;
+            for (WorkLoop<SCHED> wl(a, range); wl.more(a) && ok; wl.advance()) {
+                for (int u = 0; u < wl.kSub && ok; ++u) {
+                    Stretch st;
+                    if (!wl.get(a, u, st)) continue;
+                    const int n = st.j0 + st.count(t), row = (st.pair * 2 + t) * kBlockM;
+                    for (int c = st.j0 * 4; c < n * 4 && ok; ++c) {
+                        ok = mbar_wait(&bars[Cfg::kBiasEmpty + t * NB + slot], ph, abort_flag);
+                        if (!ok) break;
+                        mbar_expect_tx(&bars[Cfg::kBiasFull + t * NB + slot], kBoxBytes);
+                        tma_load_4d(sBias + (t * NB + slot) * kBoxBytes, &map_bias, &bars[Cfg::kBiasFull + t * NB + slot],
+                                    c * 32, a.bias_h ? st.h : 0, row, a.bias_b ? st.b : 0);
+                        ++done;
+                        if (++slot == NB) { slot = 0; ph ^= 1u; }
+                    }
+                }
+            }
+            for (int s = 0; s < NB && !ok; ++s) {           // unwinding: the copies in flight land first
+                const int nf = (done + NB - 1 - s) / NB;
+                for (int spin = 0; spin < 4096 && nf > 0 &&
+                     !mbar_try_wait(&bars[Cfg::kBiasFull + t * NB + s], (uint32_t)(nf - 1) & 1u); ++spin) {}
+            }
+        }
+        __syncwarp();
       }   // fp16 inputs: warps 10-11 idle, they complete the third warpgroup
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
@@ -650,6 +693,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         int s_waits = 0;                 // S_t hand-offs so far (S_full phase)
         int o_waits = 0;                 // pairs finished so far (O_done phase)
         [[maybe_unused]] int stretches = 0;
+        [[maybe_unused]] int bias_slot = 0;       // PREC = 2: next chunk's slot and phase
+        [[maybe_unused]] uint32_t bias_ph = 0u;
         bool ok = true;
 
         if (FREE && threadIdx.x == 0) a.part_meta[blockIdx.x] = make_int4(0, 0, 0, 0);
@@ -687,7 +732,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 float m = -INFINITY, l = 0.f;
                 // my row of the bias (a row beyond Nq, whose results nobody keeps, reads the last one)
                 const float* brow = nullptr;
-                if (PREC != 0 && a.bias)
+                if (PREC == 1 && a.bias)
                     brow = a.bias + st.b * a.bias_sb + h * a.bias_sh + (int64_t)(i < a.Nq ? i : a.Nq - 1) * a.bias_sn;
 
                 for (int j = first; j < n; j += kStep) {
@@ -717,7 +762,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         // scores in the log2 domain, the bias added before the mask
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
-                            if (!a.bias) {
+                            if constexpr (PREC == 2) {
+                                // my row of the chunk: 16-byte pieces, swizzled by the row (no bank conflicts)
+                                const int at = t * Cfg::kBiasSlots + bias_slot;
+                                ok = mbar_wait(&bars[Cfg::kBiasFull + at], bias_ph, abort_flag);
+                                ok = __all_sync(0xffffffffu, ok);
+                                if (!ok) break;
+                                const uint8_t* chunk = sBias + at * kBoxBytes + r * 128;
+#pragma unroll
+                                for (int c = 0; c < 32; c += 4) {
+                                    const float4 b4 = *reinterpret_cast<const float4*>(chunk + (((c >> 2) ^ (r & 7)) << 4));
+                                    SSET(q4 * 32 + c, fmaf(b4.x, kLog2e, SF(q4 * 32 + c) * a.scale_log2));
+                                    SSET(q4 * 32 + c + 1, fmaf(b4.y, kLog2e, SF(q4 * 32 + c + 1) * a.scale_log2));
+                                    SSET(q4 * 32 + c + 2, fmaf(b4.z, kLog2e, SF(q4 * 32 + c + 2) * a.scale_log2));
+                                    SSET(q4 * 32 + c + 3, fmaf(b4.w, kLog2e, SF(q4 * 32 + c + 3) * a.scale_log2));
+                                }
+                                mbar_arrive_read_done(&bars[Cfg::kBiasEmpty + at]);
+                                if (++bias_slot == Cfg::kBiasSlots) { bias_slot = 0; bias_ph ^= 1u; }
+                            } else if (!a.bias) {
 #pragma unroll
                                 for (int c = 0; c < 32; ++c) SSET(q4 * 32 + c, SF(q4 * 32 + c) * a.scale_log2);
                             } else {
@@ -741,6 +803,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                             }
                         }
                     }
+                    if (PREC == 2 && !ok) break;
                     const bool need_mask = (a.causal && col0 + kBlockN - 1 > tile * q_per_tile + a.shift) || (col0 + kBlockN > nk);
                     if (need_mask) {
                         // my row sees the block's first `seen` columns: keys below the count, at most i + shift
@@ -985,7 +1048,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     if (row_ok()) {
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
-                            if (PREC == 1 && c0 + g * 8 >= a.d) break;
+                            if (PREC != 0 && c0 + g * 8 >= a.d) break;
                             uint4 v4;
                             v4.x = pack2<BF16>(__uint_as_float(orr[g * 8 + 0]) * inv, __uint_as_float(orr[g * 8 + 1]) * inv);
                             v4.y = pack2<BF16>(__uint_as_float(orr[g * 8 + 2]) * inv, __uint_as_float(orr[g * 8 + 3]) * inv);
@@ -1168,7 +1231,15 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
         set_error("cuTensorMapEncodeTiled failed (%d)", r);
         return FA_ECUDA;
     }
+    CUtensorMap mb = mq;
+    const int bias_b = p.bias.stride_b != 0 && p.B > 1, bias_h = p.bias.stride_h != 0 && p.H > 1;
+    if (PREC == 2 && (r = cached_tmap_bnhd(&mb, p.bias.ptr, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, bias_b ? p.B : 1, p.Nq, bias_h ? p.H : 1, p.Nk,
+                                           p.bias.stride_b, p.bias.stride_n, p.bias.stride_h, 128, 32, 1))) {
+        set_error("cuTensorMapEncodeTiled failed for the bias (%d)", r);
+        return FA_ECUDA;
+    }
     FwdArgs a;
+    a.bias_b = bias_b; a.bias_h = bias_h;
     a.o = p.o.ptr;
     a.o_sb = p.o.stride_b; a.o_sn = p.o.stride_n; a.o_sh = p.o.stride_h;
     a.o_lo = p.o_lo.ptr;
@@ -1215,8 +1286,8 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
         a.mq = (const uint4*)p.dropout_bits;
         drop = 2;
     }
-    auto kernel = drop == 2 ? fwd_sm100_kernel<D, BF16, 2, PREC, 0>
-                            : (drop == 1 ? fwd_sm100_kernel<D, BF16, 1, PREC, 0> : fwd_sm100_kernel<D, BF16, 0, PREC, 0>);
+    auto kernel = drop == 2 ? fwd_sm100_kernel<D, BF16, 2, PREC, 0> : fwd_sm100_kernel<D, BF16, 0, PREC, 0>;
+    if constexpr (PREC != 2) if (drop == 1) kernel = fwd_sm100_kernel<D, BF16, 1, PREC, 0>;      // bias_is_staged()
     int smem = FwdCfg<D, PREC, 0>::kSmemBytes;
     if constexpr (PREC == 0) {
         if (plan.sched == 1) kernel = fwd_sm100_kernel<D, BF16, 0, PREC, 1>;
@@ -1228,7 +1299,7 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
         FA_CUDA_CHECK(set_smem_limit_once(kernel, smem, p.device, &done[plan.sched ? 2 + plan.sched : drop], &mu));
     }
     const int grid = plan.sched ? plan.ctas : (a.n_items < sms ? a.n_items : sms);     // one persistent CTA per SM
-    kernel<<<grid, kThreads, smem, (cudaStream_t)p.stream>>>(mq, mk, mv, a);
+    kernel<<<grid, kThreads, smem, (cudaStream_t)p.stream>>>(mq, mk, mv, mb, a);
     FA_CUDA_CHECK(cudaGetLastError());
     if constexpr (PREC == 0) if (plan.sched) {
         cudaLaunchConfig_t cfg = {};
@@ -1300,7 +1371,20 @@ size_t sm100_fwd_workspace_bytes(const fa_b200_params& p) {
 #else
 }  // namespace
 
+// Whether a call's bias comes to the kernels by TMA (PREC = 2): rows of whole 16-byte pieces, one per query.  Not where
+// the kernels draw their dropout bits themselves (`bits`: the buffer they would load them from otherwise), whose masks
+// take the room in shared memory.
+bool bias_is_staged(const fa_b200_params& p, size_t bits) {
+    if (!p.bias.ptr || p.bias.stride_n == 0 || ((uintptr_t)p.bias.ptr & 15u) != 0) return false;
+    if ((p.bias.stride_b | p.bias.stride_n | p.bias.stride_h) % 4 != 0) return false;
+    return dropout_threshold(p.dropout_p) == 0u || (p.dropout_bits && p.dropout_bits_bytes >= bits);
+}
+
 int sm100_pair_fwd(const fa_b200_params& p) {
+    if (bias_is_staged(p, dropout_bits_bytes(p))) {
+        if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, 2>(p, nullptr, 0) : launch<64, true, 2>(p, nullptr, 0);
+        return p.D > 64 ? launch<128, false, 2>(p, nullptr, 0) : launch<64, false, 2>(p, nullptr, 0);
+    }
     if (p.dtype == FA_B200_BF16) return p.D > 64 ? launch<128, true, 1>(p, nullptr, 0) : launch<64, true, 1>(p, nullptr, 0);
     return p.D > 64 ? launch<128, false, 1>(p, nullptr, 0) : launch<64, false, 1>(p, nullptr, 0);
 }

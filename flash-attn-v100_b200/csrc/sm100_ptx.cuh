@@ -107,6 +107,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+// A warp has read (plain loads) what a TMA copy will overwrite: tell the producer.  The fence orders the reads before
+// the copy, which goes through another proxy; without it the arrival overtook loads still queued behind those of
+// fifteen other warps, and a late one got values of the next tile.
+__device__ __forceinline__ void mbar_arrive_read_done(uint64_t* bar) {
+    fence_proxy_async_smem();
+    mbar_arrive_warp(bar);
+}
 
 // ---- global reductions ---------------------------------------------------------
 // Four fp32 additions to 16 consecutive bytes of global memory in one request (no return value).

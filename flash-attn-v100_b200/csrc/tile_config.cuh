@@ -16,6 +16,8 @@ constexpr int kFwdQTilesPerCta = 2;     // two query tiles in flight: the softma
 constexpr int kFwdWarps = 12;           // 8 softmax + MMA + TMA + 2 converting (bf16) / spare (fp16) warps
 constexpr int fwd_kv_stages(int D) { return D == 128 ? 2 : 4; }      // K and V rings: what 227 KB hold
 constexpr int fwd_one_tile_kv_stages(int D) { return D == 128 ? 3 : 6; }   // one query tile: the other's room too
+constexpr int fwd_bias_kv_stages(int D) { return D == 128 ? 1 : 2; }       // with a staged bias: its chunks take the room
+constexpr int fwd_bias_slots(int D) { return D == 128 ? 3 : 4; }           // of 16 KB per query tile (a block has four)
 constexpr int kFwdRegsSoftmax = 208;    // setmaxnreg split; best of 224/56, 216/72, 208/88, 200/104
 constexpr int kFwdRegsOther = 88;
 constexpr int kFwdPolyPeriod = 2;       // of every kFwdPolyPeriod groups of four exponentials, kFwdPolyCount
@@ -30,6 +32,8 @@ constexpr int kBwdWarps = 4 * kBwdWarpgroups + 4;                    // + MMA, T
 // stages took 16 % off the dQ kernel), W within one step; the key-stationary dropout instance at
 // D = 128 gives 4 KB to its masks and keeps two and two
 constexpr int bwd_u_stages(int D, bool masks) { return D == 64 ? 4 : (masks ? 2 : 3); }
+constexpr int bwd_bias_u_stages(int D) { return D == 64 ? 4 : 2; }         // with a staged bias tile of 64 KB
+constexpr int bwd_bias_w_stages(int D) { return D == 64 ? 3 : 1; }
 constexpr int bwd_w_stages(int D) { return D == 64 ? 3 : 2; }
 // the dQ kernel is launched programmatically behind the dK/dV kernel while one head's K and V take at
 // most this many bytes (N = 4096 at D = 128: -1 % of the backward; longer sequences showed no gain)

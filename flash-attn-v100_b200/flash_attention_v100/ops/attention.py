@@ -420,8 +420,10 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
         if bias is not None and ctx.needs_input_grad[6]:
             # the reference returns zeros here (ops/attention.py:297-301); this is the real gradient:
             # d loss / d scores, dense, summed over the dimensions the bias broadcasts
-            d_scores = torch.zeros(q.shape[0], q.shape[2], q.shape[1], k.shape[1], dtype=torch.float32,
-                                   device=q.device)
+            # (without a mask the kernels write every score's entry, and nothing has to be zero before)
+            shape = (q.shape[0], q.shape[2], q.shape[1], k.shape[1])
+            masked = ctx.causal or ctx.key_lengths is not None
+            d_scores = (q.new_zeros if masked else q.new_empty)(shape, dtype=torch.float32)
         dq, dk, dv = launch_backward(grad_output, q, k, v, o, lse, ctx.scale, ctx.causal,
                                      ctx.dropout_p, ctx.seed, ctx.offset, bias=bias, d_scores=d_scores,
                                      key_lengths=ctx.key_lengths, causal_shift=ctx.causal_shift,
