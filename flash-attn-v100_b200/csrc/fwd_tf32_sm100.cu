@@ -12,10 +12,15 @@
 // contractions: S = Q K^T with Q and K split in shared memory, and O += P V with P split by the
 // softmax threads as they write it to tensor memory and V split in shared memory.
 //
-// One CTA per 128-row query tile of one (batch, head); key/value blocks of 64 rows, two stages.
-//   warps 0-3   one thread per query row: operand splits, softmax (exact fp32, log2 domain), epilogue
-//   warp 4      one elected thread: TMA loads and MMA issue
-// TMEM columns: S [0,64)  P_hi [64,128)  P_lo [128,192)  O [192,192+D).
+// One CTA per 128-row query tile of one (batch, head); key/value blocks of 64 rows, two stages each of K and V.
+//   warps 0-3   one thread per query row: split of Q, softmax (exact fp32, log2 domain), epilogue
+//   warp 4      MMA issuer       order  S(0) | S(j+1) PV(j)
+//   warp 5      TMA producer
+//   warps 6-9   split of the K and V blocks as they land
+// TMEM columns: S, two buffers [0,64) and [256,320); P_hi [64,128)  P_lo [128,192)  O [192,192+D).
+// S(j+1) is computed and K(j+1), V(j+1) are split while the softmax of block j runs: with the splits in the softmax
+// warps, one S buffer and one ring for K and V together, a block was one serial chain of 2.8 us (B2 N1024 H12 causal
+// forward 45 -> 32 us).
 // Head dimension 64; no dropout and no bias (those calls, other head dimensions and the fp32 backward
 // are served by the CUDA-core tiles).  Every mbarrier wait is bounded (sm100_ptx.cuh).
 #include "fa_common.cuh"
@@ -35,13 +40,13 @@ constexpr int kQBox = kM * 128;    // one TMA box of Q: 128 rows x 32 fp32
 constexpr int kKBox = kN * 128;    // one TMA box of K or V: 64 rows x 32 fp32
 constexpr int kQTile = (kD / 32) * kQBox;      // 32 KB
 constexpr int kKTile = (kD / 32) * kKBox;      // 16 KB
-constexpr int kThreads = 160;
+constexpr int kThreads = 320;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
 // barrier slots
-enum { kBarQ = 0, kBarQSplit = 1, kBarKV = 2 /*[2]*/, kBarKVSplit = 4 /*[2]*/, kBarKVFree = 6 /*[2]*/,
-       kBarS = 8, kBarP = 9, kBarO = 10, kNumBars = 11 };
+enum { kBarQ = 0, kBarK = 1 /*[2]*/, kBarV = 3 /*[2]*/, kBarKFree = 5 /*[2]*/, kBarVFree = 7 /*[2]*/, kBarS = 9 /*[2]*/, kBarO = 11,
+       kBarQSplit = 12, kBarKSplit = 13 /*[2]*/, kBarVSplit = 15 /*[2]*/, kBarP = 17, kNumBars = 18 };
 // Q hi | Q lo | per stage: K hi, K lo, V hi, V lo | barriers | tmem slot, wait control
 constexpr int kSmemBytes = 2 * kQTile + kStages * 4 * kKTile + kNumBars * 8 + 64 + 1024;
 
@@ -124,14 +129,13 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kNumBars; ++i) {
-            const bool workers = (i == kBarQSplit || i == kBarKVSplit || i == kBarKVSplit + 1 || i == kBarP);
-            mbar_init(&bars[i], workers ? 4u : 1u);       // one arrival per worker warp
+            mbar_init(&bars[i], i >= kBarQSplit ? 4u : 1u);       // one arrival per warp of a group of four
         }
         wait_control_init(abort_flag, a.wait_limit_ms);
         fence_mbar_init();
     }
     if (warp == 4) {
-        tmem_alloc(tmem_slot, 256);
+        tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
         if (lane == 0) { prefetch_tensormap(&map_q); prefetch_tensormap(&map_k); prefetch_tensormap(&map_v); }
     }
@@ -139,10 +143,66 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tS = tmem, tPh = tmem + 64u, tPl = tmem + 128u, tO = tmem + 192u;
+    auto tS = [&](int j) { return tmem + ((uint32_t)(j & 1) << 8); };
+    const uint32_t tPh = tmem + 64u, tPl = tmem + 128u, tO = tmem + 192u;
 
-    if (warp == 4) {
-        // ------------------------------------------------------------ TMA + MMA (one thread)
+    if (warp == 5) {
+        // ------------------------------------------------------------ TMA producer
+        if (elect_one() && nblk > 0) {
+            mbar_expect_tx(&bars[kBarQ], kQTile);
+#pragma unroll
+            for (int bx = 0; bx < kD / 32; ++bx)
+                tma_load_4d(sQh + bx * kQBox, &map_q, &bars[kBarQ], bx * 32, h, tile * kM, b);
+            bool ok = true;
+            int k_done = 0, v_done = 0;
+            for (int j = 0; j < nblk; ++j) {
+                const int s = j % kStages;
+                const uint32_t ph = ((uint32_t)(j / kStages) & 1u) ^ 1u;
+                uint8_t* base = sKV + s * 4 * kKTile;
+                ok = mbar_wait(&bars[kBarKFree + s], ph, abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(&bars[kBarK + s], kKTile);
+#pragma unroll
+                for (int bx = 0; bx < kD / 32; ++bx) tma_load_4d(base + bx * kKBox, &map_k, &bars[kBarK + s], bx * 32, hk, j * kN, b);
+                ++k_done;
+                ok = mbar_wait(&bars[kBarVFree + s], ph, abort_flag);
+                if (!ok) break;
+                mbar_expect_tx(&bars[kBarV + s], kKTile);
+#pragma unroll
+                for (int bx = 0; bx < kD / 32; ++bx) tma_load_4d(base + 2 * kKTile + bx * kKBox, &map_v, &bars[kBarV + s], bx * 32, hk, j * kN, b);
+                ++v_done;
+            }
+            if (!ok) {
+                // unwinding: let the copies in flight land before shared memory is given up
+                for (int s = 0; s < kStages; ++s) {
+                    const int fk = (k_done + kStages - 1 - s) / kStages, fv = (v_done + kStages - 1 - s) / kStages;
+                    for (int spin = 0; spin < 4096 && fk > 0 && !mbar_try_wait(&bars[kBarK + s], (uint32_t)(fk - 1) & 1u); ++spin) {}
+                    for (int spin = 0; spin < 4096 && fv > 0 && !mbar_try_wait(&bars[kBarV + s], (uint32_t)(fv - 1) & 1u); ++spin) {}
+                }
+                for (int spin = 0; spin < 4096 && !mbar_try_wait(&bars[kBarQ], 0u); ++spin) {}
+            }
+        }
+        __syncwarp();
+    } else if (warp >= 6) {
+        // ------------------------------------------------------------ K and V blocks -> hi, lo
+        const int t = (int)threadIdx.x - 192;
+        bool ok = true;
+        for (int j = 0; j < nblk && ok; ++j) {
+            const int s = j % kStages;
+            const uint32_t ph = (uint32_t)(j / kStages) & 1u;
+            uint8_t* base = sKV + s * 4 * kKTile;
+#pragma unroll
+            for (int kv = 0; kv < 2 && ok; ++kv) {
+                ok = mbar_wait(&bars[(kv ? kBarV : kBarK) + s], ph, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                split_tile(base + 2 * kv * kKTile, base + (2 * kv + 1) * kKTile, kKTile, t);
+                fence_proxy_async_smem();
+                mbar_arrive_warp(&bars[(kv ? kBarVSplit : kBarKSplit) + s]);
+            }
+        }
+    } else if (warp == 4) {
+        // ------------------------------------------------------------ MMA issuer (one thread)
         if (elect_one()) {
             constexpr uint32_t idesc_s = make_idesc_tf32(kM, kN, false);      // S: B = K block, K-major
             constexpr uint32_t idesc_pv = make_idesc_tf32(kM, kD, true);      // O: B = V block, MN-major
@@ -151,24 +211,14 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             // V is MN-major (N = head dim): a 32-bit MN-major operand has one arrangement, the 128-byte
             // swizzle in 32-byte pieces (TMA delivers it so): 4-row groups of 512 bytes along K
             const uint64_t dmn_major = make_smem_desc(0, kKBox, 512, 1u);
-            auto load_kv = [&](int j) {
-                const int s = j % kStages;
-                uint8_t* base = sKV + s * 4 * kKTile;
-                mbar_expect_tx(&bars[kBarKV + s], 2 * kKTile);
-#pragma unroll
-                for (int bx = 0; bx < kD / 32; ++bx) {
-                    tma_load_4d(base + bx * kKBox, &map_k, &bars[kBarKV + s], bx * 32, hk, j * kN, b);
-                    tma_load_4d(base + 2 * kKTile + bx * kKBox, &map_v, &bars[kBarKV + s], bx * 32, hk, j * kN, b);
-                }
-            };
             // S (+)= A[tile] * B[tile]^T, both K-major: D / 8 K-steps of 8 fp32 (32 bytes); a box holds 32
-            auto issue_s = [&](uint32_t a_u, uint32_t b_u, bool acc) {
+            auto issue_s = [&](uint32_t d_tmem, uint32_t a_u, uint32_t b_u, bool acc) {
                 const uint64_t a0 = dk_major + (uint64_t)(a_u >> 4), b0 = dk_major + (uint64_t)(b_u >> 4);
 #pragma unroll
                 for (int kk = 0; kk < kD / 8; ++kk) {
                     const uint32_t ao = ((uint32_t)(kk >> 2) * kQBox + (uint32_t)(kk & 3) * 32u) >> 4;
                     const uint32_t bo = ((uint32_t)(kk >> 2) * kKBox + (uint32_t)(kk & 3) * 32u) >> 4;
-                    mma_ss_tf32(tS, a0 + ao, b0 + bo, idesc_s, (acc || kk > 0) ? 1u : 0u);
+                    mma_ss_tf32(d_tmem, a0 + ao, b0 + bo, idesc_s, (acc || kk > 0) ? 1u : 0u);
                 }
             };
             // O (+)= P[TMEM] * V[tile], V MN-major: kN / 8 K-steps of 8 keys (8 rows of 128 bytes)
@@ -179,45 +229,39 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     mma_ts_tf32(tO, p_tmem + (uint32_t)kk * 8u, b0 + (uint64_t)((kk * 1024) >> 4), idesc_pv,
                                 (acc || kk > 0) ? 1u : 0u);
             };
-            bool ok = true;
-            if (nblk > 0) {
-                mbar_expect_tx(&bars[kBarQ], kQTile);
-#pragma unroll
-                for (int bx = 0; bx < kD / 32; ++bx)
-                    tma_load_4d(sQh + bx * kQBox, &map_q, &bars[kBarQ], bx * 32, h, tile * kM, b);
-                load_kv(0);
-                if (nblk > 1) load_kv(1);
-                ok = mbar_wait(&bars[kBarQSplit], 0u, abort_flag);
-            }
+            auto s_block = [&](int j) {
+                const int s = j % kStages;
+                if (!mbar_wait(&bars[kBarKSplit + s], (uint32_t)(j / kStages) & 1u, abort_flag)) return false;
+                tc_fence_after_sync();
+                const uint32_t base = sKV_u + (uint32_t)(s * 4 * kKTile);
+                issue_s(tS(j), sQh_u, base, false);                 // Q_hi K_hi
+                issue_s(tS(j), sQl_u, base, true);                  // Q_lo K_hi
+                issue_s(tS(j), sQh_u, base + kKTile, true);         // Q_hi K_lo
+                mma_commit(&bars[kBarS + (j & 1)]);
+                mma_commit(&bars[kBarKFree + s]);
+                return true;
+            };
+            bool ok = nblk == 0 || mbar_wait(&bars[kBarQSplit], 0u, abort_flag);
+            if (ok && nblk > 0) ok = s_block(0);
             for (int j = 0; j < nblk && ok; ++j) {
                 const int s = j % kStages;
-                const uint32_t ph = (uint32_t)(j / kStages) & 1u;
                 const uint32_t base = sKV_u + (uint32_t)(s * 4 * kKTile);
-                ok = mbar_wait(&bars[kBarKVSplit + s], ph, abort_flag);
-                if (!ok) break;
-                tc_fence_after_sync();
-                issue_s(sQh_u, base, false);                 // Q_hi K_hi
-                issue_s(sQl_u, base, true);                  // Q_lo K_hi
-                issue_s(sQh_u, base + kKTile, true);         // Q_hi K_lo
-                mma_commit(&bars[kBarS]);
-                ok = mbar_wait(&bars[kBarP], (uint32_t)j & 1u, abort_flag);
+                // the buffer of S(j+1) held S(j-1), which the threads had read when they handed over P(j-1)
+                if (j + 1 < nblk) { ok = s_block(j + 1); if (!ok) break; }
+                ok = mbar_wait(&bars[kBarVSplit + s], (uint32_t)(j / kStages) & 1u, abort_flag);
+                if (ok) ok = mbar_wait(&bars[kBarP], (uint32_t)j & 1u, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
                 issue_pv(tPh, base + 2 * kKTile, j > 0);     // P_hi V_hi
                 issue_pv(tPl, base + 2 * kKTile, true);      // P_lo V_hi
                 issue_pv(tPh, base + 3 * kKTile, true);      // P_hi V_lo
-                mma_commit(&bars[kBarKVFree + s]);           // the stage's tiles have been read
+                mma_commit(&bars[kBarVFree + s]);
                 mma_commit(&bars[kBarO]);
-                if (j + kStages < nblk) {
-                    ok = mbar_wait(&bars[kBarKVFree + s], ph, abort_flag);
-                    if (!ok) break;
-                    load_kv(j + kStages);
-                }
             }
         }
         __syncwarp();
     } else {
-        // ------------------------------------------------------------ splits, softmax, epilogue
+        // ------------------------------------------------------------ split of Q, softmax, epilogue
         const int t = threadIdx.x;                        // 0..127: query row of the tile = TMEM lane
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
         const int i = tile * kM + t;                      // global query row
@@ -233,24 +277,13 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
         }
         for (int j = 0; j < nblk && ok; ++j) {
-            const int s = j % kStages;
-            const uint32_t ph = (uint32_t)(j / kStages) & 1u;
-            uint8_t* base = sKV + s * 4 * kKTile;
-            ok = mbar_wait(&bars[kBarKV + s], ph, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            split_tile(base, base + kKTile, kKTile, t);                     // K
-            split_tile(base + 2 * kKTile, base + 3 * kKTile, kKTile, t);    // V
-            fence_proxy_async_smem();
-            mbar_arrive_warp(&bars[kBarKVSplit + s]);
-
-            ok = mbar_wait(&bars[kBarS], (uint32_t)j & 1u, abort_flag);
+            ok = mbar_wait(&bars[kBarS + (j & 1)], (uint32_t)(j >> 1) & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
             uint32_t sr[2][32];
-            tmem_ld_32x32(tS + lane_off, sr[0]);
-            tmem_ld_32x32(tS + lane_off + 32u, sr[1]);
+            tmem_ld_32x32(tS(j) + lane_off, sr[0]);
+            tmem_ld_32x32(tS(j) + lane_off + 32u, sr[1]);
             tmem_wait_ld();
             // my row sees the block's first `seen` columns: keys below the count, at most i + shift
             const int col0 = j * kN;
@@ -268,32 +301,9 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             // a row that has seen no key yet (possible only beyond Nq) keeps m = -inf: its P are exp2(-inf - (-inf));
             // use 0 as the reference there so that they come out as 0
             const float m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-            // the accumulator is rescaled by the whole warp or not at all (tensor-memory accesses are
-            // warp-collective): a row whose maximum stays gets alpha = 1
-            if (__any_sync(0xffffffffu, m_new > m)) {
-                const float alpha = exp2f(m - m_ref);              // 0 on the first block
-                l *= alpha;
-                if (j > 0) {
-                    // O(j-1) is complete: its MMAs were committed to the O barrier before S(j) was issued
-                    ok = mbar_wait(&bars[kBarO], (uint32_t)(j - 1) & 1u, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (ok) {
-                        tc_fence_after_sync();
-#pragma unroll
-                        for (int c0 = 0; c0 < kD; c0 += 32) {
-                            uint32_t orr[32];
-                            tmem_ld_32x32(tO + lane_off + c0, orr);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int c = 0; c < 32; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
-                            tmem_st_32x32(tO + lane_off + c0, orr);
-                        }
-                    }
-                }
-                m = m_new;
-            }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            const float alpha = exp2f(m - m_ref);                      // 0 on the first block, 1 where the maximum stays
+            const bool rescale = __any_sync(0xffffffffu, m_new > m);
+            if (rescale) { l *= alpha; m = m_new; }
             float sum = 0.f;
             uint32_t plo[2][32];
 #pragma unroll
@@ -303,6 +313,26 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 const uint32_t hi = __float_as_uint(p) & 0xFFFFE000u;
                 sr[c >> 5][c & 31] = hi;
                 plo[c >> 5][c & 31] = __float_as_uint(p - __uint_as_float(hi));
+            }
+            if (j > 0) {
+                // PV(j-1) has read P's columns and left O(j-1)
+                ok = mbar_wait(&bars[kBarO], (uint32_t)(j - 1) & 1u, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after_sync();
+                // the accumulator is rescaled by the whole warp or not at all (tensor-memory accesses are
+                // warp-collective): a row whose maximum stays gets alpha = 1
+                if (rescale) {
+#pragma unroll
+                    for (int c0 = 0; c0 < kD; c0 += 32) {
+                        uint32_t orr[32];
+                        tmem_ld_32x32(tO + lane_off + c0, orr);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
+                        tmem_st_32x32(tO + lane_off + c0, orr);
+                    }
+                }
             }
             l += sum;
             tmem_st_32x32(tPh + lane_off, sr[0]);
@@ -339,7 +369,7 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 4) tmem_dealloc(tmem, 256);
+    if (warp == 4) tmem_dealloc(tmem, 512);
     if (threadIdx.x == 0 && *abort_flag) report_status(a.status, 5);
 }
 
