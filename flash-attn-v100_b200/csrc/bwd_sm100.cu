@@ -138,6 +138,7 @@ struct BwdArgs {
     const float* lse2;     // [B*H][nq_pad]  kPShift - lse * log2(e), -inf in the padding
     const float* delta;    // [B*H][nq_pad]  -delta, 0 in the padding
     const float* ranges;   // [B*Hkv][2]     max |dO| over the column's query heads, max |V|
+    const float* lse;      // [B*H][Nq]      as the forward left it (PREC != 0, query-stationary)
     const float* erow;     // [B*H][nq_pad]  row exponents e_i of the fp16 dO copy (row form only)
     float* dq_acc;         // fused kernel: fp32 dQ sums, [B*H][nq_pad/128] tiles of [D/4][128 rows][4]
     const int32_t* kv_len; // optional per-batch key counts
@@ -684,6 +685,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 my_nlse2 -= (float)e_i;            // -inf in the padding stays -inf
                 my_ndelta *= pow2i(e_i);
             }
+            // pairs: P = 2^((S scale - lse + bias) log2 e) 2^kPShift, the exponent's terms in this order because it is
+            // small wherever P is not, and the shift exact behind it.  With kPShift inside, the exponent was rounded at
+            // 14, and d(loss)/d(scores), an fp32 result, was up to 1.7 times further from float64.
+            if (PREC != 0) my_nlse2 = row_g < a.Nq ? -a.lse[((int64_t)b * a.H + head_x) * a.Nq + row_g] : -INFINITY;
         }
         // dS' = P' o (dP * tt_mul o Z + (-delta) * nd_mul): see "number formats" above
         const uint64_t ttm2 = f2_pack(sc.tt_mul, sc.tt_mul), ndm2 = f2_pack(sc.nd_mul, sc.nd_mul);
@@ -1081,16 +1086,18 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_st();
             } else {
                 const uint64_t neg2 = f2_pack(my_nlse2, my_nlse2);
+                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale);
+                [[maybe_unused]] constexpr float kShift = 16384.f;          // 2^kPShift
                 [[maybe_unused]] float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < CPT; c += 2) {
                     float x0, x1;
-                    f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), sc2, neg2), x0, x1);
+                    f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), PREC ? scn2 : sc2, neg2), x0, x1);
                     if constexpr (PREC == 2) {
                         // my row's 32 keys are the wg-th box, its 16-byte pieces swizzled by the row
                         if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4));
-                        PSET(c, ex2(fmaf((c & 2) ? bv.z : bv.x, kLog2e, x0)));
-                        PSET(c + 1, ex2(fmaf((c & 2) ? bv.w : bv.y, kLog2e, x1)));
+                        PSET(c, ex2((x0 + ((c & 2) ? bv.z : bv.x)) * kLog2e) * kShift);
+                        PSET(c + 1, ex2((x1 + ((c & 2) ? bv.w : bv.y)) * kLog2e) * kShift);
                         continue;
                     }
                     if constexpr (PREC == 1) {
@@ -1098,15 +1105,15 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             const float* bp = bias_h + (int64_t)(row_g < a.Nq ? row_g : a.Nq - 1) * a.bias_sn + col_g0 + c;
                             if (a.bias_vec && col_g0 + (c & ~3) + 4 <= a.Nk) {
                                 if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(bp);
-                                x0 = fmaf((c & 2) ? bv.z : bv.x, kLog2e, x0);
-                                x1 = fmaf((c & 2) ? bv.w : bv.y, kLog2e, x1);
+                                x0 += (c & 2) ? bv.z : bv.x;
+                                x1 += (c & 2) ? bv.w : bv.y;
                             } else {
-                                if (col_g0 + c < a.Nk) x0 = fmaf(bp[0], kLog2e, x0);
-                                if (col_g0 + c + 1 < a.Nk) x1 = fmaf(bp[1], kLog2e, x1);
+                                if (col_g0 + c < a.Nk) x0 += bp[0];
+                                if (col_g0 + c + 1 < a.Nk) x1 += bp[1];
                             }
                         }
-                        PSET(c, ex2(x0));
-                        PSET(c + 1, ex2(x1));
+                        PSET(c, ex2(x0 * kLog2e) * kShift);
+                        PSET(c + 1, ex2(x1 * kLog2e) * kShift);
                         continue;
                     }
                     // a quarter of the exponentials as a polynomial on the FMA pipes (this kernel keeps the
@@ -1558,6 +1565,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         set_error("cuTensorMapEncodeTiled failed for the bias (%d)", r);
         return FA_ECUDA;
     }
+    a.lse = p.lse;
     a.lse2 = lse2; a.delta = delta; a.ranges = ranges; a.dq_acc = dq_acc; a.status = p.status_word; a.wait_limit_ms = p.wait_limit_ms;
     a.erow = COPIES ? (const float*)(wsp + ws.erow_off) : nullptr;
     a.kv_len = p.kv_lengths;

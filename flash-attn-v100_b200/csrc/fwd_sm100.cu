@@ -759,7 +759,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
                     const int col0 = j * kBlockN;
                     if constexpr (PREC != 0) {
-                        // scores in the log2 domain, the bias added before the mask
+                        // scores in the log2 domain, the bias added before the mask (the small term is the one rounded)
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
                             if constexpr (PREC == 2) {
@@ -772,10 +772,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                                 for (int c = 0; c < 32; c += 4) {
                                     const float4 b4 = *reinterpret_cast<const float4*>(chunk + (((c >> 2) ^ (r & 7)) << 4));
-                                    SSET(q4 * 32 + c, fmaf(b4.x, kLog2e, SF(q4 * 32 + c) * a.scale_log2));
-                                    SSET(q4 * 32 + c + 1, fmaf(b4.y, kLog2e, SF(q4 * 32 + c + 1) * a.scale_log2));
-                                    SSET(q4 * 32 + c + 2, fmaf(b4.z, kLog2e, SF(q4 * 32 + c + 2) * a.scale_log2));
-                                    SSET(q4 * 32 + c + 3, fmaf(b4.w, kLog2e, SF(q4 * 32 + c + 3) * a.scale_log2));
+                                    SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b4.x * kLog2e));
+                                    SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale_log2, b4.y * kLog2e));
+                                    SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale_log2, b4.z * kLog2e));
+                                    SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale_log2, b4.w * kLog2e));
                                 }
                                 mbar_arrive_read_done(&bars[Cfg::kBiasEmpty + at]);
                                 if (++bias_slot == Cfg::kBiasSlots) { bias_slot = 0; bias_ph ^= 1u; }
@@ -788,16 +788,16 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                                     for (int c = 0; c < 32; c += 4) {
                                         const float4 b4 = *reinterpret_cast<const float4*>(bp + c);
-                                        SSET(q4 * 32 + c, fmaf(b4.x, kLog2e, SF(q4 * 32 + c) * a.scale_log2));
-                                        SSET(q4 * 32 + c + 1, fmaf(b4.y, kLog2e, SF(q4 * 32 + c + 1) * a.scale_log2));
-                                        SSET(q4 * 32 + c + 2, fmaf(b4.z, kLog2e, SF(q4 * 32 + c + 2) * a.scale_log2));
-                                        SSET(q4 * 32 + c + 3, fmaf(b4.w, kLog2e, SF(q4 * 32 + c + 3) * a.scale_log2));
+                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b4.x * kLog2e));
+                                        SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale_log2, b4.y * kLog2e));
+                                        SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale_log2, b4.z * kLog2e));
+                                        SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale_log2, b4.w * kLog2e));
                                     }
                                 } else {
 #pragma unroll
                                     for (int c = 0; c < 32; ++c) {
                                         const float b1 = col0 + q4 * 32 + c < a.Nk ? bp[c] : 0.f;
-                                        SSET(q4 * 32 + c, fmaf(b1, kLog2e, SF(q4 * 32 + c) * a.scale_log2));
+                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b1 * kLog2e));
                                     }
                                 }
                             }
