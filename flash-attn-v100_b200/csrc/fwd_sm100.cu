@@ -1331,7 +1331,8 @@ bool tensor_ok(const fa_b200_tensor& t, int64_t B, int64_t N, int64_t H) {
 // Which calls the tensor-core family covers.  `why` names the first reason it does not.
 bool sm100_supports(const fa_b200_params& p, bool backward, const char** why) {
     if (p.dtype == FA_B200_F32) {
-        // fp32: the forward has a tensor-core kernel (TF32 products taken three times); the backward is CUDA-core tiles
+        // fp32: the forward has a tensor-core kernel (TF32 products taken three times); the backward has one that AUTO
+        // takes when the caller offers scratch (sm100_f32_bwd_scratch_bytes), CUDA-core tiles otherwise
         if (backward) { *why = "the fp32 backward is served by the CUDA-core kernels"; return false; }
         return sm100_tf32_fwd_supports(p, why);
     }
