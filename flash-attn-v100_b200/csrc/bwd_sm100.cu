@@ -164,6 +164,7 @@ struct BwdArgs {
     int bias_vec;                  // its rows can be read as float4
     int bias_b, bias_h;            // PREC = 2: whether it has a batch / head dimension
     int ds_vec;                    // rows of d_scores can be written as float4
+    int ds_staged;                 // PREC = 2: d_scores leaves by TMA
     float* d_scores;               // optional dense (B, H, Nq, Nk) gradient of the scores (written by MODE 1)
 };
 
@@ -262,7 +263,8 @@ __global__ void __launch_bounds__(128 * NWG + kExtraThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                  const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_out1, const __grid_constant__ CUtensorMap map_out2,
-                 const __grid_constant__ CUtensorMap map_aux, const __grid_constant__ CUtensorMap map_bias, const BwdArgs a) {
+                 const __grid_constant__ CUtensorMap map_aux, const __grid_constant__ CUtensorMap map_bias,
+                 const __grid_constant__ CUtensorMap map_ds, const BwdArgs a) {
     using Cfg = BwdCfg<D, MODE, DROP, PREC>;
     constexpr bool KS = (MODE != 1);        // key-stationary: K, V stay, query tiles stream
     constexpr bool FUSED = (MODE == 2);     // key-stationary and dQ too
@@ -646,11 +648,20 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (elect_one()) {
             int qi = 0, hg = 0, done = 0;
             bool ok = true;
+            // dQ kernel: the threads leave d(loss)/d(scores) of a step in the place of its bias tile
+            auto store_ds = [&](int it) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (it * kTile + 32 * c < a.Nk) tma_store_4d(&map_ds, sBias + c * kBoxBytes, it * kTile + 32 * c, head_x, tile * kTile, b);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+            };
             for (int it = 0; it < n_iter; ++it) {
                 const int head = KS ? head_x * group + hg : head_x;
                 const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : it) * kTile;
                 ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)it & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
+                if (MODE == 1 && a.ds_staged && it > 0) store_ds(it - 1);
                 mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
@@ -659,6 +670,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 ++done;
                 if (++qi == n_per_head) { qi = 0; ++hg; }
             }
+            if (MODE == 1 && a.ds_staged && ok && n_iter > 0 && mbar_wait(&bars[Cfg::kBiasEmpty], (uint32_t)(n_iter - 1) & 1u, abort_flag))
+                store_ds(n_iter - 1);
             for (int spin = 0; !ok && spin < 4096 && done > 0 && !mbar_try_wait(&bars[Cfg::kBiasFull], (uint32_t)(done - 1) & 1u); ++spin) {}
         }
         __syncwarp();
@@ -1128,7 +1141,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         PSET(c + 1, ex2(x1));
                     }
                 }
-                if (PREC == 2) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
+                if (PREC == 2 && !a.ds_staged) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
                 const bool diag = a.causal && strm_tile * kTile + kTile - 1 > tile * kTile + a.shift;
                 if (diag || strm_tile * kTile + kTile > nk) {
                     // my row sees my first `seen` columns: keys below the count, at most row + shift
@@ -1208,7 +1221,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             const int e = (c4 - hf * (CPT / 8)) * 2;
                             pack2_pair<P_BF16>(d0, d1, pk[e], pl[e]);
                             pack2_pair<P_BF16>(d2v, d3, pk[e + 1], pl[e + 1]);
-                            if (ds_row && row_g < a.Nq) {
+                            if (PREC == 2 && a.ds_staged) {
+                                // ... by way of the bias tile's place (only I read these 16 bytes) and a TMA store: a
+                                // thread's own stores would go to 32 rows a warp
+                                *reinterpret_cast<float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4)) =
+                                    make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
+                            } else if (ds_row && row_g < a.Nq) {
                                 // d loss / d scores, the power of two of dS' taken out (exact)
                                 float* dst = ds_row + col_g0 + c;
                                 if (a.ds_vec) {
@@ -1242,6 +1260,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 if (FUSED) fence_proxy_async_smem();
                 tmem_wait_st();
+                if (PREC == 2 && MODE == 1 && a.ds_staged) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);     // (written, here)
             }
 #undef PF
 #undef PSET
@@ -1557,12 +1576,18 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
             return FA_ECUDA;
         }
     }
-    CUtensorMap mb = mq;
+    CUtensorMap mb = mq, mds = mq;
     BwdArgs a;
     a.bias_b = p.bias.stride_b != 0 && p.B > 1; a.bias_h = p.bias.stride_h != 0 && p.H > 1;
     if (PREC == 2 && (r = cached_tmap_bnhd(&mb, p.bias.ptr, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.bias_b ? p.B : 1, p.Nq, a.bias_h ? p.H : 1,
                                            p.Nk, p.bias.stride_b, p.bias.stride_n, p.bias.stride_h, 128, 32, 1))) {
         set_error("cuTensorMapEncodeTiled failed for the bias (%d)", r);
+        return FA_ECUDA;
+    }
+    a.ds_staged = PREC == 2 && p.d_scores && p.Nk % 4 == 0 && ((uintptr_t)p.d_scores & 15u) == 0;
+    if (a.ds_staged && (r = cached_tmap_bnhd(&mds, p.d_scores, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.B, p.Nq, p.H, p.Nk,
+                                             (int64_t)p.H * p.Nq * p.Nk, p.Nk, (int64_t)p.Nq * p.Nk, 128, 32, 1))) {
+        set_error("cuTensorMapEncodeTiled failed for d_scores (%d)", r);
         return FA_ECUDA;
     }
     a.lse = p.lse;
@@ -1609,7 +1634,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         const int smem2 = pick_smem<D, 2, PREC>(drop);
         FA_CUDA_CHECK(set_smem_limit_once(k2, smem2, p.device, &smem_done[6 + drop], &smem_mu));
         if (phases & 2) {
-            k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, mb, a);
+            k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, mb, mds, a);
             FA_CUDA_CHECK(cudaGetLastError());
         }
         if (phases & 4) {
@@ -1629,7 +1654,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     if (phases & 2) {
         // stationary K_j, V_j; streamed Q_i, dO_i (bf16 with copies: their fp16 copies; the kernel leaves
         // the fp16 copy of K behind for the dQ kernel)
-        k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, mb, a);
+        k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, mb, mds, a);
         FA_CUDA_CHECK(cudaGetLastError());
     }
     if (phases & 4) {
@@ -1646,7 +1671,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         // that the dK/dV kernel is still writing.
         cfg.numAttrs = (!COPIES && (phases & 2) && (int64_t)p.Nk * D * 4 <= (int64_t)tile::kBwdOverlapMaxKvBytes) ? 1 : 0;
         // stationary Q_i (its fp16 copy), dO_i; streamed K_j (its fp16 copy), V_j
-        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k1, mq16, mg, mk16, mv, mdq, mdq, mdq, mb, a));
+        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k1, mq16, mg, mk16, mv, mdq, mdq, mdq, mb, mds, a));
     }
     return FA_OK;
 }
