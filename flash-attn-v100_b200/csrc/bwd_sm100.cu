@@ -135,10 +135,9 @@ struct BwdCfg {
 };
 
 struct BwdArgs {
-    const float* lse2;     // [B*H][nq_pad]  kPShift - lse * log2(e), -inf in the padding
+    const float* lse2;     // [B*H][nq_pad]  kPShift - lse * log2(e), pairs: -lse; -inf in the padding
     const float* delta;    // [B*H][nq_pad]  -delta, 0 in the padding
     const float* ranges;   // [B*Hkv][2]     max |dO| over the column's query heads, max |V|
-    const float* lse;      // [B*H][Nq]      as the forward left it (PREC != 0, query-stationary)
     const float* erow;     // [B*H][nq_pad]  row exponents e_i of the fp16 dO copy (row form only)
     float* dq_acc;         // fused kernel: fp32 dQ sums, [B*H][nq_pad/128] tiles of [D/4][128 rows][4]
     const int32_t* kv_len; // optional per-batch key counts
@@ -698,10 +697,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 my_nlse2 -= (float)e_i;            // -inf in the padding stays -inf
                 my_ndelta *= pow2i(e_i);
             }
-            // pairs: P = 2^((S scale - lse + bias) log2 e) 2^kPShift, the exponent's terms in this order because it is
-            // small wherever P is not, and the shift exact behind it.  With kPShift inside, the exponent was rounded at
-            // 14, and d(loss)/d(scores), an fp32 result, was up to 1.7 times further from float64.
-            if (PREC != 0) my_nlse2 = row_g < a.Nq ? -a.lse[((int64_t)b * a.H + head_x) * a.Nq + row_g] : -INFINITY;
+            // pairs: P = 2^((S scale + bias - lse) log2 e) 2^kPShift with the terms in the forward's order, so that a mask
+            // of the type's lowest value or of -1e9 leaves in both what its rounding leaves (the difference is small
+            // wherever P is not), and the shift exact behind it: d(loss)/d(scores) is an fp32 result.
         }
         // dS' = P' o (dP * tt_mul o Z + (-delta) * nd_mul): see "number formats" above
         const uint64_t ttm2 = f2_pack(sc.tt_mul, sc.tt_mul), ndm2 = f2_pack(sc.nd_mul, sc.nd_mul);
@@ -867,7 +865,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 kbits |= (((uint32_t)mbuf[col * 8 + (row >> 4)] >> (row & 15)) & 1u) << (16 * h + 4 * j + 2 * k + e);
                             }
             }
-            const uint64_t sc2 = f2_pack(a.scale_log2, a.scale_log2);
+            const float sc1 = PREC ? a.scale : a.scale_log2;
+            const uint64_t sc2 = f2_pack(sc1, sc1);
             // key row > query column + shift is hidden: only tiles the mask's edge crosses need the test
             const bool diag = a.causal && strm_tile * kTile + a.shift < tile * kTile + kTile - 1;
             const bool tail = tile * kTile + kTile > nk;            // the tile holds padding keys
@@ -895,21 +894,27 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         for (int k = 0; k < 2; ++k) {
                             const int i0 = 4 * j + 2 * k;
                             float x0, x1;
-                            f2_unpack(f2_fma(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), sc2, L), x0, x1);
+                            uint64_t add = L;                  // pairs with a bias: the bias first, in natural units, then -lse
+                            float b0 = 0.f, b1 = 0.f;
                             if constexpr (PREC == 2) {
                                 // bias[query][key] from the tile: eight keys (two 16-byte pieces) of four queries a load,
                                 // which the swizzle spreads over all banks
                                 const int kk = lr + 16 * h + 8 * k;
                                 const uint8_t* bp = sBias + (warp & 3) * kBoxBytes + (cb + 8 * j + 2 * lq) * 128 + (kk & 3) * 4;
-                                x0 = fmaf(*reinterpret_cast<const float*>(bp + (((kk >> 2) ^ (2 * lq)) << 4)), kLog2e, x0);
-                                x1 = fmaf(*reinterpret_cast<const float*>(bp + 128 + (((kk >> 2) ^ (2 * lq + 1)) << 4)), kLog2e, x1);
+                                b0 = *reinterpret_cast<const float*>(bp + (((kk >> 2) ^ (2 * lq)) << 4));
+                                b1 = *reinterpret_cast<const float*>(bp + 128 + (((kk >> 2) ^ (2 * lq + 1)) << 4));
                             } else if (PREC && a.bias) {
                                 // bias[query][key]: eight lanes read eight neighbouring keys of one query
                                 const int key = tile * kTile + rbase + 16 * h + 8 * k, qr = col_g0 + 8 * j + 2 * lq;
                                 const float* bp = bias_h + (int64_t)qr * a.bias_sn + key;
-                                if (key < a.Nk && qr < a.Nq) x0 = fmaf(bp[0], kLog2e, x0);
-                                if (key < a.Nk && qr + 1 < a.Nq) x1 = fmaf(bp[a.bias_sn], kLog2e, x1);
+                                if (key < a.Nk && qr < a.Nq) b0 = bp[0];
+                                if (key < a.Nk && qr + 1 < a.Nq) b1 = bp[a.bias_sn];
                             }
+                            if (PREC == 2 || (PREC == 1 && a.bias)) add = f2_pack(b0, b1);
+                            uint64_t x = f2_fma(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), sc2, add);
+                            if (PREC == 2 || (PREC == 1 && a.bias)) x = f2_add(x, L);
+                            if (PREC) x = f2_fma(x, f2_pack(kLog2e, kLog2e), f2_pack(kPShift, kPShift));
+                            f2_unpack(x, x0, x1);
                             pf[h][i0] = __float_as_uint(ex2(x0));
                             pf[h][i0 + 1] = __float_as_uint(ex2(x1));
                         }
@@ -1099,36 +1104,43 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_st();
             } else {
                 const uint64_t neg2 = f2_pack(my_nlse2, my_nlse2);
-                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale);
-                [[maybe_unused]] constexpr float kShift = 16384.f;          // 2^kPShift
+                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(16384.f, 16384.f);
                 [[maybe_unused]] float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < CPT; c += 2) {
                     float x0, x1;
-                    f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), PREC ? scn2 : sc2, neg2), x0, x1);
-                    if constexpr (PREC == 2) {
-                        // my row's 32 keys are the wg-th box, its 16-byte pieces swizzled by the row
-                        if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4));
-                        PSET(c, ex2((x0 + ((c & 2) ? bv.z : bv.x)) * kLog2e) * kShift);
-                        PSET(c + 1, ex2((x1 + ((c & 2) ? bv.w : bv.y)) * kLog2e) * kShift);
-                        continue;
-                    }
-                    if constexpr (PREC == 1) {
-                        if (a.bias) {
-                            const float* bp = bias_h + (int64_t)(row_g < a.Nq ? row_g : a.Nq - 1) * a.bias_sn + col_g0 + c;
-                            if (a.bias_vec && col_g0 + (c & ~3) + 4 <= a.Nk) {
-                                if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(bp);
-                                x0 += (c & 2) ? bv.z : bv.x;
-                                x1 += (c & 2) ? bv.w : bv.y;
+                    if constexpr (PREC != 0) {
+                        const uint64_t s2 = f2_pack(PF(c), PF(c + 1));
+                        uint64_t x;
+                        if (PREC == 2 || a.bias) {
+                            float b0 = 0.f, b1 = 0.f;
+                            if constexpr (PREC == 2) {
+                                // my row's 32 keys are the wg-th box, its 16-byte pieces swizzled by the row
+                                if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4));
+                                b0 = (c & 2) ? bv.z : bv.x;
+                                b1 = (c & 2) ? bv.w : bv.y;
                             } else {
-                                if (col_g0 + c < a.Nk) x0 += bp[0];
-                                if (col_g0 + c + 1 < a.Nk) x1 += bp[1];
+                                const float* bp = bias_h + (int64_t)(row_g < a.Nq ? row_g : a.Nq - 1) * a.bias_sn + col_g0 + c;
+                                if (a.bias_vec && col_g0 + (c & ~3) + 4 <= a.Nk) {
+                                    if ((c & 3) == 0) bv = *reinterpret_cast<const float4*>(bp);
+                                    b0 = (c & 2) ? bv.z : bv.x;
+                                    b1 = (c & 2) ? bv.w : bv.y;
+                                } else {
+                                    if (col_g0 + c < a.Nk) b0 = bp[0];
+                                    if (col_g0 + c + 1 < a.Nk) b1 = bp[1];
+                                }
                             }
+                            x = f2_add(f2_fma(s2, scn2, f2_pack(b0, b1)), neg2);
+                        } else {
+                            x = f2_fma(s2, scn2, neg2);
                         }
-                        PSET(c, ex2(x0 * kLog2e) * kShift);
-                        PSET(c + 1, ex2(x1 * kLog2e) * kShift);
+                        f2_unpack(f2_mul(x, log2e2), x0, x1);
+                        f2_unpack(f2_mul(f2_pack(ex2(x0), ex2(x1)), up2), x0, x1);
+                        PSET(c, x0);
+                        PSET(c + 1, x1);
                         continue;
                     }
+                    f2_unpack(f2_fma(f2_pack(PF(c), PF(c + 1)), sc2, neg2), x0, x1);
                     // a quarter of the exponentials as a polynomial on the FMA pipes (this kernel keeps the
                     // special-function unit busiest; measured 0.7 % over the backward, half: 0.2 %)
                     if (((c >> 1) & 3) == 0) {
@@ -1375,6 +1387,7 @@ struct PreprocessCopies {
     const void* o_lo; int64_t l_sb, l_sn, l_sh;     // optional residual of O (any dtype)
     const void* q; int64_t q_sb, q_sn, q_sh;
     uint16_t* q16; uint16_t* do16; float* erow;
+    int pairs;                                      // PREC != 0: -lse instead of kPShift - lse*log2(e)
 };
 // A head size below D (pair instances) leaves the lanes beyond it idle.
 template <typename T, int D, bool COPIES>
@@ -1455,7 +1468,7 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
             }
         }
         if (sub == 0) {
-            if (in) { delta[row] = -s * pow2i(-e_i); lse2[row] = kPShift - lse[bh * Nq + i] * kLog2e + (float)e_i; }
+            if (in) { delta[row] = -s * pow2i(-e_i); lse2[row] = cp.pairs ? -lse[bh * Nq + i] : kPShift - lse[bh * Nq + i] * kLog2e + (float)e_i; }
             else    { delta[row] = 0.f; lse2[row] = -INFINITY; }
             if (COPIES) cp.erow[row] = in ? (float)e_i : 0.f;
         }
@@ -1538,6 +1551,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         if (n_blocks > 0x7fffffff) { set_error("problem too large for the preprocess grid"); return FA_EUNSUPPORTED; }
         const int n_row_blocks = (int)n_row_blocks64;
         PreprocessCopies cp = {};
+        cp.pairs = PREC != 0;
         cp.o_lo = p.o_lo.ptr; cp.l_sb = p.o_lo.stride_b; cp.l_sn = p.o_lo.stride_n; cp.l_sh = p.o_lo.stride_h;
         if (COPIES) {
             cp.q = p.q.ptr; cp.q_sb = p.q.stride_b; cp.q_sn = p.q.stride_n; cp.q_sh = p.q.stride_h;
@@ -1590,7 +1604,6 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         set_error("cuTensorMapEncodeTiled failed for d_scores (%d)", r);
         return FA_ECUDA;
     }
-    a.lse = p.lse;
     a.lse2 = lse2; a.delta = delta; a.ranges = ranges; a.dq_acc = dq_acc; a.status = p.status_word; a.wait_limit_ms = p.wait_limit_ms;
     a.erow = COPIES ? (const float*)(wsp + ws.erow_off) : nullptr;
     a.kv_len = p.kv_lengths;

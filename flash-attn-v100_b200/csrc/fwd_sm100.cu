@@ -135,7 +135,8 @@ struct FwdArgs {
     int items_per_head;            // causal: ceil(n_pairs / 2) mirrored items; else n_pairs
     int n_items;                   // items_per_head * B * H
     int wait_limit_ms;             // limit of one mbarrier wait (0: the default)
-    float scale_log2;              // scale * log2(e)
+    float scale_log2;
+    float scale;                   // PREC != 0: scores stay in natural units              // scale * log2(e)
     uint32_t drop_thr;
     float inv_keep;
     PhiloxKey key;
@@ -341,6 +342,7 @@ template <> struct SoftmaxLoop<2> : SplitSoftmaxLoop { using SplitSoftmaxLoop::S
 // P is stored as 2^(S c - m + kPShift): with the lazily refreshed maximum P <= 2^8, so the shifted value
 // stays below 2^14 in fp16 and entries down to 2^-20 of the row's largest keep full precision.
 constexpr float kPShift = 6.0f;
+constexpr float kPScale = 64.0f;            // 2^kPShift
 
 // DROP: 0 no dropout; 1 the keep bits are drawn here, by the softmax threads (no workspace);
 // 2 they are loaded from the workspace, where dropout_bits_kernel has written the call's bits.
@@ -759,7 +761,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
                     const int col0 = j * kBlockN;
                     if constexpr (PREC != 0) {
-                        // scores in the log2 domain, the bias added before the mask (the small term is the one rounded)
+                        // Scores in natural units, the bias added as it is and before the mask: masks of the type's lowest
+                        // value, of -1e9 or of its largest have to keep x - m (and, in the backward, x - lse) what the
+                        // subtraction gives, and bias * log2 e overflows or is rounded by more than a whole unit there.
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
                             if constexpr (PREC == 2) {
@@ -772,32 +776,32 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                                 for (int c = 0; c < 32; c += 4) {
                                     const float4 b4 = *reinterpret_cast<const float4*>(chunk + (((c >> 2) ^ (r & 7)) << 4));
-                                    SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b4.x * kLog2e));
-                                    SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale_log2, b4.y * kLog2e));
-                                    SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale_log2, b4.z * kLog2e));
-                                    SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale_log2, b4.w * kLog2e));
+                                    SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale, b4.x));
+                                    SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale, b4.y));
+                                    SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale, b4.z));
+                                    SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale, b4.w));
                                 }
                                 mbar_arrive_read_done(&bars[Cfg::kBiasEmpty + at]);
                                 if (++bias_slot == Cfg::kBiasSlots) { bias_slot = 0; bias_ph ^= 1u; }
                             } else if (!a.bias) {
 #pragma unroll
-                                for (int c = 0; c < 32; ++c) SSET(q4 * 32 + c, SF(q4 * 32 + c) * a.scale_log2);
+                                for (int c = 0; c < 32; ++c) SSET(q4 * 32 + c, SF(q4 * 32 + c) * a.scale);
                             } else {
                                 const float* bp = brow + col0 + q4 * 32;
                                 if (a.bias_vec && col0 + q4 * 32 + 32 <= a.Nk) {
 #pragma unroll
                                     for (int c = 0; c < 32; c += 4) {
                                         const float4 b4 = *reinterpret_cast<const float4*>(bp + c);
-                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b4.x * kLog2e));
-                                        SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale_log2, b4.y * kLog2e));
-                                        SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale_log2, b4.z * kLog2e));
-                                        SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale_log2, b4.w * kLog2e));
+                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale, b4.x));
+                                        SSET(q4 * 32 + c + 1, fmaf(SF(q4 * 32 + c + 1), a.scale, b4.y));
+                                        SSET(q4 * 32 + c + 2, fmaf(SF(q4 * 32 + c + 2), a.scale, b4.z));
+                                        SSET(q4 * 32 + c + 3, fmaf(SF(q4 * 32 + c + 3), a.scale, b4.w));
                                     }
                                 } else {
 #pragma unroll
                                     for (int c = 0; c < 32; ++c) {
                                         const float b1 = col0 + q4 * 32 + c < a.Nk ? bp[c] : 0.f;
-                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale_log2, b1 * kLog2e));
+                                        SSET(q4 * 32 + c, fmaf(SF(q4 * 32 + c), a.scale, b1));
                                     }
                                 }
                             }
@@ -821,10 +825,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     }
                     const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * (PREC ? 1.f : a.scale_log2);
                     const float m_new = fmaxf(m, mx);
-                    const bool grow = (m_new - m) > kRescaleThreshold;   // first block: inf > 8
+                    const bool grow = (m_new - m) > (PREC ? kRescaleThreshold * kLn2 : kRescaleThreshold);   // first block: inf > 8
                     if (__any_sync(0xffffffffu, grow)) {
                         // 0 on the first block; a row may have seen nothing but -inf so far (a bias; a stretch of a pair)
-                        const float alpha = ((PREC || FREE) && m_new == -INFINITY) ? 0.f : ex2(m - m_new);
+                        const float alpha = ((PREC || FREE) && m_new == -INFINITY) ? 0.f : ex2(PREC ? (m - m_new) * kLog2e : m - m_new);
                         m = m_new;
                         l *= alpha;
                         if (j > first) {
@@ -841,9 +845,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                     if constexpr (PREC != 0) {
-                        // P = 2^(x - m) as hi + lo.  A row that has seen only -inf so far keeps m = -inf; 0 in its
-                        // place lets its P come out as 0.
-                        const float ms = kPShift - (m == -INFINITY ? 0.f : m);
+                        // P = e^(x - m) 2^kPShift as hi + lo, base 2 and the shift behind the difference, which is small
+                        // where P is not.  A row that has seen only -inf so far keeps m = -inf; 0 in its place lets its
+                        // P come out as 0.
+                        const float nm = m == -INFINITY ? 0.f : -m;
+                        const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale);
                         float l0 = 0.f, l1 = 0.f;
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
@@ -856,7 +862,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
                             for (int cc = 0; cc < 32; cc += 2) {
                                 const int c = q4 * 32 + cc;
-                                float p0 = ex2(SF(c) + ms), p1 = ex2(SF(c + 1) + ms);
+                                float p0, p1;
+                                f2_unpack(f2_mul(f2_add(f2_pack(SF(c), SF(c + 1)), nm2), log2e2), p0, p1);
+                                f2_unpack(f2_mul(f2_pack(ex2(p0), ex2(p1)), up2), p0, p1);
                                 l0 += p0; l1 += p1;
                                 if constexpr (DROP == 2) {
                                     const uint32_t word = q4 == 0 ? kb4.x : (q4 == 1 ? kb4.y : (q4 == 2 ? kb4.z : kb4.w));
@@ -1071,7 +1079,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                 }
-                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = kLn2 * ((m - kPShift) + log2f(l));
+                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = PREC ? fmaf(kLn2, log2f(l) - kPShift, m) : kLn2 * ((m - kPShift) + log2f(l));
                 // the O_t reads above are complete (wait::ld); the next pair's first PV_t MMA waits for
                 // this warpgroup's next P_t, so it cannot overwrite O_t earlier
             }
@@ -1262,6 +1270,7 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
     if (n_items > 0x7fffffff - 65536) { set_error("too many work items"); return FA_EUNSUPPORTED; }
     a.n_items = (int)n_items;
     a.scale_log2 = p.scale * kLog2e;
+    a.scale = p.scale;
     a.d = d;
     a.bias = (const float*)p.bias.ptr;
     a.bias_sb = p.bias.stride_b; a.bias_sn = p.bias.stride_n; a.bias_sh = p.bias.stride_h;

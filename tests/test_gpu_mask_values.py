@@ -1,0 +1,53 @@
+"""Additive masks of large finite values on the tensor-core kernels: the lowest (and largest) values of a type and -1e9,
+where multiplying the bias by log2(e) overflows or is rounded by more than a unit.
+
+A row all of whose keys carry such a value is uniform over them (its scores vanish in the rounding of score + bias), as
+on the CUDA-core tiles and in torch.  Both kernel families round that sum alike, so they have to agree to the rounding
+of the 16-bit results (tolerances of test_gpu_pair_kernels); d(loss)/d(scores) and lse are fp32.
+"""
+import pytest
+import torch
+
+import flash_attention_v100 as fa
+from flash_attention_v100.ops.attention import launch_backward, launch_forward
+from test_gpu_pair_kernels import TOL, _rand, _rel
+
+pytestmark = pytest.mark.gpu
+VALUES = {"fp32-min": torch.finfo(torch.float32).min, "bf16-min": torch.finfo(torch.bfloat16).min, "fp32-max": torch.finfo(torch.float32).max,
+          "-1e9": -1e9, "-1e4": -1e4}
+
+
+def _masked(form, value, H, Nq, Nk):
+    if form == "padding":                       # (B, 1, 1, Nk): the second batch entry has no key at all
+        bias = torch.zeros(2, 1, 1, Nk)
+        bias[0, ..., Nk - 20:] = value
+        bias[1] = value
+        return bias
+    bias = _rand((1, H, Nq, Nk), torch.float32, 9)
+    if form == "rows":
+        bias[:, :, 7::50] = value               # whole rows among ordinary ones
+    else:
+        bias[..., :30] = value                  # left padding: with a causal mask the first rows see nothing else
+    return bias
+
+
+def _run(q, k, v, g, bias, causal):
+    scale = q.shape[3] ** -0.5
+    o, lse = launch_forward(q, k, v, scale, causal, bias=bias)
+    ds = torch.zeros(q.shape[0], q.shape[2], q.shape[1], k.shape[1], device=q.device)
+    return dict(zip(("o", "lse", "ds", "dq", "dk", "dv"), (o, lse, ds, *launch_backward(g, q, k, v, o, lse, scale, causal, bias=bias, d_scores=ds))))
+
+
+@pytest.mark.parametrize("value", VALUES)
+@pytest.mark.parametrize("form,causal", [("rows", False), ("rows", True), ("left", True), ("padding", False)])
+@pytest.mark.parametrize("dtype,D,N", [(torch.bfloat16, 64, 200), (torch.float16, 64, 201), (torch.bfloat16, 128, 260), (torch.float16, 96, 132)],
+                         ids=["bf16-d64", "fp16-d64-direct", "bf16-d128", "fp16-d96"])
+def test_as_on_the_cuda_cores(device, dtype, D, N, form, causal, value):
+    q, k, v, g = (_rand((2, N, 2, D), dtype, s).to(device) for s in range(4))
+    bias = _masked(form, VALUES[value], 2, N, N).to(device)
+    with fa.kernel_variant("simt"):
+        want = _run(q, k, v, g, bias, causal)
+    got = _run(q, k, v, g, bias, causal)
+    for n in want:
+        assert torch.isfinite(want[n]).all() and torch.isfinite(got[n]).all(), n
+        assert _rel(got[n], want[n]) <= TOL[dtype], (n, _rel(got[n], want[n]))
