@@ -40,9 +40,12 @@ inline int make_tmap_bnhd(CUtensorMap* map, const void* ptr, CUtensorMapDataType
                           int box_rows, int box_cols, int swizzle, int box_heads = 1) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return -1;
-    // size-1 dimensions may carry arbitrary strides in a tensor view: give them a legal one
-    if (H == 1) sh = D;
-    if (N == 1) sn = (sh * H > D ? sh * H : D);
+    // size-1 dimensions may carry arbitrary strides in a tensor view: give them a legal one, whole 16-byte pieces (D is
+    // any number of elements where the map is over a bias, whose rows are keys)
+    const int64_t piece = elem_bytes < 16 ? 16 / (int64_t)elem_bytes : 1;
+    const int64_t row = (D + piece - 1) / piece * piece;
+    if (H == 1) sh = row;
+    if (N == 1) sn = (sh * H > row ? sh * H : row);
     if (B == 1) sb = sn * N;
     cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)N, (cuuint64_t)B};
     cuuint64_t strides[3] = {(cuuint64_t)(sh * elem_bytes), (cuuint64_t)(sn * elem_bytes),

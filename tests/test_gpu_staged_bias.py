@@ -63,3 +63,24 @@ def test_bias_views(device):
         got = (o, lse, ds, *launch_backward(g, q, k, v, o, lse, 0.125, False, bias=bias, d_scores=ds))
         want = want or got
         assert all(_rel(a, b) <= TOL[torch.float16] for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("Nk", [197, 129, 3])
+@pytest.mark.parametrize("shape,H", [((1, 1), 2), ((2, 1), 2), ((2, 1), 1), ((1, 1), 1), ((2, 2), 2)])
+def test_masks_cut_out_of_wider_rows(device, D, Nk, shape, H):
+    """mask[..., :Nq, :Nk] of a buffer whose rows are a multiple of 16 bytes apart while Nk is none, with dimensions of
+    size one in front.  The same values in rows TMA cannot address take the direct loads: equal bit for bit."""
+    Nq, dtype = 130, torch.bfloat16
+    q, g = (_rand((2, Nq, H, D), dtype, s).to(device) for s in (1, 2))
+    k, v = (_rand((2, Nk, H, D), dtype, s).to(device) for s in (3, 4))
+    values = _rand((*shape, Nq, Nk), torch.float32, 5).to(device)
+
+    def run(pitch):
+        wide = torch.full((*shape, Nq + 7, pitch), 100.0, device=device)
+        wide[:, :, :Nq, :Nk] = values
+        bias = wide[:, :, :Nq, :Nk]
+        o, lse = launch_forward(q, k, v, D ** -0.5, False, bias=bias)
+        ds = torch.zeros(2, H, Nq, Nk, device=device)
+        return (o, lse, ds, *launch_backward(g, q, k, v, o, lse, D ** -0.5, False, bias=bias, d_scores=ds))
+    assert all(torch.equal(a, b) for a, b in zip(run(200), run(201)))
