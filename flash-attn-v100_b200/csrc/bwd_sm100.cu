@@ -870,6 +870,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             // key row > query column + shift is hidden: only tiles the mask's edge crosses need the test
             const bool diag = a.causal && strm_tile * kTile + a.shift < tile * kTile + kTile - 1;
             const bool tail = tile * kTile + kTile > nk;            // the tile holds padding keys
+            // query columns below `lim` do not see a key row: all of them for a
+            // padding key, those with column + shift < row under the mask's edge
+            auto hidden_below = [&](int h, int k) {
+                const int row_k = tile * kTile + rbase + 16 * h + 8 * k;
+                return (tail && row_k >= nk) ? 0x7fffffff : (diag ? row_k - a.shift : -0x7fffffff);
+            };
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 uint32_t pk[2][4], pl[2][4];                        // [h][2j' + k], j' = j - 2hf; pairs: the low parts
@@ -929,11 +935,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
                             for (int k = 0; k < 2; ++k) {
                                 const int j = 2 * hf + jj, i0 = 4 * j + 2 * k;
-                                const int row_k = tile * kTile + rbase + 16 * h + 8 * k;
-                                const int col = col_g0 + 8 * j + 2 * lq;
-                                // query columns below `lim` do not see this key row: all of them for a
-                                // padding key, those with column + shift < row under the mask's edge
-                                const int lim = (tail && row_k >= nk) ? 0x7fffffff : (diag ? row_k - a.shift : -0x7fffffff);
+                                const int col = col_g0 + 8 * j + 2 * lq, lim = hidden_below(h, k);
                                 if (col < lim) pf[h][i0] = 0u;
                                 if (col + 1 < lim) pf[h][i0 + 1] = 0u;
                             }
@@ -1006,6 +1008,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 }
                                 float d0, d1;
                                 f2_unpack(f2_mul(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), tt), d0, d1);
+                                if (PREC && (diag || tail)) {       // as in the other kernel: none, not 0 times what delta is
+                                    const int col = col_g0 + 8 * j + 2 * lq, lim = hidden_below(h, k);
+                                    if (col < lim) d0 = 0.f;
+                                    if (col + 1 < lim) d1 = 0.f;
+                                }
                                 if (PREC) pack2_pair<P_BF16>(d0, d1, pk[h][2 * jj + k], pl[h][2 * jj + k]);
                                 else      pk[h][2 * jj + k] = pack2<false>(d0, d1);
                             }
@@ -1050,6 +1057,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 mbar_arrive_warp(&bars[Cfg::kPReady]);
             }
             const uint64_t sc2 = f2_pack(a.scale_log2, a.scale_log2);
+            [[maybe_unused]] int seen = CPT;           // pairs, query-stationary: my first columns that my row sees
             if (KS) {
                 // P = 2^(S*c - lse): the staged vector holds -lse*log2(e), two columns per 64-bit word.
                 // Two halves of CPT / 2 columns: the first is packed, stored to TMEM and handed to the
@@ -1157,7 +1165,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const bool diag = a.causal && strm_tile * kTile + kTile - 1 > tile * kTile + a.shift;
                 if (diag || strm_tile * kTile + kTile > nk) {
                     // my row sees my first `seen` columns: keys below the count, at most row + shift
-                    int seen = nk - col_g0;
+                    seen = nk - col_g0;
                     if (diag && row_g + a.shift + 1 - col_g0 < seen) seen = row_g + a.shift + 1 - col_g0;
 #pragma unroll
                     for (int c = 0; c < CPT; ++c)
@@ -1230,6 +1238,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         f2_unpack(f2_mul(f2_pack(PF(c), PF(c + 1)), ta), d0, d1);
                         f2_unpack(f2_mul(f2_pack(PF(c + 2), PF(c + 3)), tb), d2v, d3);
                         if constexpr (PREC != 0) {
+                            // a hidden score has no gradient, also where delta or dP is no number (0 times that is none)
+                            if (seen < CPT) {
+                                if (c >= seen) d0 = 0.f;
+                                if (c + 1 >= seen) d1 = 0.f;
+                                if (c + 2 >= seen) d2v = 0.f;
+                                if (c + 3 >= seen) d3 = 0.f;
+                            }
                             const int e = (c4 - hf * (CPT / 8)) * 2;
                             pack2_pair<P_BF16>(d0, d1, pk[e], pl[e]);
                             pack2_pair<P_BF16>(d2v, d3, pk[e + 1], pl[e + 1]);

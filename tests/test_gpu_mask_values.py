@@ -51,3 +51,19 @@ def test_as_on_the_cuda_cores(device, dtype, D, N, form, causal, value):
     for n in want:
         assert torch.isfinite(want[n]).all() and torch.isfinite(got[n]).all(), n
         assert _rel(got[n], want[n]) <= TOL[dtype], (n, _rel(got[n], want[n]))
+
+
+@pytest.mark.parametrize("dtype,D,N", [(torch.bfloat16, 64, 200), (torch.float16, 64, 201), (torch.bfloat16, 128, 260), (torch.float16, 96, 132)],
+                         ids=["bf16-d64", "fp16-d64-direct", "bf16-d128", "fp16-d96"])
+@pytest.mark.parametrize("row", [float("-inf"), float("nan")], ids=["-inf", "nan"])
+def test_a_row_without_a_result_has_no_gradient_where_it_sees_nothing(device, dtype, D, N, row):
+    """Under a causal mask d(loss)/d(scores) of a row that is no number stays zero beyond the diagonal (which the sum over
+    a broadcast bias' batch would spread to other entries), and dK of keys no such row sees stays a number."""
+    q, k, v, g = (_rand((2, N, 2, D), dtype, s).to(device) for s in range(4))
+    bias = _rand((1, 2, N, N), torch.float32, 9).to(device)
+    bias[:, :, 70] = row
+    with fa.kernel_variant("simt"):
+        want = _run(q, k, v, g, bias, True)
+    got = _run(q, k, v, g, bias, True)
+    assert (got["ds"][:, :, 70, 71:] == 0).all() and torch.equal(torch.isnan(got["ds"]), torch.isnan(want["ds"]))
+    assert torch.isfinite(got["dk"][:, 71:]).all()
