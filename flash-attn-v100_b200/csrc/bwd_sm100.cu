@@ -210,6 +210,7 @@ __device__ __forceinline__ float pow2i(int e) {
 }
 // How dO reaches the key-stationary kernels' MMAs, which decides where its normalisation sits:
 //   kDoAsIs     fp16 inputs: dO is used as it is
+//   kDoPairs    bf16 as hi + lo pairs: dO is used as it is, and neither P nor dS needs a scale
 //   kDoInline   bf16, converted tile by tile inside the kernel: one factor 2^-e_col for the whole column
 //   kDoRowCopy  bf16, converted once by the preprocess launch into an fp16 copy, every row by its own
 //               2^-e_i (the column's maximum is not known while the copy is written); the staged vectors
@@ -217,21 +218,41 @@ __device__ __forceinline__ float pow2i(int e) {
 // With e_col = (bound of the column's max |dO|) - 15 the constants below are the same in the last two
 // forms except for l_add and nd_mul.  The query-stationary kernel multiplies the bf16 dO itself
 // (kDoAsIs arithmetic; it undoes e_i in its per-row scalars when the vectors are in the row form).
-enum DoForm { kDoAsIs = 0, kDoInline = 1, kDoRowCopy = 2 };
+enum DoForm { kDoAsIs = 0, kDoInline = 1, kDoRowCopy = 2, kDoPairs = 3 };
 __device__ __forceinline__ BwdScales make_scales(const float* rng, int D, float inv_keep, float scale, DoForm form) {
     const int k_do = log2_bound(rng[0]), k_v = log2_bound(rng[1]);
-    const int e_col = form == kDoAsIs ? 0 : k_do - 15;
-    const int g = 15 - (k_do + k_v + (D > 64 ? 8 : 7) + log2_bound(inv_keep));
+    const int e_col = (form == kDoAsIs || form == kDoPairs) ? 0 : k_do - 15;
+    // pairs of bf16 have fp32's exponents; elsewhere the factors are whole only within the exponents of normal numbers
+    int g = form == kDoPairs ? 0 : 15 - (k_do + k_v + (D > 64 ? 8 : 7) + log2_bound(inv_keep));
+    if (form == kDoAsIs) g = g < -112 ? -112 : (g > 126 ? 126 : g);
     BwdScales sc;
-    sc.tt_mul = pow2i(g - (int)kPShift + e_col);
-    sc.nd_mul = pow2i(g - (int)kPShift + (form == kDoRowCopy ? e_col : 0));
+    const int up = form == kDoPairs ? 0 : (int)kPShift;       // P' = P * 2^up
+    sc.tt_mul = pow2i(g - up + e_col);
+    sc.nd_mul = pow2i(g - up + (form == kDoRowCopy ? e_col : 0));
     sc.l_add = form == kDoRowCopy ? (float)(-e_col) : 0.f;
     sc.acc1_mul = scale * pow2i(-g);
-    sc.acc2_mul = inv_keep * pow2i(e_col - (int)kPShift);
+    sc.acc2_mul = inv_keep * pow2i(e_col - up);
     sc.do_mul = pow2i(-e_col);
     return sc;
 }
 
+// Largest magnitude among the eight 16-bit values of a 16-byte piece, folded into a running maximum
+// of magnitude bit patterns (two per word; for fp16 and bf16 alike a larger magnitude is a larger
+// unsigned pattern).
+__device__ __forceinline__ uint32_t absmax16_acc(uint32_t m, const uint4& v) {
+    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.x & 0x7FFF7FFFu));
+    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.y & 0x7FFF7FFFu));
+    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.z & 0x7FFF7FFFu));
+    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.w & 0x7FFF7FFFu));
+    return m;
+}
+// Pairs: the magnitudes of a 16-byte piece that holds an infinity or a NaN are left out.  Such a row's results are no
+// numbers whatever the scale; as the column's maximum it pushed the scale of every other row out of range.
+template <typename T>
+__device__ __forceinline__ uint32_t finite_piece(uint32_t m) {
+    constexpr uint32_t inf = std::is_same<T, __half>::value ? 0x7C00u : 0x7F80u;
+    return max(m & 0xFFFFu, m >> 16) < inf ? m : 0u;
+}
 // Which (tile, head, batch) a CTA works on.  The grid is (tiles, heads, batch) and CTAs start in the
 // order of their linear index.  Under a causal mask tiles cost between 1 and `tiles` steps, so the
 // order decides how evenly the SMs finish: the (batch, head) columns are taken in groups of
@@ -375,8 +396,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // fused kernel: the per-step dQ tile has columns of its own when D = 64 and shares T2's when D = 128
     constexpr bool kDqAliasesT2 = (D > 64);
     const uint32_t tDq = kDqAliasesT2 ? tT2 : tmem + 448u;
-    const BwdScales sc = make_scales(a.ranges + 2 * ((int64_t)b * a.Hkv + head_kv), D, a.inv_keep, a.scale,
-                                     !(CONV && KS) ? kDoAsIs : (INLINE ? kDoInline : kDoRowCopy));
+    const float* col_range = a.ranges + 2 * ((int64_t)b * a.Hkv + head_kv);
+    BwdScales sc = make_scales(col_range, D, a.inv_keep, a.scale,
+                               P_BF16 ? kDoPairs : (!(CONV && KS) ? kDoAsIs : (INLINE ? kDoInline : kDoRowCopy)));
 
     // Registers: without dropout the launch allocation of 96 per thread lets no role spill, and moving
     // registers from the MMA / TMA warps to the elementwise ones (104 / 64, 104 / 40) made one side or the
@@ -699,7 +721,23 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
             // pairs: P = 2^((S scale + bias - lse) log2 e) 2^kPShift with the terms in the forward's order, so that a mask
             // of the type's lowest value or of -1e9 leaves in both what its rounding leaves (the difference is small
-            // wherever P is not), and the shift exact behind it: d(loss)/d(scores) is an fp32 result.
+            // wherever P is not), and the shift (fp16 only) exact behind it: d(loss)/d(scores) is an fp32 result.
+        }
+        if constexpr (PREC != 0 && !BF16 && MODE == 1) {
+            // fp16 pairs: dS of my row scaled by a power of two of its own, from its own max |dO|, so that rows far
+            // below the column's largest keep their bits (dQ and d(loss)/d(scores) of a row need no common scale; the
+            // other kernel sums over rows and has to have one)
+            if (n_iter > 0 && mbar_wait(&bars[Cfg::kXYFull], 0u, abort_flag)) {
+                uint32_t m = 0u;
+#pragma unroll
+                for (int c = 0; c < Cfg::kNBox * 8; ++c) {
+                    const uint32_t mp = finite_piece<__half>(absmax16_acc(
+                        0u, *reinterpret_cast<const uint4*>(sY + (c >> 3) * kBoxBytes + r * 128 + (((c ^ r) & 7) << 4))));
+                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(mp));
+                }
+                const float rng[2] = {__half2float(__ushort_as_half((unsigned short)max(m & 0xFFFFu, m >> 16))), col_range[1]};
+                sc = make_scales(rng, D, a.inv_keep, a.scale, kDoAsIs);
+            }
         }
         // dS' = P' o (dP * tt_mul o Z + (-delta) * nd_mul): see "number formats" above
         const uint64_t ttm2 = f2_pack(sc.tt_mul, sc.tt_mul), ndm2 = f2_pack(sc.nd_mul, sc.nd_mul);
@@ -919,7 +957,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             if (PREC == 2 || (PREC == 1 && a.bias)) add = f2_pack(b0, b1);
                             uint64_t x = f2_fma(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), sc2, add);
                             if (PREC == 2 || (PREC == 1 && a.bias)) x = f2_add(x, L);
-                            if (PREC) x = f2_fma(x, f2_pack(kLog2e, kLog2e), f2_pack(kPShift, kPShift));
+                            if (P_BF16)    x = f2_mul(x, f2_pack(kLog2e, kLog2e));
+                            else if (PREC) x = f2_fma(x, f2_pack(kLog2e, kLog2e), f2_pack(kPShift, kPShift));
                             f2_unpack(x, x0, x1);
                             pf[h][i0] = __float_as_uint(ex2(x0));
                             pf[h][i0 + 1] = __float_as_uint(ex2(x1));
@@ -1143,7 +1182,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             x = f2_fma(s2, scn2, neg2);
                         }
                         f2_unpack(f2_mul(x, log2e2), x0, x1);
-                        f2_unpack(f2_mul(f2_pack(ex2(x0), ex2(x1)), up2), x0, x1);
+                        x0 = ex2(x0);
+                        x1 = ex2(x1);
+                        if (!P_BF16) f2_unpack(f2_mul(f2_pack(x0, x1), up2), x0, x1);
                         PSET(c, x0);
                         PSET(c + 1, x1);
                         continue;
@@ -1363,17 +1404,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (MODE == 1) grid_dependency_wait();
 }
 
-// Largest magnitude among the eight 16-bit values of a 16-byte piece, folded into a running maximum
-// of magnitude bit patterns (two per word; for fp16 and bf16 alike a larger magnitude is a larger
-// unsigned pattern).
-__device__ __forceinline__ uint32_t absmax16_acc(uint32_t m, const uint4& v) {
-    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.x & 0x7FFF7FFFu));
-    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.y & 0x7FFF7FFFu));
-    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.z & 0x7FFF7FFFu));
-    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.w & 0x7FFF7FFFu));
-    return m;
-}
-// Block-wide maximum of those patterns, as a float, folded into *slot (an fp32 bit pattern; for
+// Block-wide maximum of absmax16_acc's patterns, as a float, folded into *slot (an fp32 bit pattern; for
 // non-negative floats the unsigned order is the numeric order, so atomicMax on the bits is exact).
 template <typename T>
 __device__ __forceinline__ void absmax16_commit(uint32_t m, float* slot, uint32_t* red) {
@@ -1402,7 +1433,7 @@ struct PreprocessCopies {
     const void* o_lo; int64_t l_sb, l_sn, l_sh;     // optional residual of O (any dtype)
     const void* q; int64_t q_sb, q_sn, q_sh;
     uint16_t* q16; uint16_t* do16; float* erow;
-    int pairs;                                      // PREC != 0: -lse instead of kPShift - lse*log2(e)
+    int pairs;                                      // PREC != 0: -lse instead of kPShift - lse*log2(e), maxima of finite values
 };
 // A head size below D (pair instances) leaves the lanes beyond it idle.
 template <typename T, int D, bool COPIES>
@@ -1426,7 +1457,12 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
         uint32_t m = 0u;
         const int j_end = min(nk, (slab + 1) * kVRows);
         for (int j = slab * kVRows + (int)(threadIdx.x / LPR); j < j_end && sub * 8 < d; j += 256 / LPR)
-            m = absmax16_acc(m, *reinterpret_cast<const uint4*>(v + b * v_sb + (int64_t)j * v_sn + hk * v_sh + sub * 8));
+        {
+            const uint4 piece = *reinterpret_cast<const uint4*>(v + b * v_sb + (int64_t)j * v_sn + hk * v_sh + sub * 8);
+            if (!cp.pairs) { m = absmax16_acc(m, piece); continue; }
+            const uint32_t mp = finite_piece<T>(absmax16_acc(0u, piece));
+            asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(mp));
+        }
         absmax16_commit<T>(m, ranges + 2 * (int64_t)col + 1, red);
         return;
     }
@@ -1464,7 +1500,8 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
         for (int e = 0; e < 8; ++e) s = fmaf(to_f32<T>(eo[e]) + to_f32<T>(el[e]), to_f32<T>(eg[e]), s);
 #pragma unroll
         for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        const uint32_t m_mine = absmax16_acc(0u, vg);
+        uint32_t m_mine = absmax16_acc(0u, vg);
+        if (cp.pairs) m_mine = finite_piece<T>(m_mine);
         m = max(m, max(m_mine & 0xFFFFu, m_mine >> 16));
         int e_i = 0;
         if (COPIES) {

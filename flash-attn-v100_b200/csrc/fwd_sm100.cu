@@ -845,8 +845,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                     if constexpr (PREC != 0) {
-                        // P = e^(x - m) 2^kPShift as hi + lo, base 2 and the shift behind the difference, which is small
-                        // where P is not.  A row that has seen only -inf so far keeps m = -inf; 0 in its place lets its
+                        // P = e^(x - m) as hi + lo (fp16: times 2^kPShift), base 2 and the shift behind the difference, which is
+                        // small where P is not.  A row that has seen only -inf so far keeps m = -inf; 0 in its place lets its
                         // P come out as 0.
                         const float nm = m == -INFINITY ? 0.f : -m;
                         const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale);
@@ -864,7 +864,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                                 const int c = q4 * 32 + cc;
                                 float p0, p1;
                                 f2_unpack(f2_mul(f2_add(f2_pack(SF(c), SF(c + 1)), nm2), log2e2), p0, p1);
-                                f2_unpack(f2_mul(f2_pack(ex2(p0), ex2(p1)), up2), p0, p1);
+                                p0 = ex2(p0);
+                                p1 = ex2(p1);
+                                if (!P_BF16) f2_unpack(f2_mul(f2_pack(p0, p1), up2), p0, p1);
                                 l0 += p0; l1 += p1;
                                 if constexpr (DROP == 2) {
                                     const uint32_t word = q4 == 0 ? kb4.x : (q4 == 1 ? kb4.y : (q4 == 2 ? kb4.z : kb4.w));
@@ -1079,7 +1081,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                 }
-                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = PREC ? fmaf(kLn2, log2f(l) - kPShift, m) : kLn2 * ((m - kPShift) + log2f(l));
+                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = PREC ? fmaf(kLn2, log2f(l) - (P_BF16 ? 0.f : kPShift), m) : kLn2 * ((m - kPShift) + log2f(l));
                 // the O_t reads above are complete (wait::ld); the next pair's first PV_t MMA waits for
                 // this warpgroup's next P_t, so it cannot overwrite O_t earlier
             }

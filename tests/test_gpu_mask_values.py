@@ -67,3 +67,32 @@ def test_a_row_without_a_result_has_no_gradient_where_it_sees_nothing(device, dt
     got = _run(q, k, v, g, bias, True)
     assert (got["ds"][:, :, 70, 71:] == 0).all() and torch.equal(torch.isnan(got["ds"]), torch.isnan(want["ds"]))
     assert torch.isfinite(got["dk"][:, 71:]).all()
+
+
+@pytest.mark.parametrize("dtype,D,N", [(torch.bfloat16, 64, 200), (torch.float16, 64, 201), (torch.bfloat16, 128, 260), (torch.float16, 96, 132)],
+                         ids=["bf16-d64", "fp16-d64-direct", "bf16-d128", "fp16-d96"])
+@pytest.mark.parametrize("where", ["g", "v"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), "max"])
+def test_one_value_that_is_no_number_leaves_the_other_rows_alone(device, dtype, D, N, where, value):
+    """An infinity, a NaN or the type's largest value in one row of dO or V (an overflowing loss scale): gradients that
+    are numbers on the CUDA cores are the same numbers here, but for a dP that overflows the tensor core's sum."""
+    t = {n: _rand((2, N, 2, D), dtype, s) for s, n in enumerate("qkvg")}
+    if value == "max":
+        # (the largest bf16 value times another one is an infinity in fp32 arithmetic as well)
+        value = 65504.0 if dtype == torch.float16 else 2.0 ** 120
+    t[where][0, 100, 0, 3] = value
+    bias = _rand((1, 2, N, N), torch.float32, 9).to(device)
+    q, k, v, g = (x.to(device) for x in t.values())
+    with fa.kernel_variant("simt"):
+        want = _run(q, k, v, g, bias, False)
+    got = _run(q, k, v, g, bias, False)
+    for n in ("ds", "dq", "dk", "dv"):
+        assert torch.isfinite(got[n][torch.isfinite(want[n])]).all(), n
+    if where == "g":
+        for b in range(2):
+            for h in range(2):
+                for n in ("ds", "dq"):
+                    a, w = ((x[b, h] if n == "ds" else x[b, :, h]).double() for x in (got[n], want[n]))
+                    rows = torch.arange(N, device=device) != 100
+                    err = ((a - w).norm(dim=1) / w.norm(dim=1))[rows].max().item()
+                    assert err <= 2 * TOL[dtype], (n, b, h, err)
