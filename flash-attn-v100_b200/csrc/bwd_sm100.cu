@@ -121,8 +121,10 @@ struct BwdCfg {
     static constexpr int kWConv = kUConv + kUStages;             // [kWStages] streamed W, key-stationary kernels only
     static constexpr int kBiasFull = kWConv + kWStages;          // PREC = 2: the step's bias tile has landed
     static constexpr int kBiasEmpty = kBiasFull + 1;             // ... and has been read (one arrival per elementwise warp)
-    static constexpr int kNumBars = kBiasEmpty + 1;
-    static constexpr int kVecBytes = (MODE != 1) ? 2 * 1024 : 0; // two slots of lse[128] | delta[128]
+    static constexpr int kSums = kBiasEmpty + 1;                 // pairs, MODE 1: the rows' partial sums (elementwise warps)
+    static constexpr int kNumBars = kSums + 1;
+    // two slots of lse[128] | delta[128]; pairs, MODE 1: a partial sum of each row from every warpgroup
+    static constexpr int kVecBytes = MODE != 1 ? 2 * 1024 : (PREC ? 128 * 4 * kNWG : 0);
     static constexpr int kDsBytes = 128 * 128 * 2;               // fused kernel: dS^T tile for the dQ MMA
     // bytes used from the 1024-aligned base: X, Y, U ring, W ring, [dS], [vectors], barriers, TMEM slot + flag, [masks]
     static constexpr int kUsedBytes = (2 + kUStages + kWStages) * kTileBytes + kBiasBytes + (kFused ? kDsBytes : 0) + kVecBytes +
@@ -307,7 +309,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint8_t* sW = sU + UST * TILE;                  // W ring
     uint8_t* sBias = sW + WST * TILE;               // PREC = 2
     uint8_t* sDs = sBias + Cfg::kBiasBytes;         // fused kernel only
-    float* sVec = (float*)(sDs + (FUSED ? Cfg::kDsBytes : 0));      // key-stationary only: 2 x (lse[128] | delta[128])
+    float* sVec = (float*)(sDs + (FUSED ? Cfg::kDsBytes : 0));      // key-stationary: 2 x (lse[128] | delta[128]); see kVecBytes
     uint64_t* bars = (uint64_t*)((uint8_t*)sVec + Cfg::kVecBytes);
     uint32_t* tmem_slot = (uint32_t*)(bars + Cfg::kNumBars);
     volatile uint32_t* abort_flag = (volatile uint32_t*)(tmem_slot + 1);
@@ -330,7 +332,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
     // iteration space (uniform over the CTA)
     const int nk = kv_len_of(a.kv_len, b, a.Nk);    // keys this batch entry attends to
-    int tile, head_x, it0, n_per_head, n_iter;
+    int tile, head_x, it0, n_per_head, n_iter, sum_steps = 0;
     if (KS) {
         tile = cw.tile_rank;                        // key tile: the first one sees the most query tiles
         head_x = cw.head;                           // kv head
@@ -346,8 +348,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         int kv_end = nk;
         if (a.causal && tile * kTile + kTile + a.shift < kv_end) kv_end = tile * kTile + kTile + a.shift;
         n_per_head = (kv_end + kTile - 1) / kTile;
-        n_iter = n_per_head;
+        // pairs with d(loss)/d(scores) wanted: the steps are walked twice (kernel comment at `summing` below)
+        if (PREC && a.d_scores) sum_steps = n_per_head;
+        n_iter = sum_steps + n_per_head;
     }
+    // query-stationary: key tile of step `it`
+    auto k_tile_of = [&](int it) { return PREC && it >= n_per_head ? it - n_per_head : it; };
     const int head_kv = (KS) ? head_x : head_x / group;
     // Key-stationary kernels: query tile of step `it`.  The fused kernel without a causal mask starts
     // each key tile's walk at a different query tile, so that the CTAs of one head, which run at
@@ -365,7 +371,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int i = 0; i < Cfg::kNumBars; ++i) {
             const bool wide = (i == Cfg::kPReady || i == Cfg::kDsReady || i == Cfg::kMask || i == Cfg::kEpi ||
                                i == Cfg::kDqRead || i == Cfg::kPHalf || i == Cfg::kDsHalf ||
-                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i == Cfg::kXYConv || i == Cfg::kBiasEmpty);
+                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i == Cfg::kXYConv || i >= Cfg::kBiasEmpty);
             const bool conv2 = i >= Cfg::kUConv && i < Cfg::kBiasFull;          // the two converting warps
             mbar_init(&bars[i], wide ? 4u * NWG : (conv2 ? 2u : 1u));    // one arrival per elementwise warp
         }
@@ -433,7 +439,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             for (int it = 0; it < n_iter; ++it) {
                 int head_u, row_u;
                 if (KS) { head_u = head_x * group + hg; row_u = q_tile_of(qi) * kTile; }
-                else    { head_u = head_kv; row_u = it * kTile; }
+                else    { head_u = head_kv; row_u = k_tile_of(it) * kTile; }
                 ok = mbar_wait(&bars[Cfg::kUEmpty + us], (uph & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
                 mbar_expect_tx(&bars[Cfg::kUFull + us], TILE);
@@ -602,11 +608,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 ok = mbar_wait(&bars[b_half], ds_par, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
-                issue_acc_half(tAcc1, tDs, cur_u, it > 0, 0);                    // dK += dS^T Q  /  dQ += dS K
+                const bool acc = !PREC || it >= sum_steps;                       // (no dS in the steps that only sum)
+                if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 0);   // dK += dS^T Q  /  dQ += dS K
                 ok = mbar_wait(&bars[b_ready], ds_par, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
-                issue_acc_half(tAcc1, tDs, cur_u, it > 0, 1);
+                if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 1);
                 mma_commit(&bars[Cfg::kUEmpty + us]);                            // last reader of U(it)
                 if (FUSED) {
                     // dQ tile of this step = dS K_j: A is the dS^T tile the threads left in shared memory,
@@ -673,16 +680,17 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             auto store_ds = [&](int it) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    if (it * kTile + 32 * c < a.Nk) tma_store_4d(&map_ds, sBias + c * kBoxBytes, it * kTile + 32 * c, head_x, tile * kTile, b);
+                    if (k_tile_of(it) * kTile + 32 * c < a.Nk)
+                        tma_store_4d(&map_ds, sBias + c * kBoxBytes, k_tile_of(it) * kTile + 32 * c, head_x, tile * kTile, b);
                 tma_store_commit();
                 tma_store_wait_read<0>();
             };
             for (int it = 0; it < n_iter; ++it) {
                 const int head = KS ? head_x * group + hg : head_x;
-                const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : it) * kTile;
+                const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : k_tile_of(it)) * kTile;
                 ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)it & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (MODE == 1 && a.ds_staged && it > 0) store_ds(it - 1);
+                if (MODE == 1 && a.ds_staged && it > sum_steps) store_ds(it - 1);
                 mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
@@ -791,10 +799,16 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             return true;
         };
 
+        // Pairs with d(loss)/d(scores) wanted (MODE 1).  That output is fp32, but delta comes from an O rounded to 16 bits
+        // (or 16 + 16) that was summed with P as a pair, and P from an lse rounded once: together more than the CUDA
+        // cores' error.  So a first walk over the keys sums P and P o dP Z of every row in fp32; their quotient is
+        // delta, and the sum of P, one but for rounding, divides P.  Only dQ's and d(scores)' kernel, only these calls.
+        [[maybe_unused]] uint64_t sum_p2 = 0ull, sum_pd2 = 0ull;           // {0.f, 0.f}
+        [[maybe_unused]] float p_mul = P_BF16 ? 1.f : 16384.f;             // 2^kPShift where P carries it
         int qi = 0, hg = 0;                 // step within the query head, query heads done (key-stationary)
         int prev_tile = 0, prev_head = 0;   // query tile and head of the previous step
         for (int it = 0; it < n_iter; ++it) {
-            const int strm_tile = (KS) ? q_tile_of(qi) : it;     // query tile (0) / key tile (1)
+            const int strm_tile = (KS) ? q_tile_of(qi) : k_tile_of(it);     // query tile (0) / key tile (1)
             const int col_g0 = strm_tile * kTile + cb;                          // global index of my first column
             const int head_q = (KS) ? head_x * group + hg : head_x;
             const uint32_t bh = dropout_column(a.rng, b, head_q);
@@ -1096,6 +1110,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 mbar_arrive_warp(&bars[Cfg::kPReady]);
             }
             const uint64_t sc2 = f2_pack(a.scale_log2, a.scale_log2);
+            [[maybe_unused]] const bool summing = PREC != 0 && MODE == 1 && it < sum_steps;
             [[maybe_unused]] int seen = CPT;           // pairs, query-stationary: my first columns that my row sees
             if (KS) {
                 // P = 2^(S*c - lse): the staged vector holds -lse*log2(e), two columns per 64-bit word.
@@ -1151,7 +1166,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_st();
             } else {
                 const uint64_t neg2 = f2_pack(my_nlse2, my_nlse2);
-                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(16384.f, 16384.f);
+                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(p_mul, p_mul);
                 [[maybe_unused]] float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < CPT; c += 2) {
@@ -1182,9 +1197,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             x = f2_fma(s2, scn2, neg2);
                         }
                         f2_unpack(f2_mul(x, log2e2), x0, x1);
-                        x0 = ex2(x0);
-                        x1 = ex2(x1);
-                        if (!P_BF16) f2_unpack(f2_mul(f2_pack(x0, x1), up2), x0, x1);
+                        f2_unpack(f2_mul(f2_pack(ex2(x0), ex2(x1)), up2), x0, x1);
                         PSET(c, x0);
                         PSET(c + 1, x1);
                         continue;
@@ -1202,7 +1215,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         PSET(c + 1, ex2(x1));
                     }
                 }
-                if (PREC == 2 && !a.ds_staged) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
+                if (PREC == 2 && (!a.ds_staged || summing)) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
                 const bool diag = a.causal && strm_tile * kTile + kTile - 1 > tile * kTile + a.shift;
                 if (diag || strm_tile * kTile + kTile > nk) {
                     // my row sees my first `seen` columns: keys below the count, at most row + shift
@@ -1243,8 +1256,29 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 // the first is stored and handed over while the second is computed.
                 const ulonglong2* d2 = reinterpret_cast<const ulonglong2*>(del_s + cb);
                 const uint64_t my_nd2 = f2_pack(my_ndelta, my_ndelta);
+                if (summing) {
+                    tc_fence_before_sync();
+                    mbar_arrive_warp(&bars[b_half]);
+                    uint64_t sp = 0ull, spd = 0ull;
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
+                    for (int c = 0; c < CPT; c += 2) {
+                        const uint64_t p2 = f2_pack(PF(c), PF(c + 1));
+                        uint64_t z2 = ttm2;
+                        if (drop) z2 = f2_pack(((kb[0] >> c) & 1u) ? zk : 0.f, ((kb[0] >> c) & 2u) ? zk : 0.f);
+                        sp = f2_add(sp, p2);
+                        uint64_t t2 = f2_mul(p2, f2_mul(f2_pack(__uint_as_float(dr[0][c]), __uint_as_float(dr[0][c + 1])), z2));
+                        if (seen < CPT) {              // hidden: no part of the sum, also where dP is no number
+                            float t0, t1;
+                            f2_unpack(t2, t0, t1);
+                            t2 = f2_pack(c < seen ? t0 : 0.f, c + 1 < seen ? t1 : 0.f);
+                        }
+                        spd = f2_add(spd, t2);
+                    }
+                    sum_p2 = f2_add(sum_p2, sp);
+                    sum_pd2 = f2_add(sum_pd2, spd);
+                }
+#pragma unroll
+                for (int hf = 0; hf < 2 && !summing; ++hf) {
                     uint32_t pk[CPT / 4], pl[CPT / 4];
                     if (hf == 1) {
                         tmem_wait_st();                            // the first half, stored just now
@@ -1328,12 +1362,38 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 if (FUSED) fence_proxy_async_smem();
                 tmem_wait_st();
-                if (PREC == 2 && MODE == 1 && a.ds_staged) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);     // (written, here)
+                if (PREC == 2 && MODE == 1 && a.ds_staged && !summing) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);     // (written, here)
             }
 #undef PF
 #undef PSET
             tc_fence_before_sync();
             mbar_arrive_warp(&bars[b_ready]);
+            if (summing && it == sum_steps - 1) {
+                // the row's four threads put their sums together, in a fixed order
+                uint32_t meet = 0u;
+                auto all_met = [&] {
+                    mbar_arrive_warp(&bars[Cfg::kSums]);
+                    const bool good = mbar_wait(&bars[Cfg::kSums], meet & 1u, abort_flag);
+                    ++meet;
+                    return __all_sync(0xffffffffu, good);
+                };
+                auto row_sum = [&](uint64_t mine, float& out) {
+                    float x0, x1;
+                    f2_unpack(mine, x0, x1);
+                    sVec[wg * 128 + r] = x0 + x1;
+                    if (!all_met()) return false;
+                    out = (sVec[r] + sVec[128 + r]) + (sVec[256 + r] + sVec[384 + r]);
+                    return true;
+                };
+                float sum_p = 0.f, sum_pd = 0.f;
+                ok = row_sum(sum_p2, sum_p) && all_met() && row_sum(sum_pd2, sum_pd);
+                if (!ok) break;
+                // a row without a result, or one whose lse has lost its sum (all of it masked with a lowest value),
+                // keeps what it has
+                if (sum_p > 0.f && fabsf(sum_pd) < INFINITY) my_ndelta = -sum_pd / sum_p;
+                const float unit = p_mul / sum_p;
+                if (fabsf(unit - 1.f) < 0.25f) p_mul *= unit;
+            }
             }
             if (KS) mbar_arrive_warp(&bars[Cfg::kVEmpty + (it & 1)]);      // this step's lse / delta rows are read
             prev_tile = strm_tile; prev_head = head_q;

@@ -344,6 +344,9 @@ template <> struct SoftmaxLoop<2> : SplitSoftmaxLoop { using SplitSoftmaxLoop::S
 constexpr float kPShift = 6.0f;
 constexpr float kPScale = 64.0f;            // 2^kPShift
 
+// log(x) rounded once: the hardware's base-2 logarithm is off by up to 2^-22 and would be the largest error of an lse.
+__device__ __noinline__ float exact_log(float x) { return (float)log((double)x); }
+
 // DROP: 0 no dropout; 1 the keep bits are drawn here, by the softmax threads (no workspace);
 // 2 they are loaded from the workspace, where dropout_bits_kernel has written the call's bits.
 // SCHED: see FwdCfg.
@@ -1081,7 +1084,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     }
                 }
-                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = PREC ? fmaf(kLn2, log2f(l) - (P_BF16 ? 0.f : kPShift), m) : kLn2 * ((m - kPShift) + log2f(l));
+                if (row_ok()) a.lse[((int64_t)st.b * a.H + h) * a.Nq + i] = PREC ? m + exact_log(P_BF16 ? l : l * (1.f / kPScale))
+                                                                                 : kLn2 * ((m - kPShift) + log2f(l));
                 // the O_t reads above are complete (wait::ld); the next pair's first PV_t MMA waits for
                 // this warpgroup's next P_t, so it cannot overwrite O_t earlier
             }
