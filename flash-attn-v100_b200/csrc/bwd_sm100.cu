@@ -280,7 +280,9 @@ __device__ __forceinline__ CtaWork cta_work(int cols_per_group) {
 // INLINE (bf16 inputs only): the streamed tiles arrive as bf16 and the two spare warps convert them;
 // otherwise bf16 calls stream the fp16 copies the preprocess launch (Q, dO) and the dK/dV kernel (K:
 // map_aux, a by-product of its stationary tile) have written to the workspace.
-template <int D, bool BF16, int MODE, int NWG, int DROP, bool INLINE, int PREC>
+// DS (pairs, MODE 1): the call wants d(loss)/d(scores).  An instance of its own: as a branch its code cost the kernel of
+// calls that do not want it 10 of 56 us (B4 N1024 H16 D96 causal).
+template <int D, bool BF16, int MODE, int NWG, int DROP, bool INLINE, int PREC, bool DS>
 __global__ void __launch_bounds__(128 * NWG + kExtraThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                  const __grid_constant__ CUtensorMap map_u, const __grid_constant__ CUtensorMap map_w,
@@ -349,11 +351,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         if (a.causal && tile * kTile + kTile + a.shift < kv_end) kv_end = tile * kTile + kTile + a.shift;
         n_per_head = (kv_end + kTile - 1) / kTile;
         // pairs with d(loss)/d(scores) wanted: the steps are walked twice (kernel comment at `summing` below)
-        if (PREC && a.d_scores) sum_steps = n_per_head;
+        if (DS) sum_steps = n_per_head;
         n_iter = sum_steps + n_per_head;
     }
     // query-stationary: key tile of step `it`
-    auto k_tile_of = [&](int it) { return PREC && it >= n_per_head ? it - n_per_head : it; };
+    auto k_tile_of = [&](int it) { return DS && it >= n_per_head ? it - n_per_head : it; };
     const int head_kv = (KS) ? head_x : head_x / group;
     // Key-stationary kernels: query tile of step `it`.  The fused kernel without a causal mask starts
     // each key tile's walk at a different query tile, so that the CTAs of one head, which run at
@@ -608,7 +610,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 ok = mbar_wait(&bars[b_half], ds_par, abort_flag);
                 if (!ok) break;
                 tc_fence_after_sync();
-                const bool acc = !PREC || it >= sum_steps;                       // (no dS in the steps that only sum)
+                const bool acc = !DS || it >= sum_steps;                       // (no dS in the steps that only sum)
                 if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 0);   // dK += dS^T Q  /  dQ += dS K
                 ok = mbar_wait(&bars[b_ready], ds_par, abort_flag);
                 if (!ok) break;
@@ -690,7 +692,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : k_tile_of(it)) * kTile;
                 ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)it & 1u) ^ 1u, abort_flag);
                 if (!ok) break;
-                if (MODE == 1 && a.ds_staged && it > sum_steps) store_ds(it - 1);
+                if (DS && a.ds_staged && it > sum_steps) store_ds(it - 1);
                 mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
@@ -699,7 +701,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 ++done;
                 if (++qi == n_per_head) { qi = 0; ++hg; }
             }
-            if (MODE == 1 && a.ds_staged && ok && n_iter > 0 && mbar_wait(&bars[Cfg::kBiasEmpty], (uint32_t)(n_iter - 1) & 1u, abort_flag))
+            if (DS && a.ds_staged && ok && n_iter > 0 && mbar_wait(&bars[Cfg::kBiasEmpty], (uint32_t)(n_iter - 1) & 1u, abort_flag))
                 store_ds(n_iter - 1);
             for (int spin = 0; !ok && spin < 4096 && done > 0 && !mbar_try_wait(&bars[Cfg::kBiasFull], (uint32_t)(done - 1) & 1u); ++spin) {}
         }
@@ -753,7 +755,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const uint64_t ladd2 = f2_pack(sc.l_add, sc.l_add);
         my_ndelta *= sc.nd_mul;
         // PREC = 1, query-stationary: my row of d loss / d scores, and what undoes dS' = dS * 2^g
-        [[maybe_unused]] float* ds_row = (PREC && MODE == 1 && a.d_scores)
+        [[maybe_unused]] float* ds_row = DS
             ? a.d_scores + (((int64_t)b * a.H + head_x) * a.Nq + row_g) * (int64_t)a.Nk : nullptr;
         [[maybe_unused]] const float ds_mul = sc.acc1_mul / a.scale;
         bool ok = true;
@@ -1061,7 +1063,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 }
                                 float d0, d1;
                                 f2_unpack(f2_mul(f2_pack(__uint_as_float(pf[h][i0]), __uint_as_float(pf[h][i0 + 1])), tt), d0, d1);
-                                if (PREC && (diag || tail)) {       // as in the other kernel: none, not 0 times what delta is
+                                // as in the other kernel: none, not 0 times what delta is (only a bias makes rows without a result)
+                                if ((PREC == 2 || (PREC == 1 && a.bias)) && (diag || tail)) {
                                     const int col = col_g0 + 8 * j + 2 * lq, lim = hidden_below(h, k);
                                     if (col < lim) d0 = 0.f;
                                     if (col + 1 < lim) d1 = 0.f;
@@ -1110,7 +1113,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 mbar_arrive_warp(&bars[Cfg::kPReady]);
             }
             const uint64_t sc2 = f2_pack(a.scale_log2, a.scale_log2);
-            [[maybe_unused]] const bool summing = PREC != 0 && MODE == 1 && it < sum_steps;
+            [[maybe_unused]] const bool summing = DS && it < sum_steps;
             [[maybe_unused]] int seen = CPT;           // pairs, query-stationary: my first columns that my row sees
             if (KS) {
                 // P = 2^(S*c - lse): the staged vector holds -lse*log2(e), two columns per 64-bit word.
@@ -1197,7 +1200,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                             x = f2_fma(s2, scn2, neg2);
                         }
                         f2_unpack(f2_mul(x, log2e2), x0, x1);
-                        f2_unpack(f2_mul(f2_pack(ex2(x0), ex2(x1)), up2), x0, x1);
+                        x0 = ex2(x0);
+                        x1 = ex2(x1);
+                        if (DS || !P_BF16) f2_unpack(f2_mul(f2_pack(x0, x1), up2), x0, x1);
                         PSET(c, x0);
                         PSET(c + 1, x1);
                         continue;
@@ -1215,7 +1220,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         PSET(c + 1, ex2(x1));
                     }
                 }
-                if (PREC == 2 && (!a.ds_staged || summing)) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
+                if (PREC == 2 && (!DS || !a.ds_staged || summing)) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);
                 const bool diag = a.causal && strm_tile * kTile + kTile - 1 > tile * kTile + a.shift;
                 if (diag || strm_tile * kTile + kTile > nk) {
                     // my row sees my first `seen` columns: keys below the count, at most row + shift
@@ -1276,99 +1281,100 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     }
                     sum_p2 = f2_add(sum_p2, sp);
                     sum_pd2 = f2_add(sum_pd2, spd);
-                }
+                } else {
 #pragma unroll
-                for (int hf = 0; hf < 2 && !summing; ++hf) {
-                    uint32_t pk[CPT / 4], pl[CPT / 4];
-                    if (hf == 1) {
-                        tmem_wait_st();                            // the first half, stored just now
-                        tc_fence_before_sync();
-                        mbar_arrive_warp(&bars[b_half]);
-                    }
-#pragma unroll
-                    for (int c4 = hf * (CPT / 8); c4 < (hf + 1) * (CPT / 8); ++c4) {
-                        ulonglong2 nd;
-                        if (KS) { nd = d2[c4]; nd.x = f2_mul(nd.x, ndm2); nd.y = f2_mul(nd.y, ndm2); }
-                        else { nd.x = my_nd2; nd.y = my_nd2; }
-                        const int c = c4 * 4;
-                        uint64_t dpa = f2_pack(__uint_as_float(dr[c >> 5][c & 31]), __uint_as_float(dr[c >> 5][(c + 1) & 31]));
-                        uint64_t dpb = f2_pack(__uint_as_float(dr[c >> 5][(c + 2) & 31]), __uint_as_float(dr[c >> 5][(c + 3) & 31]));
-                        uint64_t ta, tb;
-                        if (drop) {
-                            // dropped entries: dS = P o (-delta), selected after the FMA
-                            const uint32_t kw = kb[c >> 5] >> (c & 31);
-                            const uint64_t zk2 = f2_pack(zk, zk);
-                            float t0, t1, t2, t3, n0, n1, n2, n3;
-                            f2_unpack(f2_fma(dpa, zk2, nd.x), t0, t1);
-                            f2_unpack(f2_fma(dpb, zk2, nd.y), t2, t3);
-                            f2_unpack(nd.x, n0, n1);
-                            f2_unpack(nd.y, n2, n3);
-                            ta = f2_pack((kw & 1u) ? t0 : n0, (kw & 2u) ? t1 : n1);
-                            tb = f2_pack((kw & 4u) ? t2 : n2, (kw & 8u) ? t3 : n3);
-                        } else {
-                            ta = f2_fma(dpa, ttm2, nd.x);
-                            tb = f2_fma(dpb, ttm2, nd.y);
+                    for (int hf = 0; hf < 2; ++hf) {
+                        uint32_t pk[CPT / 4], pl[CPT / 4];
+                        if (hf == 1) {
+                            tmem_wait_st();                            // the first half, stored just now
+                            tc_fence_before_sync();
+                            mbar_arrive_warp(&bars[b_half]);
                         }
-                        float d0, d1, d2v, d3;
-                        f2_unpack(f2_mul(f2_pack(PF(c), PF(c + 1)), ta), d0, d1);
-                        f2_unpack(f2_mul(f2_pack(PF(c + 2), PF(c + 3)), tb), d2v, d3);
-                        if constexpr (PREC != 0) {
-                            // a hidden score has no gradient, also where delta or dP is no number (0 times that is none)
-                            if (seen < CPT) {
-                                if (c >= seen) d0 = 0.f;
-                                if (c + 1 >= seen) d1 = 0.f;
-                                if (c + 2 >= seen) d2v = 0.f;
-                                if (c + 3 >= seen) d3 = 0.f;
+#pragma unroll
+                        for (int c4 = hf * (CPT / 8); c4 < (hf + 1) * (CPT / 8); ++c4) {
+                            ulonglong2 nd;
+                            if (KS) { nd = d2[c4]; nd.x = f2_mul(nd.x, ndm2); nd.y = f2_mul(nd.y, ndm2); }
+                            else { nd.x = my_nd2; nd.y = my_nd2; }
+                            const int c = c4 * 4;
+                            uint64_t dpa = f2_pack(__uint_as_float(dr[c >> 5][c & 31]), __uint_as_float(dr[c >> 5][(c + 1) & 31]));
+                            uint64_t dpb = f2_pack(__uint_as_float(dr[c >> 5][(c + 2) & 31]), __uint_as_float(dr[c >> 5][(c + 3) & 31]));
+                            uint64_t ta, tb;
+                            if (drop) {
+                                // dropped entries: dS = P o (-delta), selected after the FMA
+                                const uint32_t kw = kb[c >> 5] >> (c & 31);
+                                const uint64_t zk2 = f2_pack(zk, zk);
+                                float t0, t1, t2, t3, n0, n1, n2, n3;
+                                f2_unpack(f2_fma(dpa, zk2, nd.x), t0, t1);
+                                f2_unpack(f2_fma(dpb, zk2, nd.y), t2, t3);
+                                f2_unpack(nd.x, n0, n1);
+                                f2_unpack(nd.y, n2, n3);
+                                ta = f2_pack((kw & 1u) ? t0 : n0, (kw & 2u) ? t1 : n1);
+                                tb = f2_pack((kw & 4u) ? t2 : n2, (kw & 8u) ? t3 : n3);
+                            } else {
+                                ta = f2_fma(dpa, ttm2, nd.x);
+                                tb = f2_fma(dpb, ttm2, nd.y);
                             }
-                            const int e = (c4 - hf * (CPT / 8)) * 2;
-                            pack2_pair<P_BF16>(d0, d1, pk[e], pl[e]);
-                            pack2_pair<P_BF16>(d2v, d3, pk[e + 1], pl[e + 1]);
-                            if (PREC == 2 && a.ds_staged) {
-                                // ... by way of the bias tile's place (only I read these 16 bytes) and a TMA store: a
-                                // thread's own stores would go to 32 rows a warp
-                                *reinterpret_cast<float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4)) =
-                                    make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
-                            } else if (ds_row && row_g < a.Nq) {
-                                // d loss / d scores, the power of two of dS' taken out (exact)
-                                float* dst = ds_row + col_g0 + c;
-                                if (a.ds_vec) {
-                                    if (col_g0 + c < a.Nk)
-                                        *reinterpret_cast<float4*>(dst) = make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
-                                } else {
-                                    if (col_g0 + c < a.Nk) dst[0] = d0 * ds_mul;
-                                    if (col_g0 + c + 1 < a.Nk) dst[1] = d1 * ds_mul;
-                                    if (col_g0 + c + 2 < a.Nk) dst[2] = d2v * ds_mul;
-                                    if (col_g0 + c + 3 < a.Nk) dst[3] = d3 * ds_mul;
+                            float d0, d1, d2v, d3;
+                            f2_unpack(f2_mul(f2_pack(PF(c), PF(c + 1)), ta), d0, d1);
+                            f2_unpack(f2_mul(f2_pack(PF(c + 2), PF(c + 3)), tb), d2v, d3);
+                            if constexpr (PREC != 0) {
+                                // a hidden score has no gradient, also where delta or dP is no number (0 times that is none)
+                                if (DS && seen < CPT) {
+                                    if (c >= seen) d0 = 0.f;
+                                    if (c + 1 >= seen) d1 = 0.f;
+                                    if (c + 2 >= seen) d2v = 0.f;
+                                    if (c + 3 >= seen) d3 = 0.f;
                                 }
+                                const int e = (c4 - hf * (CPT / 8)) * 2;
+                                pack2_pair<P_BF16>(d0, d1, pk[e], pl[e]);
+                                pack2_pair<P_BF16>(d2v, d3, pk[e + 1], pl[e + 1]);
+                                if (DS && PREC == 2 && a.ds_staged) {
+                                    // ... by way of the bias tile's place (only I read these 16 bytes) and a TMA store: a
+                                    // thread's own stores would go to 32 rows a warp
+                                    *reinterpret_cast<float4*>(sBias + wg * kBoxBytes + r * 128 + (((c >> 2) ^ (r & 7)) << 4)) =
+                                        make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
+                                } else if (DS && row_g < a.Nq) {
+                                    // d loss / d scores, the power of two of dS' taken out (exact)
+                                    float* dst = ds_row + col_g0 + c;
+                                    if (a.ds_vec) {
+                                        if (col_g0 + c < a.Nk)
+                                            *reinterpret_cast<float4*>(dst) = make_float4(d0 * ds_mul, d1 * ds_mul, d2v * ds_mul, d3 * ds_mul);
+                                    } else {
+                                        if (col_g0 + c < a.Nk) dst[0] = d0 * ds_mul;
+                                        if (col_g0 + c + 1 < a.Nk) dst[1] = d1 * ds_mul;
+                                        if (col_g0 + c + 2 < a.Nk) dst[2] = d2v * ds_mul;
+                                        if (col_g0 + c + 3 < a.Nk) dst[3] = d3 * ds_mul;
+                                    }
+                                }
+                            } else {
+                                pk[(c4 - hf * (CPT / 8)) * 2 + 0] = pack2<false>(d0, d1);
+                                pk[(c4 - hf * (CPT / 8)) * 2 + 1] = pack2<false>(d2v, d3);
                             }
-                        } else {
-                            pk[(c4 - hf * (CPT / 8)) * 2 + 0] = pack2<false>(d0, d1);
-                            pk[(c4 - hf * (CPT / 8)) * 2 + 1] = pack2<false>(d2v, d3);
                         }
-                    }
-                    tmem_st_32x8(tD + lane_off + cb + hf * (CPT / 4), pk);
-                    if (PREC) tmem_st_32x8(tD + lane_off + cb + CPT / 2 + hf * (CPT / 4), pl);
-                    if (FUSED) {
-                        // the same dS^T values as a shared-memory tile [key row][query], 64-query boxes with
-                        // the 128-byte swizzle: the A operand (MN-major) of the dQ MMA.  The previous
-                        // step's dQ MMA has finished reading it: its completion was awaited in drain_dq.
+                        tmem_st_32x8(tD + lane_off + cb + hf * (CPT / 4), pk);
+                        if (PREC) tmem_st_32x8(tD + lane_off + cb + CPT / 2 + hf * (CPT / 4), pl);
+                        if (FUSED) {
+                            // the same dS^T values as a shared-memory tile [key row][query], 64-query boxes with
+                            // the 128-byte swizzle: the A operand (MN-major) of the dQ MMA.  The previous
+                            // step's dQ MMA has finished reading it: its completion was awaited in drain_dq.
 #pragma unroll
-                        for (int v = 0; v < CPT / 16; ++v) {
-                            const int q0 = cb + hf * (CPT / 2) + v * 8;                 // first of 8 queries
-                            uint8_t* dst = sDs + (q0 >> 6) * kBoxBytes + r * 128 + ((((q0 & 63) >> 3) ^ (r & 7)) << 4);
-                            *reinterpret_cast<uint4*>(dst) = make_uint4(pk[4 * v], pk[4 * v + 1], pk[4 * v + 2], pk[4 * v + 3]);
+                            for (int v = 0; v < CPT / 16; ++v) {
+                                const int q0 = cb + hf * (CPT / 2) + v * 8;                 // first of 8 queries
+                                uint8_t* dst = sDs + (q0 >> 6) * kBoxBytes + r * 128 + ((((q0 & 63) >> 3) ^ (r & 7)) << 4);
+                                *reinterpret_cast<uint4*>(dst) = make_uint4(pk[4 * v], pk[4 * v + 1], pk[4 * v + 2], pk[4 * v + 3]);
+                            }
                         }
                     }
                 }
                 if (FUSED) fence_proxy_async_smem();
                 tmem_wait_st();
-                if (PREC == 2 && MODE == 1 && a.ds_staged && !summing) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);     // (written, here)
+                if (PREC == 2 && DS && a.ds_staged && !summing) mbar_arrive_read_done(&bars[Cfg::kBiasEmpty]);     // (written, here)
             }
 #undef PF
 #undef PSET
             tc_fence_before_sync();
             mbar_arrive_warp(&bars[b_ready]);
-            if (summing && it == sum_steps - 1) {
+            if (DS && it == sum_steps - 1) {
                 // the row's four threads put their sums together, in a fixed order
                 uint32_t meet = 0u;
                 auto all_met = [&] {
@@ -1620,11 +1626,11 @@ bwd_dq_convert_kernel(const float* __restrict__ acc, T* __restrict__ dq, int Nq,
 // convert their tiles themselves.
 // the kernel instance and its shared memory for a dropout form (0 none, 1 drawn in the kernel, 2 loaded;
 // the converting-in-kernel instances, which serve the entry without a workspace, never load)
-template <int D, bool BF16, int MODE, bool INLINE, int PREC>
+template <int D, bool BF16, int MODE, bool INLINE, int PREC, bool DS = false>
 auto pick_kernel(int drop) {
-    if (drop == 2 && !INLINE) return bwd_sm100_kernel<D, BF16, MODE, kNWG, INLINE ? 1 : 2, INLINE, PREC>;
-    if constexpr (PREC == 2) return bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;       // bias_is_staged(): never drop = 1
-    else return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE, PREC> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC>;
+    if (drop == 2 && !INLINE) return bwd_sm100_kernel<D, BF16, MODE, kNWG, INLINE ? 1 : 2, INLINE, PREC, DS>;
+    if constexpr (PREC == 2) return bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC, DS>;       // bias_is_staged(): never drop = 1
+    else return drop ? bwd_sm100_kernel<D, BF16, MODE, kNWG, 1, INLINE, PREC, DS> : bwd_sm100_kernel<D, BF16, MODE, kNWG, 0, INLINE, PREC, DS>;
 }
 template <int D, int MODE, int PREC>
 int pick_smem(int drop) {
@@ -1773,9 +1779,10 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     if (COPIES && ws.k16_bytes == 0) { set_error("workspace layout lacks the fp16 copy of K"); return FA_EWORKSPACE; }
     auto k0 = pick_kernel<D, BF16, 0, INLINE, PREC>(drop);
     auto k1 = pick_kernel<D, BF16, 1, INLINE, PREC>(drop);
+    if constexpr (PREC != 0) if (p.d_scores) k1 = pick_kernel<D, BF16, 1, INLINE, PREC, true>(drop);
     const int smem0 = pick_smem<D, 0, PREC>(drop), smem1 = pick_smem<D, 1, PREC>(drop);
     FA_CUDA_CHECK(set_smem_limit_once(k0, smem0, p.device, &smem_done[drop], &smem_mu));
-    FA_CUDA_CHECK(set_smem_limit_once(k1, smem1, p.device, &smem_done[3 + drop], &smem_mu));
+    FA_CUDA_CHECK(set_smem_limit_once(k1, smem1, p.device, &smem_done[(PREC && p.d_scores ? 6 : 3) + drop], &smem_mu));
     if (phases & 2) {
         // stationary K_j, V_j; streamed Q_i, dO_i (bf16 with copies: their fp16 copies; the kernel leaves
         // the fp16 copy of K behind for the dQ kernel)
