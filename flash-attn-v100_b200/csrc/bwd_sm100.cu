@@ -150,6 +150,8 @@ struct BwdArgs {
     int causal;
     int shift;                     // key j is visible to query i iff j <= i + shift
     float scale, scale_log2;
+    float score_scale;             // pairs: scale for the scores, with the truncation of their sums given back
+    float dp_gain;                 // pairs: the same factor for dP
     uint32_t drop_thr;
     float inv_keep;
     PhiloxKey key;
@@ -750,8 +752,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             }
         }
         // dS' = P' o (dP * tt_mul o Z + (-delta) * nd_mul): see "number formats" above
-        const uint64_t ttm2 = f2_pack(sc.tt_mul, sc.tt_mul), ndm2 = f2_pack(sc.nd_mul, sc.nd_mul);
-        const float zk = a.inv_keep * sc.tt_mul;
+        const float tt_mul = DS ? sc.tt_mul * a.dp_gain : sc.tt_mul;
+        const uint64_t ttm2 = f2_pack(tt_mul, tt_mul), ndm2 = f2_pack(sc.nd_mul, sc.nd_mul);
+        const float zk = a.inv_keep * tt_mul;
         const uint64_t ladd2 = f2_pack(sc.l_add, sc.l_add);
         my_ndelta *= sc.nd_mul;
         // PREC = 1, query-stationary: my row of d loss / d scores, and what undoes dS' = dS * 2^g
@@ -919,7 +922,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                 kbits |= (((uint32_t)mbuf[col * 8 + (row >> 4)] >> (row & 15)) & 1u) << (16 * h + 4 * j + 2 * k + e);
                             }
             }
-            const float sc1 = PREC ? a.scale : a.scale_log2;
+            const float sc1 = PREC ? a.score_scale : a.scale_log2;
             const uint64_t sc2 = f2_pack(sc1, sc1);
             // key row > query column + shift is hidden: only tiles the mask's edge crosses need the test
             const bool diag = a.causal && strm_tile * kTile + a.shift < tile * kTile + kTile - 1;
@@ -1169,7 +1172,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 tmem_wait_st();
             } else {
                 const uint64_t neg2 = f2_pack(my_nlse2, my_nlse2);
-                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.scale, a.scale), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(p_mul, p_mul);
+                [[maybe_unused]] const uint64_t scn2 = f2_pack(a.score_scale, a.score_scale), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(p_mul, p_mul);
                 [[maybe_unused]] float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int c = 0; c < CPT; c += 2) {
@@ -1736,6 +1739,8 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     a.shift = p.causal ? p.causal_shift : 0;
     a.scale = p.scale;
     a.scale_log2 = p.scale * kLog2e;
+    a.score_scale = pair_score_scale(p);
+    a.dp_gain = 1.f + pair_truncation(p);
     a.drop_thr = dropout_threshold(p.dropout_p);
     a.inv_keep = 1.f / (1.f - dropout_effective_p(p.dropout_p));
     a.key = philox_make_key(p.seed, p.offset);

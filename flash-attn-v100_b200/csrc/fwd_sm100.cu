@@ -853,7 +853,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         // P come out as 0.
                         const float nm = m == -INFINITY ? 0.f : -m;
                         const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale);
-                        float l0 = 0.f, l1 = 0.f;
+                        uint64_t la = 0ull, lb = 0ull;             // {0.f, 0.f}: four short chains, whose roundings lse shows
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
                             if (q4 == 3) {
@@ -867,10 +867,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                                 const int c = q4 * 32 + cc;
                                 float p0, p1;
                                 f2_unpack(f2_mul(f2_add(f2_pack(SF(c), SF(c + 1)), nm2), log2e2), p0, p1);
-                                p0 = ex2(p0);
-                                p1 = ex2(p1);
-                                if (!P_BF16) f2_unpack(f2_mul(f2_pack(p0, p1), up2), p0, p1);
-                                l0 += p0; l1 += p1;
+                                uint64_t p2 = f2_pack(ex2(p0), ex2(p1));
+                                if (!P_BF16) p2 = f2_mul(p2, up2);
+                                if (cc & 2) lb = f2_add(lb, p2); else la = f2_add(la, p2);
+                                f2_unpack(p2, p0, p1);
                                 if constexpr (DROP == 2) {
                                     const uint32_t word = q4 == 0 ? kb4.x : (q4 == 1 ? kb4.y : (q4 == 2 ? kb4.z : kb4.w));
                                     if (!((word >> cc) & 1u)) p0 = 0.f;
@@ -886,6 +886,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                             tmem_st_32x16(tS + (q4 >> 1) * 64 + (q4 & 1) * 16, hi);
                             tmem_st_32x16(tS + (q4 >> 1) * 64 + 32 + (q4 & 1) * 16, lo);
                         }
+                        float l0, l1;
+                        f2_unpack(f2_add(la, lb), l0, l1);
                         l += l0 + l1;
                         tmem_wait_st();
                         tc_fence_before_sync();
@@ -1276,7 +1278,7 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
     if (n_items > 0x7fffffff - 65536) { set_error("too many work items"); return FA_EUNSUPPORTED; }
     a.n_items = (int)n_items;
     a.scale_log2 = p.scale * kLog2e;
-    a.scale = p.scale;
+    a.scale = pair_score_scale(p);
     a.d = d;
     a.bias = (const float*)p.bias.ptr;
     a.bias_sb = p.bias.stride_b; a.bias_sn = p.bias.stride_n; a.bias_sh = p.bias.stride_h;
