@@ -35,8 +35,10 @@
 // cores -> here: N2048 full 2.9e-6 -> 2.7e-6, N1024 causal 1.8e-6 -> 1.5e-6, with scores 16 times as large
 // 6.1e-5 -> 5.8e-5.  From a forward without error it would be 1.0e-6 -> 5.2e-7, 8.0e-7 -> 3.8e-7 and 3.6e-6 -> 7.3e-6:
 // inside one MMA the tensor core aligns sixteen products and drops what lies below, which shows when scores are large.
-// So the rule takes the one head size whose forward is the TF32 kernel, D = 64, and leaves the others, whose forward
-// is as exact as the CUDA cores', where they were.
+// So the rule takes the calls whose forward is the TF32 kernel (D = 64, aligned tensors, positive scale) and leaves the
+// others, whose forward is as exact as the CUDA cores', where they were; a caller whose o and lse come from another
+// forward offers no scratch.  An infinite operand (or one beyond bf16's largest value) gives NaN here where the
+// CUDA-core kernels may give an infinity: its planes are inf, NaN, NaN.
 #include "fa_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"
@@ -472,11 +474,12 @@ F32Layout f32_layout(const fa_b200_params& p) {
 
 }  // namespace
 
-// Which backward calls the planes serve, and the scratch they take (0: not served).  Other head sizes (kernel comment),
-// a bias and dropout stay on the CUDA cores.
+// Which backward calls the planes serve, and the scratch they take (0: not served): those whose forward the TF32 kernel
+// serves (kernel comment).  Other head sizes, a bias, dropout and tensors that kernel refuses stay on the CUDA cores.
 size_t sm100_f32_bwd_scratch_bytes(const fa_b200_params& p) {
     if (p.dtype != FA_B200_F32 || p.variant != FA_B200_VARIANT_AUTO || p.D != kDim) return 0;
-    if (p.bias.ptr || p.d_scores || p.o_lo.ptr || dropout_threshold(p.dropout_p) != 0u) return 0;
+    const char* why = "";
+    if (p.d_scores || !sm100_tf32_fwd_supports(p, &why)) return 0;
     if (p.B > 65535 / kPlanes || p.H > 65535 || p.B < 1 || p.Nq < 1 || p.Nk < 1) return 0;
     return f32_layout(p).bytes;
 }

@@ -263,12 +263,14 @@ def launch_forward(q, k, v, scale, causal, dropout_p=0.0, seed=0, offset=0, out=
 
 def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, offset=0, out=None,
                     workspace=None, bias=None, d_scores=None, key_lengths=None, causal_shift=0,
-                    dropout_origin=None, o_residual=None, fast=False, keep_bits=None):
+                    dropout_origin=None, o_residual=None, fast=False, keep_bits=None, foreign_forward=False):
     """dq, dk, dv <- fa_b200_bwd.  Counterpart of
     flash_attention_backward_triton_enhanced (kernels/backward_kernel.py:208-318).
     `out=(dq, dk, dv)` and `workspace` (uint8, at least fa_b200_bwd_workspace_bytes)
     use caller-owned buffers instead of allocating (an fp32 call without a `workspace` gets more scratch and, where
-    they serve it, the tensor-core kernels).  `fast`: allow the one-kernel backward where it
+    they serve it, the tensor-core kernels).  `foreign_forward`: o and lse may come from another forward than
+    launch_forward's own choice; fp32 calls then keep the CUDA-core kernels, whose error does not grow behind an exact
+    one.  `fast`: allow the one-kernel backward where it
     is faster (D = 64); dQ is then summed in no fixed order and is not bit-reproducible.
     `keep_bits`: as in launch_forward; (buffer, True) reuses the bits the forward wrote."""
     d_o = _last_dim_contiguous(d_o)
@@ -292,7 +294,7 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
             raise ValueError("d_scores must be a contiguous fp32 (B, H, Nq, Nk) tensor")
         p.d_scores = d_scores.data_ptr()
     lib = _cabi.load()
-    if workspace is None and q.dtype == torch.float32:
+    if workspace is None and q.dtype == torch.float32 and not foreign_forward:
         # planes for the tensor-core backward of fp32 calls; a caller with a workspace of its own gets the CUDA-core one
         nbytes = int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
         if nbytes:
@@ -393,6 +395,7 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
                              keep_bits="new" if dropout_p > 0.0 else None, forward_only=not needs_grad,
                              split_keys=not needs_grad)
         o, lse = res[0], res[1]
+        ctx.simt_forward = getattr(_variant_override, "value", _cabi.VARIANT_AUTO) == _cabi.VARIANT_SIMT
         ctx.keep_bits = res[2] if (len(res) > 2 and needs_grad) else None
         ctx.dropout_origin = dropout_origin
         ctx.has_bias, ctx.has_residual = bias is not None, o_lo is not None
@@ -428,7 +431,8 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
                                      ctx.dropout_p, ctx.seed, ctx.offset, bias=bias, d_scores=d_scores,
                                      key_lengths=ctx.key_lengths, causal_shift=ctx.causal_shift,
                                      dropout_origin=ctx.dropout_origin, o_residual=o_lo, fast=ctx.fast and bias is None,
-                                     keep_bits=(ctx.keep_bits, True) if ctx.keep_bits is not None else None)
+                                     keep_bits=(ctx.keep_bits, True) if ctx.keep_bits is not None else None,
+                                     foreign_forward=ctx.simt_forward)
         if d_scores is not None:
             dims = [i for i in range(4) if bias.shape[i] == 1 and d_scores.shape[i] != 1]
             grad_bias = (d_scores.sum(dim=dims, keepdim=True) if dims else d_scores).to(bias.dtype)
@@ -464,7 +468,8 @@ def flash_attention_backward_enhanced(grad_output, q, k, v, output, lse, max_val
     accepted and ignored: the kernels recompute P from the log-sum-exp alone.
     kwargs: dropout_p and dropout_stream=(seed, offset) to replay a mask; output_residual (the tensor the
     forward filled when it was given one: removes the output's rounding from dQ and dK); bias (the
-    forward's additive bias) and d_scores (zero-filled fp32 (B, H, Nq, Nk) that receives d loss / d scores)."""
+    forward's additive bias) and d_scores (zero-filled fp32 (B, H, Nq, Nk) that receives d loss / d scores);
+    own_forward=True: output and lse are this library's, which lets fp32 calls with D = 64 use the tensor cores."""
     q, k, v, scale = validate_inputs(q, k, v, scale, kwargs.get("bias"), kwargs.get("dropout_p", 0.0))
     seed, offset = kwargs.get("dropout_stream", (0, 0))
     with torch.no_grad():
@@ -473,7 +478,8 @@ def flash_attention_backward_enhanced(grad_output, q, k, v, output, lse, max_val
                                bias=kwargs.get("bias"), d_scores=kwargs.get("d_scores"),
                                key_lengths=kwargs.get("key_lengths"), dropout_origin=kwargs.get("dropout_origin"),
                                o_residual=kwargs.get("output_residual"),
-                               fast=kwargs.get("performance_mode") == "speed")
+                               fast=kwargs.get("performance_mode") == "speed",
+                               foreign_forward=not kwargs.get("own_forward", False))
 
 
 def compare_with_pytorch_attention_enhanced(q, k, v, causal: bool = False,

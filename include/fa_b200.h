@@ -207,9 +207,11 @@ size_t fa_b200_fwd_workspace_bytes(const fa_b200_params* p);
 int fa_b200_bwd(const fa_b200_params* p);
 
 /* Backward with optional scratch beside the workspace.  With at least fa_b200_bwd_scratch_bytes(p) bytes (256-byte
- * aligned; 0: the call has no use for it), fp32 calls of variant AUTO with D = 64, without bias and dropout, run on
- * the tensor cores, every fp32 operand split into three bf16 planes that the scratch holds, with an error no larger
- * than the CUDA-core kernels' behind the same forward; the workspace is not used then.  With less, the same as fa_b200_bwd. */
+ * aligned; 0: the call has no use for it), fp32 calls of variant AUTO whose forward runs on the tensor cores (D = 64,
+ * aligned tensors, positive scale, no bias or dropout) do so too, every fp32 operand split into three bf16 planes that
+ * the scratch holds.  Behind that forward the error is no larger than the CUDA-core kernels'; with o and lse of a more
+ * exact one it can be twice theirs for scores in the tens, so offer no scratch then.  An infinite operand gives NaN.
+ * The workspace is not used.  With less scratch, the same as fa_b200_bwd. */
 int fa_b200_bwd_with_scratch(const fa_b200_params* p, void* scratch, size_t scratch_bytes);
 size_t fa_b200_bwd_scratch_bytes(const fa_b200_params* p);
 

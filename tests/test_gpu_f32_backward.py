@@ -91,3 +91,31 @@ def test_rule_and_strided_gradients(device):
     assert all(torch.equal(a, b) for a, b in zip(out, want))
     assert all((t[..., 0] == 7.0).all() and (t[..., 65:] == 7.0).all() for t in wide)
     assert lib.fa_b200_bwd_with_scratch(ctypes.byref(params(out)), buf.data_ptr(), n - 1) == _cabi.FA_EWORKSPACE   # and no workspace
+
+
+def test_other_forwards_and_what_their_kernel_refuses_stay_on_the_cuda_cores(device):
+    """The planes' error is the CUDA cores' behind the TF32 forward only: an explicit backward, whose o and lse may come
+    from anywhere, a forward run on the CUDA cores, and tensors or scales that forward does not take keep theirs."""
+    gen = torch.Generator().manual_seed(3)
+    q, k, v, g = (torch.randn(1, 130, 2, 64, generator=gen).to(device) for _ in range(4))
+    o, lse = ops.launch_forward(q, k, v, 0.125, True)
+    planes = ops.launch_backward(g, q, k, v, o, lse, 0.125, True)
+    with ops.kernel_variant("simt"):
+        plain = ops.launch_backward(g, q, k, v, o, lse, 0.125, True)
+        o1, lse1 = ops.launch_forward(q, k, v, 0.125, True)
+        plain1 = ops.launch_backward(g, q, k, v, o1, lse1, 0.125, True)
+    same = lambda a, b: all(torch.equal(x, y) for x, y in zip(a, b))
+    assert not same(planes, plain)
+    explicit = lambda **kw: ops.flash_attention_backward_enhanced(g, q, k, v, o, lse, scale=0.125, causal=True, **kw)
+    assert same(explicit(), plain) and same(explicit(own_forward=True), planes)
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    with ops.kernel_variant("simt"):
+        out = ops.EnhancedFlashAttentionV100Function.apply(*leaves, 0.125, True)
+    assert same(torch.autograd.grad(out, leaves, g), plain1)
+    lib = _cabi.load()
+
+    def size(t, scale):
+        p = ops._base_params(t, k, v, o, lse, scale, True, 0.0, 0, 0, d_o=g, dq=q, dk=k, dv=v)
+        return int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
+    odd = torch.zeros(1, 130, 2, 67, device=device)[..., :64]
+    assert size(q, 0.125) > 0 and size(odd, 0.125) == 0 and size(q, -0.125) == 0
