@@ -198,6 +198,20 @@ def saves_output_residual(dtype: torch.dtype) -> bool:
 KEEP_BITS_MAX_BYTES = 4 << 30
 
 
+# The planes of an fp32 backward take one and a half times q, k, v and dO together.  Beyond this size, and where the
+# allocator has no such block, the call runs on the CUDA-core kernels, which need next to nothing.
+F32_PLANES_MAX_BYTES = 8 << 30
+
+
+def _planes_scratch(q: torch.Tensor, nbytes: int) -> Optional[torch.Tensor]:
+    if nbytes == 0 or nbytes > F32_PLANES_MAX_BYTES:
+        return None
+    try:
+        return q.new_empty(nbytes, dtype=torch.uint8)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def _dropout_bits_operand(p, keep_bits, forward_only=False):
     """Point the call at a buffer for its dropout keep bits.  `keep_bits`: None (the kernels draw their
     bits themselves), "new" (allocate; returned for a later call to reuse), or (tensor, ready) with a
@@ -296,10 +310,9 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
     lib = _cabi.load()
     if workspace is None and q.dtype == torch.float32 and not foreign_forward:
         # planes for the tensor-core backward of fp32 calls; a caller with a workspace of its own gets the CUDA-core one
-        nbytes = int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
-        if nbytes:
-            ws = q.new_empty(nbytes, dtype=torch.uint8)
-            rc = lib.fa_b200_bwd_with_scratch(ctypes.byref(p), ws.data_ptr(), nbytes)
+        ws = _planes_scratch(q, int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p))))
+        if ws is not None:
+            rc = lib.fa_b200_bwd_with_scratch(ctypes.byref(p), ws.data_ptr(), ws.numel())
             _cabi.raise_for_status(rc, "fa_b200_bwd")
             return dq, dk, dv
     nbytes = int(lib.fa_b200_bwd_workspace_bytes(ctypes.byref(p)))

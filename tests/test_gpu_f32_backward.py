@@ -119,3 +119,25 @@ def test_other_forwards_and_what_their_kernel_refuses_stay_on_the_cuda_cores(dev
         return int(lib.fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
     odd = torch.zeros(1, 130, 2, 67, device=device)[..., :64]
     assert size(q, 0.125) > 0 and size(odd, 0.125) == 0 and size(q, -0.125) == 0
+
+
+def test_without_room_for_the_planes_the_cuda_cores_serve_the_call(device, monkeypatch):
+    q = torch.randn(1, 70, 3, 64, device=device)
+    o, lse = ops.launch_forward(q, q, q, 0.125, True)
+    run = lambda: ops.launch_backward(q, q, q, q, o, lse, 0.125, True)
+    planes = run()
+    with ops.kernel_variant("simt"):
+        plain = run()
+    same = lambda a, b: all(torch.equal(x, y) for x, y in zip(a, b))
+    assert not same(planes, plain)
+    with monkeypatch.context() as m:
+        m.setattr(ops, "F32_PLANES_MAX_BYTES", 1000)
+        assert same(run(), plain)
+
+    def full(self, size, **kw):                       # the allocator has nothing for a large byte buffer
+        if kw.get("dtype") == torch.uint8 and size > 100000:
+            raise torch.cuda.OutOfMemoryError("no block")
+        return torch.empty(size, dtype=kw.get("dtype", self.dtype), device=self.device)
+    with monkeypatch.context() as m:
+        m.setattr(torch.Tensor, "new_empty", full)
+        assert same(run(), plain)
