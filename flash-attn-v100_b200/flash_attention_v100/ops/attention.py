@@ -285,9 +285,11 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
     they serve it, the tensor-core kernels).  `foreign_forward`: o and lse may come from another forward than
     launch_forward's own choice; fp32 calls then keep the CUDA-core kernels, whose error does not grow behind an exact
     one.  `fast`: allow the one-kernel backward where it
-    is faster (D = 64); dQ is then summed in no fixed order and is not bit-reproducible.
+    is faster (16-bit calls with D = 64 and no bias; others run as without it); dQ is then summed in no fixed order and is not bit-reproducible.
     `keep_bits`: as in launch_forward; (buffer, True) reuses the bits the forward wrote."""
     d_o = _last_dim_contiguous(d_o)
+    # a preference, not a demand on the library: an explicit variant would be refused for the other calls
+    fast = fast and q.dtype != torch.float32 and q.shape[3] == 64 and bias is None
     if out is not None:
         dq, dk, dv = out
     else:
@@ -443,7 +445,7 @@ class EnhancedFlashAttentionV100Function(torch.autograd.Function):
         dq, dk, dv = launch_backward(grad_output, q, k, v, o, lse, ctx.scale, ctx.causal,
                                      ctx.dropout_p, ctx.seed, ctx.offset, bias=bias, d_scores=d_scores,
                                      key_lengths=ctx.key_lengths, causal_shift=ctx.causal_shift,
-                                     dropout_origin=ctx.dropout_origin, o_residual=o_lo, fast=ctx.fast and bias is None,
+                                     dropout_origin=ctx.dropout_origin, o_residual=o_lo, fast=ctx.fast,
                                      keep_bits=(ctx.keep_bits, True) if ctx.keep_bits is not None else None,
                                      foreign_forward=ctx.simt_forward)
         if d_scores is not None:
