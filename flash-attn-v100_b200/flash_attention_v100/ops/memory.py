@@ -34,6 +34,28 @@ def backward_workspace_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, nu
     return int(_cabi.load().fa_b200_bwd_workspace_bytes(ctypes.byref(p)))
 
 
+def backward_scratch_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, num_heads: int, head_dim: int,
+                           dtype: torch.dtype, num_heads_kv: int = None) -> int:
+    """Bytes the default backward allocates in place of that workspace where the tensor cores serve an fp32 call (the
+    bf16 planes of q, dO, k and v), or 0."""
+    from .attention import F32_PLANES_MAX_BYTES
+    p = _sizes_params(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype, num_heads_kv)
+    n = int(_cabi.load().fa_b200_bwd_scratch_bytes(ctypes.byref(p)))
+    return n if n <= F32_PLANES_MAX_BYTES else 0
+
+
+def forward_scratch_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, num_heads: int, head_dim: int,
+                          dtype: torch.dtype, num_heads_kv: int = None) -> int:
+    """Most bytes a forward without gradients allocates to share its keys out over the SMs (with or without a causal
+    mask and key counts); 0 without a GPU."""
+    p = _sizes_params(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype, num_heads_kv)
+    most = 0
+    for p.causal in (0, 1):
+        for p.kv_lengths in (None, 16):               # (a size query does not read them)
+            most = max(most, int(_cabi.load().fa_b200_fwd_workspace_bytes(ctypes.byref(p))))
+    return most
+
+
 def dropout_bits_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, num_heads: int, head_dim: int,
                        dtype: torch.dtype, dropout_p: float, num_heads_kv: int = None) -> int:
     """Bytes of the buffer that holds a call's dropout keep bits (two bits of storage per score: one per
@@ -83,7 +105,11 @@ def estimate_peak_memory_usage(batch_size: int, seq_len_q: int, seq_len_k: int, 
     bwd = 0
     if include_gradients:
         bwd = t_q * 2 + t_k * 2                        # dO, dQ, dK, dV
-        bwd += backward_workspace_bytes(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype)
+        sizes = (batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype)
+        planes = backward_scratch_bytes(*sizes) if dropout_p == 0.0 else 0
+        bwd += planes or backward_workspace_bytes(*sizes)
+    elif dropout_p == 0.0:
+        fwd += forward_scratch_bytes(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype)
     bits = dropout_bits_bytes(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype, dropout_p) \
         if dropout_p > 0.0 else 0
     if not include_gradients:
@@ -104,5 +130,5 @@ def get_memory_statistics(device=None) -> Dict[str, float]:
             "peak_allocated_mb": torch.cuda.max_memory_allocated(device) * mb}
 
 
-__all__ = ["backward_workspace_bytes", "allocate_attention_workspace", "free_attention_workspace",
+__all__ = ["backward_workspace_bytes", "backward_scratch_bytes", "forward_scratch_bytes", "allocate_attention_workspace", "free_attention_workspace",
            "estimate_peak_memory_usage", "get_memory_statistics"]

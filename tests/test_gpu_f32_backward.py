@@ -141,3 +141,18 @@ def test_without_room_for_the_planes_the_cuda_cores_serve_the_call(device, monke
     with monkeypatch.context() as m:
         m.setattr(torch.Tensor, "new_empty", full)
         assert same(run(), plain)
+
+
+def test_memory_estimate_covers_the_planes(device):
+    from flash_attention_v100.ops import memory
+    B, N, H = 2, 1000, 4
+    q, g = (torch.randn(B, N, H, 64, device=device) for _ in range(2))
+    o, lse = ops.launch_forward(q, q, q, 0.125, True)
+    est = memory.estimate_peak_memory_usage(B, N, N, H, 64, torch.float32)["total_memory_mb"] * 2 ** 20
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated(device)
+    torch.cuda.reset_peak_memory_stats(device)
+    ops.launch_backward(g, q, q, q, o, lse, 0.125, True)
+    torch.cuda.synchronize()
+    held = (3 * q.numel() + 2 * o.numel()) * 4 + lse.numel() * 4          # q, k, v, o, dO and lse of the estimate
+    assert held + torch.cuda.max_memory_allocated(device) - before <= est + (1 << 16)

@@ -105,6 +105,12 @@ def test_workspace_estimates():
     est = memory.estimate_peak_memory_usage(4, 4096, 4096, 32, 128, torch.bfloat16)
     assert est["total_memory_mb"] > 8 * 128          # eight 134 MB tensors at least
     assert est["total_memory_mb"] < 4 * 32 * 4096 * 4096 * 2 / 2 ** 20   # far below the N^2 scores
+    # fp32 on the tensor cores: three 16-bit planes of q, dO, k and v in the backward
+    planes = memory.backward_scratch_bytes(2, 1024, 1024, 12, 64, torch.float32)
+    assert planes >= 4 * 3 * 2 * 2 * 1024 * 12 * 64
+    small = memory.estimate_peak_memory_usage(2, 1024, 1024, 12, 64, torch.float32)
+    assert small["gradient_memory_mb"] * 2 ** 20 >= planes + 4 * 4 * 2 * 1024 * 12 * 64
+    assert memory.backward_scratch_bytes(2, 1024, 1024, 12, 96, torch.float32) == 0
     # dropout on the tensor-core kernels: the call's keep bits, two bits of storage per score
     bits = memory.dropout_bits_bytes(32, 2048, 2048, 16, 64, torch.bfloat16, 0.1)
     assert bits == 32 * 16 * 2048 * 2048 // 4
