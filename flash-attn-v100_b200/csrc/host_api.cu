@@ -431,16 +431,20 @@ int fa_b200_bwd_static(const fa_b200_params* p) {
     return variant != FA_B200_VARIANT_SIMT ? sm100_bwd(q, ws) : simt_bwd(q, ws);
 }
 
-// Static tile table.  Tensor-core rows report the constants the sm_100a kernels are compiled from
-// (tile_config.cuh); everything else is served by 64x64 CUDA-core tiles.  The same tiles serve both
+// Static tile table.  16-bit rows whose head size is a multiple of 8 report the constants the sm_100a kernels are
+// compiled from (tile_config.cuh; sizes other than 64 and 128 run in tiles padded to the next of the two); everything
+// else reports the 64x64 CUDA-core tiles that any such call can run on (fp32 calls with D = 64 go to tensor-core
+// kernels with tiles of their own where those cover them, fwd_tf32_sm100.cu and bwd_f32_sm100.cu).  The same tiles serve both
 // masks: `causal` is part of the reference's lookup key (config.py:288-348) and changes no row here.
 int fa_b200_tile_config(int D, int dtype, int causal, int backward, fa_b200_tile* out) {
     if (!out) { set_error("out is null"); return FA_EINVAL; }
     if (D <= 0 || D > 128) { set_error("no tile for D=%d", D); return FA_EUNSUPPORTED; }
     (void)causal;
     memset(out, 0, sizeof(*out));
-    bool tc = (dtype == FA_B200_F16 || dtype == FA_B200_BF16) && (D == 64 || D == 128);
+    const bool tc = (dtype == FA_B200_F16 || dtype == FA_B200_BF16) && D % 8 == 0;
+    const bool one_kernel = tile::bwd_one_kernel(D);
     if (tc) {
+        D = D <= 64 ? 64 : 128;
         out->variant = FA_B200_VARIANT_TCGEN05_2PASS;     // what AUTO runs
         out->block_m = tile::kBlockM;
         out->block_n = tile::kBlockN;
@@ -450,7 +454,7 @@ int fa_b200_tile_config(int D, int dtype, int causal, int backward, fa_b200_tile
         out->num_warps = backward ? tile::kBwdWarps : tile::kFwdWarps;
         out->regs_softmax = backward ? 0 : tile::kFwdRegsSoftmax;
         out->regs_other = backward ? 0 : tile::kFwdRegsOther;
-        out->one_kernel_backward = backward && tile::bwd_one_kernel(D) ? 1 : 0;   // available on request (TCGEN05)
+        out->one_kernel_backward = backward && one_kernel ? 1 : 0;   // available on request (TCGEN05)
     } else {
         out->variant = FA_B200_VARIANT_SIMT;
         out->block_m = 64;

@@ -4,8 +4,10 @@ Replaces the reference's run-time tuner (kernels/autotuning.py:118-1018,
 never reached from its call path) and the seq-len buckets of
 config.get_enhanced_config (config.py:288-348).  The table lives in the shared
 library: fa_b200_tile_config reports the constants of csrc/tile_config.cuh, the
-header the kernels themselves are compiled from, so what this module returns is
-what runs.
+header the kernels themselves are compiled from, so for 16-bit calls without a
+bias what this module returns is what runs.  fp32 rows report the CUDA-core
+tiles; fp32 calls with D = 64 mostly run on tensor-core kernels whose tiles are
+their own.
 """
 from __future__ import annotations
 

@@ -56,8 +56,9 @@ typedef enum fa_b200_status {
 } fa_b200_status;
 
 /* Which kernel family serves the call.  AUTO: the tensor-core family where it covers the call
- * (fp16/bf16, D in {64, 128}, aligned tensors, no bias), in its deterministic form, else CUDA-core
- * tiles. */
+ * (fp16/bf16, D a multiple of 8 up to 128, aligned tensors, positive scale, with or without a bias; fp32 with
+ * D = 64, no bias or dropout), in its deterministic form, else CUDA-core tiles.  An explicit TCGEN05 or
+ * TCGEN05_2PASS asks for the instances with one 16-bit P (D in {64, 128}, no bias) and is refused elsewhere. */
 typedef enum fa_b200_variant {
     FA_B200_VARIANT_AUTO    = 0,
     FA_B200_VARIANT_SIMT    = 1,  /* CUDA-core tiles: any D <= 128, all dtypes, fp32 exact */

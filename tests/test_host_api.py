@@ -92,7 +92,12 @@ def test_tile_table_keys_and_families():
         assert key in cfg
     assert cfg["BLOCK_K"] == 128 and cfg["VARIANT"] == "tcgen05_2pass"     # what AUTO runs: the deterministic form
     assert tile_table.lookup(64, torch.float32)["VARIANT"] == "simt"
-    assert tile_table.lookup(96, torch.float16)["VARIANT"] == "simt"
+    # 16-bit head sizes that are multiples of 8 run on the tensor cores, in tiles padded to 64 or 128 columns
+    assert tile_table.lookup(96, torch.float16)["VARIANT"] == "tcgen05_2pass"
+    assert tile_table.lookup(96, torch.float16)["NUM_STAGES"] == tile_table.lookup(128, torch.float16)["NUM_STAGES"]
+    assert tile_table.lookup(40, torch.bfloat16, backward=True)["W_STAGES"] == tile_table.lookup(64, torch.bfloat16, backward=True)["W_STAGES"]
+    assert not tile_table.lookup(40, torch.bfloat16, backward=True)["ONE_KERNEL_BACKWARD"]
+    assert tile_table.lookup(20, torch.float16)["VARIANT"] == "simt"
     with pytest.raises(ValueError):
         tile_table.lookup(256, torch.float16)
     cfg8 = fa.get_enhanced_config(4096, 128, 8)
