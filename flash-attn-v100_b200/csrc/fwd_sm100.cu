@@ -1188,14 +1188,20 @@ int64_t column_units(const fa_b200_params& p, int q_per_tile, int n_pairs) {
 // Packing.  The query heads that share a K/V head read the same keys, so with few queries they belong into one tile:
 // 128 / pack queries of `pack` = H / Hkv heads.  Taken when it leaves at least 5 % fewer (pair, key block) units;
 // with many queries both forms have the same number and the plain one stays.
-// Splitting.  Whole pairs dealt round robin leave SMs idle when there are few of them, or when a few keys of one
-// batch entry make one pair long.  The call's units are then cut into one equal range per SM.  What that costs
+// Splitting.  Whole pairs dealt round robin leave SMs idle when there are few of them, or when one batch entry's many
+// keys make its pairs long.  The call's units are then cut into one equal range per SM.  What that costs
 // (partial sums through memory and a second launch) is about kMergeUnits units, so the ranges have to be that much
 // shorter than the longest round-robin share, and a tenth.  B200, before -> after, both rules together:
 // 32 requests of 2048-4096 keys, 1 query, H32 Hkv8 D128 bf16: 304 -> 84 us (403 MB of keys and values, 62 us at the
 // copy rate); 1 request, 700 queries on 8892 keys, same heads: 240 -> 112 us (98 GFLOP, 60 us at cuBLAS's rate).
 // Decoding as one pair per unit, without the one-tile kernel (SCHED = 2), took 116 us: S, softmax and P V of one tile
 // are a serial chain of about 2.7 us a block, and two stages of K and V cover too little of the memory's latency.
+// Key counts are on the device, so the rule sees Nk.  Ranges are as even for unequal counts as for equal ones, whole
+// pairs are not, and a block of the one-tile kernel takes about three quarters of the other kernel's time: with counts
+// its ranges are taken at that.  Whole pairs -> ranges, 148 requests, 1 query, H8 Hkv8 D128, Nk 4096 (eight whole pairs
+// an SM): all counts 4096 516 -> 384 us, counts from half of it 418 -> 300, all 1024 119 -> 114, all 256 48 -> 61.
+// Calls of several tiles have no such gain: 8 requests of 2048 queries on 2048 keys, H16 D128, all counts 2048
+// 282 -> 292 us, from half of it 242 -> 283, so nothing is taken off there.
 constexpr int kMergeUnits = 4;
 FwdPlan plan_schedule(const fa_b200_params& p, int D, int sms, bool free) {
     FwdPlan pl;
@@ -1216,9 +1222,10 @@ FwdPlan plan_schedule(const fa_b200_params& p, int D, int sms, bool free) {
     const int64_t total = (int64_t)p.B * pl.heads * col;
     pl.ctas = (int)(total < sms ? total : sms);
     int64_t ranges = (total + pl.ctas - 1) / pl.ctas;
-    if (p.kv_lengths) ranges = (3 * ranges + 3) / 4;         // counts below Nk: the longest share is Nk's, a range the mean's
+    const bool one_tile = p.Nq <= pl.q_per_tile;
+    if (p.kv_lengths && one_tile) ranges = (3 * ranges + 3) / 4;
     if (total < (1 << 30) && whole * 9 > (ranges + kMergeUnits) * 10) {
-        pl.sched = p.Nq <= pl.q_per_tile ? 2 : 1;
+        pl.sched = one_tile ? 2 : 1;
         const int tiles = (int)(((int64_t)p.Nq + pl.q_per_tile - 1) / pl.q_per_tile);
         const int rows = tiles > 1 ? 2 * kBlockM : p.Nq * pl.pack;
         pl.part_rows = (int)align_up((size_t)rows, 32);

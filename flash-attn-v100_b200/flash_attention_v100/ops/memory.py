@@ -47,7 +47,7 @@ def backward_scratch_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, num_
 def forward_scratch_bytes(batch_size: int, seq_len_q: int, seq_len_k: int, num_heads: int, head_dim: int,
                           dtype: torch.dtype, num_heads_kv: int = None) -> int:
     """Most bytes a forward without gradients allocates to share its keys out over the SMs (with or without a causal
-    mask and key counts); 0 without a GPU."""
+    mask, with or without key counts); 0 without a GPU."""
     p = _sizes_params(batch_size, seq_len_q, seq_len_k, num_heads, head_dim, dtype, num_heads_kv)
     most = 0
     for p.causal in (0, 1):

@@ -102,6 +102,18 @@ def test_rule_leaves_the_rest_alone(device):
         assert torch.equal(o, o0) and torch.equal(lse, lse0)
 
 
+def test_key_counts_alone_do_not_cut_calls_of_several_tiles(device):
+    """Whole pairs that fill the SMs evenly stay whole where a unit costs the same either way, whatever the counts."""
+    sms = torch.cuda.get_device_properties(device).multi_processor_count
+    q, k = (torch.zeros(sms // 2, n, 2, 128, device=device, dtype=torch.bfloat16) for n in (256, 3000))
+    counts = torch.full((sms // 2,), 3000, device=device, dtype=torch.int32)
+    for given in (False, True):
+        p = ops._base_params(q, k, k, q, torch.empty(1, device=device), 0.125, False, 0.0, 0, 0)
+        if given:
+            p.kv_lengths = counts.data_ptr()
+        assert _cabi.load().fa_b200_fwd_workspace_bytes(ctypes.byref(p)) == 0
+
+
 def test_rows_with_nan_and_infinite_scores(device):
     """A NaN in one range's keys reaches the row's result, as with whole pairs; other columns stay clean."""
     q, k = _rand((1, 4, 2, 64), torch.float16, 1).to(device), _rand((1, 1500, 2, 64), torch.float16, 2).to(device)
