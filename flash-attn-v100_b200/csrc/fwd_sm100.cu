@@ -154,6 +154,7 @@ struct FwdArgs {
     // Split schedule: the call's (pair, key block) units are cut into gridDim.x equal ranges; a pair that lies in
     // several ranges leaves partial results for fwd_merge_kernel.
     int part_rows;                 // rows a partial's slot holds
+    int start_cost;                // one tile: units a pair's start counts as, in front of its key blocks (plan_schedule)
     float4* part_o;                // [2 * gridDim.x slots][D / 4][part_rows], sums not yet divided
     float2* part_ml;               // [2 * gridDim.x slots][part_rows]: maximum (log2 units), row sum (< 0: no block visited)
     int4* part_meta;               // [gridDim.x]: batch, column, pair, number of ranges (0: none starts here)
@@ -179,9 +180,10 @@ __device__ __forceinline__ int pair_blocks(const FwdArgs& a, int pair, int nk) {
     return n0 > n1 ? n0 : n1;
 }
 
-// Where a CTA's range of units starts and how long it is (split schedule), left in shared memory for every role.
+// Where a CTA's range of units starts and how long it is (split schedule), left in shared memory for every role.  A pair
+// has start_cost units that stand for its start, then one for each key block; `at` is the range's place in its first pair.
 // `ctas`: CTAs that have a range (with per-batch key counts the units can be fewer than the CTAs; every range has one).
-struct RangeStart { int b, h, pair, block, units, total, ctas; };
+struct RangeStart { int b, h, pair, at, units, total, ctas; };
 __device__ __forceinline__ int range_begin(int cta, int ctas, int total) { return (int)((int64_t)cta * total / ctas); }
 
 __device__ __forceinline__ int warp_scan(int v, int lane) {
@@ -205,12 +207,25 @@ __device__ __forceinline__ int warp_find(int n, int lane, int& target, Cost cost
     }
     return n - 1;
 }
-// One warp: the costs are the pairs' key blocks; with per-batch key counts a batch entry has a total of its own.
+// The units of a pair that a walk with `units` left takes from place `at` on, as key blocks [j0, j1); returns what is left
+// for the next pairs, nothing where it would end before a pair's first block (find_range sees to the first pair).
+template <int SCHED> __device__ __forceinline__ int start_cost(const FwdArgs& a) { return SCHED == 2 ? a.start_cost : 0; }
+template <int SCHED>
+__device__ __forceinline__ int take_units(const FwdArgs& a, int at, int units, Stretch& s) {
+    const int n = s.n[0] > s.n[1] ? s.n[0] : s.n[1], c0 = start_cost<SCHED>(a);
+    s.j0 = max(at - c0, 0);
+    s.j1 = min(n, at + units - c0);
+    const int left = at + units - c0 - n;
+    return left > c0 ? left : 0;
+}
+// One warp: the costs are the pairs' units; with per-batch key counts a batch entry has a total of its own.
+template <int SCHED>
 __device__ __forceinline__ void find_range(const FwdArgs& a, int lane, volatile RangeStart* out) {
+    const int c0 = start_cost<SCHED>(a);
     auto column = [&](int b) {                       // units of one (batch, column): serial, every lane its own b
         const int nk = kv_len_of(a.kv_len, b, a.Nk);
         int sum = 0;
-        for (int pr = 0; pr < a.n_pairs; ++pr) sum += pair_blocks(a, pr, nk);
+        for (int pr = 0; pr < a.n_pairs; ++pr) sum += pair_blocks(a, pr, nk) + c0;
         return sum;
     };
     int total = 0, col = 0;
@@ -218,7 +233,7 @@ __device__ __forceinline__ void find_range(const FwdArgs& a, int lane, volatile 
         for (int b = lane; b < a.B; b += 32) total += a.heads * column(b);
         total = __shfl_sync(0xffffffffu, warp_scan(total, lane), 31);
     } else {
-        for (int pr = lane; pr < a.n_pairs; pr += 32) col += pair_blocks(a, pr, a.Nk);
+        for (int pr = lane; pr < a.n_pairs; pr += 32) col += pair_blocks(a, pr, a.Nk) + c0;
         col = __shfl_sync(0xffffffffu, warp_scan(col, lane), 31);
         total = a.B * a.heads * col;
     }
@@ -237,9 +252,9 @@ __device__ __forceinline__ void find_range(const FwdArgs& a, int lane, volatile 
     const int h = at / col;
     at -= h * col;
     const int nk = kv_len_of(a.kv_len, b, a.Nk);
-    const int pair = warp_find(a.n_pairs, lane, at, [&](int i) { return pair_blocks(a, i, nk); });
+    const int pair = warp_find(a.n_pairs, lane, at, [&](int i) { return pair_blocks(a, i, nk) + c0; });
     if (lane == 0) {
-        out->b = b; out->h = h; out->pair = pair; out->block = at; out->units = units; out->total = total; out->ctas = ctas;
+        out->b = b; out->h = h; out->pair = pair; out->at = at; out->units = at + units > c0 ? units : 0; out->total = total; out->ctas = ctas;
     }
 }
 
@@ -275,57 +290,52 @@ template <> struct WorkLoop<0> {       // whole pairs, round robin
         return true;
     }
 };
-template <> struct WorkLoop<1> {       // split schedule: the CTA's range of units
+template <int SCHED> struct WorkLoop {       // split schedule: the CTA's range of units
     static constexpr int kSub = 1;
-    int b, h, pair, block, units;
+    int b, h, pair, at, units;
     __device__ __forceinline__ WorkLoop(const FwdArgs&, const volatile RangeStart* r)
-        : b(r->b), h(r->h), pair(r->pair), block(r->block), units(r->units) {}
+        : b(r->b), h(r->h), pair(r->pair), at(r->at), units(r->units) {}
     __device__ __forceinline__ bool more(const FwdArgs&) const { return units > 0; }
     __device__ __forceinline__ void advance() {}
     __device__ __forceinline__ bool get(const FwdArgs& a, int, Stretch& s) {
         s.pair = pair; s.h = h; s.b = b;
         s.nk = kv_len_of(a.kv_len, b, a.Nk);
         s.n[0] = num_blocks(a, a.q_per_tile, pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, pair, 1, s.nk);
-        const int n = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
-        s.j0 = block;
-        s.j1 = n - block < units ? n : block + units;
-        units -= s.j1 - s.j0;
-        block = 0;
+        units = take_units<SCHED>(a, at, units, s);
+        at = 0;
         if (++pair == a.n_pairs) { pair = 0; if (++h == a.heads) { h = 0; ++b; } }
         return true;
     }
 };
-template <> struct WorkLoop<2> : WorkLoop<1> { using WorkLoop<1>::WorkLoop; };
 
 // The softmax warps' form of the walk: its state and the current stretch lie in shared memory, a record per warp, and
 // the epilogue reads the stretch again, so that no register holds them while a block's 128 scores are worked on.
 // Held in registers, the D = 128 kernel spilled 424 bytes instead of 60 and the chunk below took 152 us instead of 112.
-struct WalkRecord { int b, h, pair, block, units, cur_pair, cur_h, cur_b, cur_j0, cur_j1; };
-template <int SCHED> struct SoftmaxLoop : WorkLoop<SCHED> {
-    __device__ __forceinline__ SoftmaxLoop(const FwdArgs& a, const volatile RangeStart* r, volatile WalkRecord*) : WorkLoop<SCHED>(a, r) {}
+struct WalkRecord { int b, h, pair, at, units, cur_pair, cur_h, cur_b, cur_j0, cur_j1; };
+template <int SCHED> struct SoftmaxLoop;
+template <> struct SoftmaxLoop<0> : WorkLoop<0> {
+    __device__ __forceinline__ SoftmaxLoop(const FwdArgs& a, const volatile RangeStart* r, volatile WalkRecord*) : WorkLoop<0>(a, r) {}
     __device__ __forceinline__ void again(const FwdArgs&, Stretch&) const {}
 };
-struct SplitSoftmaxLoop {
+template <int SCHED> struct SoftmaxLoop {
     static constexpr int kSub = 1;
     volatile WalkRecord* rec;
-    __device__ __forceinline__ SplitSoftmaxLoop(const FwdArgs&, const volatile RangeStart* r, volatile WalkRecord* w) : rec(w) {
-        rec->b = r->b; rec->h = r->h; rec->pair = r->pair; rec->block = r->block; rec->units = r->units;    // every lane the same
+    __device__ __forceinline__ SoftmaxLoop(const FwdArgs&, const volatile RangeStart* r, volatile WalkRecord* w) : rec(w) {
+        rec->b = r->b; rec->h = r->h; rec->pair = r->pair; rec->at = r->at; rec->units = r->units;    // every lane the same
         __syncwarp();
     }
     __device__ __forceinline__ bool more(const FwdArgs&) const { return rec->units > 0; }
     __device__ __forceinline__ void advance() {}
     __device__ __forceinline__ bool get(const FwdArgs& a, int, Stretch& s) {
         int b = rec->b, h = rec->h, pair = rec->pair;
-        const int block = rec->block, units = rec->units;
+        const int at = rec->at, units = rec->units;
         s.pair = pair; s.h = h; s.b = b;
         s.nk = kv_len_of(a.kv_len, b, a.Nk);
         s.n[0] = num_blocks(a, a.q_per_tile, pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, pair, 1, s.nk);
-        const int n = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
-        s.j0 = block;
-        s.j1 = n - block < units ? n : block + units;
+        const int left = take_units<SCHED>(a, at, units, s);
         if (++pair == a.n_pairs) { pair = 0; if (++h == a.heads) { h = 0; ++b; } }
         __syncwarp();                                  // every lane has read
-        rec->b = b; rec->h = h; rec->pair = pair; rec->block = 0; rec->units = units - (s.j1 - s.j0);
+        rec->b = b; rec->h = h; rec->pair = pair; rec->at = 0; rec->units = left;
         rec->cur_pair = s.pair; rec->cur_h = s.h; rec->cur_b = s.b; rec->cur_j0 = s.j0; rec->cur_j1 = s.j1;
         __syncwarp();
         return true;
@@ -336,8 +346,6 @@ struct SplitSoftmaxLoop {
         s.n[0] = num_blocks(a, a.q_per_tile, s.pair, 0, s.nk); s.n[1] = num_blocks(a, a.q_per_tile, s.pair, 1, s.nk);
     }
 };
-template <> struct SoftmaxLoop<1> : SplitSoftmaxLoop { using SplitSoftmaxLoop::SplitSoftmaxLoop; };
-template <> struct SoftmaxLoop<2> : SplitSoftmaxLoop { using SplitSoftmaxLoop::SplitSoftmaxLoop; };
 
 // P is stored as 2^(S c - m + kPShift): with the lazily refreshed maximum P <= 2^8, so the shifted value
 // stays below 2^14 in fp16 and entries down to 2^-20 of the row's largest keep full precision.
@@ -397,7 +405,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         prefetch_tensormap(&map_k);
         prefetch_tensormap(&map_v);
     }
-    if (FREE && warp == 11) find_range(a, lane, range);
+    if (FREE && warp == 11) find_range<SCHED>(a, lane, range);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -1167,6 +1175,7 @@ struct FwdPlan {
     int pack, q_per_tile, heads, n_pairs;
     int sched;                     // FwdCfg's SCHED
     int ctas, part_rows;           // split schedule: ranges, rows per slot
+    int start_cost;                // FwdArgs
     size_t ml_off, meta_off, bytes;        // workspace: partial sums | maxima and row sums | ranges' pairs
 };
 
@@ -1203,6 +1212,14 @@ int64_t column_units(const fa_b200_params& p, int q_per_tile, int n_pairs) {
 // Calls of several tiles have no such gain: 8 requests of 2048 queries on 2048 keys, H16 D128, all counts 2048
 // 282 -> 292 us, from half of it 242 -> 283, so nothing is taken off there.
 constexpr int kMergeUnits = 4;
+// Starts.  Q, the first S and the epilogue of a pair take as long as three blocks of the one-tile kernel (4.5 of
+// 1.3 us), and ranges equal in blocks alone are not equal in time where counts make some pairs short.  With counts a
+// pair's start therefore counts as that many units there, unless ranges are so short (in blocks, by Nk) that hardly any
+// holds a whole pair.  Ranges equal in blocks -> so, 1 query, counts from 1 to an eighth of the cache: 148 requests, H8
+// Hkv8 D64, Nk 8192 109 -> 83 us, D128, Nk 4096 115 -> 101, 37 requests, H32 Hkv8 D128, Nk 4096 38 -> 30; 32 requests
+// of 2048-4096 keys, H32 Hkv8 D128 84 -> 82.  Without counts pairs are alike, and in the kernel of several tiles the
+// walk with starts took registers from the softmax (700 queries on 8892 keys 93 -> 100 us).
+constexpr int kLongRange = 8;
 FwdPlan plan_schedule(const fa_b200_params& p, int D, int sms, bool free) {
     FwdPlan pl;
     memset(&pl, 0, sizeof(pl));
@@ -1224,8 +1241,9 @@ FwdPlan plan_schedule(const fa_b200_params& p, int D, int sms, bool free) {
     int64_t ranges = (total + pl.ctas - 1) / pl.ctas;
     const bool one_tile = p.Nq <= pl.q_per_tile;
     if (p.kv_lengths && one_tile) ranges = (3 * ranges + 3) / 4;
-    if (total < (1 << 30) && whole * 9 > (ranges + kMergeUnits) * 10) {
+    if (total < (1 << 28) && whole * 9 > (ranges + kMergeUnits) * 10) {
         pl.sched = one_tile ? 2 : 1;
+        pl.start_cost = p.kv_lengths && one_tile && ranges >= kLongRange ? 3 : 0;
         const int tiles = (int)(((int64_t)p.Nq + pl.q_per_tile - 1) / pl.q_per_tile);
         const int rows = tiles > 1 ? 2 * kBlockM : p.Nq * pl.pack;
         pl.part_rows = (int)align_up((size_t)rows, 32);
@@ -1277,6 +1295,7 @@ int launch(const fa_b200_params& p, void* ws, size_t ws_bytes) {
     a.pack = plan.pack; a.q_per_tile = plan.q_per_tile; a.heads = plan.heads;
     a.n_pairs = plan.n_pairs;
     a.part_rows = plan.part_rows;
+    a.start_cost = plan.start_cost;
     a.part_o = (float4*)ws;
     a.part_ml = (float2*)((char*)ws + plan.ml_off);
     a.part_meta = (int4*)((char*)ws + plan.meta_off);

@@ -76,6 +76,17 @@ def test_many_batch_entries(device):
     _check(device, torch.bfloat16, 40, 1, 1280, 4, 1, 128)
 
 
+@pytest.mark.parametrize("longest", [128, 300, 2900])
+def test_many_pairs_of_a_few_blocks(device, longest):
+    """Ranges that hold many pairs, end inside the units that stand for a pair's start, or hold nothing else."""
+    gen = torch.Generator().manual_seed(longest)
+    lengths = torch.randint(1, longest + 1, (64,), generator=gen).tolist()
+    _check(device, torch.float16, 64, 1, 3000, 4, 4, 64, lengths=lengths)
+    _check(device, torch.bfloat16, 64, 3, 3000, 8, 2, 128, lengths=lengths[::-1])
+    _check(device, torch.float16, 25, 150, 3000, 4, 4, 128, lengths=lengths[:25])
+    _check(device, torch.float16, 5, 1, 6000, 32, 32, 64, lengths=[longest, 1, 1, 6000, 1])
+
+
 @pytest.mark.parametrize("N", [1664, 2501])
 def test_prompts(device, N):
     """Self-attention of one request with few heads: pairs of very different length under the causal mask."""
