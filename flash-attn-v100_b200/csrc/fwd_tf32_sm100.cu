@@ -21,8 +21,8 @@
 // S(j+1) is computed and K(j+1), V(j+1) are split while the softmax of block j runs: with the splits in the softmax
 // warps, one S buffer and one ring for K and V together, a block was one serial chain of 2.8 us (B2 N1024 H12 causal
 // forward 45 -> 32 us).
-// Head dimension 64; no dropout and no bias (those calls, other head dimensions and the fp32 backward
-// are served by the CUDA-core tiles).  Every mbarrier wait is bounded (sm100_ptx.cuh).
+// Head dimension 64; no dropout and no bias (those calls and other head dimensions are served by the CUDA-core
+// tiles; the fp32 backward has kernels of its own, bwd_f32_sm100.cu).  Every mbarrier wait is bounded (sm100_ptx.cuh).
 #include "fa_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tma_host.cuh"

@@ -1,8 +1,10 @@
 // C-ABI layer of libfa_b200.so: argument validation, kernel-family choice,
 // workspace layout, the static tile table, error strings and the host side of
-// the dropout stream.  Everything here is O(1) host work per call: no tensor
-// scans and no device synchronisation (the reference's launchers do both:
-// utils.py:227-254, kernels/forward_kernel.py:308-313).
+// the dropout stream.  No tensor scans and no device synchronisation (the
+// reference's launchers do both: utils.py:227-254, kernels/forward_kernel.py:308-313);
+// the host work of a call does not grow with its tensors, but for the forward's
+// split schedule, which adds up a causal call's pairs of query tiles (one step per
+// 256 queries).
 #include "fa_common.cuh"
 #include "sm100_ptx.cuh"
 #include "tile_config.cuh"

@@ -10,8 +10,8 @@ the kernels underneath:
   views, no transposes or copies;
 * a boolean key-padding mask on its own (no attn_mask, no causal mask) costs no bias at all:
   attention does not depend on the order of the keys, so the kept keys of every batch entry are
-  moved to the front (one gather of K and V, undone for dK and dV by autograd) and the call runs
-  on the tensor-core kernels with per-batch key counts;
+  moved to the front (on the GPU one scan of the mask and one launch that moves the rows of K and V,
+  the gradients back the same way) and the call runs with per-batch key counts;
 * other masks become the smallest bias that expresses them - a key-padding mask is a
   (B, 1, 1, Nk) bias, a 2-D attn_mask a (1, 1, Nq, Nk) one - instead of a dense
   (B, H, Nq, Nk) tensor (reference :228-250); boolean masks hide where True,

@@ -304,7 +304,8 @@ def launch_backward(d_o, q, k, v, o, lse, scale, causal, dropout_p=0.0, seed=0, 
         _check_residual(o_residual, o)
         p.o_lo = _tensor4(o_residual)
     if d_scores is not None:
-        # dense (B, H, Nq, Nk) fp32, zero-filled by the caller: receives d loss / d scores
+        # dense (B, H, Nq, Nk) fp32 that receives d loss / d scores; entries that causal or key_lengths hide are not
+        # written, so with either the caller fills it with zeros first
         if d_scores.dtype != torch.float32 or not d_scores.is_contiguous() or \
                 tuple(d_scores.shape) != (q.shape[0], q.shape[2], q.shape[1], k.shape[1]):
             raise ValueError("d_scores must be a contiguous fp32 (B, H, Nq, Nk) tensor")

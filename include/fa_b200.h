@@ -127,7 +127,9 @@ typedef struct fa_b200_params {
        batch, head and QUERY index, the key index has stride 1; a stride of 0 broadcasts (a key-padding
        mask is (B, 1, 1, Nk): stride_h = stride_n = 0).  -inf entries mask keys.  ptr = NULL: no bias.
        With 16-bit inputs and a head size that is a multiple of 8 the tensor-core kernels serve such calls (P and
-       dS as hi + lo pairs); other calls with a bias run on the CUDA-core kernels. */
+       dS as hi + lo pairs); other calls with a bias run on the CUDA-core kernels.  Masks of finite values, down to
+       the lowest of fp32, give the same results on both; an infinite element of V or dO gives an infinity or a NaN
+       in the elements it reaches on the former, an infinity on the latter. */
     fa_b200_tensor bias;
     /* backward, optional: dense (B, H, Nq, Nk) fp32 buffer, zero-filled by the caller, that receives
        d(loss)/d(scores) = P o (dP o Z - delta); the caller sums it over the bias' broadcast
@@ -137,7 +139,8 @@ typedef struct fa_b200_params {
        batch entry b attends to keys [0, kv_lengths[b]) only, the rest of its K/V rows are padding.
        Values are clamped to [1, Nk].  dK and dV rows of the padding are written as zeros.  No counterpart
        in the reference, which expresses padding as a dense -inf bias (examples/basic_usage.py:243-248);
-       here whole key blocks beyond the count are skipped, on every kernel family. */
+       here whole key blocks beyond the count are skipped, on every kernel family.  Padding in the last block visited
+       (128 keys on the tensor-core kernels, 64 on the CUDA cores) is multiplied by zero: it has to hold numbers. */
     const int32_t* kv_lengths;
     /* Dropout stream of a call over a slice of a larger problem (a head or batch shard, one chunk of a
        batch).  The mask of column (b, h) is indexed by (b + rng_batch_offset) * rng_heads + h +

@@ -116,3 +116,31 @@ def test_rows_whose_first_keys_are_hidden(device):
     assert torch.isnan(o[0, 5]).all() and torch.isnan(o2[0, 5]).all() and lse[0, 0, 5] == lse2[0, 0, 5] == float("-inf")
     keep = torch.arange(64, device=device) != 5
     assert _rel(o[:, keep], o2[:, keep]) <= 4.2e-4 and _rel(lse[:, :, keep], lse2[:, :, keep]) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=["fp16", "bf16"])
+@pytest.mark.parametrize("D,N,causal", [(64, 440, False), (128, 440, False), (64, 385, True), (96, 900, False)])
+def test_fp32_results_are_as_exact_as_on_the_cuda_cores(device, dtype, D, N, causal):
+    """lse and d(loss)/d(scores) against float64: the CUDA-core tiles' distance is the bound.  lse is rounded once behind
+    either sum, by up to half a unit of its last place, which is most of both distances: a quarter more is allowed."""
+    gen = torch.Generator(device=device).manual_seed(N)
+    q, k, v, g = (torch.randn(2, N, 4, D, generator=gen, device=device).to(dtype) for _ in range(4))
+    bias = torch.randn(1, 4, N, N, generator=gen, device=device) * 0.5
+    qd, kd, vd, gd = (t.double().transpose(1, 2) for t in (q, k, v, g))
+    s = qd @ kd.transpose(-1, -2) * D ** -0.5 + bias.double()
+    if causal:
+        s = s.masked_fill(torch.ones(N, N, device=device, dtype=torch.bool).triu(1), float("-inf"))
+    lse_ref = torch.logsumexp(s, -1)
+    p = torch.exp(s - lse_ref[..., None])
+    ds_ref = p * (gd @ vd.transpose(-1, -2) - (gd * (p @ vd)).sum(-1, keepdim=True))
+
+    def errors():
+        res = torch.empty_like(q)
+        o, lse = launch_forward(q, k, v, D ** -0.5, causal, bias=bias, o_residual=res)
+        ds = torch.zeros(2, 4, N, N, device=device)
+        launch_backward(g, q, k, v, o, lse, D ** -0.5, causal, bias=bias, d_scores=ds, o_residual=res)
+        return [((a.double() - r).norm() / r.norm()).item() for a, r in ((lse, lse_ref), (ds, ds_ref))]
+    with fa.kernel_variant("simt"):
+        lse_simt, ds_simt = errors()
+    lse_pair, ds_pair = errors()
+    assert lse_pair <= 1.25 * lse_simt and ds_pair <= ds_simt, (lse_pair, lse_simt, ds_pair, ds_simt)
