@@ -282,8 +282,9 @@ __device__ __forceinline__ CtaWork cta_work(int cols_per_group) {
 // INLINE (bf16 inputs only): the streamed tiles arrive as bf16 and the two spare warps convert them;
 // otherwise bf16 calls stream the fp16 copies the preprocess launch (Q, dO) and the dK/dV kernel (K:
 // map_aux, a by-product of its stationary tile) have written to the workspace.
-// DS (pairs, MODE 1): the call wants d(loss)/d(scores).  An instance of its own: as a branch its code cost the kernel of
-// calls that do not want it 10 of 56 us (B4 N1024 H16 D96 causal).
+// DS (pairs, MODE 1): the call wants d(loss)/d(scores).  An instance of its own: as branches its code cost the kernel of
+// calls that do not want it 13 of 66 us (B4 N1024 H16 D96 causal).  Two walks over the keys take 95 us where one took 71
+// (B8 N512 H12 D64 bf16); see `sum_p2` for what they give.
 template <int D, bool BF16, int MODE, int NWG, int DROP, bool INLINE, int PREC, bool DS>
 __global__ void __launch_bounds__(128 * NWG + kExtraThreads, 1)
 bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
@@ -352,7 +353,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         int kv_end = nk;
         if (a.causal && tile * kTile + kTile + a.shift < kv_end) kv_end = tile * kTile + kTile + a.shift;
         n_per_head = (kv_end + kTile - 1) / kTile;
-        // pairs with d(loss)/d(scores) wanted: the steps are walked twice (kernel comment at `summing` below)
+        // d(loss)/d(scores) wanted: the steps are walked twice (comment at `sum_p2` below)
         if (DS) sum_steps = n_per_head;
         n_iter = sum_steps + n_per_head;
     }
@@ -807,7 +808,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // Pairs with d(loss)/d(scores) wanted (MODE 1).  That output is fp32, but delta comes from an O rounded to 16 bits
         // (or 16 + 16) that was summed with P as a pair, and P from an lse rounded once: together more than the CUDA
         // cores' error.  So a first walk over the keys sums P and P o dP Z of every row in fp32; their quotient is
-        // delta, and the sum of P, one but for rounding, divides P.  Only dQ's and d(scores)' kernel, only these calls.
+        // delta, and the sum of P, one but for rounding, divides P (distance from float64 at B2 N440 H4 D64 bf16, CUDA cores
+        // 3.5e-7: 5.6e-7 -> 2.4e-7; N385 causal 1.05e-6: 1.23e-6 -> 1.8e-7).
         [[maybe_unused]] uint64_t sum_p2 = 0ull, sum_pd2 = 0ull;           // {0.f, 0.f}
         [[maybe_unused]] float p_mul = P_BF16 ? 1.f : 16384.f;             // 2^kPShift where P carries it
         int qi = 0, hg = 0;                 // step within the query head, query heads done (key-stationary)

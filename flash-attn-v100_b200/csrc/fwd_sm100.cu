@@ -28,7 +28,7 @@
 //               f16 x f16 with P rounded to fp16 instead of bf16 (see sm100_ptx.cuh); fp16 inputs: idle
 //               (the two warps complete the third warpgroup for setmaxnreg)
 //
-// Online softmax in the log2 domain with scale*log2(e) folded into one FMA.
+// Online softmax in the log2 domain with scale*log2(e) folded into one FMA (pair instances: in natural units, see there).
 // The running maximum is only refreshed when it grows by more than 2^8 (warp
 // vote), so the O accumulator in TMEM is rescaled rarely; the final division
 // by the row sum makes the result exact either way.  P is rounded to fp16 (whatever
