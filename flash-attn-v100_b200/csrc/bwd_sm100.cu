@@ -194,6 +194,7 @@ struct BwdScales {
     float tt_mul;     // dP (as the MMA delivers it) * tt_mul
     float nd_mul;     // the staged -delta vector * nd_mul
     float l_add;      // added to the staged lse vector (key-stationary kernels)
+    float ds_mul;     // dS = dS' * ds_mul            (2^-g)
     float acc1_mul;   // dK or dQ  = ACC1 * acc1_mul  (scale * 2^-g)
     float acc2_mul;   // dV        = ACC2 * acc2_mul
     float do_mul;     // inline conversion: dO' = dO * do_mul
@@ -234,7 +235,8 @@ __device__ __forceinline__ BwdScales make_scales(const float* rng, int D, float 
     sc.tt_mul = pow2i(g - up + e_col);
     sc.nd_mul = pow2i(g - up + (form == kDoRowCopy ? e_col : 0));
     sc.l_add = form == kDoRowCopy ? (float)(-e_col) : 0.f;
-    sc.acc1_mul = scale * pow2i(-g);
+    sc.ds_mul = pow2i(-g);
+    sc.acc1_mul = scale * sc.ds_mul;
     sc.acc2_mul = inv_keep * pow2i(e_col - up);
     sc.do_mul = pow2i(-e_col);
     return sc;
@@ -761,7 +763,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // PREC = 1, query-stationary: my row of d loss / d scores, and what undoes dS' = dS * 2^g
         [[maybe_unused]] float* ds_row = DS
             ? a.d_scores + (((int64_t)b * a.H + head_x) * a.Nq + row_g) * (int64_t)a.Nk : nullptr;
-        [[maybe_unused]] const float ds_mul = sc.acc1_mul / a.scale;
+        [[maybe_unused]] const float ds_mul = sc.ds_mul;
         bool ok = true;
         if (XY_CONV && n_iter > 0) {
             // the stationary tiles, once per CTA: K_j and V_j, or Q_i (dO_i is only ever multiplied
