@@ -97,8 +97,14 @@ struct BwdCfg {
     static constexpr int kWStages = PREC == 2 ? tile::bwd_bias_w_stages(D) : tile::bwd_w_stages(D);
     static constexpr int kBiasBytes = PREC == 2 ? 4 * kBoxBytes : 0;    // four boxes of 128 queries x 32 keys
     static constexpr int kMaskBytes = 2 * 128 * 8 * 2;          // two buffers of 128 x 8 uint16 keep masks
-    static constexpr int kXYFull = 0;
-    static constexpr int kUFull = 1;                             // [kUStages]
+    static constexpr int kXFull = 0;
+    static constexpr int kYFull = 1;
+    static constexpr int kXEmpty = 2;                            // the item's last reader of X (see kXEmptyArrivals)
+    static constexpr int kYEmpty = 3;
+    static constexpr int kSchedFull = 4;                         // [2] the next item's place is in its slot
+    static constexpr int kSchedEmpty = 6;                        // [2] ... and has been read (one arrival per reading warp)
+    static constexpr int kClc = 8;                               // the answer to the request for another item has landed
+    static constexpr int kUFull = 9;                             // [kUStages]
     static constexpr int kUEmpty = kUFull + kUStages;            // [kUStages]
     static constexpr int kWFull = kUEmpty + kUStages;            // [kWStages]
     static constexpr int kWEmpty = kWFull + kWStages;            // [kWStages]
@@ -108,27 +114,35 @@ struct BwdCfg {
     static constexpr int kDsReady = kPReady + 1;                 // one arrival per elementwise warp
     static constexpr int kAccDone = kDsReady + 1;
     static constexpr int kMask = kAccDone + 1;                   // one arrival per elementwise warp
-    static constexpr int kEpi = kMask + 1;                       // one arrival per elementwise warp
-    static constexpr int kDqFull = kEpi + 1;                     // fused kernel: dQ tile of the step complete
+    static constexpr int kEpi = kMask + 1;                       // one arrival per elementwise warp: results are staged
+    static constexpr int kRowFull = kEpi + 1;                    // query-stationary: the rows' -lse, -delta and exponents landed
+    static constexpr int kRowEmpty = kRowFull + 1;               // ... and read (one arrival per elementwise warp)
+    static constexpr int kDqFull = kRowEmpty + 1;                // fused kernel: dQ tile of the step complete
     static constexpr int kDqRead = kDqFull + 1;                  // ... and read out (one arrival per warp)
     static constexpr int kPHalf = kDqRead + 1;                   // key-stationary: first half of each P^T slice stored
     static constexpr int kDsHalf = kPHalf + 1;                   // first half of each dS slice stored
     static constexpr int kVFull = kDsHalf + 1;                   // [2] key-stationary: -lse, -delta rows of a step landed
     static constexpr int kVEmpty = kVFull + 2;                   // [2] ... and read (one arrival per elementwise warp)
     // bf16 inputs: tiles converted to fp16 in place (arrivals: one per converting warp)
-    static constexpr int kXYConv = kVEmpty + 2;                  // stationary tiles (elementwise warps)
-    static constexpr int kUConv = kXYConv + 1;                   // [kUStages] streamed U (the two spare warps)
+    static constexpr int kXConv = kVEmpty + 2;                   // stationary tiles (one arrival per elementwise warp)
+    static constexpr int kYConv = kXConv + 1;
+    static constexpr int kUConv = kYConv + 1;                    // [kUStages] streamed U (the two spare warps)
     static constexpr int kWConv = kUConv + kUStages;             // [kWStages] streamed W, key-stationary kernels only
     static constexpr int kBiasFull = kWConv + kWStages;          // PREC = 2: the step's bias tile has landed
     static constexpr int kBiasEmpty = kBiasFull + 1;             // ... and has been read (one arrival per elementwise warp)
     static constexpr int kSums = kBiasEmpty + 1;                 // pairs, MODE 1: the rows' partial sums (elementwise warps)
     static constexpr int kNumBars = kSums + 1;
-    // two slots of lse[128] | delta[128]; pairs, MODE 1: a partial sum of each row from every warpgroup
-    static constexpr int kVecBytes = MODE != 1 ? 2 * 1024 : (PREC ? 128 * 4 * kNWG : 0);
+    // two slots of lse[128] | delta[128]; MODE 1: the rows' lse[128] | delta[128] | exponents[128], pairs: later a partial
+    // sum of each row from every warpgroup
+    static constexpr int kVecBytes = MODE != 1 ? 2 * 1024 : (PREC ? 128 * 4 * kNWG : 3 * 512);
     static constexpr int kDsBytes = 128 * 128 * 2;               // fused kernel: dS^T tile for the dQ MMA
-    // bytes used from the 1024-aligned base: X, Y, U ring, W ring, [dS], [vectors], barriers, TMEM slot + flag, [masks]
+    static constexpr int kBarBytes = (kNumBars * 8 + 15) / 16 * 16;
+    // behind the barriers: TMEM slot, abort flag and wait limit (16 bytes), the answer to a request for a block (16),
+    // two BwdItem
+    static constexpr int kCtlBytes = 32 + 2 * 48;
+    // bytes used from the 1024-aligned base: X, Y, U ring, W ring, [dS], [vectors], barriers, control words, [masks]
     static constexpr int kUsedBytes = (2 + kUStages + kWStages) * kTileBytes + kBiasBytes + (kFused ? kDsBytes : 0) + kVecBytes +
-                                      kNumBars * 8 + 64 + (kMasks ? kMaskBytes : 0);
+                                      kBarBytes + kCtlBytes + (kMasks ? kMaskBytes : 0);
     static constexpr int kMaxSmem = 232448;                      // 227 KB: the most one CTA can ask for
     static_assert(128 * kNWG + 128 == 32 * tile::kBwdWarps, "thread count and table disagree");
     static_assert(kUsedBytes <= kMaxSmem, "shared-memory plan does not fit");
@@ -145,6 +159,7 @@ struct BwdArgs {
     const int32_t* kv_len; // optional per-batch key counts
     int32_t* status;
     int B, Nq, Nk, H, Hkv, nq_pad;
+    int group;                     // H / Hkv
     int wait_limit_ms;             // limit of one mbarrier wait (0: the default)
     int cols_per_group;            // CTA order: (batch, head) columns per group, see cta_work()
     int causal;
@@ -152,6 +167,9 @@ struct BwdArgs {
     float scale, scale_log2;
     float score_scale;             // pairs: scale for the scores, with the truncation of their sums given back
     float dp_gain;                 // pairs: the same factor for dP
+    // dQ, or dK and dV: 16-byte pieces, element strides
+    void* out1; int64_t o1_sb, o1_sn, o1_sh;
+    void* out2; int64_t o2_sb, o2_sn, o2_sh;
     uint32_t drop_thr;
     float inv_keep;
     PhiloxKey key;
@@ -259,16 +277,16 @@ __device__ __forceinline__ uint32_t finite_piece(uint32_t m) {
     constexpr uint32_t inf = std::is_same<T, __half>::value ? 0x7C00u : 0x7F80u;
     return max(m & 0xFFFFu, m >> 16) < inf ? m : 0u;
 }
-// Which (tile, head, batch) a CTA works on.  The grid is (tiles, heads, batch) and CTAs start in the
+// Which (tile, head, batch) a block of the grid stands for.  The grid is (tiles, heads, batch) and blocks are taken in the
 // order of their linear index.  Under a causal mask tiles cost between 1 and `tiles` steps, so the
 // order decides how evenly the SMs finish: the (batch, head) columns are taken in groups of
 // `cols_per_group`, and within a group all columns' most expensive tile comes first, then the next
 // one, ... (longest first).  A group is sized so that its Q, K, V and dO stay in L2 while its CTAs
 // run; the cheap tiles that end one group fill the SMs beside the expensive ones that start the next.
 struct CtaWork { int tile_rank, head, b; };
-__device__ __forceinline__ CtaWork cta_work(int cols_per_group) {
+__device__ __forceinline__ CtaWork cta_work(int cols_per_group, uint3 block) {
     const int X = (int)gridDim.x, Y = (int)gridDim.y, cols = Y * (int)gridDim.z;
-    const int L = (int)blockIdx.x + X * ((int)blockIdx.y + Y * (int)blockIdx.z);
+    const int L = (int)block.x + X * ((int)block.y + Y * (int)block.z);
     const int G = cols_per_group < 1 ? 1 : cols_per_group;
     const int grp = L / (G * X), r = L - grp * (G * X);
     const int gcols = (cols - grp * G) < G ? (cols - grp * G) : G;
@@ -278,6 +296,50 @@ __device__ __forceinline__ CtaWork cta_work(int cols_per_group) {
     w.head = col % Y;
     w.b = col / Y;
     return w;
+}
+
+// A block of the grid as the producer leaves it in shared memory for the other roles (twelve words).
+struct BwdItem {
+    int tile, head_x, b;               // stationary tile; its K/V head (key-stationary) or query head
+    int nk;                            // keys the batch entry attends to
+    int it0, n_per_head;               // key-stationary: first query tile that sees the tile; steps of a query head
+    int n_iter;                        // steps in all; -1: no block any more
+    int rot;                           // FUSED: see q_tile_of
+    float range[2];                    // max |dO|, max |V| of the column
+    int head_kv, pad;
+};
+static_assert(sizeof(BwdItem) == 48, "kCtlBytes");
+template <bool KS, bool FUSED, bool DS>
+__device__ __forceinline__ BwdItem make_item(const BwdArgs& a, const CtaWork& cw) {
+    BwdItem m;
+    m.b = cw.b;
+    m.head_x = cw.head;
+    m.nk = kv_len_of(a.kv_len, cw.b, a.Nk);
+    m.rot = 0;
+    if (KS) {
+        m.tile = cw.tile_rank;                        // key tile: the first one sees the most query tiles
+        m.head_kv = cw.head;
+        // first query tile that sees this key tile: query i sees key j iff j <= i + shift
+        m.it0 = a.causal ? (m.tile * kTile > a.shift ? (m.tile * kTile - a.shift) / kTile : 0) : 0;
+        const int nq_tiles = (a.Nq + kTile - 1) / kTile;
+        m.n_per_head = nq_tiles > m.it0 ? nq_tiles - m.it0 : 0;
+        if (m.tile * kTile >= m.nk) m.n_per_head = 0;   // a tile of padding keys: dK = dV = 0
+        m.n_iter = m.n_per_head * a.group;
+        // The fused kernel without a causal mask starts each key tile's walk at a different query tile, so that the CTAs
+        // of one head, which run at the same time, add to different dQ tiles (under a causal mask the walks are
+        // staggered already).
+        if (FUSED && !a.causal && m.n_per_head > 0) m.rot = m.tile % m.n_per_head;
+    } else {
+        m.tile = a.causal ? (int)gridDim.x - 1 - cw.tile_rank : cw.tile_rank;     // query tile, heavy first
+        m.head_kv = cw.head / a.group;
+        m.it0 = 0;
+        int kv_end = m.nk;
+        if (a.causal && m.tile * kTile + kTile + a.shift < kv_end) kv_end = m.tile * kTile + kTile + a.shift;
+        m.n_per_head = kv_end > 0 ? (kv_end + kTile - 1) / kTile : 0;
+        // d(loss)/d(scores) wanted: the steps are walked twice (comment at `sum_p2` below)
+        m.n_iter = DS ? 2 * m.n_per_head : m.n_per_head;
+    }
+    return m;
 }
 
 // MODE 0: dK, dV (key-stationary).  MODE 1: dQ (query-stationary).
@@ -301,9 +363,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     constexpr bool P_BF16 = BF16 && PREC != 0;  // ... except that pairs of bf16 need no conversion
     static_assert(PREC == 0 || (MODE != 2 && !INLINE), "the pair instances are the two-pass form");
     constexpr bool STREAM_CONV = CONV && INLINE;             // ... the streamed ones by the spare warps
-    constexpr bool XY_CONV = CONV && (KS || INLINE);         // ... the stationary ones by the elementwise warps
+    constexpr bool XY_CONV = CONV && (KS || INLINE);         // ... the stationary ones (X; key-stationary also Y), too
     constexpr bool ROWFORM = CONV && !INLINE;                // staged vectors are in the row form (see DoForm)
     constexpr bool K_COPY = ROWFORM && MODE == 0;            // this kernel writes the fp16 copy of K
+    constexpr bool ROW_MAX = PREC != 0 && !BF16 && MODE == 1;   // the threads read Y, too
     static_assert(BF16 || !INLINE, "inline conversion is a bf16 variant");
     constexpr int UST = Cfg::kUStages, WST = Cfg::kWStages;
     constexpr int TILE = Cfg::kTileBytes;
@@ -318,9 +381,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint8_t* sDs = sBias + Cfg::kBiasBytes;         // fused kernel only
     float* sVec = (float*)(sDs + (FUSED ? Cfg::kDsBytes : 0));      // key-stationary: 2 x (lse[128] | delta[128]); see kVecBytes
     uint64_t* bars = (uint64_t*)((uint8_t*)sVec + Cfg::kVecBytes);
-    uint32_t* tmem_slot = (uint32_t*)(bars + Cfg::kNumBars);
+    uint32_t* tmem_slot = (uint32_t*)((uint8_t*)bars + Cfg::kBarBytes);
     volatile uint32_t* abort_flag = (volatile uint32_t*)(tmem_slot + 1);
-    uint16_t* sMask = (uint16_t*)((uint8_t*)bars + Cfg::kNumBars * 8 + 64);    // present with dropout only
+    uint32_t* clc_answer = tmem_slot + 4;
+    volatile BwdItem* sched = (volatile BwdItem*)(tmem_slot + 8);              // [2]: block k of this CTA in slot k & 1
+    uint16_t* sMask = (uint16_t*)((uint8_t*)bars + Cfg::kBarBytes + Cfg::kCtlBytes);    // present with dropout only
     {
         // the launch may have had no room for a full kilobyte of alignment slack
         uint32_t dyn;
@@ -332,61 +397,38 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const CtaWork cw = cta_work(a.cols_per_group);
-    const int b = cw.b;
-    const int group = a.H / a.Hkv;
-    const int nq_tiles = (a.Nq + kTile - 1) / kTile;
-
-    // iteration space (uniform over the CTA)
-    const int nk = kv_len_of(a.kv_len, b, a.Nk);    // keys this batch entry attends to
-    int tile, head_x, it0, n_per_head, n_iter, sum_steps = 0;
-    if (KS) {
-        tile = cw.tile_rank;                        // key tile: the first one sees the most query tiles
-        head_x = cw.head;                           // kv head
-        // first query tile that sees this key tile: query i sees key j iff j <= i + shift
-        it0 = a.causal ? (tile * kTile > a.shift ? (tile * kTile - a.shift) / kTile : 0) : 0;
-        n_per_head = nq_tiles > it0 ? nq_tiles - it0 : 0;
-        if (tile * kTile >= nk) n_per_head = 0;     // a tile of padding keys: dK = dV = 0
-        n_iter = n_per_head * group;
-    } else {
-        tile = a.causal ? (int)gridDim.x - 1 - cw.tile_rank : cw.tile_rank;     // query tile, heavy first
-        head_x = cw.head;                           // query head
-        it0 = 0;
-        int kv_end = nk;
-        if (a.causal && tile * kTile + kTile + a.shift < kv_end) kv_end = tile * kTile + kTile + a.shift;
-        n_per_head = (kv_end + kTile - 1) / kTile;
-        // d(loss)/d(scores) wanted: the steps are walked twice (comment at `sum_p2` below)
-        if (DS) sum_steps = n_per_head;
-        n_iter = sum_steps + n_per_head;
-    }
     // query-stationary: key tile of step `it`
-    auto k_tile_of = [&](int it) { return DS && it >= n_per_head ? it - n_per_head : it; };
-    const int head_kv = (KS) ? head_x : head_x / group;
-    // Key-stationary kernels: query tile of step `it`.  The fused kernel without a causal mask starts
-    // each key tile's walk at a different query tile, so that the CTAs of one head, which run at
-    // the same time, add to different dQ tiles (under a causal mask the walks are staggered already).
-    const int rot = (FUSED && !a.causal && n_per_head > 0) ? tile % n_per_head : 0;
-    // qi = index of the step within its query head (each role keeps qi and the head count as
-    // running counters: a division per step and warp is a visible share of the issue slots)
-    auto q_tile_of = [&](int qi) {
+    auto k_tile_of = [&](int n_per_head, int it) { return DS && it >= n_per_head ? it - n_per_head : it; };
+    // Key-stationary kernels: query tile of a step, qi = its index within its query head (each role keeps qi and the head
+    // count as running counters: a division per step and warp is a visible share of the issue slots).
+    auto q_tile_of = [&](int it0, int n_per_head, int rot, int qi) {
         int t = qi + rot;
         if (t >= n_per_head) t -= n_per_head;
         return it0 + t;
     };
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < Cfg::kNumBars; ++i) {
-            const bool wide = (i == Cfg::kPReady || i == Cfg::kDsReady || i == Cfg::kMask || i == Cfg::kEpi ||
-                               i == Cfg::kDqRead || i == Cfg::kPHalf || i == Cfg::kDsHalf ||
-                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i == Cfg::kXYConv || i >= Cfg::kBiasEmpty);
-            const bool conv2 = i >= Cfg::kUConv && i < Cfg::kBiasFull;          // the two converting warps
-            mbar_init(&bars[i], wide ? 4u * NWG : (conv2 ? 2u : 1u));    // one arrival per elementwise warp
-        }
-        wait_control_init(abort_flag, a.wait_limit_ms);
-        fence_mbar_init();
-    }
     constexpr int kMmaWarp = 4 * NWG, kTmaWarp = 4 * NWG + 1;
     constexpr int CPT = kTile / NWG;                    // columns of T1/T2 one elementwise thread owns
+    constexpr int kAllThreads = 128 * NWG + kExtraThreads;
+    if (warp == kTmaWarp) {
+        // the producer's warp sets the barriers up, so that the first loads need not wait for the other warps
+        constexpr uint32_t kReaders = 4u * NWG + 2u + ((STREAM_CONV || PREC == 2) ? 1u : 0u);
+        for (int i = lane; i < Cfg::kNumBars; i += 32) {
+            const bool wide = (i == Cfg::kPReady || i == Cfg::kDsReady || i == Cfg::kMask || i == Cfg::kEpi || i == Cfg::kRowEmpty ||
+                               i == Cfg::kXConv || i == Cfg::kYConv ||
+                               i == Cfg::kDqRead || i == Cfg::kPHalf || i == Cfg::kDsHalf ||
+                               i == Cfg::kVEmpty || i == Cfg::kVEmpty + 1 || i >= Cfg::kBiasEmpty);
+            const bool conv2 = i >= Cfg::kUConv && i < Cfg::kBiasFull;          // the two converting warps
+            uint32_t count = wide ? 4u * NWG : (conv2 ? 2u : 1u);    // one arrival per elementwise warp
+            if (i == Cfg::kSchedEmpty || i == Cfg::kSchedEmpty + 1) count = kReaders;
+            if (i == Cfg::kXEmpty && K_COPY) count = 2u;              // the MMAs and the copy of K
+            if (i == Cfg::kYEmpty && ROW_MAX) count = 1u + 4u * NWG;
+            mbar_init(&bars[i], count);
+        }
+        if (lane == 0) wait_control_init(abort_flag, a.wait_limit_ms);
+        fence_mbar_init();
+        __syncwarp();
+    }
     // The dQ kernel reads nothing the dK/dV kernel writes: it may take the SMs this grid's last wave
     // leaves idle (it is launched serialized behind this grid, and waits for it only before it ends).
     if (MODE == 0) grid_launch_dependents();
@@ -394,24 +436,29 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
-    if (warp == kTmaWarp && lane == 0) {
-        prefetch_tensormap(&map_x); prefetch_tensormap(&map_y);
-        prefetch_tensormap(&map_u); prefetch_tensormap(&map_w);
-        prefetch_tensormap(&map_out1);
-        if (KS) prefetch_tensormap(&map_out2);
-        if (K_COPY) prefetch_tensormap(&map_aux);
+    if (warp == kTmaWarp) {
+        asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kAllThreads) : "memory");
+    } else {
+        tc_fence_before_sync();
+        asm volatile("barrier.cta.sync 1, %0;" ::"n"(kAllThreads) : "memory");
+        tc_fence_after_sync();
     }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
     const uint32_t tmem = *tmem_slot;
     const uint32_t tT1 = tmem, tT2 = tmem + 128u, tAcc1 = tmem + 256u, tAcc2 = tmem + 384u;
     // fused kernel: the per-step dQ tile has columns of its own when D = 64 and shares T2's when D = 128
     constexpr bool kDqAliasesT2 = (D > 64);
     const uint32_t tDq = kDqAliasesT2 ? tT2 : tmem + 448u;
-    const float* col_range = a.ranges + 2 * ((int64_t)b * a.Hkv + head_kv);
-    BwdScales sc = make_scales(col_range, D, a.inv_keep, a.scale,
-                               P_BF16 ? kDoPairs : (!(CONV && KS) ? kDoAsIs : (INLINE ? kDoInline : kDoRowCopy)));
+    constexpr DoForm kForm = P_BF16 ? kDoPairs : (!(CONV && KS) ? kDoAsIs : (INLINE ? kDoInline : kDoRowCopy));
+
+    // Persistent: a CTA goes on to a further block of the grid, which it takes from the blocks not yet launched
+    // (clusterlaunchcontrol), so the order above and its balance stay what the hardware's dispatch gives, and the streamed
+    // tiles, the rings' and barriers' phases and tensor memory carry on.  As a CTA per block, the start (barriers, tensor
+    // memory, the first loads), the end and the gap between two CTAs cost 13900 cycles a block of the dK/dV kernel and
+    // 11000 of the dQ kernel at D = 128 bf16, 8900 and 8700 at D = 64 fp16, next to 2700, 1570, 2350 and 1460 a step.
+    // The producer asks for the next block and leaves it in one of two slots; k counts a role's blocks.  A role that is
+    // done with a slot arrives on its barrier (the elementwise warps at a block's end: they read the slot again instead of
+    // holding it in registers).
+    auto item_there = [&](int k) { return mbar_wait(&bars[Cfg::kSchedFull + (k & 1)], (uint32_t)(k >> 1) & 1u, abort_flag); };
 
     // Registers: without dropout the launch allocation of 96 per thread lets no role spill, and moving
     // registers from the MMA / TMA warps to the elementwise ones (104 / 64, 104 / 40) made one side or the
@@ -430,76 +477,117 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       if (warp == kTmaWarp) {
         // ---------------------------------------------------------------- TMA producer
         if (elect_one()) {
-            int u_issued = 0, w_issued = 0, v_issued = 0;
-            bool ok = true;
-            if (n_iter > 0) {
-                mbar_expect_tx(&bars[Cfg::kXYFull], 2 * TILE);
-#pragma unroll
-                for (int bx = 0; bx < Cfg::kNBox; ++bx) {
-                    tma_load_4d(sX + bx * kBoxBytes, &map_x, &bars[Cfg::kXYFull], bx * 64, head_x, tile * kTile, b);
-                    tma_load_4d(sY + bx * kBoxBytes, &map_y, &bars[Cfg::kXYFull], bx * 64, head_x, tile * kTile, b);
-                }
-            }
-            int qi = 0, hg = 0;
+            prefetch_tensormap(&map_x); prefetch_tensormap(&map_u);
+            int u_issued = 0, w_issued = 0, v_issued = 0, r_issued = 0, items = 0, asked = 0;     // items: blocks with steps
             int us = 0, ws = 0;                      // ring slots of this step
             uint32_t uph = 0, wph = 0;               // how often each ring has wrapped (parity)
-            for (int it = 0; it < n_iter; ++it) {
-                int head_u, row_u;
-                if (KS) { head_u = head_x * group + hg; row_u = q_tile_of(qi) * kTile; }
-                else    { head_u = head_kv; row_u = k_tile_of(it) * kTile; }
-                ok = mbar_wait(&bars[Cfg::kUEmpty + us], (uph & 1u) ^ 1u, abort_flag);
-                if (!ok) break;
-                mbar_expect_tx(&bars[Cfg::kUFull + us], TILE);
+            int xy_issued[2] = {0, 0};
+            bool ok = true;
+            CtaWork w = cta_work(a.cols_per_group, blockIdx);
+            BwdItem m = make_item<KS, FUSED, DS>(a, w);
+            auto publish = [&](int k) {
+                const int slot = k & 1;
+                float2 rg = make_float2(0.f, 0.f);
+                if (m.n_iter >= 0) rg = *reinterpret_cast<const float2*>(a.ranges + 2 * ((int64_t)m.b * a.Hkv + m.head_kv));
+                ok = mbar_wait(&bars[Cfg::kSchedEmpty + slot], ((uint32_t)(k >> 1) & 1u) ^ 1u, abort_flag);
+                if (!ok) return;
+                volatile BwdItem* d = sched + slot;
+                d->tile = m.tile; d->head_x = m.head_x; d->b = m.b; d->nk = m.nk; d->it0 = m.it0; d->n_per_head = m.n_per_head;
+                d->n_iter = m.n_iter; d->rot = m.rot; d->range[0] = rg.x; d->range[1] = rg.y; d->head_kv = m.head_kv;
+                mbar_arrive(&bars[Cfg::kSchedFull + slot]);
+            };
+            for (int k = 0; ok; ++k) {
+                bool published = k > 0;              // (the first block's loads go out first)
+                auto load_xy = [&](int y) {
+                    ok = mbar_wait(&bars[Cfg::kXEmpty + y], ((uint32_t)items & 1u) ^ 1u, abort_flag);
+                    if (!ok) return;
+                    mbar_expect_tx(&bars[Cfg::kXFull + y], TILE);
 #pragma unroll
-                for (int bx = 0; bx < Cfg::kNBox; ++bx)
-                    tma_load_4d(sU + us * TILE + bx * kBoxBytes, &map_u, &bars[Cfg::kUFull + us], bx * 64, head_u, row_u, b);
-                ++u_issued;
-                ok = mbar_wait(&bars[Cfg::kWEmpty + ws], (wph & 1u) ^ 1u, abort_flag);
-                if (!ok) break;
-                mbar_expect_tx(&bars[Cfg::kWFull + ws], TILE);
-#pragma unroll
-                for (int bx = 0; bx < Cfg::kNBox; ++bx)
-                    tma_load_4d(sW + ws * TILE + bx * kBoxBytes, &map_w, &bars[Cfg::kWFull + ws], bx * 64, head_u, row_u, b);
-                ++w_issued;
-                if (KS) {
-                    // the step's -lse*log2(e) and -delta rows: a two-slot ring of their own
-                    const int vs = it & 1;
-                    ok = mbar_wait(&bars[Cfg::kVEmpty + vs], ((uint32_t)(it >> 1) & 1u) ^ 1u, abort_flag);
+                    for (int bx = 0; bx < Cfg::kNBox; ++bx)
+                        tma_load_4d(sX + y * TILE + bx * kBoxBytes, y ? &map_y : &map_x, &bars[Cfg::kXFull + y], bx * 64, m.head_x, m.tile * kTile, m.b);
+                    ++xy_issued[y];
+                };
+                int qi = 0, hg = 0;
+                for (int it = 0; it < m.n_iter; ++it) {
+                    int head_u, row_u;
+                    if (KS) { head_u = m.head_x * a.group + hg; row_u = q_tile_of(m.it0, m.n_per_head, m.rot, qi) * kTile; }
+                    else    { head_u = m.head_kv; row_u = k_tile_of(m.n_per_head, it) * kTile; }
+                    ok = mbar_wait(&bars[Cfg::kUEmpty + us], (uph & 1u) ^ 1u, abort_flag);
                     if (!ok) break;
-                    const int64_t off = ((int64_t)b * a.H + head_u) * a.nq_pad + row_u;
-                    mbar_expect_tx(&bars[Cfg::kVFull + vs], 1024);
-                    bulk_load_1d(sVec + vs * 256, a.lse2 + off, 512, &bars[Cfg::kVFull + vs]);
-                    bulk_load_1d(sVec + vs * 256 + 128, a.delta + off, 512, &bars[Cfg::kVFull + vs]);
-                    ++v_issued;
+                    mbar_expect_tx(&bars[Cfg::kUFull + us], TILE);
+#pragma unroll
+                    for (int bx = 0; bx < Cfg::kNBox; ++bx)
+                        tma_load_4d(sU + us * TILE + bx * kBoxBytes, &map_u, &bars[Cfg::kUFull + us], bx * 64, head_u, row_u, m.b);
+                    ++u_issued;
+                    if (it == 0) { load_xy(0); if (!ok) break; }
+                    ok = mbar_wait(&bars[Cfg::kWEmpty + ws], (wph & 1u) ^ 1u, abort_flag);
+                    if (!ok) break;
+                    mbar_expect_tx(&bars[Cfg::kWFull + ws], TILE);
+#pragma unroll
+                    for (int bx = 0; bx < Cfg::kNBox; ++bx)
+                        tma_load_4d(sW + ws * TILE + bx * kBoxBytes, &map_w, &bars[Cfg::kWFull + ws], bx * 64, head_u, row_u, m.b);
+                    ++w_issued;
+                    if (KS) {
+                        // the step's -lse*log2(e) and -delta rows: a two-slot ring of their own
+                        const int vs = v_issued & 1;
+                        ok = mbar_wait(&bars[Cfg::kVEmpty + vs], ((uint32_t)(v_issued >> 1) & 1u) ^ 1u, abort_flag);
+                        if (!ok) break;
+                        const int64_t off = ((int64_t)m.b * a.H + head_u) * a.nq_pad + row_u;
+                        mbar_expect_tx(&bars[Cfg::kVFull + vs], 1024);
+                        bulk_load_1d(sVec + vs * 256, a.lse2 + off, 512, &bars[Cfg::kVFull + vs]);
+                        bulk_load_1d(sVec + vs * 256 + 128, a.delta + off, 512, &bars[Cfg::kVFull + vs]);
+                        ++v_issued;
+                    } else if (it == 0) {
+                        // the stationary rows' own: read by the threads when the block begins
+                        ok = mbar_wait(&bars[Cfg::kRowEmpty], ((uint32_t)items & 1u) ^ 1u, abort_flag);
+                        if (!ok) break;
+                        const int64_t off = ((int64_t)m.b * a.H + m.head_x) * a.nq_pad + m.tile * kTile;
+                        mbar_expect_tx(&bars[Cfg::kRowFull], ROWFORM ? 1536 : 1024);
+                        bulk_load_1d(sVec, a.lse2 + off, 512, &bars[Cfg::kRowFull]);
+                        bulk_load_1d(sVec + 128, a.delta + off, 512, &bars[Cfg::kRowFull]);
+                        if (ROWFORM) bulk_load_1d(sVec + 256, a.erow + off, 512, &bars[Cfg::kRowFull]);
+                        ++r_issued;
+                    }
+                    if (it == 0) { load_xy(1); if (!ok) break; }
+                    if (++us == UST) { us = 0; ++uph; }
+                    if (++ws == WST) { ws = 0; ++wph; }
+                    if (++qi == m.n_per_head) { qi = 0; ++hg; }
+                    if (!published) { publish(k); published = true; if (!ok) break; }
+                    // a request two steps before the last one: its answer is there in time, and the block is
+                    // not taken from a CTA that would have come to it sooner
+                    if (it + 3 >= m.n_iter && asked == k) { clc_request(clc_answer, &bars[Cfg::kClc]); ++asked; }
                 }
-                if (++us == UST) { us = 0; ++uph; }
-                if (++ws == WST) { ws = 0; ++wph; }
-                if (++qi == n_per_head) { qi = 0; ++hg; }
+                if (ok && !published) publish(k);
+                if (!ok) break;
+                if (m.n_iter > 0) ++items;
+                if (asked == k) { clc_request(clc_answer, &bars[Cfg::kClc]); ++asked; }
+                ok = mbar_wait(&bars[Cfg::kClc], (uint32_t)k & 1u, abort_flag);
+                if (!ok) break;
+                uint3 block;
+                const bool another = clc_answer_block(clc_answer, block);
+                fence_proxy_async_smem();            // read before the next answer is written
+                if (another) m = make_item<KS, FUSED, DS>(a, cta_work(a.cols_per_group, block));
+                else m.n_iter = -1;
+                publish(k + 1);
+                if (!another) break;
             }
             if (!ok) {
                 // unwinding: let copies already issued land before shared memory is given up
-                for (int st = 0; st < UST; ++st) {
-                    const int nf = (u_issued + UST - 1 - st) / UST;
-                    for (int spin = 0; spin < 4096 && nf > 0 &&
-                         !mbar_try_wait(&bars[Cfg::kUFull + st], (uint32_t)(nf - 1) & 1u); ++spin) {}
-                }
-                for (int st = 0; st < WST; ++st) {
-                    const int nf = (w_issued + WST - 1 - st) / WST;
-                    for (int spin = 0; spin < 4096 && nf > 0 &&
-                         !mbar_try_wait(&bars[Cfg::kWFull + st], (uint32_t)(nf - 1) & 1u); ++spin) {}
-                }
-                for (int st = 0; st < 2; ++st) {
-                    const int nf = (v_issued + 1 - st) / 2;
-                    for (int spin = 0; spin < 4096 && nf > 0 &&
-                         !mbar_try_wait(&bars[Cfg::kVFull + st], (uint32_t)(nf - 1) & 1u); ++spin) {}
-                }
-                for (int spin = 0; spin < 4096 && n_iter > 0 && !mbar_try_wait(&bars[Cfg::kXYFull], 0u); ++spin) {}
+                auto landed = [&](int bar, int n) {
+                    for (int spin = 0; spin < 4096 && n > 0 && !mbar_try_wait(&bars[bar], (uint32_t)(n - 1) & 1u); ++spin) {}
+                };
+                for (int st = 0; st < UST; ++st) landed(Cfg::kUFull + st, (u_issued + UST - 1 - st) / UST);
+                for (int st = 0; st < WST; ++st) landed(Cfg::kWFull + st, (w_issued + WST - 1 - st) / WST);
+                for (int st = 0; st < 2; ++st) landed(Cfg::kVFull + st, (v_issued + 1 - st) / 2);
+                for (int y = 0; y < 2; ++y) landed(Cfg::kXFull + y, xy_issued[y]);
+                landed(Cfg::kRowFull, r_issued);
+                landed(Cfg::kClc, asked);
             }
         }
         __syncwarp();
       } else if (warp == kMmaWarp) {
         // ---------------------------------------------------------------- MMA issuer
-        if (elect_one() && n_iter > 0) {
+        if (elect_one()) {
             // operand formats: converted tiles, P and dS are fp16; the query-stationary kernel's dP keeps
             // its two bf16 tiles (dO_i, V_j) as they are
             constexpr bool T1_BF16 = BF16 && !CONV, T2_BF16 = BF16 && !(CONV && KS);
@@ -509,7 +597,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                             : make_idesc_f16(false, false, kTile, D, false, true);
             constexpr int kUReady = STREAM_CONV ? Cfg::kUConv : Cfg::kUFull;
             constexpr int kWReady = (STREAM_CONV && KS) ? Cfg::kWConv : Cfg::kWFull;
-            constexpr int kXYReady = XY_CONV ? Cfg::kXYConv : Cfg::kXYFull;
+            constexpr int kXReady = XY_CONV ? Cfg::kXConv : Cfg::kXFull;
+            constexpr int kYReady = (XY_CONV && KS) ? Cfg::kYConv : Cfg::kYFull;
             const uint32_t sX_u = smem_u32(sX), sY_u = smem_u32(sY), sU_u = smem_u32(sU), sW_u = smem_u32(sW);
 
             // Descriptors differ only in the 16-byte-granular start address held in their low
@@ -533,11 +622,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 static_assert(CPT == 32, "one K-step of 16 per half slice");
                 const uint64_t b0 = dmn_major + (uint64_t)(strm_u >> 4);
 #pragma unroll
-                for (int g = 0; g < kTile / 32; ++g) {
-                    const int kk = 2 * g + hf;
-                    const uint32_t a_col = (uint32_t)g * CPT + (uint32_t)hf * 8u;
+                for (int q = 0; q < kTile / 32; ++q) {
+                    const int kk = 2 * q + hf;
+                    const uint32_t a_col = (uint32_t)q * CPT + (uint32_t)hf * 8u;
                     mma_ts_f16(d_tmem, a_tmem + a_col, b0 + (uint64_t)((kk * 2048) >> 4), idesc_acc,
-                               (acc || hf > 0 || g > 0) ? 1u : 0u);
+                               (acc || hf > 0 || q > 0) ? 1u : 0u);
                     if (PREC) mma_ts_f16(d_tmem, a_tmem + a_col + CPT / 2, b0 + (uint64_t)((kk * 2048) >> 4), idesc_acc, 1u);
                 }
             };
@@ -553,161 +642,244 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                kk > 0);
             };
 
-            bool ok = mbar_wait(&bars[kXYReady], 0u, abort_flag);
-            if (ok) ok = mbar_wait(&bars[kUReady + 0], 0u, abort_flag);
-            if (ok) ok = mbar_wait(&bars[kWReady + 0], 0u, abort_flag);
-            if (ok) {
-                tc_fence_after_sync();
-                issue_t(tT1, sX_u, sU_u, idesc_t1);
+            // n_iter, sum_steps: of the block at work, from its last step on of the one behind it; `items` blocks with steps
+            // came before.  A block's first S and dP are issued beside the last step of the block before it, its
+            // accumulators are first written behind a hand-off that the threads make when they have read those of the
+            // block before.
+            bool ok = true;
+            int n_next = 0, sum_next = 0;
+            int blocks = 0, items = 0, g = 0;        // g: steps so far
+            auto next_block = [&] {
+                ok = item_there(blocks);
+                if (!ok) return;
+                n_next = sched[blocks & 1].n_iter;
+                if (DS) sum_next = sched[blocks & 1].n_per_head;
+                mbar_arrive(&bars[Cfg::kSchedEmpty + (blocks & 1)]);
+                ++blocks;
+            };
+            // S (dP) of the next step; `item` the number of its block, `first`, `last`: whether it is that one's first, last step
+            auto next_t1 = [&](uint32_t strm_u, int item, bool first, bool last) {
+                if (first) {
+                    ok = mbar_wait(&bars[kXReady], (uint32_t)item & 1u, abort_flag);
+                    if (!ok) return;
+                    tc_fence_after_sync();
+                }
+                issue_t(tT1, sX_u, strm_u, idesc_t1);
                 mma_commit(&bars[Cfg::kT1Full]);
-                issue_t(tT2, sY_u, sW_u, idesc_t2);
-                mma_commit(&bars[Cfg::kT2Full]);
-                if (!KS) mma_commit(&bars[Cfg::kWEmpty + 0]);        // MODE 1: V_j is read by dP(j) only
-            }
+                if (last && !FUSED) mma_commit(&bars[Cfg::kXEmpty]);
+            };
+            auto next_t2 = [&](uint32_t strm_u, int slot, uint32_t ph, int step, int item, bool first, bool last) {
+                ok = mbar_wait(&bars[kWReady + slot], ph & 1u, abort_flag);
+                if (ok && first) ok = mbar_wait(&bars[kYReady], (uint32_t)item & 1u, abort_flag);
+                if (!ok) return;
+                tc_fence_after_sync();
+                // query-stationary: the buffer of this step held dS of two steps ago, whose dQ MMAs were issued before
+                const bool odd = !KS && (step & 1);
+                issue_t(odd ? tAcc2 : tT2, sY_u, strm_u, idesc_t2);
+                mma_commit(&bars[odd ? Cfg::kT1Full + 1 : Cfg::kT2Full]);
+                if (!KS) mma_commit(&bars[Cfg::kWEmpty + slot]);             // MODE 1: V_j is read by dP(j) only
+                if (last) mma_commit(&bars[Cfg::kYEmpty]);
+            };
             int us = 0, ws = 0;                      // ring slots of this step's U and W
             uint32_t uph = 0, wph = 0;               // wrap counts (parity of the slots' phases)
-            for (int it = 0; it < n_iter && ok; ++it) {
-                int nus = us + 1, nws = ws + 1;      // slots of the next step
-                uint32_t nuph = uph, nwph = wph;
-                if (nus == UST) { nus = 0; ++nuph; }
-                if (nws == WST) { nws = 0; ++nwph; }
-                const uint32_t cur_u = sU_u + us * TILE, nxt_u = sU_u + nus * TILE;
-                const uint32_t cur_w = sW_u + ws * TILE, nxt_w = sW_u + nws * TILE;
-                const bool more = it + 1 < n_iter;
-                if (more) { ok = mbar_wait(&bars[kUReady + nus], nuph & 1u, abort_flag); if (!ok) break; }
-                if (KS) {
-                    ok = mbar_wait(&bars[Cfg::kPHalf], (uint32_t)it & 1u, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    issue_acc_half(tAcc2, tT1, cur_w, it > 0, 0);                // dV += (P o Z)^T dO, first halves
-                    ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)it & 1u, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    issue_acc_half(tAcc2, tT1, cur_w, it > 0, 1);
-                    mma_commit(&bars[Cfg::kWEmpty + ws]);                        // dO_i: dP^T(i) earlier, dV(i) last
-                    if (more) { issue_t(tT1, sX_u, nxt_u, idesc_t1); mma_commit(&bars[Cfg::kT1Full]); }
-                } else if (more) {
-                    // dQ needs no second accumulator, and P never goes back to tensor memory here: S has one
-                    // buffer, free again as soon as the threads hold S(it) in registers, and dP / dS have
-                    // two (T2 and the columns a second accumulator would take).  S(it+1) and dP(it+1) are
-                    // both issued before this thread waits for dS(it), so the threads find their next
-                    // inputs ready; with one dP buffer, dP(it+1) could only follow dQ(it), and
-                    // dS -> dQ -> dP -> dS was the loop that set the step time.
-                    ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)it & 1u, abort_flag);     // S(it) is in registers
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    issue_t(tT1, sX_u, nxt_u, idesc_t1);
-                    mma_commit(&bars[Cfg::kT1Full]);
-                    ok = mbar_wait(&bars[kWReady + nws], nwph & 1u, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after_sync();
-                    // the buffer of step it+1 held dS(it-1), which dQ(it-1) read: issued before, in order
-                    issue_t(((it + 1) & 1) ? tAcc2 : tT2, sY_u, nxt_w, idesc_t2);
-                    mma_commit(&bars[((it + 1) & 1) ? Cfg::kT1Full + 1 : Cfg::kT2Full]);
-                    mma_commit(&bars[Cfg::kWEmpty + nws]);
+            bool begun = false;                      // whether the block's first S and dP are out
+            next_block();
+            for (; ok; ++items) {
+                // blocks without steps: one at a time, since the threads are done with a block's slot when they have ended
+                // the block, and there are two slots
+                while (ok && n_next == 0) next_block();
+                if (!ok || n_next < 0) break;
+                const int n_iter = n_next, sum_steps = sum_next;
+                if (!begun) {
+                    ok = mbar_wait(&bars[kUReady + us], uph & 1u, abort_flag);
+                    if (ok) next_t1(sU_u + us * TILE, items, true, n_iter == 1);
+                    if (ok) next_t2(sW_u + ws * TILE, ws, wph, g, items, true, n_iter == 1);
                 }
-                // query-stationary: a barrier pair per dP / dS buffer (phase = uses of that buffer), which
-                // the threads cannot lap: dS(it+2) needs dP(it+2), issued after these waits
-                const int b_half = (!KS && (it & 1)) ? Cfg::kPHalf : Cfg::kDsHalf;
-                const int b_ready = (!KS && (it & 1)) ? Cfg::kDqRead : Cfg::kDsReady;
-                const uint32_t ds_par = KS ? ((uint32_t)it & 1u) : ((uint32_t)(it >> 1) & 1u);
-                const uint32_t tDs = (!KS && (it & 1)) ? tAcc2 : tT2;
-                ok = mbar_wait(&bars[b_half], ds_par, abort_flag);
-                if (!ok) break;
-                tc_fence_after_sync();
-                const bool acc = !DS || it >= sum_steps;                       // (no dS in the steps that only sum)
-                if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 0);   // dK += dS^T Q  /  dQ += dS K
-                ok = mbar_wait(&bars[b_ready], ds_par, abort_flag);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 1);
-                mma_commit(&bars[Cfg::kUEmpty + us]);                            // last reader of U(it)
-                if (FUSED) {
-                    // dQ tile of this step = dS K_j: A is the dS^T tile the threads left in shared memory,
-                    // read MN-major (M = queries), B is the stationary K tile read MN-major (N = D)
-                    if (!kDqAliasesT2 && it > 0) {
-                        // own columns: only the previous tile's read-out has to precede (issuing
-                        // dP^T(it+1) ahead of this MMA measured slower)
-                        ok = mbar_wait(&bars[Cfg::kDqRead], (uint32_t)(it - 1) & 1u, abort_flag);
+                for (int it = 0; it < n_iter && ok; ++it, ++g) {
+                    int nus = us + 1, nws = ws + 1;      // slots of the next step
+                    uint32_t nuph = uph, nwph = wph;
+                    if (nus == UST) { nus = 0; ++nuph; }
+                    if (nws == WST) { nws = 0; ++nwph; }
+                    const uint32_t cur_u = sU_u + us * TILE, nxt_u = sU_u + nus * TILE;
+                    const uint32_t cur_w = sW_u + ws * TILE, nxt_w = sW_u + nws * TILE;
+                    const bool last = it + 1 == n_iter;
+                    if (last) { next_block(); if (!ok) break; }
+                    const bool more = !last || n_next > 0;
+                    begun = more;
+                    const int nitem = items + (last ? 1 : 0);
+                    const bool nlast = last ? n_next == 1 : it + 2 == n_iter;
+                    if (more) { ok = mbar_wait(&bars[kUReady + nus], nuph & 1u, abort_flag); if (!ok) break; }
+                    // the next block's S goes out early where its stationary tile is there
+                    auto t1_now = [&] { return more && (!last || (!FUSED && mbar_test(&bars[kXReady], (uint32_t)nitem & 1u))); };
+                    bool t1_out = false;
+                    if (KS) {
+                        ok = mbar_wait(&bars[Cfg::kPHalf], (uint32_t)g & 1u, abort_flag);
                         if (!ok) break;
                         tc_fence_after_sync();
-                    }
-                    issue_dq();
-                    mma_commit(&bars[Cfg::kDqFull]);
-                    if (more && kDqAliasesT2) {
-                        // the tile sits in T2's columns: dP^T(it+1) may only follow its read-out
-                        ok = mbar_wait(&bars[Cfg::kDqRead], (uint32_t)it & 1u, abort_flag);
+                        issue_acc_half(tAcc2, tT1, cur_w, it > 0, 0);                // dV += (P o Z)^T dO, first halves
+                        ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)g & 1u, abort_flag);
                         if (!ok) break;
                         tc_fence_after_sync();
+                        issue_acc_half(tAcc2, tT1, cur_w, it > 0, 1);
+                        if (!last) mma_commit(&bars[Cfg::kWEmpty + ws]);             // dO_i: dP^T(i) earlier, dV(i) last
+                        if ((t1_out = t1_now())) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
+                    } else {
+                        // dQ needs no second accumulator, and P never goes back to tensor memory here: S has one
+                        // buffer, free again as soon as the threads hold S(it) in registers, and dP / dS have
+                        // two (T2 and the columns a second accumulator would take).  S(it+1) and dP(it+1) are
+                        // both issued before this thread waits for dS(it), so the threads find their next
+                        // inputs ready; with one dP buffer, dP(it+1) could only follow dQ(it), and
+                        // dS -> dQ -> dP -> dS was the loop that set the step time.
+                        ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)g & 1u, abort_flag);     // S(it) is in registers
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        if ((t1_out = t1_now())) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
+                        if (more && !last) { next_t2(nxt_w, nws, nwph, g + 1, nitem, false, nlast); if (!ok) break; }
                     }
-                }
-                if (KS && more) {
-                    ok = mbar_wait(&bars[kWReady + nws], nwph & 1u, abort_flag);
+                    // query-stationary: a barrier pair per dP / dS buffer (phase = uses of that buffer), which
+                    // the threads cannot lap: dS(it+2) needs dP(it+2), issued after these waits
+                    const int b_half = (!KS && (g & 1)) ? Cfg::kPHalf : Cfg::kDsHalf;
+                    const int b_ready = (!KS && (g & 1)) ? Cfg::kDqRead : Cfg::kDsReady;
+                    const uint32_t ds_par = KS ? ((uint32_t)g & 1u) : ((uint32_t)(g >> 1) & 1u);
+                    const uint32_t tDs = (!KS && (g & 1)) ? tAcc2 : tT2;
+                    ok = mbar_wait(&bars[b_half], ds_par, abort_flag);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    issue_t(tT2, sY_u, nxt_w, idesc_t2);
-                    mma_commit(&bars[Cfg::kT2Full]);
+                    const bool acc = !DS || it >= sum_steps;                       // (no dS in the steps that only sum)
+                    if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 0);   // dK += dS^T Q  /  dQ += dS K
+                    ok = mbar_wait(&bars[b_ready], ds_par, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 1);
+                    // last reader of U(it); a block's last U and W tiles' places take its results first
+                    mma_commit(&bars[last ? Cfg::kAccDone : Cfg::kUEmpty + us]);
+                    if (FUSED) {
+                        // dQ tile of this step = dS K_j: A is the dS^T tile the threads left in shared memory,
+                        // read MN-major (M = queries), B is the stationary K tile read MN-major (N = D).  Only the previous
+                        // tile's read-out has to precede (issuing dP^T(it+1) ahead of this MMA measured slower)
+                        if (g > 0) {
+                            ok = mbar_wait(&bars[Cfg::kDqRead], (uint32_t)(g - 1) & 1u, abort_flag);
+                            if (!ok) break;
+                            tc_fence_after_sync();
+                        }
+                        issue_dq();
+                        mma_commit(&bars[Cfg::kDqFull]);
+                        if (last) mma_commit(&bars[Cfg::kXEmpty]);
+                    }
+                    if (more && !t1_out) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
+                    if (more && (KS || last)) { next_t2(nxt_w, nws, nwph, g + 1, nitem, last, nlast); if (!ok) break; }
+                    us = nus; uph = nuph; ws = nws; wph = nwph;
                 }
-                us = nus; uph = nuph; ws = nws; wph = nwph;
             }
-            if (ok) mma_commit(&bars[Cfg::kAccDone]);
         }
         __syncwarp();
-      } else if (STREAM_CONV) {
-        // ---------------------------------------------------------------- warps 18-19: streamed tiles -> fp16
-        // the producer's walk; a tile is touched between its arrival (U_full / W_full) and its first
-        // reader (the MMAs wait for U_conv / W_conv).  dO tiles are normalised on the way.
+      } else if (warp == kTmaWarp + 2 || STREAM_CONV) {
+        // ---------------------------------------------------------------- warp 19: TMA stores (K's copy, the results)
+        // INLINE, with warp 18: the streamed tiles bf16 -> fp16, between their arrival (U_full, W_full) and their first
+        // reader (the MMAs wait for U_conv, W_conv), dO tiles normalised on the way.
         const int ct = (warp - kTmaWarp - 1) * 32 + lane;
-        int us = 0, ws = 0;
+        const bool stores = warp == kTmaWarp + 2 && lane == 0;
+        int us = 0, ws = 0, items = 0, steps = 0;
         uint32_t uph = 0, wph = 0;
-        for (int it = 0; it < n_iter; ++it) {
-            bool ok = mbar_wait(&bars[Cfg::kUFull + us], uph & 1u, abort_flag);
+        bool ok = true;
+        auto convert = [&](int full, int conv, uint32_t parity, uint8_t* tile, bool scaled, float mul) {
+            ok = mbar_wait(&bars[full], parity & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            if (scaled) convert_tile_bf16_to_f16<true>(tile, TILE, ct, 64, mul);
+            else        convert_tile_bf16_to_f16<false>(tile, TILE, ct, 64, 1.f);
+            fence_proxy_async_smem();
+            mbar_arrive_warp(&bars[conv]);
+        };
+        for (int k = 0; ; ++k) {
+            ok = ok && item_there(k);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-            convert_tile_bf16_to_f16<false>(sU + us * TILE, TILE, ct, 64, 1.f);
-            fence_proxy_async_smem();
-            mbar_arrive_warp(&bars[Cfg::kUConv + us]);
-            if (KS) {
-                ok = mbar_wait(&bars[Cfg::kWFull + ws], wph & 1u, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                convert_tile_bf16_to_f16<true>(sW + ws * TILE, TILE, ct, 64, sc.do_mul);
-                fence_proxy_async_smem();
-                mbar_arrive_warp(&bars[Cfg::kWConv + ws]);
+            const volatile BwdItem* m = sched + (k & 1);
+            const int n_iter = m->n_iter, row0 = m->tile * kTile, head = m->head_x, b = m->b;
+            const float range[2] = {m->range[0], m->range[1]};
+            mbar_arrive_warp(&bars[Cfg::kSchedEmpty + (k & 1)]);
+            if (n_iter < 0) break;
+            if (n_iter == 0) continue;
+            if (K_COPY && stores && mbar_wait(&bars[Cfg::kXConv], (uint32_t)items & 1u, abort_flag)) {
+                // the fp16 K tile is what the dQ kernel streams: keep a copy (rows beyond Nk are clipped)
+#pragma unroll
+                for (int bx = 0; bx < Cfg::kNBox; ++bx)
+                    tma_store_4d(&map_aux, sX + bx * kBoxBytes, bx * 64, head, row0, b);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(&bars[Cfg::kXEmpty]);
             }
-            if (++us == UST) { us = 0; ++uph; }
-            if (++ws == WST) { ws = 0; ++wph; }
+            __syncwarp();
+            if (STREAM_CONV) {
+                const float do_mul = make_scales(range, D, a.inv_keep, a.scale, kForm).do_mul;
+                for (int it = 0; it < n_iter && ok; ++it) {
+                    convert(Cfg::kUFull + us, Cfg::kUConv + us, uph, sU + us * TILE, false, 1.f);
+                    if (KS && ok) convert(Cfg::kWFull + ws, Cfg::kWConv + ws, wph, sW + ws * TILE, true, do_mul);
+                    if (++us == UST) { us = 0; ++uph; }
+                    if (++ws == WST) { ws = 0; ++wph; }
+                }
+                if (!ok) break;
+            }
+            steps += n_iter;
+            if (stores && mbar_wait(&bars[Cfg::kEpi], (uint32_t)items & 1u, abort_flag)) {
+                const int su = (steps - 1) % UST, sw = (steps - 1) % WST;
+#pragma unroll
+                for (int bx = 0; bx < Cfg::kNBox; ++bx) {
+                    tma_store_4d(&map_out1, sU + su * TILE + bx * kBoxBytes, bx * 64, head, row0, b);
+                    if (KS) tma_store_4d(&map_out2, sW + sw * TILE + bx * kBoxBytes, bx * 64, head, row0, b);
+                }
+                tma_store_commit();
+                tma_store_wait_read<0>();          // (the writes complete on their own)
+                mbar_arrive(&bars[Cfg::kUEmpty + su]);
+                if (KS) mbar_arrive(&bars[Cfg::kWEmpty + sw]);
+            }
+            __syncwarp();
+            ++items;
         }
       } else if (PREC == 2 && warp == kTmaWarp + 1) {
         // ---------------------------------------------------------------- warp 18: the steps' bias tiles
         if (elect_one()) {
-            int qi = 0, hg = 0, done = 0;
+            int done = 0;                        // tiles loaded so far
             bool ok = true;
-            // dQ kernel: the threads leave d(loss)/d(scores) of a step in the place of its bias tile
-            auto store_ds = [&](int it) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (k_tile_of(it) * kTile + 32 * c < a.Nk)
-                        tma_store_4d(&map_ds, sBias + c * kBoxBytes, k_tile_of(it) * kTile + 32 * c, head_x, tile * kTile, b);
-                tma_store_commit();
-                tma_store_wait_read<0>();
-            };
-            for (int it = 0; it < n_iter; ++it) {
-                const int head = KS ? head_x * group + hg : head_x;
-                const int q_row = (KS ? q_tile_of(qi) : tile) * kTile, k_col = (KS ? tile : k_tile_of(it)) * kTile;
-                ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)it & 1u) ^ 1u, abort_flag);
+            for (int k = 0; ok; ++k) {
+                ok = item_there(k);
                 if (!ok) break;
-                if (DS && a.ds_staged && it > sum_steps) store_ds(it - 1);
-                mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
+                const volatile BwdItem* m = sched + (k & 1);
+                const int n_iter = m->n_iter, n_per_head = m->n_per_head, it0 = m->it0, head_x = m->head_x, tile = m->tile, b = m->b;
+                mbar_arrive(&bars[Cfg::kSchedEmpty + (k & 1)]);
+                if (n_iter < 0) break;
+                const int sum_steps = DS ? n_per_head : 0;
+                int qi = 0, hg = 0;
+                // dQ kernel: the threads leave d(loss)/d(scores) of a step in the place of its bias tile
+                auto store_ds = [&](int it) {
+                    const int k_col = k_tile_of(n_per_head, it) * kTile;
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    tma_load_4d(sBias + c * kBoxBytes, &map_bias, &bars[Cfg::kBiasFull], k_col + 32 * c, a.bias_h ? head : 0, q_row,
-                                a.bias_b ? b : 0);
-                ++done;
-                if (++qi == n_per_head) { qi = 0; ++hg; }
+                    for (int c = 0; c < 4; ++c)
+                        if (k_col + 32 * c < a.Nk) tma_store_4d(&map_ds, sBias + c * kBoxBytes, k_col + 32 * c, head_x, tile * kTile, b);
+                    tma_store_commit();
+                    tma_store_wait_read<0>();
+                };
+                for (int it = 0; it < n_iter; ++it) {
+                    const int head = KS ? head_x * a.group + hg : head_x;
+                    const int q_row = (KS ? q_tile_of(it0, n_per_head, 0, qi) : tile) * kTile;
+                    const int k_col = (KS ? tile : k_tile_of(n_per_head, it)) * kTile;
+                    ok = mbar_wait(&bars[Cfg::kBiasEmpty], ((uint32_t)done & 1u) ^ 1u, abort_flag);
+                    if (!ok) break;
+                    if (DS && a.ds_staged && it > sum_steps) store_ds(it - 1);
+                    mbar_expect_tx(&bars[Cfg::kBiasFull], 4 * kBoxBytes);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        tma_load_4d(sBias + c * kBoxBytes, &map_bias, &bars[Cfg::kBiasFull], k_col + 32 * c, a.bias_h ? head : 0, q_row,
+                                    a.bias_b ? b : 0);
+                    ++done;
+                    if (++qi == n_per_head) { qi = 0; ++hg; }
+                }
+                if (DS && a.ds_staged && ok && n_iter > 0) {
+                    ok = mbar_wait(&bars[Cfg::kBiasEmpty], (uint32_t)(done - 1) & 1u, abort_flag);
+                    if (ok) store_ds(n_iter - 1);
+                }
             }
-            if (DS && a.ds_staged && ok && n_iter > 0 && mbar_wait(&bars[Cfg::kBiasEmpty], (uint32_t)(n_iter - 1) & 1u, abort_flag))
-                store_ds(n_iter - 1);
             for (int spin = 0; !ok && spin < 4096 && done > 0 && !mbar_try_wait(&bars[Cfg::kBiasFull], (uint32_t)(done - 1) & 1u); ++spin) {}
         }
         __syncwarp();
@@ -721,16 +893,52 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const int cb = wg * CPT;
         const int tid = wg * 128 + r;                          // 0 .. 128*NWG-1
         const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-        const int row_g = tile * kTile + r;                    // MODE 0: key index; MODE 1: query index
         constexpr bool drop = DROP != 0;
+        // bf16: a stationary tile to fp16 in place (K_j and V_j, or Q_i; dO_i is only ever multiplied with the bf16 V_j
+        // tiles and stays as it is), by all elementwise warps: a block's X while the one before it still waits for its
+        // accumulators, its Y behind that one's epilogue.  By the two spare warps it took 4000 cycles a tile.
+        auto convert_xy = [&](int y, uint32_t parity) {
+            bool good = mbar_wait(&bars[Cfg::kXFull + y], parity, abort_flag);
+            good = __all_sync(0xffffffffu, good);
+            if (!good) return false;
+            convert_tile_bf16_to_f16<false>(sX + y * TILE, TILE, tid, 128 * NWG, 1.f);
+            fence_proxy_async_smem();
+            mbar_arrive_warp(&bars[Cfg::kXConv + y]);
+            return true;
+        };
+        bool ok = true;
+        int g = 0;                           // steps so far
+        uint32_t count = 0u;                 // blocks (bits 0-1), blocks with steps (bit 2): as much as the barriers' phases need
+        ok = __all_sync(0xffffffffu, item_there(0));
+        if (XY_CONV && ok && sched[0].n_iter > 0) ok = convert_xy(0, 0u);
+        while (ok) {
+        const volatile BwdItem* m = sched + (count & 1u);
+        const int tile = m->tile, head_x = m->head_x, b = m->b, nk = m->nk, it0 = m->it0, n_per_head = m->n_per_head, n_iter = m->n_iter;
+        [[maybe_unused]] const int sum_steps = DS ? n_per_head : 0;
+        [[maybe_unused]] const int rot = FUSED ? m->rot : 0;
+        if (n_iter < 0) break;
+        if (XY_CONV && KS && n_iter > 0) {
+            ok = convert_xy(1, (count >> 2) & 1u);
+            if (!ok) break;
+        }
+        const int row_g = tile * kTile + r;                    // MODE 0: key index; MODE 1: query index
+        auto scales = [&] {
+            const float range[2] = {m->range[0], m->range[1]};
+            return make_scales(range, D, a.inv_keep, a.scale, kForm);
+        };
+        BwdScales sc = scales();
         float my_nlse2 = 0.f, my_ndelta = 0.f;      // -lse*log2(e) and -delta of my query row (MODE 1)
-        if (MODE == 1) {
-            const int64_t off = ((int64_t)b * a.H + head_x) * a.nq_pad + row_g;
-            my_nlse2 = a.lse2[off];
-            my_ndelta = a.delta[off];
+        if (MODE == 1 && n_iter > 0) {
+            ok = mbar_wait(&bars[Cfg::kRowFull], (count >> 2) & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            my_nlse2 = sVec[r];
+            my_ndelta = sVec[128 + r];
+            const float e = ROWFORM ? sVec[256 + r] : 0.f;
+            if (!DS) mbar_arrive_read_done(&bars[Cfg::kRowEmpty]);       // (else its room holds sums first)
             if (ROWFORM) {
                 // the vectors are staged for the key-stationary kernels: take the row exponent out again
-                const int e_i = (int)a.erow[off];
+                const int e_i = (int)e;
                 my_nlse2 -= (float)e_i;            // -inf in the padding stays -inf
                 my_ndelta *= pow2i(e_i);
             }
@@ -738,20 +946,23 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             // of the type's lowest value or of -1e9 leaves in both what its rounding leaves (the difference is small
             // wherever P is not), and the shift (fp16 only) exact behind it: d(loss)/d(scores) is an fp32 result.
         }
-        if constexpr (PREC != 0 && !BF16 && MODE == 1) {
+        if constexpr (ROW_MAX) {
             // fp16 pairs: dS of my row scaled by a power of two of its own, from its own max |dO|, so that rows far
             // below the column's largest keep their bits (dQ and d(loss)/d(scores) of a row need no common scale; the
             // other kernel sums over rows and has to have one)
-            if (n_iter > 0 && mbar_wait(&bars[Cfg::kXYFull], 0u, abort_flag)) {
-                uint32_t m = 0u;
+            if (n_iter > 0) ok = mbar_wait(&bars[Cfg::kYFull], (count >> 2) & 1u, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (n_iter > 0 && ok) {
+                uint32_t top = 0u;
 #pragma unroll
                 for (int c = 0; c < Cfg::kNBox * 8; ++c) {
                     const uint32_t mp = finite_piece<__half>(absmax16_acc(
                         0u, *reinterpret_cast<const uint4*>(sY + (c >> 3) * kBoxBytes + r * 128 + (((c ^ r) & 7) << 4))));
-                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(mp));
+                    asm("max.u16x2 %0, %0, %1;" : "+r"(top) : "r"(mp));
                 }
-                const float rng[2] = {__half2float(__ushort_as_half((unsigned short)max(m & 0xFFFFu, m >> 16))), col_range[1]};
+                const float rng[2] = {__half2float(__ushort_as_half((unsigned short)max(top & 0xFFFFu, top >> 16))), m->range[1]};
                 sc = make_scales(rng, D, a.inv_keep, a.scale, kDoAsIs);
+                mbar_arrive_read_done(&bars[Cfg::kYEmpty]);
             }
         }
         // dS' = P' o (dP * tt_mul o Z + (-delta) * nd_mul): see "number formats" above
@@ -764,26 +975,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         [[maybe_unused]] float* ds_row = DS
             ? a.d_scores + (((int64_t)b * a.H + head_x) * a.Nq + row_g) * (int64_t)a.Nk : nullptr;
         [[maybe_unused]] const float ds_mul = sc.ds_mul;
-        bool ok = true;
-        if (XY_CONV && n_iter > 0) {
-            // the stationary tiles, once per CTA: K_j and V_j, or Q_i (dO_i is only ever multiplied
-            // with the bf16 V_j tiles and stays as it is)
-            ok = mbar_wait(&bars[Cfg::kXYFull], 0u, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (ok) {
-                convert_tile_bf16_to_f16<false>(sX, (KS ? 2 : 1) * TILE, tid, 128 * NWG, 1.f);   // Y follows X
-                fence_proxy_async_smem();
-                mbar_arrive_warp(&bars[Cfg::kXYConv]);
-                if (K_COPY && tid == 0 && mbar_wait(&bars[Cfg::kXYConv], 0u, abort_flag)) {
-                    // the fp16 K tile is what the dQ kernel streams: keep a copy (rows beyond Nk are clipped)
-#pragma unroll
-                    for (int bx = 0; bx < Cfg::kNBox; ++bx)
-                        tma_store_4d(&map_aux, sX + bx * kBoxBytes, bx * 64, head_x, tile * kTile, b);
-                    tma_store_commit();       // read out before the kernel ends: the epilogue waits for all groups
-                }
-            }
-        }
-
         // fused kernel: add the dQ tile of step `jt` (queries on the TMEM lanes, my D / NWG columns)
         // to the fp32 sums in global memory; the order of additions across CTAs is not fixed
         auto drain_dq = [&](int jt, int q_tile, int head_q) -> bool {
@@ -816,14 +1007,15 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         [[maybe_unused]] float p_mul = P_BF16 ? 1.f : 16384.f;             // 2^kPShift where P carries it
         int qi = 0, hg = 0;                 // step within the query head, query heads done (key-stationary)
         int prev_tile = 0, prev_head = 0;   // query tile and head of the previous step
-        for (int it = 0; it < n_iter; ++it) {
-            const int strm_tile = (KS) ? q_tile_of(qi) : k_tile_of(it);     // query tile (0) / key tile (1)
+        for (const int g0 = g, g_end = g + n_iter; g < g_end && ok; ++g) {
+            const int it = g - g0;          // (query-stationary)
+            const int strm_tile = (KS) ? q_tile_of(it0, n_per_head, rot, qi) : k_tile_of(n_per_head, it);     // query tile (0) / key tile (1)
             const int col_g0 = strm_tile * kTile + cb;                          // global index of my first column
-            const int head_q = (KS) ? head_x * group + hg : head_x;
+            const int head_q = (KS) ? head_x * a.group + hg : head_x;
             const uint32_t bh = dropout_column(a.rng, b, head_q);
             [[maybe_unused]] const float* bias_h = PREC ? a.bias + b * a.bias_sb + head_q * a.bias_sh : nullptr;
-            // key-stationary: -lse*log2(e) and -delta of this step's 128 queries (slot it & 1)
-            const float* lse_s = sVec + (it & 1) * 256;
+            // key-stationary: -lse*log2(e) and -delta of this step's 128 queries (slot g & 1)
+            const float* lse_s = sVec + (g & 1) * 256;
             const float* del_s = lse_s + 128;
 
             // ---- dropout keep bits of my CPT columns (bit c of kb[c / 32])
@@ -856,14 +1048,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     // keys are rows here: build the tile's masks cooperatively, query-major, then read
                     // one bit per (query column, my key row)
                     constexpr int PER = 8 / NWG;               // 16-key blocks each thread generates
-                    uint16_t* mbuf = sMask + (it & 1) * (128 * 8);
+                    uint16_t* mbuf = sMask + (g & 1) * (128 * 8);
                     const int ql = tid & 127, jb0 = (tid >> 7) * PER;
 #pragma unroll
-                    for (int g = 0; g < PER; ++g)
-                        mbuf[ql * 8 + jb0 + g] = (uint16_t)dropout_keep_bits(
-                            a.key, bh, (uint32_t)(strm_tile * kTile + ql), (uint32_t)(tile * 8 + jb0 + g), a.drop_thr);
+                    for (int q = 0; q < PER; ++q)
+                        mbuf[ql * 8 + jb0 + q] = (uint16_t)dropout_keep_bits(
+                            a.key, bh, (uint32_t)(strm_tile * kTile + ql), (uint32_t)(tile * 8 + jb0 + q), a.drop_thr);
                     mbar_arrive_warp(&bars[Cfg::kMask]);
-                    ok = mbar_wait(&bars[Cfg::kMask], (uint32_t)it & 1u, abort_flag);
+                    ok = mbar_wait(&bars[Cfg::kMask], (uint32_t)g & 1u, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     if (FUSED) {      // (the fragment-layout phases read their keep bits from mbuf themselves)
@@ -892,9 +1084,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
                     for (int k = 0; k < 2; ++k) kwr[h][k] = w[16 * h + 8 * k];
             }
-            ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)it & 1u, abort_flag);
-            if (ok) ok = mbar_wait(&bars[Cfg::kVFull + (it & 1)], (uint32_t)(it >> 1) & 1u, abort_flag);
-            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)it & 1u, abort_flag);
+            ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)g & 1u, abort_flag);
+            if (ok) ok = mbar_wait(&bars[Cfg::kVFull + (g & 1)], (uint32_t)(g >> 1) & 1u, abort_flag);
+            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)g & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -912,7 +1104,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 #pragma unroll
                     for (int k = 0; k < 2; ++k) kwr[h][k] >>= ((cb & 31) + 2 * lq);
             } else if (drop) {
-                const uint16_t* mbuf = sMask + (it & 1) * (128 * 8);
+                const uint16_t* mbuf = sMask + (g & 1) * (128 * 8);
                 kbits = 0u;
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
@@ -1034,7 +1226,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             tc_fence_before_sync();
             mbar_arrive_warp(&bars[Cfg::kPReady]);
 
-            ok = mbar_wait(&bars[Cfg::kT2Full], (uint32_t)it & 1u, abort_flag);
+            ok = mbar_wait(&bars[Cfg::kT2Full], (uint32_t)g & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1102,9 +1294,9 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             // written with 16-byte stores from this layout (with the fragment layout above it measured
             // 5-10 % slower)
             // ---- phase A: P from T1
-            ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)it & 1u, abort_flag);
-            if (KS && ok) ok = mbar_wait(&bars[Cfg::kVFull + (it & 1)], (uint32_t)(it >> 1) & 1u, abort_flag);
-            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)it & 1u, abort_flag);
+            ok = mbar_wait(&bars[Cfg::kT1Full], (uint32_t)g & 1u, abort_flag);
+            if (KS && ok) ok = mbar_wait(&bars[Cfg::kVFull + (g & 1)], (uint32_t)(g >> 1) & 1u, abort_flag);
+            if (PREC == 2 && ok) ok = mbar_wait(&bars[Cfg::kBiasFull], (uint32_t)g & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1243,19 +1435,19 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 mbar_arrive_warp(&bars[Cfg::kPReady]);
             }
 
-            if (FUSED && it > 0) {
+            if (FUSED && qi + hg > 0) {
                 // dQ of the previous step: its MMAs ran while phase A above did
-                ok = drain_dq(it - 1, prev_tile, prev_head);
+                ok = drain_dq(g - 1, prev_tile, prev_head);
                 if (!ok) break;
             }
 
             // ---- phase B: dS from T2
             // query-stationary: dP / dS alternate between two buffers, each with its own barriers
-            const bool odd_buf = !KS && (it & 1);
+            const bool odd_buf = !KS && (g & 1);
             const uint32_t tD = odd_buf ? tAcc2 : tT2;
             const int b_half = odd_buf ? Cfg::kPHalf : Cfg::kDsHalf, b_ready = odd_buf ? Cfg::kDqRead : Cfg::kDsReady;
-            ok = KS ? mbar_wait(&bars[Cfg::kT2Full], (uint32_t)it & 1u, abort_flag)
-                    : mbar_wait(&bars[odd_buf ? Cfg::kT1Full + 1 : Cfg::kT2Full], (uint32_t)(it >> 1) & 1u, abort_flag);
+            ok = KS ? mbar_wait(&bars[Cfg::kT2Full], (uint32_t)g & 1u, abort_flag)
+                    : mbar_wait(&bars[odd_buf ? Cfg::kT1Full + 1 : Cfg::kT2Full], (uint32_t)(g >> 1) & 1u, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
@@ -1383,7 +1575,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive_warp(&bars[b_ready]);
             if (DS && it == sum_steps - 1) {
                 // the row's four threads put their sums together, in a fixed order
-                uint32_t meet = 0u;
+                uint32_t meet = ((count >> 2) & 1u);         // three times a block
                 auto all_met = [&] {
                     mbar_arrive_warp(&bars[Cfg::kSums]);
                     const bool good = mbar_wait(&bars[Cfg::kSums], meet & 1u, abort_flag);
@@ -1401,6 +1593,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 float sum_p = 0.f, sum_pd = 0.f;
                 ok = row_sum(sum_p2, sum_p) && all_met() && row_sum(sum_pd2, sum_pd);
                 if (!ok) break;
+                mbar_arrive_read_done(&bars[Cfg::kRowEmpty]);
                 // a row without a result, or one whose lse has lost its sum (all of it masked with a lowest value),
                 // keeps what it has
                 if (sum_p > 0.f && fabsf(sum_pd) < INFINITY) my_ndelta = -sum_pd / sum_p;
@@ -1408,67 +1601,67 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (fabsf(unit - 1.f) < 0.25f) p_mul *= unit;
             }
             }
-            if (KS) mbar_arrive_warp(&bars[Cfg::kVEmpty + (it & 1)]);      // this step's lse / delta rows are read
+            if (KS) mbar_arrive_warp(&bars[Cfg::kVEmpty + (g & 1)]);      // this step's lse / delta rows are read
             prev_tile = strm_tile; prev_head = head_q;
             if (++qi == n_per_head) { qi = 0; ++hg; }
         }
 
-        if (FUSED && n_iter > 0 && ok) ok = drain_dq(n_iter - 1, prev_tile, prev_head);
+        if (FUSED && n_iter > 0 && ok) ok = drain_dq(g - 1, prev_tile, prev_head);
 
-        // ---- epilogue: accumulators -> 16-bit -> swizzled staging -> TMA store
-        if (n_iter > 0 && ok) ok = mbar_wait(&bars[Cfg::kAccDone], 0u, abort_flag);
+        // ---- epilogue: accumulators -> 16-bit -> swizzled staging -> TMA store.  dK or dQ goes to the place of the block's
+        // last U tile, dV to that of its last W tile; warp 19 sends them off and gives the places back to the producer.
+        // (Straight from registers a warp's 16-byte stores go to 32 rows each: 2200 cycles at D = 64, 4000 at D = 128.)
+        if (ok) ok = item_there((int)((count + 1u) & 3u));
         ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-            tc_fence_after_sync();
-            constexpr int kCols = D / NWG;                     // my share of the D accumulator columns: 16..64
-            constexpr int kOuts = (KS) ? 2 : 1;
+        if (!ok) break;
+        if (XY_CONV && sched[(count & 1u) ^ 1u].n_iter > 0) ok = convert_xy(0, ((count >> 2) & 1u) ^ (n_iter > 0 ? 1u : 0u));
+        if (!ROW_MAX) sc = scales();                       // (not kept through the steps)
+        if (n_iter > 0 && ok) ok = mbar_wait(&bars[Cfg::kAccDone], (count >> 2) & 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after_sync();
+        constexpr int kCols = D / NWG;                     // my share of the D accumulator columns: 16 or 32
+        constexpr int kOuts = (KS) ? 2 : 1;
+        if (n_iter > 0) {
 #pragma unroll
             for (int o = 0; o < kOuts; ++o) {
                 const uint32_t tacc = (o == 0 ? tAcc1 : tAcc2) + lane_off + (uint32_t)(wg * kCols);
                 const float mul = (o == 0) ? sc.acc1_mul : sc.acc2_mul;
-                uint8_t* stage = sU + o * TILE;                // the U ring is idle once all MMAs completed
+                uint8_t* stage = o == 0 ? sU + ((g - 1) % UST) * TILE : sW + ((g - 1) % WST) * TILE;
+                uint32_t acc[kCols];
+                if constexpr (kCols == 32) tmem_ld_32x32(tacc, acc);
+                else                       tmem_ld_32x16(tacc, acc);
+                tmem_wait_ld();
 #pragma unroll
-                for (int c0 = 0; c0 < kCols; c0 += 32) {
-                    constexpr int kN = kCols < 32 ? kCols : 32;
-                    uint32_t acc[kN];
-                    if (n_iter > 0) {
-                        if constexpr (kN == 32) tmem_ld_32x32(tacc + c0, acc);
-                        else                    tmem_ld_32x16(tacc + c0, acc);
-                        tmem_wait_ld();
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < kN; ++c) acc[c] = 0u;    // no query sees this key tile
-                    }
-#pragma unroll
-                    for (int g = 0; g < kN / 8; ++g) {
-                        uint4 v4;
-                        v4.x = pack2<BF16>(__uint_as_float(acc[g * 8 + 0]) * mul, __uint_as_float(acc[g * 8 + 1]) * mul);
-                        v4.y = pack2<BF16>(__uint_as_float(acc[g * 8 + 2]) * mul, __uint_as_float(acc[g * 8 + 3]) * mul);
-                        v4.z = pack2<BF16>(__uint_as_float(acc[g * 8 + 4]) * mul, __uint_as_float(acc[g * 8 + 5]) * mul);
-                        v4.w = pack2<BF16>(__uint_as_float(acc[g * 8 + 6]) * mul, __uint_as_float(acc[g * 8 + 7]) * mul);
-                        const int col = wg * kCols + c0 + g * 8;
-                        const int chunk = (col & 63) >> 3;
-                        uint8_t* dst = stage + (col >> 6) * kBoxBytes + r * 128 + ((chunk ^ (r & 7)) << 4);
-                        *reinterpret_cast<uint4*>(dst) = v4;
-                    }
+                for (int q = 0; q < kCols / 8; ++q) {
+                    uint4 v4;
+                    v4.x = pack2<BF16>(__uint_as_float(acc[q * 8 + 0]) * mul, __uint_as_float(acc[q * 8 + 1]) * mul);
+                    v4.y = pack2<BF16>(__uint_as_float(acc[q * 8 + 2]) * mul, __uint_as_float(acc[q * 8 + 3]) * mul);
+                    v4.z = pack2<BF16>(__uint_as_float(acc[q * 8 + 4]) * mul, __uint_as_float(acc[q * 8 + 5]) * mul);
+                    v4.w = pack2<BF16>(__uint_as_float(acc[q * 8 + 6]) * mul, __uint_as_float(acc[q * 8 + 7]) * mul);
+                    const int col = wg * kCols + q * 8;
+                    *reinterpret_cast<uint4*>(stage + (col >> 6) * kBoxBytes + r * 128 + ((((col & 63) >> 3) ^ (r & 7)) << 4)) = v4;
                 }
             }
+            tc_fence_before_sync();                        // (the next block's first hand-off lets them be overwritten)
             fence_proxy_async_smem();
             mbar_arrive_warp(&bars[Cfg::kEpi]);
-            if (tid == 0 && mbar_wait(&bars[Cfg::kEpi], 0u, abort_flag)) {
+        } else if (row_g < (KS ? a.Nk : a.Nq)) {
+            // no query sees this key tile
+            uint16_t* dst1 = (uint16_t*)a.out1 + b * a.o1_sb + (int64_t)row_g * a.o1_sn + head_x * a.o1_sh;
+            uint16_t* dst2 = (uint16_t*)a.out2 + b * a.o2_sb + (int64_t)row_g * a.o2_sn + head_x * a.o2_sh;
 #pragma unroll
-                for (int bx = 0; bx < Cfg::kNBox; ++bx) {
-                    tma_store_4d(&map_out1, sU + bx * kBoxBytes, bx * 64, head_x, tile * kTile, b);
-                    if (KS)
-                        tma_store_4d(&map_out2, sU + TILE + bx * kBoxBytes, bx * 64, head_x, tile * kTile, b);
-                }
-                tma_store_commit();
-                tma_store_wait_read<0>();   // the staging tile has been read; the writes complete on their own
+            for (int col = wg * kCols; col < (wg + 1) * kCols; col += 8) {
+                if (PREC != 0 && col >= a.d) break;
+                *reinterpret_cast<uint4*>(dst1 + col) = make_uint4(0u, 0u, 0u, 0u);
+                if (KS) *reinterpret_cast<uint4*>(dst2 + col) = make_uint4(0u, 0u, 0u, 0u);
             }
+        }
+        mbar_arrive_warp(&bars[Cfg::kSchedEmpty + (count & 1u)]);
+        count = ((count + 1u) & 3u) | ((count & 4u) ^ (n_iter > 0 ? 4u : 0u));
         }
     }
 
-    if (K_COPY && threadIdx.x == 0) tma_store_wait_read<0>();   // the K copy's source tile (also when unwinding)
     tc_fence_before_sync();
     __syncthreads();
     if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
@@ -1739,6 +1932,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         const int64_t g = (int64_t)tile::kBwdGroupBytes / (col_bytes > 0 ? col_bytes : 1);
         a.cols_per_group = (int)(g < 1 ? 1 : (g > 65535 ? 65535 : g));
     }
+    a.group = p.H / p.Hkv;
     a.causal = p.causal;
     a.shift = p.causal ? p.causal_shift : 0;
     a.scale = p.scale;
@@ -1763,6 +1957,10 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         if (rc) return rc;
     }
 
+    auto outputs = [&](const fa_b200_tensor& t1, const fa_b200_tensor& t2) {
+        a.out1 = t1.ptr; a.o1_sb = t1.stride_b; a.o1_sn = t1.stride_n; a.o1_sh = t1.stride_h;
+        a.out2 = t2.ptr; a.o2_sb = t2.stride_b; a.o2_sn = t2.stride_n; a.o2_sh = t2.stride_h;
+    };
     static std::mutex smem_mu;             // per (D, dtype, INLINE) instance of this function
     static uint64_t smem_done[9] = {};     // [kernel mode x dropout form] -> devices whose limit is set
     constexpr int kThreads = 128 * kNWG + kExtraThreads;
@@ -1774,6 +1972,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         const int smem2 = pick_smem<D, 2, PREC>(drop);
         FA_CUDA_CHECK(set_smem_limit_once(k2, smem2, p.device, &smem_done[6 + drop], &smem_mu));
         if (phases & 2) {
+            outputs(p.dk, p.dv);
             k2<<<grid_kv, kThreads, smem2, st>>>(mk, mv, mq16, mg16, mdk, mdv, mdk, mb, mds, a);
             FA_CUDA_CHECK(cudaGetLastError());
         }
@@ -1795,6 +1994,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
     if (phases & 2) {
         // stationary K_j, V_j; streamed Q_i, dO_i (bf16 with copies: their fp16 copies; the kernel leaves
         // the fp16 copy of K behind for the dQ kernel)
+        outputs(p.dk, p.dv);
         k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, mb, mds, a);
         FA_CUDA_CHECK(cudaGetLastError());
     }
@@ -1812,6 +2012,7 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         // that the dK/dV kernel is still writing.
         cfg.numAttrs = (!COPIES && (phases & 2) && (int64_t)p.Nk * D * 4 <= (int64_t)tile::kBwdOverlapMaxKvBytes) ? 1 : 0;
         // stationary Q_i (its fp16 copy), dO_i; streamed K_j (its fp16 copy), V_j
+        outputs(p.dq, p.dq);
         FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k1, mq16, mg, mk16, mv, mdq, mdq, mdq, mb, mds, a));
     }
     return FA_OK;

@@ -63,6 +63,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Whether the phase with the given parity is complete, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 
 // Wall-clock limit of one wait.  The longest legitimate wait inside a CTA is
 // one pipeline step (microseconds); the default of two seconds means a protocol
@@ -445,6 +457,27 @@ __device__ __forceinline__ void convert_tile_bf16_to_f16(uint8_t* tile, int byte
         }
         p[i * nthreads] = v;
     }
+}
+
+// Work of blocks that have not been launched yet (clusterlaunchcontrol, sm_100).  A request takes the next block of the
+// grid off the hardware's list; its answer (16 bytes, 16-byte aligned) arrives on `bar`.  After an answer without a block
+// no further request may be made.
+__device__ __forceinline__ void clc_request(uint32_t* answer, uint64_t* bar) {
+    mbar_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool clc_answer_block(const uint32_t* answer, uint3& block) {
+    uint32_t got;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+        "ld.shared.b128 r, [%4];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "selp.u32 %3, 1, 0, p;\n\t"
+        "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n\t}"
+        : "=r"(block.x), "=r"(block.y), "=r"(block.z), "=r"(got) : "r"(smem_u32(answer)) : "memory");
+    return got != 0;
 }
 
 // Programmatic dependent launch.  launch_dependents: the next kernel in the stream, if it was launched
