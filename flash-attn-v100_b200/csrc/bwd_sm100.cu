@@ -642,76 +642,50 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                                kk > 0);
             };
 
-            // n_iter, sum_steps: of the block at work, from its last step on of the one behind it; `items` blocks with steps
-            // came before.  A block's first S and dP are issued beside the last step of the block before it, its
-            // accumulators are first written behind a hand-off that the threads make when they have read those of the
-            // block before.
+            // A block's first S and dP are issued behind the last MMAs of the block before it; its accumulators are first
+            // written behind a hand-off that the threads make when they have read those of the block before.
+            // The loop over the steps holds nothing but a step: this thread is what a step waits for, and with a block's start
+            // folded into the loop the dQ kernel took 154 us for 128 steps instead of 138 (one head, N 16384, D 128), the
+            // other one 225 instead of 218.
             bool ok = true;
-            int n_next = 0, sum_next = 0;
-            int blocks = 0, items = 0, g = 0;        // g: steps so far
-            auto next_block = [&] {
-                ok = item_there(blocks);
-                if (!ok) return;
-                n_next = sched[blocks & 1].n_iter;
-                if (DS) sum_next = sched[blocks & 1].n_per_head;
-                mbar_arrive(&bars[Cfg::kSchedEmpty + (blocks & 1)]);
-                ++blocks;
-            };
-            // S (dP) of the next step; `item` the number of its block, `first`, `last`: whether it is that one's first, last step
-            auto next_t1 = [&](uint32_t strm_u, int item, bool first, bool last) {
-                if (first) {
-                    ok = mbar_wait(&bars[kXReady], (uint32_t)item & 1u, abort_flag);
-                    if (!ok) return;
-                    tc_fence_after_sync();
-                }
-                issue_t(tT1, sX_u, strm_u, idesc_t1);
-                mma_commit(&bars[Cfg::kT1Full]);
-                if (last && !FUSED) mma_commit(&bars[Cfg::kXEmpty]);
-            };
-            auto next_t2 = [&](uint32_t strm_u, int slot, uint32_t ph, int step, int item, bool first, bool last) {
-                ok = mbar_wait(&bars[kWReady + slot], ph & 1u, abort_flag);
-                if (ok && first) ok = mbar_wait(&bars[kYReady], (uint32_t)item & 1u, abort_flag);
-                if (!ok) return;
-                tc_fence_after_sync();
-                // query-stationary: the buffer of this step held dS of two steps ago, whose dQ MMAs were issued before
-                const bool odd = !KS && (step & 1);
-                issue_t(odd ? tAcc2 : tT2, sY_u, strm_u, idesc_t2);
-                mma_commit(&bars[odd ? Cfg::kT1Full + 1 : Cfg::kT2Full]);
-                if (!KS) mma_commit(&bars[Cfg::kWEmpty + slot]);             // MODE 1: V_j is read by dP(j) only
-                if (last) mma_commit(&bars[Cfg::kYEmpty]);
-            };
+            int blocks = 0, items = 0, g = 0;        // blocks, blocks with steps, steps so far
             int us = 0, ws = 0;                      // ring slots of this step's U and W
             uint32_t uph = 0, wph = 0;               // wrap counts (parity of the slots' phases)
-            bool begun = false;                      // whether the block's first S and dP are out
-            next_block();
-            for (; ok; ++items) {
-                // blocks without steps: one at a time, since the threads are done with a block's slot when they have ended
-                // the block, and there are two slots
-                while (ok && n_next == 0) next_block();
-                if (!ok || n_next < 0) break;
-                const int n_iter = n_next, sum_steps = sum_next;
-                if (!begun) {
-                    ok = mbar_wait(&bars[kUReady + us], uph & 1u, abort_flag);
-                    if (ok) next_t1(sU_u + us * TILE, items, true, n_iter == 1);
-                    if (ok) next_t2(sW_u + ws * TILE, ws, wph, g, items, true, n_iter == 1);
-                }
-                for (int it = 0; it < n_iter && ok; ++it, ++g) {
+            for (;;) {
+                // (blocks without steps one at a time: the threads are done with a block's slot when they have ended the block,
+                // and there are two slots)
+                ok = item_there(blocks);
+                if (!ok) break;
+                const int n_iter = sched[blocks & 1].n_iter;
+                [[maybe_unused]] const int sum_steps = DS ? sched[blocks & 1].n_per_head : 0;
+                mbar_arrive(&bars[Cfg::kSchedEmpty + (blocks & 1)]);
+                ++blocks;
+                if (n_iter < 0) break;
+                if (n_iter == 0) continue;
+                ok = mbar_wait(&bars[kUReady + us], uph & 1u, abort_flag);
+                if (ok) ok = mbar_wait(&bars[kXReady], (uint32_t)items & 1u, abort_flag);
+                if (!ok) break;
+                tc_fence_after_sync();
+                issue_t(tT1, sX_u, sU_u + us * TILE, idesc_t1);
+                mma_commit(&bars[Cfg::kT1Full]);
+                if (n_iter == 1 && !FUSED) mma_commit(&bars[Cfg::kXEmpty]);
+                ok = mbar_wait(&bars[kWReady + ws], wph & 1u, abort_flag);
+                if (ok) ok = mbar_wait(&bars[kYReady], (uint32_t)items & 1u, abort_flag);
+                if (!ok) break;
+                tc_fence_after_sync();
+                issue_t((!KS && (g & 1)) ? tAcc2 : tT2, sY_u, sW_u + ws * TILE, idesc_t2);
+                mma_commit(&bars[(!KS && (g & 1)) ? Cfg::kT1Full + 1 : Cfg::kT2Full]);
+                if (!KS) mma_commit(&bars[Cfg::kWEmpty + ws]);               // MODE 1: V_j is read by dP(j) only
+                if (n_iter == 1) mma_commit(&bars[Cfg::kYEmpty]);
+                for (int it = 0; it < n_iter; ++it, ++g) {
                     int nus = us + 1, nws = ws + 1;      // slots of the next step
                     uint32_t nuph = uph, nwph = wph;
                     if (nus == UST) { nus = 0; ++nuph; }
                     if (nws == WST) { nws = 0; ++nwph; }
                     const uint32_t cur_u = sU_u + us * TILE, nxt_u = sU_u + nus * TILE;
                     const uint32_t cur_w = sW_u + ws * TILE, nxt_w = sW_u + nws * TILE;
-                    const bool last = it + 1 == n_iter;
-                    if (last) { next_block(); if (!ok) break; }
-                    const bool more = !last || n_next > 0;
-                    begun = more;
-                    const int nitem = items + (last ? 1 : 0);
-                    const bool nlast = last ? n_next == 1 : it + 2 == n_iter;
+                    const bool more = it + 1 < n_iter, ends = it + 2 == n_iter;      // ends: the next step is the block's last
                     if (more) { ok = mbar_wait(&bars[kUReady + nus], nuph & 1u, abort_flag); if (!ok) break; }
-                    // the next block's S goes out early where its stationary tile is there
-                    auto t1_now = [&] { return more && (!last || (!FUSED && mbar_test(&bars[kXReady], (uint32_t)nitem & 1u))); };
-                    bool t1_out = false;
                     if (KS) {
                         ok = mbar_wait(&bars[Cfg::kPHalf], (uint32_t)g & 1u, abort_flag);
                         if (!ok) break;
@@ -721,9 +695,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         if (!ok) break;
                         tc_fence_after_sync();
                         issue_acc_half(tAcc2, tT1, cur_w, it > 0, 1);
-                        if (!last) mma_commit(&bars[Cfg::kWEmpty + ws]);             // dO_i: dP^T(i) earlier, dV(i) last
-                        if ((t1_out = t1_now())) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
-                    } else {
+                        if (more) {
+                            mma_commit(&bars[Cfg::kWEmpty + ws]);                    // dO_i: dP^T(i) earlier, dV(i) last
+                            issue_t(tT1, sX_u, nxt_u, idesc_t1);
+                            mma_commit(&bars[Cfg::kT1Full]);
+                            if (ends && !FUSED) mma_commit(&bars[Cfg::kXEmpty]);
+                        }
+                    } else if (more) {
                         // dQ needs no second accumulator, and P never goes back to tensor memory here: S has one
                         // buffer, free again as soon as the threads hold S(it) in registers, and dP / dS have
                         // two (T2 and the columns a second accumulator would take).  S(it+1) and dP(it+1) are
@@ -733,8 +711,16 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)g & 1u, abort_flag);     // S(it) is in registers
                         if (!ok) break;
                         tc_fence_after_sync();
-                        if ((t1_out = t1_now())) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
-                        if (more && !last) { next_t2(nxt_w, nws, nwph, g + 1, nitem, false, nlast); if (!ok) break; }
+                        issue_t(tT1, sX_u, nxt_u, idesc_t1);
+                        mma_commit(&bars[Cfg::kT1Full]);
+                        ok = mbar_wait(&bars[kWReady + nws], nwph & 1u, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        // the buffer of step it+1 held dS(it-1), which dQ(it-1) read: issued before, in order
+                        issue_t(((g + 1) & 1) ? tAcc2 : tT2, sY_u, nxt_w, idesc_t2);
+                        mma_commit(&bars[((g + 1) & 1) ? Cfg::kT1Full + 1 : Cfg::kT2Full]);
+                        mma_commit(&bars[Cfg::kWEmpty + nws]);
+                        if (ends) { mma_commit(&bars[Cfg::kXEmpty]); mma_commit(&bars[Cfg::kYEmpty]); }
                     }
                     // query-stationary: a barrier pair per dP / dS buffer (phase = uses of that buffer), which
                     // the threads cannot lap: dS(it+2) needs dP(it+2), issued after these waits
@@ -752,7 +738,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     tc_fence_after_sync();
                     if (acc) issue_acc_half(tAcc1, tDs, cur_u, it > sum_steps, 1);
                     // last reader of U(it); a block's last U and W tiles' places take its results first
-                    mma_commit(&bars[last ? Cfg::kAccDone : Cfg::kUEmpty + us]);
+                    mma_commit(&bars[more ? Cfg::kUEmpty + us : Cfg::kAccDone]);
                     if (FUSED) {
                         // dQ tile of this step = dS K_j: A is the dS^T tile the threads left in shared memory,
                         // read MN-major (M = queries), B is the stationary K tile read MN-major (N = D).  Only the previous
@@ -764,12 +750,23 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                         }
                         issue_dq();
                         mma_commit(&bars[Cfg::kDqFull]);
-                        if (last) mma_commit(&bars[Cfg::kXEmpty]);
+                        if (!more) mma_commit(&bars[Cfg::kXEmpty]);
                     }
-                    if (more && !t1_out) { next_t1(nxt_u, nitem, last, nlast); if (!ok) break; }
-                    if (more && (KS || last)) { next_t2(nxt_w, nws, nwph, g + 1, nitem, last, nlast); if (!ok) break; }
+                    if (KS && more) {
+                        ok = mbar_wait(&bars[kWReady + nws], nwph & 1u, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        issue_t(tT2, sY_u, nxt_w, idesc_t2);
+                        mma_commit(&bars[Cfg::kT2Full]);
+                        if (ends) mma_commit(&bars[Cfg::kYEmpty]);
+                    }
                     us = nus; uph = nuph; ws = nws; wph = nwph;
                 }
+                if (!ok) break;
+                // query-stationary: the next block's S overwrites the last one's, which has to be in registers
+                if (!KS) ok = mbar_wait(&bars[Cfg::kPReady], (uint32_t)(g - 1) & 1u, abort_flag);
+                if (!ok) break;
+                ++items;
             }
         }
         __syncwarp();
@@ -779,6 +776,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // reader (the MMAs wait for U_conv, W_conv), dO tiles normalised on the way.
         const int ct = (warp - kTmaWarp - 1) * 32 + lane;
         const bool stores = warp == kTmaWarp + 2 && lane == 0;
+        constexpr uint32_t kIdleNs = 200;          // (looking all the time it slowed every step by a tenth)
         int us = 0, ws = 0, items = 0, steps = 0;
         uint32_t uph = 0, wph = 0;
         bool ok = true;
@@ -792,7 +790,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive_warp(&bars[conv]);
         };
         for (int k = 0; ; ++k) {
-            ok = ok && item_there(k);
+            ok = ok && mbar_wait(&bars[Cfg::kSchedFull + (k & 1)], (uint32_t)(k >> 1) & 1u, abort_flag, STREAM_CONV ? 0u : kIdleNs);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             const volatile BwdItem* m = sched + (k & 1);
@@ -801,7 +799,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_arrive_warp(&bars[Cfg::kSchedEmpty + (k & 1)]);
             if (n_iter < 0) break;
             if (n_iter == 0) continue;
-            if (K_COPY && stores && mbar_wait(&bars[Cfg::kXConv], (uint32_t)items & 1u, abort_flag)) {
+            if (K_COPY && stores && mbar_wait(&bars[Cfg::kXConv], (uint32_t)items & 1u, abort_flag, kIdleNs)) {
                 // the fp16 K tile is what the dQ kernel streams: keep a copy (rows beyond Nk are clipped)
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kNBox; ++bx)
@@ -822,7 +820,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (!ok) break;
             }
             steps += n_iter;
-            if (stores && mbar_wait(&bars[Cfg::kEpi], (uint32_t)items & 1u, abort_flag)) {
+            if (stores && mbar_wait(&bars[Cfg::kEpi], (uint32_t)items & 1u, abort_flag, kIdleNs)) {
                 const int su = (steps - 1) % UST, sw = (steps - 1) % WST;
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kNBox; ++bx) {
@@ -911,7 +909,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         uint32_t count = 0u;                 // blocks (bits 0-1), blocks with steps (bit 2): as much as the barriers' phases need
         ok = __all_sync(0xffffffffu, item_there(0));
         if (XY_CONV && ok && sched[0].n_iter > 0) ok = convert_xy(0, 0u);
+        auto scales = [&](const volatile BwdItem* m) {
+            const float range[2] = {m->range[0], m->range[1]};
+            return make_scales(range, D, a.inv_keep, a.scale, kForm);
+        };
         while (ok) {
+        [[maybe_unused]] BwdScales sc_row;       // ROW_MAX: the row's own
+        {
         const volatile BwdItem* m = sched + (count & 1u);
         const int tile = m->tile, head_x = m->head_x, b = m->b, nk = m->nk, it0 = m->it0, n_per_head = m->n_per_head, n_iter = m->n_iter;
         [[maybe_unused]] const int sum_steps = DS ? n_per_head : 0;
@@ -922,11 +926,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (!ok) break;
         }
         const int row_g = tile * kTile + r;                    // MODE 0: key index; MODE 1: query index
-        auto scales = [&] {
-            const float range[2] = {m->range[0], m->range[1]};
-            return make_scales(range, D, a.inv_keep, a.scale, kForm);
-        };
-        BwdScales sc = scales();
+        BwdScales sc = scales(m);
         float my_nlse2 = 0.f, my_ndelta = 0.f;      // -lse*log2(e) and -delta of my query row (MODE 1)
         if (MODE == 1 && n_iter > 0) {
             ok = mbar_wait(&bars[Cfg::kRowFull], (count >> 2) & 1u, abort_flag);
@@ -1608,14 +1608,19 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
 
         if (FUSED && n_iter > 0 && ok) ok = drain_dq(g - 1, prev_tile, prev_head);
 
+        if (ROW_MAX) sc_row = sc;
+        }
         // ---- epilogue: accumulators -> 16-bit -> swizzled staging -> TMA store.  dK or dQ goes to the place of the block's
         // last U tile, dV to that of its last W tile; warp 19 sends them off and gives the places back to the producer.
         // (Straight from registers a warp's 16-byte stores go to 32 rows each: 2200 cycles at D = 64, 4000 at D = 128.)
         if (ok) ok = item_there((int)((count + 1u) & 3u));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+        // (read again: what is not held through the steps leaves their loop its registers)
+        const volatile BwdItem* m = sched + (count & 1u);
+        const int n_iter = m->n_iter;
         if (XY_CONV && sched[(count & 1u) ^ 1u].n_iter > 0) ok = convert_xy(0, ((count >> 2) & 1u) ^ (n_iter > 0 ? 1u : 0u));
-        if (!ROW_MAX) sc = scales();                       // (not kept through the steps)
+        const BwdScales sc = ROW_MAX ? sc_row : scales(m);
         if (n_iter > 0 && ok) ok = mbar_wait(&bars[Cfg::kAccDone], (count >> 2) & 1u, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -1646,10 +1651,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             tc_fence_before_sync();                        // (the next block's first hand-off lets them be overwritten)
             fence_proxy_async_smem();
             mbar_arrive_warp(&bars[Cfg::kEpi]);
-        } else if (row_g < (KS ? a.Nk : a.Nq)) {
+        } else if (m->tile * kTile + r < (KS ? a.Nk : a.Nq)) {
             // no query sees this key tile
-            uint16_t* dst1 = (uint16_t*)a.out1 + b * a.o1_sb + (int64_t)row_g * a.o1_sn + head_x * a.o1_sh;
-            uint16_t* dst2 = (uint16_t*)a.out2 + b * a.o2_sb + (int64_t)row_g * a.o2_sn + head_x * a.o2_sh;
+            const int64_t row = m->tile * kTile + r;
+            uint16_t* dst1 = (uint16_t*)a.out1 + m->b * a.o1_sb + row * a.o1_sn + m->head_x * a.o1_sh;
+            uint16_t* dst2 = (uint16_t*)a.out2 + m->b * a.o2_sb + row * a.o2_sn + m->head_x * a.o2_sh;
 #pragma unroll
             for (int col = wg * kCols; col < (wg + 1) * kCols; col += 8) {
                 if (PREC != 0 && col >= a.d) break;

@@ -98,13 +98,15 @@ __device__ __forceinline__ void report_status(int32_t* status, int32_t code) {
     }
 }
 
-// Wait for the phase with the given parity; false when the wait ran out or the flag was raised.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+// Wait for the phase with the given parity; false when the wait ran out or the flag was raised.  `sleep_ns`: a wait that
+// nothing hurries pauses between its looks, which would take issue slots from the warps that work.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t sleep_ns = 0u) {
     if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     uint32_t spins = 0;
     while (true) {
         if (mbar_try_wait(bar, parity)) return true;
+        if (sleep_ns) __nanosleep(sleep_ns);
         if ((++spins & 63u) == 0) {
             if (abort_flag[0]) return false;
             if (globaltimer_ns() - t0 > (uint64_t)abort_flag[1] * 1000ull) {
