@@ -59,9 +59,6 @@ constexpr int kBoxBytes = 128 * 128;   // one TMA box: 128 rows x 64 16-bit elem
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = tile::kFwdRescaleLog2;   // log2 units
-// Share of the exponentials evaluated by the FMA-pipe polynomial instead of the special-function
-// unit: in kPolyCount of every kPolyPeriod groups of four, two (tile_config.cuh has the measurements).
-constexpr int kPolyPeriod = tile::kFwdPolyPeriod, kPolyCount = tile::kFwdPolyCount;
 // The first 64 keys of P are handed to the MMA warp after this many of the second half's 64
 // exponentials (a multiple of 4), when their tcgen05.st has had time to complete.
 constexpr int kHalfSignalAt = tile::kFwdHalfSignalAt;
@@ -92,6 +89,7 @@ template <int D, int PREC, int SCHED>
 struct FwdCfg {
     static constexpr int kNBox = D / 64;
     static constexpr int kTileBytes = kNBox * kBoxBytes;
+    static constexpr int kPolyPeriod = tile::fwd_poly_period(D);
     static constexpr int kQTiles = SCHED == 2 ? 1 : 2;
     static constexpr int kStages = SCHED == 2 ? tile::fwd_one_tile_kv_stages(D)
                                                  : (PREC == 2 ? tile::fwd_bias_kv_stages(D) : tile::fwd_kv_stages(D));
@@ -845,23 +843,24 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         if (j > first) {
                             // S_t(j) complete implies PV_t(j-1) complete (same issuing thread, in order)
 #pragma unroll
-                            for (int c0 = 0; c0 < D; c0 += 32) {
-                                uint32_t orr[32];
-                                tmem_ld_32x32(tO + c0, orr);
+                            for (int c0 = 0; c0 < D; c0 += 16) {        // (32 at a time: 512 bytes of spills)
+                                uint32_t orr[16];
+                                tmem_ld_32x16(tO + c0, orr);
                                 tmem_wait_ld();
 #pragma unroll
-                                for (int c = 0; c < 32; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
-                                tmem_st_32x32(tO + c0, orr);
+                                for (int c = 0; c < 16; ++c) orr[c] = __float_as_uint(__uint_as_float(orr[c]) * alpha);
+                                tmem_st_32x16(tO + c0, orr);
                             }
                         }
                     }
+                    uint64_t la = 0ull, lb = 0ull;             // {0.f, 0.f}
                     if constexpr (PREC != 0) {
                         // P = e^(x - m) as hi + lo (fp16: times 2^kPShift), base 2 and the shift behind the difference, which is
                         // small where P is not.  A row that has seen only -inf so far keeps m = -inf; 0 in its place lets its
                         // P come out as 0.
                         const float nm = m == -INFINITY ? 0.f : -m;
                         const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale);
-                        uint64_t la = 0ull, lb = 0ull;             // {0.f, 0.f}: four short chains, whose roundings lse shows
+                        // (la, lb: four short chains, whose roundings lse shows)
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
                             if (q4 == 3) {
@@ -909,45 +908,41 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     // overlap the exponentials of the other half.
                     const float ms = kPShift - (FREE && m == -INFINITY ? 0.f : m);     // nothing seen yet: P = 0
                     const uint64_t c2 = f2_pack(a.scale_log2, a.scale_log2), nm2 = f2_pack(ms, ms);
-                    uint64_t la = 0ull, lb = 0ull;             // {0.f, 0.f}
+                    uint32_t pk[32];
 #pragma unroll
-                    for (int c0 = 0; c0 < 2; ++c0) {
-                        uint32_t pk[32];
-#pragma unroll
-                        for (int cc = 0; cc < 64; cc += 4) {
-                            const int c = c0 * 64 + cc;
-                            float x0, x1, x2, x3, p0, p1, p2, p3;
-                            if (DROP != 1 && c0 == 1 && cc == kHalfSignalAt) {
-                                // the first half's store has had these groups' time to complete
-                                tmem_wait_st();
-                                tc_fence_before_sync();
-                                mbar_arrive_warp(&bars[Cfg::kPHalf + t]);
-                            }
-                            f2_unpack(f2_fma(f2_pack(SF(c), SF(c + 1)), c2, nm2), x0, x1);
-                            f2_unpack(f2_fma(f2_pack(SF(c + 2), SF(c + 3)), c2, nm2), x2, x3);
-                            p0 = ex2(x0); p1 = ex2(x1);
-                            if (((cc >> 2) % kPolyPeriod) < kPolyCount) ex2_poly2(x2, x3, p2, p3);
-                            else { p2 = ex2(x2); p3 = ex2(x3); }
-                            la = f2_add(la, f2_pack(p0, p1));
-                            lb = f2_add(lb, f2_pack(p2, p3));
-                            if constexpr (DROP == 1) {
-                                SSET(c, p0); SSET(c + 1, p1); SSET(c + 2, p2); SSET(c + 3, p3);
-                            } else {
-                                if constexpr (DROP == 2) {
-                                    // dropped entries leave the MMA's operand, not the row sum above
-                                    const uint32_t word = (c >> 5) == 0 ? kb4.x : ((c >> 5) == 1 ? kb4.y : ((c >> 5) == 2 ? kb4.z : kb4.w));
-                                    const uint32_t kw = word >> (c & 31);
-                                    if (!(kw & 1u)) p0 = 0.f;
-                                    if (!(kw & 2u)) p1 = 0.f;
-                                    if (!(kw & 4u)) p2 = 0.f;
-                                    if (!(kw & 8u)) p3 = 0.f;
-                                }
-                                pk[cc / 2] = pack2<P_BF16>(p0, p1);
-                                pk[cc / 2 + 1] = pack2<P_BF16>(p2, p3);
-                            }
+                    for (int c = 0; c < 128; c += 4) {
+                        if (DROP != 1 && c == 64) tmem_st_32x32(tS, pk);
+                        if (DROP != 1 && c == 64 + kHalfSignalAt) {
+                            // the first half's store has had these groups' time to complete
+                            tmem_wait_st();
+                            tc_fence_before_sync();
+                            mbar_arrive_warp(&bars[Cfg::kPHalf + t]);
                         }
-                        if constexpr (DROP != 1) tmem_st_32x32(tS + c0 * 32, pk);
+                        float x0, x1, x2, x3, p0, p1, p2, p3;
+                        f2_unpack(f2_fma(f2_pack(SF(c), SF(c + 1)), c2, nm2), x0, x1);
+                        f2_unpack(f2_fma(f2_pack(SF(c + 2), SF(c + 3)), c2, nm2), x2, x3);
+                        p0 = ex2(x0); p1 = ex2(x1);
+                        if ((c >> 2) % Cfg::kPolyPeriod == 0) ex2_poly2(x2, x3, p2, p3);
+                        else { p2 = ex2(x2); p3 = ex2(x3); }
+                        la = f2_add(la, f2_pack(p0, p1));
+                        lb = f2_add(lb, f2_pack(p2, p3));
+                        if constexpr (DROP == 1) {
+                            SSET(c, p0); SSET(c + 1, p1); SSET(c + 2, p2); SSET(c + 3, p3);
+                        } else {
+                            if constexpr (DROP == 2) {
+                                // dropped entries leave the MMA's operand, not the row sum above
+                                const uint32_t word = (c >> 5) == 0 ? kb4.x : ((c >> 5) == 1 ? kb4.y : ((c >> 5) == 2 ? kb4.z : kb4.w));
+                                const uint32_t kw = word >> (c & 31);
+                                if (!(kw & 1u)) p0 = 0.f;
+                                if (!(kw & 2u)) p1 = 0.f;
+                                if (!(kw & 4u)) p2 = 0.f;
+                                if (!(kw & 8u)) p3 = 0.f;
+                            }
+                            pk[(c & 63) / 2] = pack2<P_BF16>(p0, p1);
+                            pk[(c & 63) / 2 + 1] = pack2<P_BF16>(p2, p3);
+                        }
                     }
+                    if constexpr (DROP != 1) tmem_st_32x32(tS + 32, pk);
                     {
                         float s0, s1, s2, s3;
                         f2_unpack(la, s0, s1); f2_unpack(lb, s2, s3);

@@ -20,8 +20,10 @@ constexpr int fwd_bias_kv_stages(int D) { return D == 128 ? 1 : 2; }       // wi
 constexpr int fwd_bias_slots(int D) { return D == 128 ? 3 : 4; }           // of 16 KB per query tile (a block has four)
 constexpr int kFwdRegsSoftmax = 208;    // setmaxnreg split; best of 224/56, 216/72, 208/88, 200/104
 constexpr int kFwdRegsOther = 88;
-constexpr int kFwdPolyPeriod = 2;       // of every kFwdPolyPeriod groups of four exponentials, kFwdPolyCount
-constexpr int kFwdPolyCount = 1;        //   evaluate two on the FMA pipes: 0 % 0.559 ms, 25 % 0.544, 50 % 0.563
+// One of fwd_poly_period(D) groups of four exponentials evaluates two by the polynomial on the FMA pipes instead of the
+// special-function unit.  Cycles of a key block, both query tiles, N = 8192: D = 128 fp16 3030 without, 2960 with one of
+// four, 2865 with one of two; D = 64 fp16 2960, 2717, 2905 (at half the MMAs a block the threads' instructions weigh more).
+constexpr int fwd_poly_period(int D) { return D == 64 ? 4 : 2; }
 constexpr int kFwdHalfSignalAt = 16;    // first half of P handed over after this many of the second half's exps
 constexpr float kFwdRescaleLog2 = 8.f;  // the running maximum is refreshed when it grows by more than 2^8
 
