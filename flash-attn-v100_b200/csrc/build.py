@@ -1,4 +1,5 @@
-"""Build libfa_b200.so for sm_100a with bare nvcc (no torch headers needed).
+"""Build libfa_b200.so for sm_100a with bare nvcc (no torch headers needed), and fa_b200_torch.so, the native autograd
+operator on top of it (torch_op.cpp: host code, torch's headers).
 
 Usage: python build.py [--force] [--verbose]
 The library lands in ../flash_attention_v100/lib/ so it travels with the package.
@@ -10,6 +11,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_DIR = os.path.join(os.path.dirname(HERE), "flash_attention_v100", "lib")
 OUT = os.path.join(OUT_DIR, "libfa_b200.so")
+OP_OUT = os.path.join(OUT_DIR, "fa_b200_torch.so")
+OP_SOURCE = "torch_op.cpp"
 SOURCES = ["host_api.cu", "simt_kernels.cu", "fwd_sm100.cu", "fwd_tf32_sm100.cu", "bwd_sm100.cu", "bwd_f32_sm100.cu", "combine.cu", "compact.cu",
            "fwd_pair_sm100.cu", "bwd_pair_sm100.cu"]
 HEADERS = ["fa_common.cuh", "philox.cuh", "sm100_ptx.cuh", "tma_host.cuh", "tile_config.cuh",
@@ -24,7 +27,37 @@ def _newest(paths):
     return max((os.path.getmtime(p) for p in paths if os.path.exists(p)), default=0.0)
 
 
+def _op_command():
+    import importlib.util
+    import sysconfig
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include",
+            f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}", os.path.join(HERE, OP_SOURCE), "-o", OP_OUT,
+            f"-L{torch_dir}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python",
+            f"-L{OUT_DIR}", "-lfa_b200", "-Wl,-rpath,$ORIGIN"]
+
+
+def build_op(force=False):
+    """The native operator; after the library, which it is linked against."""
+    deps = [os.path.join(HERE, OP_SOURCE), os.path.join(HERE, "..", "..", "include", "fa_b200.h"), os.path.abspath(__file__)]
+    if not force and os.path.exists(OP_OUT) and os.path.getmtime(OP_OUT) >= _newest(deps):
+        return OP_OUT
+    cmd = _op_command()
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout)
+        raise RuntimeError("building the native operator failed")
+    return OP_OUT
+
+
 def build(force=False, verbose=False):
+    lib = build_library(force, verbose)
+    build_op(force)
+    return lib
+
+
+def build_library(force=False, verbose=False):
     os.makedirs(OUT_DIR, exist_ok=True)
     srcs = [os.path.join(HERE, s) for s in SOURCES]
     deps = srcs + [os.path.join(HERE, h) for h in HEADERS] + [os.path.abspath(__file__)]

@@ -19,7 +19,7 @@ import torch
 import torch.distributed as dist
 
 from .config import get_enhanced_config
-from .ops.attention import FlashAttentionV100Function
+from .ops.attention import FlashAttentionV100Function, native_call
 from .utils import validate_inputs as _validate_inputs
 
 log = logging.getLogger("flash_attention_v100")
@@ -299,15 +299,21 @@ def flash_attention_v100(
     manager = get_flash_attention_manager(enable_multi_gpu=enable_multi_gpu,
                                           optimization_strategy=optimization_strategy,
                                           enable_profiling=enable_profiling)
+    use_multi = manager.enable_multi_gpu if enable_multi_gpu is None else (
+        bool(enable_multi_gpu) and torch.cuda.is_available())
+    profile = manager.enable_profiling or enable_profiling
+    if bias is None and dropout_origin is None and dropout_p == 0.0 and not profile and not (use_multi and len(manager.devices) > 1) \
+            and causal_alignment in ("top_left", "bottom_right"):
+        result = native_call(q, k, v, scale, bool(causal), causal_alignment == "bottom_right", key_lengths,
+                             optimization_strategy == "speed")
+        if result is not None:
+            return result if return_softmax_lse else result[0]
     if validate_inputs:
         q, k, v, scale = _validate_inputs(q, k, v, scale, bias, dropout_p)
     elif scale is None:
         scale = q.shape[-1] ** -0.5
 
     shift = _causal_shift(causal, causal_alignment, q.shape[1], k.shape[1], key_lengths)
-    use_multi = manager.enable_multi_gpu if enable_multi_gpu is None else (
-        bool(enable_multi_gpu) and torch.cuda.is_available())
-    profile = manager.enable_profiling or enable_profiling
     if profile:
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record(torch.cuda.current_stream(q.device))

@@ -13,6 +13,7 @@ import threading
 
 _PKG_DIR = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(_PKG_DIR, "lib", "libfa_b200.so")
+OP_PATH = os.path.join(_PKG_DIR, "lib", "fa_b200_torch.so")
 
 ABI_VERSION = 3
 FA_B200_F16, FA_B200_BF16, FA_B200_F32 = 0, 1, 2
@@ -160,6 +161,30 @@ def load():
             raise FlashAttentionLibraryError("ABI version mismatch")
         _lib = lib
     return _lib
+
+
+_op = None
+
+
+def load_op():
+    """The native autograd operator (csrc/torch_op.cpp), which calls the library above; loaded once, loud if missing."""
+    global _op
+    if _op is not None:
+        return _op
+    load()
+    with _lock:
+        if _op is None:
+            import importlib.machinery
+            import importlib.util
+            import torch  # noqa: F401  (its libraries first)
+            if not os.path.exists(OP_PATH):
+                raise FlashAttentionLibraryError(
+                    f"{OP_PATH} not found: build it with `python {os.path.join(os.path.dirname(_PKG_DIR), 'csrc', 'build.py')}`")
+            loader = importlib.machinery.ExtensionFileLoader("fa_b200_torch", OP_PATH)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("fa_b200_torch", loader))
+            loader.exec_module(module)
+            _op = module
+    return _op
 
 
 def raise_for_status(rc: int, what: str) -> None:

