@@ -792,10 +792,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                                 }
                                 mbar_arrive_read_done(&bars[Cfg::kBiasEmpty + at]);
                                 if (++bias_slot == Cfg::kBiasSlots) { bias_slot = 0; bias_ph ^= 1u; }
-                            } else if (!a.bias) {
-#pragma unroll
-                                for (int c = 0; c < 32; ++c) SSET(q4 * 32 + c, SF(q4 * 32 + c) * a.scale);
-                            } else {
+                            } else if (a.bias) {
                                 const float* bp = brow + col0 + q4 * 32;
                                 if (a.bias_vec && col0 + q4 * 32 + 32 <= a.Nk) {
 #pragma unroll
@@ -832,7 +829,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         mx0 = max3(mx0, SF(c), SF(c + 1)); mx1 = max3(mx1, SF(c + 2), SF(c + 3));
                         if (c + 4 < 128) { mx2 = max3(mx2, SF(c + 4), SF(c + 5)); mx3 = max3(mx3, SF(c + 6), SF(c + 7)); }
                     }
-                    const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * (PREC ? 1.f : a.scale_log2);
+                    // with a bias the scores are x already, without one x = S scale is left to the FMA that takes the maximum off
+                    const float to_x = PREC == 0 ? a.scale_log2 : (PREC == 1 && !a.bias ? a.scale : 1.f);
+                    const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * to_x;
                     const float m_new = fmaxf(m, mx);
                     const bool grow = (m_new - m) > (PREC ? kRescaleThreshold * kLn2 : kRescaleThreshold);   // first block: inf > 8
                     if (__any_sync(0xffffffffu, grow)) {
@@ -859,7 +858,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         // small where P is not.  A row that has seen only -inf so far keeps m = -inf; 0 in its place lets its
                         // P come out as 0.
                         const float nm = m == -INFINITY ? 0.f : -m;
-                        const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale);
+                        const uint64_t nm2 = f2_pack(nm, nm), log2e2 = f2_pack(kLog2e, kLog2e), up2 = f2_pack(kPScale, kPScale), to_x2 = f2_pack(to_x, to_x);
                         // (la, lb: four short chains, whose roundings lse shows)
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
@@ -873,7 +872,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                             for (int cc = 0; cc < 32; cc += 2) {
                                 const int c = q4 * 32 + cc;
                                 float p0, p1;
-                                f2_unpack(f2_mul(f2_add(f2_pack(SF(c), SF(c + 1)), nm2), log2e2), p0, p1);
+                                f2_unpack(f2_mul(PREC == 1 ? f2_fma(f2_pack(SF(c), SF(c + 1)), to_x2, nm2) : f2_add(f2_pack(SF(c), SF(c + 1)), nm2), log2e2), p0, p1);
                                 uint64_t p2 = f2_pack(ex2(p0), ex2(p1));
                                 if (!P_BF16) p2 = f2_mul(p2, up2);
                                 if (cc & 2) lb = f2_add(lb, p2); else la = f2_add(la, p2);

@@ -413,9 +413,10 @@ __device__ __forceinline__ void unpack2(uint32_t v, float& lo, float& hi) {
 template <bool BF16>
 __device__ __forceinline__ void pack2_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
     hi = pack2<BF16>(x0, x1);
-    float h0, h1;
+    float h0, h1, d0, d1;
     unpack2<BF16>(hi, h0, h1);
-    lo = pack2<BF16>(x0 - h0, x1 - h1);
+    f2_unpack(f2_fma(f2_pack(h0, h1), 0xBF800000BF800000ull, f2_pack(x0, x1)), d0, d1);      // x - h, both at once
+    lo = pack2<BF16>(d0, d1);
 }
 
 // ---- bf16 -> fp16 in shared memory ---------------------------------------------------------------
