@@ -80,12 +80,14 @@ struct F32Args {
 // x -> three bf16 planes, two values packed per word
 __device__ __forceinline__ void split3(float x0, float x1, uint32_t& a, uint32_t& b, uint32_t& c) {
     float h0, h1;
+    auto less = [&] { f2_unpack(f2_fma(f2_pack(h0, h1), 0xBF800000BF800000ull, f2_pack(x0, x1)), x0, x1); };     // x -= h, both at once
     a = pack2<true>(x0, x1);
     unpack2<true>(a, h0, h1);
-    x0 -= h0; x1 -= h1;
+    less();
     b = pack2<true>(x0, x1);
     unpack2<true>(b, h0, h1);
-    c = pack2<true>(x0 - h0, x1 - h1);
+    less();
+    c = pack2<true>(x0, x1);
 }
 
 template <int MODE>
@@ -132,10 +134,6 @@ bwd_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         wait_control_init(abort_flag, a.wait_limit_ms);
         fence_mbar_init();
     }
-    // The dQ kernel reads nothing the dK/dV kernel writes: it may take the SMs that this grid's last blocks leave idle
-    // (launched serialized behind this grid, it waits for it only before it ends).  B2 N1024 H12 causal has 192 blocks
-    // of 1 to 8 units in each.  The step at B4 N2048 H8 causal 538 -> 521 us, at B4 N1500 H8 without a mask 597 -> 587.
-    if (KS) grid_launch_dependents();
     if (warp == kWorkers) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -147,6 +145,13 @@ bwd_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    if (KS) {
+        grid_dependency_wait();                 // the planes: what stands above ran beside the end of the split kernel
+        // The dQ kernel reads nothing the dK/dV kernel writes: it may take the SMs that this grid's last blocks leave idle
+        // (launched serialized behind this grid, it waits for it only before it ends).  B2 N1024 H12 causal has 192 blocks
+        // of 1 to 8 units in each.  The step at B4 N2048 H8 causal 538 -> 521 us, at B4 N1500 H8 without a mask 597 -> 587.
+        grid_launch_dependents();
+    }
     const uint32_t tmem = *tmem_slot;
     const uint32_t tT1 = tmem, tT2 = tmem + 64u, tP = tmem + 128u, tDs = tmem + 224u, tAcc1 = tmem + 320u, tAcc2 = tmem + 384u, tT1b = tmem + 448u;
 
@@ -403,61 +408,71 @@ bwd_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     if (!KS) grid_dependency_wait();            // the end of this grid must still mean the end of the dK/dV grid
 }
 
-// Planes of the four operands, delta and the padded lse: one warp per row, two columns per lane.  Rows [0, q_rows) are
-// (batch, padded query, head), the rest (batch, key, K/V head), heads fastest as in memory.
+// Planes of the four operands, delta and the padded lse.  Eight lanes share a row, eight columns each: 32 bytes of an fp32
+// operand come in two loads, 16 bytes go to each plane.  Rows [0, q_rows) are (batch, padded query, head), the rest (batch,
+// key, K/V head), heads fastest as in memory.  Bound by the stores: B2 N1024 H12 is 25 MB in (31 with o) and 38 MB out.  One
+// warp a row with 4-byte accesses and 64-bit divisions took 17.2 us there, this 9.3.
 struct SplitArgs {
     fa_b200_tensor q, k, v, o, d_o;
     const float* lse_in;
     uint32_t *q16, *g16, *k16, *v16;      // planes, two columns per word
     float *lse, *delta;
     int B, Nq, Nk, H, Hkv, nq_pad;
-    int64_t q_rows, rows;
+    uint32_t q_rows, rows;
+    int vec_q, vec_kv;                    // their rows can be read as float4
 };
 __global__ void __launch_bounds__(256) bwd_f32_split_kernel(const SplitArgs a) {
-    const int lane = threadIdx.x & 31, c = 2 * lane;
-    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (row >= a.rows) return;
-    auto load = [&](const fa_b200_tensor& t, int b, int n, int h, float& x0, float& x1) {
-        const float* src = (const float*)t.ptr + (int64_t)b * t.stride_b + (int64_t)n * t.stride_n + (int64_t)h * t.stride_h + c;
-        x0 = src[0];
-        x1 = src[1];
+    grid_launch_dependents();
+    const uint32_t sub = threadIdx.x & 7u, row = blockIdx.x * 32u + (threadIdx.x >> 3);
+    const bool in = row < a.rows;
+    auto load = [&](const fa_b200_tensor& t, bool vec, uint32_t b, uint32_t n, uint32_t h, float (&x)[8]) {
+        const float* src = (const float*)t.ptr + b * t.stride_b + n * t.stride_n + h * t.stride_h + sub * 8;
+        if (vec) {
+            const float4 lo = reinterpret_cast<const float4*>(src)[0], hi = reinterpret_cast<const float4*>(src)[1];
+            x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[e] = src[e];
+        }
     };
-    auto store = [&](uint32_t* dst, int N, int H, int b, int n, int h, float x0, float x1) {
-        uint32_t p[kPlanes];
-        split3(x0, x1, p[0], p[1], p[2]);
+    auto store = [&](uint32_t* dst, uint32_t N, uint32_t H, uint32_t b, uint32_t n, uint32_t h, const float (&x)[8]) {
+        uint32_t p[kPlanes][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split3(x[2 * e], x[2 * e + 1], p[0][e], p[1][e], p[2][e]);
 #pragma unroll
         for (int i = 0; i < kPlanes; ++i)
-            dst[((((int64_t)i * a.B + b) * N + n) * H + h) * (kDim / 2) + lane] = p[i];
+            *reinterpret_cast<uint4*>(dst + ((((int64_t)i * a.B + b) * N + n) * H + h) * (kDim / 2) + sub * 4) =
+                make_uint4(p[i][0], p[i][1], p[i][2], p[i][3]);
     };
-    float x0, x1, y0, y1;
-    if (row < a.q_rows) {
-        const int h = (int)(row % a.H);
-        const int64_t rest = row / a.H;
-        const int i = (int)(rest % a.nq_pad), b = (int)(rest / a.nq_pad);
-        const int64_t at = ((int64_t)b * a.H + h) * a.nq_pad + i;
-        if (i >= a.Nq) {
-            if (lane == 0) { a.lse[at] = INFINITY; a.delta[at] = 0.f; }
-            return;
+    float x[8], y[8];
+    float s = 0.f;                         // (every lane takes part in the sum below)
+    int64_t at = -1;
+    if (in && row < a.q_rows) {
+        const uint32_t rest = row / (uint32_t)a.H, h = row - rest * (uint32_t)a.H, b = rest / (uint32_t)a.nq_pad, i = rest - b * (uint32_t)a.nq_pad;
+        const int64_t out = ((int64_t)b * a.H + h) * a.nq_pad + i;
+        if (i >= (uint32_t)a.Nq) {
+            if (sub == 0) { a.lse[out] = INFINITY; a.delta[out] = 0.f; }
+        } else {
+            at = out;
+            load(a.q, a.vec_q, b, i, h, x);
+            store(a.q16, a.Nq, a.H, b, i, h, x);
+            load(a.d_o, a.vec_q, b, i, h, x);
+            load(a.o, a.vec_q, b, i, h, y);
+            store(a.g16, a.Nq, a.H, b, i, h, x);
+            s = (fmaf(x[0], y[0], x[1] * y[1]) + fmaf(x[2], y[2], x[3] * y[3])) + (fmaf(x[4], y[4], x[5] * y[5]) + fmaf(x[6], y[6], x[7] * y[7]));
+            if (sub == 0) a.lse[out] = a.lse_in[((int64_t)b * a.H + h) * a.Nq + i];
         }
-        load(a.q, b, i, h, x0, x1);
-        store(a.q16, a.Nq, a.H, b, i, h, x0, x1);
-        load(a.d_o, b, i, h, x0, x1);
-        store(a.g16, a.Nq, a.H, b, i, h, x0, x1);
-        load(a.o, b, i, h, y0, y1);
-        float s = fmaf(x0, y0, x1 * y1);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        if (lane == 0) { a.lse[at] = a.lse_in[((int64_t)b * a.H + h) * a.Nq + i]; a.delta[at] = s; }
-    } else {
-        const int64_t kr = row - a.q_rows;
-        const int h = (int)(kr % a.Hkv);
-        const int64_t rest = kr / a.Hkv;
-        const int j = (int)(rest % a.Nk), b = (int)(rest / a.Nk);
-        load(a.k, b, j, h, x0, x1);
-        load(a.v, b, j, h, y0, y1);
-        store(a.k16, a.Nk, a.Hkv, b, j, h, x0, x1);
-        store(a.v16, a.Nk, a.Hkv, b, j, h, y0, y1);
+    } else if (in) {
+        const uint32_t kr = row - a.q_rows, rest = kr / (uint32_t)a.Hkv, h = kr - rest * (uint32_t)a.Hkv, b = rest / (uint32_t)a.Nk,
+                       j = rest - b * (uint32_t)a.Nk;
+        load(a.k, a.vec_kv, b, j, h, x);
+        load(a.v, a.vec_kv, b, j, h, y);
+        store(a.k16, a.Nk, a.Hkv, b, j, h, x);
+        store(a.v16, a.Nk, a.Hkv, b, j, h, y);
     }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (at >= 0 && sub == 0) a.delta[at] = s;
 }
 
 struct F32Layout { size_t q, g, k, v, lse, delta, bytes; };
@@ -490,17 +505,20 @@ int sm100_f32_bwd(const fa_b200_params& p, void* scratch) {
     cudaStream_t st = (cudaStream_t)p.stream;
     const int nq_pad = (int)align_up((size_t)p.Nq, 128);
     const int phases = p.bwd_phases ? p.bwd_phases : 7;
+    auto aligned = [&](const fa_b200_tensor& t) {
+        return ((uintptr_t)t.ptr & 15u) == 0 && t.stride_b % 4 == 0 && t.stride_n % 4 == 0 && t.stride_h % 4 == 0;
+    };
     if (phases & 1) {
         SplitArgs s;
         s.q = p.q; s.k = p.k; s.v = p.v; s.o = p.o; s.d_o = p.d_o; s.lse_in = p.lse;
         s.q16 = (uint32_t*)(ws + l.q); s.g16 = (uint32_t*)(ws + l.g); s.k16 = (uint32_t*)(ws + l.k); s.v16 = (uint32_t*)(ws + l.v);
         s.lse = (float*)(ws + l.lse); s.delta = (float*)(ws + l.delta);
         s.B = p.B; s.Nq = p.Nq; s.Nk = p.Nk; s.H = p.H; s.Hkv = p.Hkv; s.nq_pad = nq_pad;
-        s.q_rows = (int64_t)p.B * nq_pad * p.H;
-        s.rows = s.q_rows + (int64_t)p.B * p.Nk * p.Hkv;
-        const int64_t blocks = (s.rows + 7) / 8;
-        if (blocks > 0x7fffffff) { set_error("problem too large for the split grid"); return FA_EUNSUPPORTED; }
-        bwd_f32_split_kernel<<<(unsigned)blocks, 256, 0, st>>>(s);
+        const int64_t q_rows = (int64_t)p.B * nq_pad * p.H, rows = q_rows + (int64_t)p.B * p.Nk * p.Hkv;
+        if (rows > 0x7fffffff) { set_error("problem too large for the split grid"); return FA_EUNSUPPORTED; }
+        s.q_rows = (uint32_t)q_rows; s.rows = (uint32_t)rows;
+        s.vec_q = aligned(p.q) && aligned(p.o) && aligned(p.d_o); s.vec_kv = aligned(p.k) && aligned(p.v);
+        bwd_f32_split_kernel<<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(s);
         FA_CUDA_CHECK(cudaGetLastError());
     }
     CUtensorMap mq, mg, mk, mv;
@@ -521,9 +539,6 @@ int sm100_f32_bwd(const fa_b200_params& p, void* scratch) {
     a.causal = p.causal; a.shift = p.causal ? p.causal_shift : 0;
     a.wait_limit_ms = p.wait_limit_ms;
     a.scale = p.scale;
-    auto aligned = [&](const fa_b200_tensor& t) {
-        return ((uintptr_t)t.ptr & 15u) == 0 && t.stride_b % 4 == 0 && t.stride_n % 4 == 0 && t.stride_h % 4 == 0;
-    };
     {
         static std::mutex mu;
         static uint64_t done[2] = {0, 0};
@@ -534,8 +549,14 @@ int sm100_f32_bwd(const fa_b200_params& p, void* scratch) {
         a.out1 = p.dk; a.out2 = p.dv;
         a.vec = aligned(p.dk) && aligned(p.dv);
         const dim3 grid((p.Nk + kRows - 1) / kRows, p.Hkv, p.B);
-        bwd_f32_kernel<0><<<grid, kThreads, kSmemBytes, st>>>(mk, mv, mq, mg, a);
-        FA_CUDA_CHECK(cudaGetLastError());
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid; cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = (phases & 1) ? 1 : 0;        // only behind the split kernel of this call
+        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, bwd_f32_kernel<0>, mk, mv, mq, mg, a));
     }
     if (phases & 4) {
         a.out1 = p.dq; a.out2 = p.dq;
