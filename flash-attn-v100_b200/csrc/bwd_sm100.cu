@@ -429,9 +429,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         fence_mbar_init();
         __syncwarp();
     }
-    // The dQ kernel reads nothing the dK/dV kernel writes: it may take the SMs this grid's last wave
-    // leaves idle (it is launched serialized behind this grid, and waits for it only before it ends).
-    if (MODE == 0) grid_launch_dependents();
     if (warp == kMmaWarp) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -442,6 +439,13 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         tc_fence_before_sync();
         asm volatile("barrier.cta.sync 1, %0;" ::"n"(kAllThreads) : "memory");
         tc_fence_after_sync();
+    }
+    if (MODE == 0) {
+        // The preprocess launch's vectors and copies: what stands above runs beside its end (3 us of a step).
+        grid_dependency_wait();
+        // The dQ kernel reads nothing the dK/dV kernel writes: it may take the SMs this grid's last wave
+        // leaves idle (it is launched serialized behind this grid, and waits for it only before it ends).
+        grid_launch_dependents();
     }
     const uint32_t tmem = *tmem_slot;
     const uint32_t tT1 = tmem, tT2 = tmem + 128u, tAcc1 = tmem + 256u, tAcc2 = tmem + 384u;
@@ -1716,6 +1720,7 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
                       int64_t o_sb, int64_t o_sn, int64_t o_sh, int64_t g_sb, int64_t g_sn, int64_t g_sh,
                       const T* __restrict__ v, int64_t v_sb, int64_t v_sn, int64_t v_sh, int Nk,
                       const int32_t* __restrict__ kv_len, int n_row_blocks, int v_slabs, const PreprocessCopies cp) {
+    grid_launch_dependents();                  // the dK/dV kernel, which waits for this grid's end
     constexpr int LPR = D / 8;                 // lanes per row
     constexpr int RPW = 32 / LPR;              // rows per warp
     constexpr int kVRows = 256;                // keys per slab of the V scan
@@ -2001,8 +2006,14 @@ int launch(const fa_b200_params& p, const BwdWorkspace& ws) {
         // stationary K_j, V_j; streamed Q_i, dO_i (bf16 with copies: their fp16 copies; the kernel leaves
         // the fp16 copy of K behind for the dQ kernel)
         outputs(p.dk, p.dv);
-        k0<<<grid_kv, kThreads, smem0, st>>>(mk, mv, mq16, mg16, mdk, mdv, mk16, mb, mds, a);
-        FA_CUDA_CHECK(cudaGetLastError());
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid_kv; cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem0; cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = (phases & 1) ? 1 : 0;        // only behind the preprocess launch of this call
+        FA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k0, mk, mv, mq16, mg16, mdk, mdv, mk16, mb, mds, a));
     }
     if (phases & 4) {
         cudaLaunchConfig_t cfg = {};

@@ -135,6 +135,7 @@ struct Attention : torch::autograd::Function<Attention> {
         ctx->saved_data["flags"] = (int64_t)c.causal | ((int64_t)c.fast << 1) | (c.shift << 2);
         if (c.lengths.defined()) ctx->saved_data["lengths"] = c.lengths;
         ctx->mark_non_differentiable({lse});
+        ctx->set_materialize_grads(false);             // (lse's would be a launch of zeros)
         return {o, lse};
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -145,6 +146,7 @@ struct Attention : torch::autograd::Function<Attention> {
                      lengths == ctx->saved_data.end() ? at::Tensor() : lengths->second.toTensor()};
         at::Tensor d[3];
         at::AutoDispatchBelowADInplaceOrView below;          // (allocations and a copy: nothing of this is recorded)
+        if (!grads[0].defined()) grads[0] = at::zeros_like(kept[3]);
         ::backward(grads[0], kept[0], kept[1], kept[2], kept[3], kept[4], kept.size() > 5 ? kept[5] : at::Tensor(), c, d[0], d[1], d[2]);
         variable_list out(4);
         for (int i = 0; i < 3; ++i)
