@@ -476,31 +476,38 @@ __device__ __forceinline__ uint32_t transpose_bits_32x32(uint32_t x, int lane) {
 // The keep bits of a whole call, written once for the tensor-core kernels to load (drawing them inside
 // those kernels costs their softmax / elementwise threads as many instructions as the attention math
 // itself; here every SM draws at full integer rate, and the forward's bits serve the backward too).
-// One warp per (column, 32 queries, 128 keys): lane = query, eight Philox blocks of 16 keys each.
+// One warp per (column, 32 R queries, 128 keys): lane = query, query + 32, .., eight Philox blocks of 16 keys each.
+// What bounds it is the integer multiplier (ncu, B4 H16 N2048: its pipe and the logic pipe both about 80 % busy), and
+// four queries a lane (R = 4) share what does not depend on the query: three of a block's twenty wide multiplies, beside
+// the two that its eight key blocks share.  343 -> 294 us at B32 H16 N2048 causal against R = 1 (R = 2: 306); high halves
+// by exact fp64 FMAs, half of them or all, took 301 and 329 us, flags without a wide multiply the same time.
 //   mq[(col * NJ + j128) * nq_pad + i]            uint4: bit c of the 128 = key j128*128 + c   (query-major)
 //   mk[((col * NI + i128) * 4 + g) * nk_pad + k]  uint32: bit q = query i128*128 + 32 g + q     (key-major:
 //       the 32 x 32 transposes of the warp's four words)
 // Tiles the causal mask hides completely hold no bits (nobody reads them: P is zero there).  Under the
-// usual mask (square, key j visible to query i iff j <= i) the 32-query blocks are dealt in pairs, block p
-// with block NIB-1-p: together they have NJ + 1 live key blocks whatever p, so every warp of the grid has
-// work (a grid over all (block, key block) items, half of them hidden, measured 0.36 against 0.33 ms on
-// B32 H16 N2048; a fixed grid that strides over the items 0.56 ms).  Other shapes walk all items and skip.
-__global__ void __launch_bounds__(256, 8)
+// usual mask (square, key j visible to query i iff j <= i) the query blocks are dealt in pairs, block p
+// with block NIB-1-p: together they have NJ + 1 live key blocks whatever p, and the middle block of an odd
+// number (R = 4) has half as many, so every warp of the grid has work (a grid over all (block, key block)
+// items, half of them hidden, measured 0.36 against 0.33 ms on B32 H16 N2048 with R = 1; a fixed grid that
+// strides over the items 0.56 ms).  Other shapes walk all items and skip.
+template <int R>
+__global__ void __launch_bounds__(256, R == 4 ? 4 : 8)
 dropout_bits_kernel(PhiloxKey key, uint32_t thr, DropoutOrigin rng, int H, int Nq, int nq_pad, int nk_pad,
                     int causal, int shift, int paired, int64_t n_items, uint4* __restrict__ mq,
                     uint32_t* __restrict__ mk) {
     const int lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (item >= n_items) return;                                     // whole warps leave together
-    const int NJ = nk_pad / 128, NIB = nq_pad / 32;
+    constexpr int kQueries = 32 * R;
+    const int NJ = nk_pad / 128, NIB = nq_pad / kQueries;
     int j128, ib;
     int64_t col;                                                      // local b * H + h
     if (paired) {
-        const int s = (int)(item % (NJ + 1));
-        const int64_t rest = item / (NJ + 1);
-        const int pr = (int)(rest % (NIB / 2));
-        col = rest / (NIB / 2);
-        const int live_lo = pr / 4 + 1;                               // live key blocks of the pair's first block
+        const uint32_t per_column = (uint32_t)NIB * (uint32_t)(NJ + 1) / 2u;       // an odd NIB ends with half a pair
+        col = item / per_column;
+        const uint32_t t = (uint32_t)(item - col * per_column);
+        const int pr = (int)(t / (uint32_t)(NJ + 1)), s = (int)(t - (uint32_t)pr * (uint32_t)(NJ + 1));
+        const int live_lo = pr * kQueries / 128 + 1;                  // live key blocks of the pair's first block
         ib = s < live_lo ? pr : NIB - 1 - pr;
         j128 = s < live_lo ? s : s - live_lo;
     } else {
@@ -508,19 +515,24 @@ dropout_bits_kernel(PhiloxKey key, uint32_t thr, DropoutOrigin rng, int H, int N
         const int64_t rest = item / NJ;
         ib = (int)(rest % NIB);
         col = rest / NIB;
-        if (causal && (int64_t)j128 * 128 > (int64_t)ib * 32 + 31 + shift) return;
+        if (causal && (int64_t)j128 * 128 > (int64_t)ib * kQueries + kQueries - 1 + shift) return;
     }
-    const int i = ib * 32 + lane;
+    const int i = ib * kQueries + lane;
     const uint32_t column = dropout_column(rng, (int)(col / H), (int)(col % H));
-    uint32_t w4[4] = {0u, 0u, 0u, 0u};
+    uint32_t w4[R][4] = {};
 #pragma unroll
     for (int g = 0; g < 8; ++g)
-        w4[g >> 1] |= dropout_keep_bits(key, column, (uint32_t)i, (uint32_t)(j128 * 8 + g), thr) << (16 * (g & 1));
-    if (mq) mq[(col * NJ + j128) * (int64_t)nq_pad + i] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-    if (mk) {
-        uint32_t* dst = mk + ((col * (nq_pad / 128) + (ib >> 2)) * 4 + (ib & 3)) * (int64_t)nk_pad + j128 * 128 + lane;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) dst[32 * x] = transpose_bits_32x32(w4[x], lane);
+        for (int r = 0; r < R; ++r)
+            w4[r][g >> 1] |= dropout_keep_bits(key, column, (uint32_t)(i + 32 * r), (uint32_t)(j128 * 8 + g), thr) << (16 * (g & 1));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        if (mq) mq[(col * NJ + j128) * (int64_t)nq_pad + i + 32 * r] = make_uint4(w4[r][0], w4[r][1], w4[r][2], w4[r][3]);
+        if (mk) {
+            uint32_t* dst = mk + (col * (nq_pad / 32) + ib * R + r) * (int64_t)nk_pad + j128 * 128 + lane;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) dst[32 * x] = transpose_bits_32x32(w4[r][x], lane);
+        }
     }
 }
 
@@ -618,12 +630,17 @@ int launch_dropout_bits(const fa_b200_params& p, void* mq, void* mk) {
     const int shift = p.causal ? p.causal_shift : 0;
     // the usual causal mask on a square problem: pairs of query blocks, no hidden items (see the kernel)
     const int paired = (p.causal && shift == 0 && nq_pad == nk_pad) ? 1 : 0;
-    const int64_t per_column = paired ? (int64_t)(nq_pad / 64) * (nk_pad / 128 + 1) : (int64_t)(nq_pad / 32) * (nk_pad / 128);
-    const int64_t n_items = (int64_t)p.B * p.H * per_column;
-    const int64_t blocks = (n_items + 7) / 8;
+    auto items = [&](int rows) {
+        return (int64_t)p.B * p.H * (nq_pad / (32 * rows)) * (paired ? nk_pad / 128 + 1 : nk_pad / 128) / (paired ? 2 : 1);
+    };
+    // four queries a lane from 2048 warps on, 14 an SM (one query -> four, us: 576 warps 4.7 -> 7.7, 1152 7.7 -> 7.8,
+    // 2176 13.6 -> 12.5, 4608 24.9 -> 22.3, 17408 85.9 -> 75.9); with fewer a warp's own chain of work is what takes the time
+    const bool wide = items(4) >= 2048;
+    const int64_t n_items = items(wide ? 4 : 1), blocks = (n_items + 7) / 8;
     if (blocks > 0x7fffffff) { set_error("problem too large for the dropout-bits grid"); return FA_EUNSUPPORTED; }
     if (blocks == 0 || (!mq && !mk)) return FA_OK;
-    dropout_bits_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)p.stream>>>(
+    auto kernel = wide ? dropout_bits_kernel<4> : dropout_bits_kernel<1>;
+    kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)p.stream>>>(
         philox_make_key(p.seed, p.offset), dropout_threshold(p.dropout_p), dropout_origin_of(p), p.H, p.Nq, nq_pad,
         nk_pad, p.causal, shift, paired, n_items, (uint4*)mq, (uint32_t*)mk);
     FA_CUDA_CHECK(cudaGetLastError());
