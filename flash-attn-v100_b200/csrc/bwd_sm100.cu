@@ -1756,12 +1756,14 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
     const T* lp = cp.o_lo ? reinterpret_cast<const T*>(cp.o_lo) + b * cp.l_sb + h * cp.l_sh + sub * 8 : nullptr;
     const T* qp = COPIES ? reinterpret_cast<const T*>(cp.q) + b * cp.q_sb + h * cp.q_sh + sub * 8 : nullptr;
     uint32_t m = 0u;
-#pragma unroll 2
+    constexpr int kTogether = COPIES ? 2 : 4;                  // passes whose loads are in flight together
+#pragma unroll kTogether
     for (int ps = 0; ps < kPasses; ++ps) {
         const int i = i0 + ps * kRowsPerPass;
         const int64_t row = bh * nq_pad + i;
         const bool in = i < Nq;
         uint4 vo = make_uint4(0, 0, 0, 0), vg = vo, vl = vo, vq = vo;
+        const float lse_i = in && sub == 0 ? lse[bh * Nq + i] : 0.f;
         if (in && sub * 8 < d) {
             vo = *reinterpret_cast<const uint4*>(op + (int64_t)i * o_sn);
             vg = *reinterpret_cast<const uint4*>(gp + (int64_t)i * g_sn);
@@ -1797,7 +1799,7 @@ bwd_preprocess_kernel(int d, const T* __restrict__ o, const T* __restrict__ d_o,
             }
         }
         if (sub == 0) {
-            if (in) { delta[row] = -s * pow2i(-e_i); lse2[row] = cp.pairs ? -lse[bh * Nq + i] : kPShift - lse[bh * Nq + i] * kLog2e + (float)e_i; }
+            if (in) { delta[row] = -s * pow2i(-e_i); lse2[row] = cp.pairs ? -lse_i : kPShift - lse_i * kLog2e + (float)e_i; }
             else    { delta[row] = 0.f; lse2[row] = -INFINITY; }
             if (COPIES) cp.erow[row] = in ? (float)e_i : 0.f;
         }
