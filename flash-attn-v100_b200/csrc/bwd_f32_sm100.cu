@@ -129,10 +129,11 @@ bwd_f32_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     auto strm_head = [&](int it) { return KS ? head_x * group + it / per_head : head_x / group; };
     auto strm_row = [&](int it) { return (KS ? it0 + it % per_head : it) * kStep; };
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kNumBars; ++i) mbar_init(&bars[i], i >= kBarT1Read ? kWorkers : 1u);
-        wait_control_init(abort_flag, a.wait_limit_ms);
+    if (warp == 0) {
+        if (lane < kNumBars) mbar_init(&bars[lane], lane >= kBarT1Read ? kWorkers : 1u);
+        if (lane == 0) wait_control_init(abort_flag, a.wait_limit_ms);
         fence_mbar_init();
+        __syncwarp();
     }
     if (warp == kWorkers) {
         tmem_alloc(tmem_slot, 512);

@@ -384,15 +384,16 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < Cfg::kNumBars; ++i) {
+    if (warp == 0) {                        // a lane a barrier: one thread for all of them took a microsecond of the launch
+        for (int i = lane; i < Cfg::kNumBars; i += 32) {
             const bool wg_bar = (i >= Cfg::kPFull && i < Cfg::kPFull + 2) || (i >= Cfg::kPHalf && i < Cfg::kPHalf + 2) ||
                                 i == Cfg::kMlFull || i == Cfg::kORead || i >= Cfg::kBiasEmpty;
             const bool conv_bar = (i >= Cfg::kVConv && i < Cfg::kVConv + ST);
             mbar_init(&bars[i], wg_bar ? 4u : (conv_bar ? 2u : 1u));
         }
-        wait_control_init(abort_flag, a.wait_limit_ms);
+        if (lane == 0) wait_control_init(abort_flag, a.wait_limit_ms);
         fence_mbar_init();
+        __syncwarp();
     }
     if (warp == 8) {
         tmem_alloc(tmem_slot, 512);

@@ -127,12 +127,11 @@ fwd_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (a.causal && tile * kM + kM + a.shift < kv_end) kv_end = tile * kM + kM + a.shift;
     const int nblk = (kv_end + kN - 1) / kN;
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kNumBars; ++i) {
-            mbar_init(&bars[i], i >= kBarQSplit ? 4u : 1u);       // one arrival per warp of a group of four
-        }
-        wait_control_init(abort_flag, a.wait_limit_ms);
+    if (warp == 0) {
+        if (lane < kNumBars) mbar_init(&bars[lane], lane >= kBarQSplit ? 4u : 1u);       // one arrival per warp of a group of four
+        if (lane == 0) wait_control_init(abort_flag, a.wait_limit_ms);
         fence_mbar_init();
+        __syncwarp();
     }
     if (warp == 4) {
         tmem_alloc(tmem_slot, 512);
