@@ -8,11 +8,12 @@
 //   1. preprocess  -delta = -rowsum(dO o O) and -lse*log2(e), both fp32, written
 //                  to the workspace in rows padded to whole 128-row tiles
 //                  (padding: delta = 0, -lse = -inf, so padded queries get P = 0)
-//   2. MODE 0      one CTA per 128-row key tile (stationary K, V), streams the
+//   2. MODE 0      a block is a 128-row key tile (stationary K, V), streams the
 //                  query tiles: writes dK and dV
-//   3. MODE 1      one CTA per 128-row query tile (stationary Q, dO), streams
+//   3. MODE 1      a block is a 128-row query tile (stationary Q, dO), streams
 //                  the key tiles: writes dQ
-// Every output element is owned by one CTA and accumulated in a fixed order, so
+// 2 starts beside the end of 1 and waits for it before it reads; 3 may run beside the end of 2 (griddepcontrol).
+// Every output element is owned by one block and accumulated in a fixed order, so
 // results are bit-reproducible (the reference accumulates dQ across CTAs with
 // an unordered read-modify-write, kernels/backward_kernel.py:179-194).
 //
@@ -48,8 +49,20 @@
 //                    step's last MMA, so it gets three stages where shared memory allows and its
 //                    next load overlaps a whole step; W gets two), and in the key-stationary
 //                    kernels the step's -lse / -delta rows into a two-slot ring
-//   warps 18-19      bf16 inputs: convert the streamed tiles to fp16 in place as they land (all MMAs run
-//                    f16 x f16, with P and dS rounded to fp16; see "number formats" below); else idle
+//   warp 18          calls with a bias: brings the steps' bias tiles (TMA)
+//   warp 19          stores by TMA: the fp16 copy of K, and each block's results once they are staged
+//   warps 18-19      INLINE: convert the streamed tiles to fp16 in place as they land (all MMAs run f16 x f16, with P
+//                    and dS rounded to fp16; see "number formats" below); stationary tiles: the elementwise warps do
+//
+// A CTA goes on from one block of the grid to the next: the producer asks for another block (clusterlaunchcontrol: the
+// answer is a block that has not been started, so the order of the grid and its balance stay what they are) when it
+// begins one, and leaves its place for the other warps in one of two slots.  Nothing is set up again; the rings, their
+// phases and tensor memory carry on.  The next block's X, U, W and its first products come while the last one's results
+// are still read out: those go to shared memory (dK or dQ over the block's last U tile, dV over its last W tile, by then
+// read by every MMA) and leave by TMA.  B32 N197 H12 D64 fp16: dK/dV and dQ 46 and 40 -> 30 and 24
+// us; backward alone under a sustained load, B8 N2048 H16 D64 fp16 688 -> 620, B4 N4096 H32 D128 bf16 causal 2011 -> 1871,
+// B1 N16384 H32 D128 6244 -> 6197 (there the board's power limit sets the pace).
+// Stored straight from registers, the results took 2200-6000 cycles a block.
 //
 // TMEM columns: T1 [0,128)  T2 [128,256)  ACC1 [256,256+D)  ACC2 [384,384+D).
 // MODE 1 has no ACC2 and never writes P back (only dS is an MMA operand there): S has the one buffer
@@ -71,8 +84,7 @@ using namespace ptx;
 constexpr int kTile = 128;
 constexpr int kBoxBytes = 128 * 128;
 constexpr int kNWG = tile::kBwdWarpgroups;   // elementwise warpgroups per CTA (each owns 128 / kNWG columns)
-constexpr int kExtraThreads = 128;       // MMA warp + TMA warp + two idle warps: registers are granted per
-                                         // four warps, so dropping the idle pair would free none
+constexpr int kExtraThreads = 128;       // MMA warp, TMA warp, warps 18 and 19: registers are granted per four warps
 constexpr float kLog2e = 1.4426950408889634f;
 
 // Shared-memory plan of one kernel instance.  The streamed tiles U and W have rings of their own:
@@ -99,7 +111,7 @@ struct BwdCfg {
     static constexpr int kMaskBytes = 2 * 128 * 8 * 2;          // two buffers of 128 x 8 uint16 keep masks
     static constexpr int kXFull = 0;
     static constexpr int kYFull = 1;
-    static constexpr int kXEmpty = 2;                            // the item's last reader of X (see kXEmptyArrivals)
+    static constexpr int kXEmpty = 2;                            // the item's last reader of X (the MMAs; with a copy of K its store, too)
     static constexpr int kYEmpty = 3;
     static constexpr int kSchedFull = 4;                         // [2] the next item's place is in its slot
     static constexpr int kSchedEmpty = 6;                        // [2] ... and has been read (one arrival per reading warp)
@@ -126,7 +138,7 @@ struct BwdCfg {
     // bf16 inputs: tiles converted to fp16 in place (arrivals: one per converting warp)
     static constexpr int kXConv = kVEmpty + 2;                   // stationary tiles (one arrival per elementwise warp)
     static constexpr int kYConv = kXConv + 1;
-    static constexpr int kUConv = kYConv + 1;                    // [kUStages] streamed U (the two spare warps)
+    static constexpr int kUConv = kYConv + 1;                    // [kUStages] streamed U (warps 18 and 19)
     static constexpr int kWConv = kUConv + kUStages;             // [kWStages] streamed W, key-stationary kernels only
     static constexpr int kBiasFull = kWConv + kWStages;          // PREC = 2: the step's bias tile has landed
     static constexpr int kBiasEmpty = kBiasFull + 1;             // ... and has been read (one arrival per elementwise warp)
@@ -343,7 +355,7 @@ __device__ __forceinline__ BwdItem make_item(const BwdArgs& a, const CtaWork& cw
 }
 
 // MODE 0: dK, dV (key-stationary).  MODE 1: dQ (query-stationary).
-// INLINE (bf16 inputs only): the streamed tiles arrive as bf16 and the two spare warps convert them;
+// INLINE (bf16 inputs only): the streamed tiles arrive as bf16 and warps 18 and 19 convert them;
 // otherwise bf16 calls stream the fp16 copies the preprocess launch (Q, dO) and the dK/dV kernel (K:
 // map_aux, a by-product of its stationary tile) have written to the workspace.
 // DS (pairs, MODE 1): the call wants d(loss)/d(scores).  An instance of its own: as branches its code cost the kernel of
@@ -362,7 +374,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     constexpr bool CONV = BF16 && PREC == 0;    // every MMA runs f16 x f16: bf16 tiles are converted
     constexpr bool P_BF16 = BF16 && PREC != 0;  // ... except that pairs of bf16 need no conversion
     static_assert(PREC == 0 || (MODE != 2 && !INLINE), "the pair instances are the two-pass form");
-    constexpr bool STREAM_CONV = CONV && INLINE;             // ... the streamed ones by the spare warps
+    constexpr bool STREAM_CONV = CONV && INLINE;             // ... the streamed ones by warps 18 and 19
     constexpr bool XY_CONV = CONV && (KS || INLINE);         // ... the stationary ones (X; key-stationary also Y), too
     constexpr bool ROWFORM = CONV && !INLINE;                // staged vectors are in the row form (see DoForm)
     constexpr bool K_COPY = ROWFORM && MODE == 0;            // this kernel writes the fp16 copy of K
@@ -449,9 +461,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
     const uint32_t tmem = *tmem_slot;
     const uint32_t tT1 = tmem, tT2 = tmem + 128u, tAcc1 = tmem + 256u, tAcc2 = tmem + 384u;
-    // fused kernel: the per-step dQ tile has columns of its own when D = 64 and shares T2's when D = 128
-    constexpr bool kDqAliasesT2 = (D > 64);
-    const uint32_t tDq = kDqAliasesT2 ? tT2 : tmem + 448u;
+    const uint32_t tDq = tmem + 448u;                   // fused kernel (D = 64 only): the per-step dQ tile
     constexpr DoForm kForm = P_BF16 ? kDoPairs : (!(CONV && KS) ? kDoAsIs : (INLINE ? kDoInline : kDoRowCopy));
 
     // Persistent: a CTA goes on to a further block of the grid, which it takes from the blocks not yet launched

@@ -1219,8 +1219,8 @@ int64_t column_units(const fa_b200_params& p, int q_per_tile, int n_pairs) {
 // keys make its pairs long.  The call's units are then cut into one equal range per SM.  What that costs
 // (partial sums through memory and a second launch) is about kMergeUnits units, so the ranges have to be that much
 // shorter than the longest round-robin share, and a tenth.  B200, before -> after, both rules together:
-// 32 requests of 2048-4096 keys, 1 query, H32 Hkv8 D128 bf16: 304 -> 84 us (403 MB of keys and values, 62 us at the
-// copy rate); 1 request, 700 queries on 8892 keys, same heads: 240 -> 112 us (98 GFLOP, 60 us at cuBLAS's rate).
+// 32 requests of 2048-4096 keys, 1 query, H32 Hkv8 D128 bf16: 304 -> 80 us (403 MB of keys and values, 62 us at the
+// copy rate); 1 request, 700 queries on 8892 keys, same heads: 240 -> 108 us (98 GFLOP, 60 us at cuBLAS's rate).
 // Decoding as one pair per unit, without the one-tile kernel (SCHED = 2), took 116 us: S, softmax and P V of one tile
 // are a serial chain of about 2.7 us a block, and two stages of K and V cover too little of the memory's latency.
 // Key counts are on the device, so the rule sees Nk.  Ranges are as even for unequal counts as for equal ones, whole

@@ -29,7 +29,7 @@ constexpr float kFwdRescaleLog2 = 8.f;  // the running maximum is refreshed when
 
 // ---- backward (bwd_sm100.cu) --------------------------------------------------------------------
 constexpr int kBwdWarpgroups = 4;       // elementwise warpgroups (2 -> 4: backward +11 %)
-constexpr int kBwdWarps = 4 * kBwdWarpgroups + 4;                    // + MMA, TMA, 2 converting / spare warps
+constexpr int kBwdWarps = 4 * kBwdWarpgroups + 4;                    // + MMA, TMA, warps 18 and 19 (bias and stores by TMA, conversions)
 // ring depth of the streamed tiles: U is read by the first and the last MMA of its step (three
 // stages took 16 % off the dQ kernel), W within one step; the key-stationary dropout instance at
 // D = 128 gives 4 KB to its masks and keeps two and two

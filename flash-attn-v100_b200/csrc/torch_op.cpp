@@ -4,7 +4,7 @@
 //
 // What it is for: the Python operator is 40 us of host work around a forward and 150 around a training step (argument
 // checks, a ctypes block, the Python side of autograd), more than the kernels of a short call take.  B200: a prompt of
-// B1 N128 H8 D64 39 -> 10 us, a training step of B32 N197 H12 D64 157 -> 95.
+// B1 N128 H8 D64 39 -> 10 us, a training step of B32 N197 H12 D64 157 -> 95 (bound by its kernels then).
 //
 // Replaces, for these calls, the reference's autograd.Function (ops/attention.py:36-333).
 #include <ATen/FunctionalTensorWrapper.h>
