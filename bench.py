@@ -178,7 +178,7 @@ def cpu_reference_throughput(w, budget_s: float = 12.0, max_heads: int = 64):
 def run_reference(args, w):
     """--impl reference: the reference's own CPU implementation of the path.  The
     reference is pure Python (nothing to compile into oracle/_ref) and its tree is
-    not present on the GPU box, so the oracle port stands in (kind "port")."""
+    not present on the GPU machine, so the oracle port stands in (kind "port")."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return

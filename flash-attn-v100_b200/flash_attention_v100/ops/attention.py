@@ -378,7 +378,7 @@ def native_call(q, k, v, scale, causal, bottom_right, key_lengths, fast):
     """(o, lse) by the native operator, or None where it does not serve the call: tensors the kernels do not take as they
     are, anything that watches operators (a transform, a tracer, a mode, a compiler), an explicit kernel_variant().  The
     public entry's calls without bias and dropout come here first; the class below is the general form.
-    A call's time on a B200 box: a short prompt's forward (B1 N128 H8 D64) 39 -> 10 us, a training step at B32 N197 H12 D64
+    A call's time on a B200: a short prompt's forward (B1 N128 H8 D64) 39 -> 10 us, a training step at B32 N197 H12 D64
     157 -> 95 (bound by its kernels then)."""
     if torch.compiler.is_compiling() or getattr(_variant_override, "value", _cabi.VARIANT_AUTO) != _cabi.VARIANT_AUTO:
         return None
