@@ -1588,8 +1588,10 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             tc_fence_before_sync();
             mbar_arrive_warp(&bars[b_ready]);
             if (DS && it == sum_steps - 1) {
-                // the row's four threads put their sums together, in a fixed order
-                uint32_t meet = ((count >> 2) & 1u);         // three times a block
+                // the row's four threads put their sums together, in a fixed order.  They meet before the first sum is left,
+                // too: the sums' room is where the rows' -lse and -delta were brought to, and with one key tile nothing else
+                // lies between a warp that is here and one that has not read them yet.
+                uint32_t meet = 0u;                          // four times a block: every block finds the first parity again
                 auto all_met = [&] {
                     mbar_arrive_warp(&bars[Cfg::kSums]);
                     const bool good = mbar_wait(&bars[Cfg::kSums], meet & 1u, abort_flag);
@@ -1605,7 +1607,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     return true;
                 };
                 float sum_p = 0.f, sum_pd = 0.f;
-                ok = row_sum(sum_p2, sum_p) && all_met() && row_sum(sum_pd2, sum_pd);
+                ok = all_met() && row_sum(sum_p2, sum_p) && all_met() && row_sum(sum_pd2, sum_pd);
                 if (!ok) break;
                 mbar_arrive_read_done(&bars[Cfg::kRowEmpty]);
                 // a row without a result, or one whose lse has lost its sum (all of it masked with a lowest value),
