@@ -172,7 +172,7 @@ struct BwdArgs {
     int32_t* status;
     int B, Nq, Nk, H, Hkv, nq_pad;
     int group;                     // H / Hkv
-    int wait_limit_ms;             // limit of one mbarrier wait (0: the default)
+    int wait_limit_ms;             // limit of a wait for one step (0: the default)
     int cols_per_group;            // CTA order: (batch, head) columns per group, see cta_work()
     int causal;
     int shift;                     // key j is visible to query i iff j <= i + shift
@@ -834,7 +834,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 if (!ok) break;
             }
             steps += n_iter;
-            if (stores && mbar_wait(&bars[Cfg::kEpi], (uint32_t)items & 1u, abort_flag, kIdleNs)) {
+            // (all the block's steps lie in this wait, beside the next one's start)
+            if (stores && mbar_wait(&bars[Cfg::kEpi], (uint32_t)items & 1u, abort_flag, kIdleNs, (uint32_t)n_iter + 1u)) {
                 const int su = (steps - 1) % UST, sw = (steps - 1) % WST;
 #pragma unroll
                 for (int bx = 0; bx < Cfg::kNBox; ++bx) {

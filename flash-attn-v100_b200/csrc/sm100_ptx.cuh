@@ -76,14 +76,13 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Wall-clock limit of one wait.  The longest legitimate wait inside a CTA is
-// one pipeline step (microseconds); the default of two seconds means a protocol
-// error.  The caller may pass a shorter one (fa_b200_params.wait_limit_ms).
+// Wall-clock limit of a wait for one pipeline step (microseconds): the default of two seconds means a protocol error.  The
+// caller may pass a shorter one (fa_b200_params.wait_limit_ms).  A wait that spans several steps names their number.
 constexpr uint32_t kDefaultWaitLimitUs = 2000000u;
 
 // The CTA's wait control block in shared memory: word 0 is the abort flag any
-// thread may raise (a raised flag ends every wait), word 1 the limit of one wait
-// in microseconds.
+// thread may raise (a raised flag ends every wait), word 1 the limit of a wait for
+// one step in microseconds.
 __device__ __forceinline__ void wait_control_init(volatile uint32_t* abort_flag, int limit_ms) {
     abort_flag[0] = 0u;
     abort_flag[1] = limit_ms > 0 ? (uint32_t)limit_ms * 1000u : kDefaultWaitLimitUs;
@@ -99,8 +98,10 @@ __device__ __forceinline__ void report_status(int32_t* status, int32_t code) {
 }
 
 // Wait for the phase with the given parity; false when the wait ran out or the flag was raised.  `sleep_ns`: a wait that
-// nothing hurries pauses between its looks, which would take issue slots from the warps that work.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t sleep_ns = 0u) {
+// nothing hurries pauses between its looks, which would take issue slots from the warps that work.  `steps`: how many
+// pipeline steps lie in the wait, each of which may take the limit.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t sleep_ns = 0u,
+                                          uint32_t steps = 1u) {
     if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     uint32_t spins = 0;
@@ -109,7 +110,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         if (sleep_ns) __nanosleep(sleep_ns);
         if ((++spins & 63u) == 0) {
             if (abort_flag[0]) return false;
-            if (globaltimer_ns() - t0 > (uint64_t)abort_flag[1] * 1000ull) {
+            if (globaltimer_ns() - t0 > (uint64_t)abort_flag[1] * 1000ull * steps) {
                 abort_flag[0] = 1u;
                 return false;
             }

@@ -149,7 +149,9 @@ typedef struct fa_b200_params {
        exactly the mask the whole call draws.  The reference has no replayable stream at all
        (kernels/forward_kernel.py:198-203). */
     int32_t        rng_batch_offset, rng_head_offset, rng_heads;
-    /* Limit of one device-side wait in milliseconds (0: the default, 2000).  A kernel whose wait on an
+    /* Limit of a device-side wait for one step of a kernel's pipeline, in milliseconds (0: the default,
+       2000; a step takes microseconds).  The one wait that lasts a whole block, the backward's for a
+       block's results, may take the limit once for each of the block's steps.  A kernel whose wait on an
        mbarrier runs out stops its pipeline, frees what it holds, returns normally and writes a non-zero
        code to *status_word; it never traps and never waits longer. */
     int32_t        wait_limit_ms;
