@@ -178,7 +178,7 @@ bool watched() {
 py::object attention(py::handle q_, py::handle k_, py::handle v_, py::handle scale_, bool causal, bool bottom_right, py::handle lengths_, bool fast) {
     const at::Tensor *qp, *kp, *vp, *lp = nullptr;
     if (watched() || !plain(q_.ptr(), qp) || !plain(k_.ptr(), kp) || !plain(v_.ptr(), vp)) return py::none();
-    const at::Tensor &q = *qp, &k = *kp, &v = *vp;
+    const at::Tensor q = *qp, k = *kp, v = *vp;          // (own references: other threads run during the call)
     const auto type = q.scalar_type();
     if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || k.sizes() != v.sizes() || q.size(0) != k.size(0) || q.size(3) != k.size(3) ||
         k.size(2) == 0 || q.size(2) % k.size(2) != 0 || q.numel() == 0 || k.numel() == 0 || q.size(3) > 128 ||
@@ -207,6 +207,9 @@ py::object attention(py::handle q_, py::handle k_, py::handle v_, py::handle sca
     const bool wants = q.requires_grad() || k.requires_grad() || v.requires_grad();
     at::Tensor o, lse, o_lo;
     try {
+        // Allocation and launches may have to wait (for memory, for room in the launch queue): other Python threads, which
+        // may be what the GPU waits for, run meanwhile.
+        py::gil_scoped_release others_run;
         if (wants && at::GradMode::is_enabled()) {
             variable_list out = Attention::apply(q, k, v, c);
             o = std::move(out[0]); lse = std::move(out[1]);

@@ -126,3 +126,33 @@ def test_refusals_keep_their_types(device):
         f(q, q, q, scale=float("nan"))
     with pytest.raises(ValueError, match="key_lengths"):
         f(q, q, q, key_lengths=torch.ones(3, dtype=torch.int32, device=device))
+
+
+def test_other_threads_run_while_a_call_waits_for_the_launch_queue(device):
+    """A kernel of about a second ahead of more calls than the launch queue holds: the calling thread has to wait for
+    room, and this one goes on ticking meanwhile.  (With the interpreter held it stood still for most of the second.)"""
+    import threading
+    import time
+    q = _rand(1, 128, 2, 64, dtype=torch.float16, device=device, seed=1)
+    assert ops.native_call(q, q, q, None, False, False, None, False) is not None
+    torch.cuda.synchronize(device)
+    took = []
+
+    def calls():
+        start = time.perf_counter()
+        with torch.no_grad():
+            for _ in range(4000):
+                ops.native_call(q, q, q, None, False, False, None, False)
+        took.append(time.perf_counter() - start)
+    torch.cuda._sleep(1_500_000_000)                                # cycles, 0.8 s or more
+    worker = threading.Thread(target=calls)
+    gap, last = 0.0, time.perf_counter()
+    worker.start()
+    while worker.is_alive():
+        time.sleep(0.001)
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+    worker.join()
+    torch.cuda.synchronize(device)
+    assert took[0] > 0.5                                            # the queue was full
+    assert gap < 0.5 * took[0]
