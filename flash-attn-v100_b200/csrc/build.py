@@ -5,6 +5,7 @@ Usage: python build.py [--force] [--verbose]
 The library lands in ../flash_attention_v100/lib/ so it travels with the package.
 """
 import os
+import re
 import subprocess
 import sys
 
@@ -27,27 +28,43 @@ def _newest(paths):
     return max((os.path.getmtime(p) for p in paths if os.path.exists(p)), default=0.0)
 
 
-def _op_command():
+def _installed_torch():
+    """Folder and version of the torch that Python would import, without importing it."""
     import importlib.util
+    folder = os.path.dirname(importlib.util.find_spec("torch").origin)
+    with open(os.path.join(folder, "version.py")) as f:
+        return folder, re.search(r"^__version__\s*=\s*['\"]([^'\"]+)", f.read(), re.M).group(1)
+
+
+def _op_command():
     import sysconfig
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    torch_dir, version = _installed_torch()
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include",
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f'-DFA_TORCH_VERSION="{version}"',
+            f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include",
             f"-I{cuda}/include", f"-I{sysconfig.get_paths()['include']}", os.path.join(HERE, OP_SOURCE), "-o", OP_OUT,
             f"-L{torch_dir}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python",
             f"-L{OUT_DIR}", "-lfa_b200", "-Wl,-rpath,$ORIGIN"]
 
 
 def build_op(force=False):
-    """The native operator; after the library, which it is linked against."""
+    """The native operator; after the library, which it is linked against.  Built again when its sources are newer or the
+    command is another one (another torch, another Python): it is laid out for the torch it was built with."""
     deps = [os.path.join(HERE, OP_SOURCE), os.path.join(HERE, "..", "..", "include", "fa_b200.h"), os.path.abspath(__file__)]
-    if not force and os.path.exists(OP_OUT) and os.path.getmtime(OP_OUT) >= _newest(deps):
-        return OP_OUT
     cmd = _op_command()
+    built_by = OP_OUT + ".cmd"
+    same = False
+    if os.path.exists(built_by):
+        with open(built_by) as f:
+            same = f.read() == " ".join(cmd)
+    if not force and same and os.path.exists(OP_OUT) and os.path.getmtime(OP_OUT) >= _newest(deps):
+        return OP_OUT
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout)
         raise RuntimeError("building the native operator failed")
+    with open(built_by, "w") as f:
+        f.write(" ".join(cmd))
     return OP_OUT
 
 

@@ -226,6 +226,12 @@ py::object attention(py::handle q_, py::handle k_, py::handle v_, py::handle sca
 
 }  // namespace
 
+#ifndef FA_TORCH_VERSION
+#error "the build names the torch whose headers these are (FA_TORCH_VERSION)"
+#endif
+// Read by kernels/_cabi.py before Python imports the module: what stands above is laid out for this torch and no other.
+extern "C" __attribute__((visibility("default"))) const char* fa_b200_torch_built_for() { return FA_TORCH_VERSION; }
+
 PYBIND11_MODULE(fa_b200_torch, m) {
     m.def("attention", &attention);
     m.def("set_status_word", [](int device, uintptr_t word) {

@@ -167,7 +167,8 @@ _op = None
 
 
 def load_op():
-    """The native autograd operator (csrc/torch_op.cpp), which calls the library above; loaded once, loud if missing."""
+    """The native autograd operator (csrc/torch_op.cpp), which calls the library above; loaded once, loud if it is missing
+    or was built for another torch, whose classes may be laid out differently."""
     global _op
     if _op is not None:
         return _op
@@ -176,10 +177,18 @@ def load_op():
         if _op is None:
             import importlib.machinery
             import importlib.util
-            import torch  # noqa: F401  (its libraries first)
+            import torch  # (its libraries first)
+            again = f"build it with `python {os.path.join(os.path.dirname(_PKG_DIR), 'csrc', 'build.py')}`"
             if not os.path.exists(OP_PATH):
-                raise FlashAttentionLibraryError(
-                    f"{OP_PATH} not found: build it with `python {os.path.join(os.path.dirname(_PKG_DIR), 'csrc', 'build.py')}`")
+                raise FlashAttentionLibraryError(f"{OP_PATH} not found: {again}")
+            try:
+                name = ctypes.CDLL(OP_PATH).fa_b200_torch_built_for
+            except (OSError, AttributeError) as e:
+                raise FlashAttentionLibraryError(f"{OP_PATH} does not fit torch {torch.__version__} ({e}): {again}") from e
+            name.restype = ctypes.c_char_p
+            built_for = name().decode()
+            if built_for != str(torch.__version__):
+                raise FlashAttentionLibraryError(f"{OP_PATH} was built for torch {built_for}, this is {torch.__version__}: {again}")
             loader = importlib.machinery.ExtensionFileLoader("fa_b200_torch", OP_PATH)
             module = importlib.util.module_from_spec(importlib.util.spec_from_loader("fa_b200_torch", loader))
             loader.exec_module(module)
