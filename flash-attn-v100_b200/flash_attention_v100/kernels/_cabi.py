@@ -164,6 +164,7 @@ def load():
 
 
 _op = None
+_status_words = {}          # device index -> address of its status word, for the operator once it is loaded
 
 
 def load_op():
@@ -192,8 +193,18 @@ def load_op():
             loader = importlib.machinery.ExtensionFileLoader("fa_b200_torch", OP_PATH)
             module = importlib.util.module_from_spec(importlib.util.spec_from_loader("fa_b200_torch", loader))
             loader.exec_module(module)
+            for device, address in _status_words.items():
+                module.set_status_word(device, address)
             _op = module
     return _op
+
+
+def serve_device(device: int, status_word: int) -> None:
+    """From here on the native operator, loaded or yet to be, serves the device's calls."""
+    with _lock:
+        _status_words[device] = status_word
+        if _op is not None:
+            _op.set_status_word(device, status_word)
 
 
 def raise_for_status(rc: int, what: str) -> None:

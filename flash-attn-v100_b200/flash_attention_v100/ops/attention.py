@@ -74,7 +74,7 @@ def _status_word(device: torch.device) -> torch.Tensor:
     if idx not in _status_words:
         word = torch.zeros(1, dtype=torch.int32).pin_memory()
         _status_words[idx] = word
-        _cabi.load_op().set_status_word(idx, _status_words[idx].data_ptr())      # (from here on it serves this device, too)
+        _cabi.serve_device(idx, word.data_ptr())
     return _status_words[idx]
 
 

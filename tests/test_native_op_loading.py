@@ -1,4 +1,5 @@
-"""Loading and building the native operator (CPU): a build for another torch is refused in words and built again."""
+"""Loading and building the native operator (CPU): a build for another torch is refused in words and built again, and what
+needs no operator does without it."""
 import importlib.util
 import os
 
@@ -6,6 +7,7 @@ import pytest
 import torch
 
 from flash_attention_v100.kernels import _cabi
+from flash_attention_v100.ops import attention as ops
 
 CSRC = os.path.join(os.path.dirname(_cabi._PKG_DIR), "csrc")
 
@@ -13,6 +15,8 @@ CSRC = os.path.join(os.path.dirname(_cabi._PKG_DIR), "csrc")
 @pytest.fixture
 def unloaded(monkeypatch):
     monkeypatch.setattr(_cabi, "_op", None)
+    monkeypatch.setattr(_cabi, "_status_words", {}, raising=False)
+    monkeypatch.setattr(ops, "_status_words", {})
     return monkeypatch
 
 
@@ -35,6 +39,28 @@ def test_an_operator_from_before_the_check_is_refused(unloaded):
     unloaded.setattr(_cabi, "OP_PATH", _cabi.LIB_PATH)              # loads, and does not say which torch it is for
     with pytest.raises(_cabi.FlashAttentionLibraryError, match="does not fit torch"):
         _cabi.load_op()
+
+
+def test_status_words_need_no_operator_and_reach_it_when_it_is_loaded(unloaded, tmp_path):
+    unloaded.setattr(torch.Tensor, "pin_memory", lambda t: t)       # (no GPU here)
+    real = _cabi.OP_PATH
+    unloaded.setattr(_cabi, "OP_PATH", str(tmp_path / "missing.so"))
+    first = ops._status_word(torch.device("cuda", 0))
+    with pytest.raises(_cabi.FlashAttentionLibraryError, match="not found"):
+        ops.native_call(first, first, first, None, False, False, None, False)
+
+    told = {}
+
+    class Op:
+        @staticmethod
+        def set_status_word(device, address):
+            told[device] = address
+    unloaded.setattr(_cabi, "OP_PATH", real)
+    unloaded.setattr("importlib.util.module_from_spec", lambda spec: Op)
+    unloaded.setattr("importlib.machinery.ExtensionFileLoader.exec_module", lambda self, module: None)
+    assert _cabi.load_op() is Op
+    second = ops._status_word(torch.device("cuda", 3))
+    assert told == {0: first.data_ptr(), 3: second.data_ptr()}
 
 
 def test_the_operator_is_built_again_for_another_torch(monkeypatch, tmp_path):
