@@ -63,18 +63,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Whether the phase with the given parity is complete, without waiting.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 
 // Wall-clock limit of a wait for one pipeline step (microseconds): the default of two seconds means a protocol error.  The
 // caller may pass a shorter one (fa_b200_params.wait_limit_ms).  A wait that spans several steps names their number.
