@@ -474,12 +474,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // holding it in registers).
     auto item_there = [&](int k) { return mbar_wait(&bars[Cfg::kSchedFull + (k & 1)], (uint32_t)(k >> 1) & 1u, abort_flag); };
 
-    // Registers: without dropout the launch allocation of 96 per thread lets no role spill, and moving
+    // Registers: without dropout the launch allocation of 96 per thread is enough for all but a few words (-Xptxas -v: 8
+    // bytes stored and 20 loaded in the bf16 dK/dV instances, which is 0.1 % of their instructions under ncu; up to 80 and
+    // 88 in those that write d(loss)/d(scores), 32 and 44 in the one-kernel form), and moving
     // registers from the MMA / TMA warps to the elementwise ones (104 / 64, 104 / 40) made one side or the
-    // other spill and measured the same or slower.  The dK/dV kernel's dropout instances do spill in the
-    // elementwise loop at 96 (28 local loads and 24 stores per step and warp, 8 % of the kernel's
-    // instructions under ncu): they take 104 and leave 64 to the other warpgroup (1.272 -> 1.216 ms at
-    // B32 H16 N2048 D64; the one-kernel backward got slower with the same split, 1.439 -> 1.466, and keeps 96).
+    // other spill and measured the same or slower.  The dK/dV kernel's dropout instances spill in the
+    // elementwise loop: they take 104 and leave 64 to the other warpgroup (1.272 -> 1.216 ms at
+    // B32 H16 N2048 D64; the one-kernel backward got slower with the same split, 1.439 -> 1.466, and keeps 96).  With 104
+    // it is 17 local loads and 12 stores a step and warp, 5 % of the instructions (ncu, B4 N2048 H16 D64 causal).
     constexpr bool kMoveRegs = DROP != 0 && MODE == 0 && !INLINE;
     // The pool is what the CTA was launched with (96 per thread): a split that asks for more makes
     // setmaxnreg.inc wait for ever (112 / 40 did: 62464 > 61440).
